@@ -21,6 +21,7 @@ COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler",
 # (source, extra flags)
 UNITS = [
     ("mhd_kernels_fp64.cu", ["-fmad=false"]),
+    ("mhd_kernels_step.cu", ["-fmad=false"]),
     ("mhd_kernels_mixed.cu", ["-fmad=false"]),
     ("mhd_krylov.cu", []),
     ("mhd_abi.cu", []),

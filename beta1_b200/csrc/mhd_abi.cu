@@ -142,15 +142,12 @@ enum TuneId
 const char *const kTuneNames[NTUNE] = {"k_pv_uplus_dt", "k_fluid_ucontra", "k_bcell_jedge",  "k_eface",
                                        "k_curl_e2f",    "k_eedge",         "k_fluid_mixed",  "k_gmres_resist",
                                        "k_hall_edge"};
-// minimum CTAs per SM of each variant (variant 0 first; 0: the compiler's
-// own allocation, no launch bounds) and the number of variants
-// per variant the reported value: the minimum CTAs per SM of its launch
-// bounds (0: none); 12 for the face-tiled k_fluid_mixed (2 CTAs per SM), 16
-// for the same with its face states staged in shared memory, 14
-// for k_pv_uplus_dt with J_cell in a pass of its own (the PV pass at 4); for
-// the persistent k_gmres_resist the CTAs of its grid (0: two per SM); for
-// k_hall_edge 2 selects the form that reads the seven cells of a staggered
-// point once
+// per variant (variant 0, the default, first) the reported value: the minimum
+// CTAs per SM of its launch bounds (0: the default's own); 12 for the
+// face-tiled k_fluid_mixed (2 CTAs per SM), 16 for the same with its face
+// states staged in shared memory, 14 for k_pv_uplus_dt with J_cell in a pass
+// of its own (the PV pass at 4); for the persistent k_gmres_resist the CTAs of
+// its grid (0: two per SM).  And the number of variants
 const int kTuneMinCtas[NTUNE][5] = {{4, 0, 5, 14, 0}, {0, 3, 0, 0, 0},        {0, 6, 0, 0, 0},
                                     {0, 6, 0, 0, 0},  {0, 6, 0, 0, 0},        {0, 8, 0, 0, 0},
                                     {3, 0, 2, 12, 16}, {0, 148, 64, 32, 0},   {0, 2, 0, 0, 0}};
@@ -177,6 +174,7 @@ struct mhd_ctx
     Consts c{};
     int G = 4;
     std::vector<BlockView> hbv;
+    HotGrid hot; // the hot kernels' launch arguments
     BlockView *dbv = nullptr;
     double *pool = nullptr;
     size_t pool_n = 0;
@@ -195,10 +193,8 @@ struct mhd_ctx
     long long *step = nullptr;
     int *err = nullptr;
     double *qref = nullptr; // [nruns][6]
-    // flattened launches (batches): block of every CTA per launch kind
-    bool flat = false;
-    int *cta_tab = nullptr;
-    int64_t cta_total[NKIND] = {};
+    int *cta_tab = nullptr; // block of every CTA of the face-tiled kernels (batches)
+    int64_t tiles = 0;      // those CTAs
     std::map<std::string, SyncMap> syncs;
     // eta Poles: (block, direction) pairs; a context with Poles runs every
     // sync in the topology order of the Pole shell
@@ -394,15 +390,6 @@ int64_t max_box(const mhd_ctx *ctx, int loc, int g)
     return m;
 }
 
-// staggered points [0, n + 1)^3 of the largest block
-int64_t max_stagger(const mhd_ctx *ctx)
-{
-    int64_t m = 0;
-    for (const auto &v : ctx->hbv)
-        m = std::max(m, int64_t(v.ni + 1) * (v.nj + 1) * (v.nk + 1));
-    return m;
-}
-
 // points of a block in a launch kind's box
 int64_t kind_points(const BlockView &v, int kind)
 {
@@ -416,15 +403,15 @@ int64_t kind_points(const BlockView &v, int kind)
     return int64_t(v.ni + 1) * (v.nj + 1) * (v.nk + 1);
 }
 
-// grid of a hot-path launch: one row of exactly the CTAs every block needs
-// (batches of uneven blocks), else one row per block sized for the largest
-dim3 grid_kind(const mhd_ctx *ctx, int kind)
+// grid of the face-tiled kernels: one row of exactly the CTAs every block
+// needs (batches of uneven blocks), else one row per block sized for the largest
+dim3 grid_tiles(const mhd_ctx *ctx)
 {
-    if (ctx->flat)
-        return dim3(unsigned(ctx->cta_total[kind]), 1);
+    if (ctx->cta_tab)
+        return dim3(unsigned(ctx->tiles), 1);
     int64_t m = 0;
     for (const auto &v : ctx->hbv)
-        m = std::max(m, kind_points(v, kind));
+        m = std::max(m, kind_points(v, KIND_TILE1));
     return dim3(unsigned(grid_for(m)), unsigned(ctx->nblocks));
 }
 
@@ -465,6 +452,8 @@ void prof_begin(mhd_ctx *ctx, const char *name)
 
 int launched(mhd_ctx *ctx, int nk = 1)
 {
+    if (nk < 0)
+        return fail(ctx, MHD_EINVAL, "unknown kernel variant");
     if (ctx->profiling)
     {
         cudaEvent_t e;
@@ -678,8 +667,7 @@ int launch_jcell_split(mhd_ctx *ctx)
     if (ctx->tune[TUNE_k_pv_uplus_dt] != kPvSplit)
         return MHD_OK;
     prof_begin(ctx, "k_jcell");
-    launch_k_jcell(ctx->pool32 != nullptr, grid_kind(ctx, KIND_CELL0), ctx->stream, ctx->dbv);
-    return launched(ctx);
+    return launched(ctx, launch_k_jcell(ctx->pool32 != nullptr, ctx->hot, ctx->stream));
 }
 
 int launch_update_derived(mhd_ctx *ctx)
@@ -688,8 +676,7 @@ int launch_update_derived(mhd_ctx *ctx)
         return launch_update_derived_pole(ctx);
     cudaStream_t s = ctx->stream;
     prof_begin(ctx, "k_bcell_jedge");
-    launch_k_bcell_jedge(ctx->tune[TUNE_k_bcell_jedge], ctx->pool32 != nullptr, grid_kind(ctx, KIND_STAG), s, ctx->dbv);
-    RUN(launched(ctx));
+    RUN(launched(ctx, launch_k_bcell_jedge(ctx->tune[TUNE_k_bcell_jedge], ctx->pool32 != nullptr, ctx->hot, s)));
     RUN(run_sync(ctx, "B_cell"));
     RUN(run_sync(ctx, "Jedge"));
     // arm the dt reduction, then J_cell, PV / U_plus and the CFL bound of the next step
@@ -700,10 +687,9 @@ int launch_update_derived(mhd_ctx *ctx)
     // of the step and are filled when read out (materialise_pv)
     RUN(launch_jcell_split(ctx));
     prof_begin(ctx, "k_pv_uplus_dt");
-    launch_k_pv_uplus_dt(ctx->tune[TUNE_k_pv_uplus_dt], ctx->pool32 != nullptr, grid_kind(ctx, KIND_CELL1), s, ctx->dbv,
-                         ctx->c, ctx->dt_key, 1, 1);
     ctx->pv_dirty = true;
-    RUN(launched(ctx));
+    RUN(launched(ctx, launch_k_pv_uplus_dt(ctx->tune[TUNE_k_pv_uplus_dt], ctx->pool32 != nullptr, ctx->hot, s, ctx->c,
+                                           ctx->dt_key)));
     RUN(run_sync(ctx, "J_cell"));
     RUN(run_sync(ctx, "Uplus"));
     return MHD_OK;
@@ -719,8 +705,7 @@ int launch_update_derived_pole(mhd_ctx *ctx)
 {
     cudaStream_t s = ctx->stream;
     prof_begin(ctx, "k_bcell_jedge");
-    launch_k_bcell_jedge(ctx->tune[TUNE_k_bcell_jedge], ctx->pool32 != nullptr, grid_kind(ctx, KIND_STAG), s, ctx->dbv);
-    RUN(launched(ctx));
+    RUN(launched(ctx, launch_k_bcell_jedge(ctx->tune[TUNE_k_bcell_jedge], ctx->pool32 != nullptr, ctx->hot, s)));
     RUN(run_sync(ctx, "B_cell"));
     RUN(launch_pole(ctx, POLE_BZETA));
     {
@@ -741,26 +726,13 @@ int launch_update_derived_pole(mhd_ctx *ctx)
     RUN(launched(ctx));
     RUN(launch_jcell_split(ctx));
     prof_begin(ctx, "k_pv_uplus_dt");
-    launch_k_pv_uplus_dt(ctx->tune[TUNE_k_pv_uplus_dt], ctx->pool32 != nullptr, grid_kind(ctx, KIND_CELL1), s, ctx->dbv,
-                         ctx->c, ctx->dt_key, 1, 1);
     ctx->pv_dirty = true;
-    RUN(launched(ctx));
+    RUN(launched(ctx, launch_k_pv_uplus_dt(ctx->tune[TUNE_k_pv_uplus_dt], ctx->pool32 != nullptr, ctx->hot, s, ctx->c,
+                                           ctx->dt_key)));
     RUN(launch_pole(ctx, POLE_JCELL));
     RUN(run_sync(ctx, "J_cell"));
     RUN(run_sync(ctx, "Uplus"));
     return MHD_OK;
-}
-
-int launch_fluid_ucontra(mhd_ctx *ctx);
-
-int launch_fluid_rhs(mhd_ctx *ctx)
-{
-    if (ctx->pool32) // the mixed form's flux pass (its FP32 U_contra are a by-product)
-        return launch_fluid_ucontra(ctx);
-    const int64_t nc = max_box(ctx, LOC_CELL, 0);
-    prof_begin(ctx, "k_fluid_rhs");
-    k_fluid_rhs<<<dim3(grid_for(nc), ctx->nblocks), kThreads, 0, ctx->stream>>>(ctx->dbv, ctx->c, nc);
-    return launched(ctx);
 }
 
 // fluid RHS together with the contravariant velocities of the EMF stencils
@@ -770,12 +742,11 @@ int launch_fluid_ucontra(mhd_ctx *ctx)
     {
         prof_begin(ctx, "k_fluid_mixed");
         const int var = ctx->tune[TUNE_k_fluid_mixed];
-        launch_k_fluid_mixed(var, grid_kind(ctx, var >= 3 ? KIND_TILE1 : KIND_CELL1), ctx->stream, ctx->dbv, ctx->c);
-        return launched(ctx);
+        return launched(ctx, launch_k_fluid_mixed(var, ctx->hot, grid_tiles(ctx), ctx->stream, ctx->dbv,
+                                                  ctx->c));
     }
     prof_begin(ctx, "k_fluid_ucontra");
-    launch_k_fluid_ucontra(ctx->tune[TUNE_k_fluid_ucontra], grid_kind(ctx, KIND_CELL1), ctx->stream, ctx->dbv, ctx->c);
-    return launched(ctx);
+    return launched(ctx, launch_k_fluid_ucontra(ctx->tune[TUNE_k_fluid_ucontra], ctx->hot, ctx->stream, ctx->c));
 }
 
 // AssembleRHS_Induction_CT_; with_ucontra unless the fluid pass computed them
@@ -790,26 +761,22 @@ int launch_induction(mhd_ctx *ctx, bool update_b, bool with_ucontra = true)
         RUN(launched(ctx));
     }
     prof_begin(ctx, "k_eface");
-    launch_k_eface(ctx->tune[TUNE_k_eface], grid_kind(ctx, KIND_STAG), s, ctx->dbv);
-    RUN(launched(ctx));
+    RUN(launched(ctx, launch_k_eface(ctx->tune[TUNE_k_eface], ctx->hot, s)));
     RUN(run_sync(ctx, "Eface"));
     // inner edges; ghost edges keep their zero of AssembleRHS_Induction_CT_
     // except where the Eedge sync writes them
     prof_begin(ctx, "k_eedge");
-    launch_k_eedge(ctx->tune[TUNE_k_eedge], grid_kind(ctx, KIND_STAG), s, ctx->dbv);
-    RUN(launched(ctx));
+    RUN(launched(ctx, launch_k_eedge(ctx->tune[TUNE_k_eedge], ctx->hot, s)));
     RUN(run_sync(ctx, "Eedge"));
     prof_begin(ctx, "k_curl_e2f");
-    launch_k_curl_e2f(ctx->tune[TUNE_k_curl_e2f], grid_kind(ctx, KIND_STAG), s, ctx->dbv, F_Exi, F_RBxi, update_b ? F_Bxi : -1, -1.0,
-                                                             ctx->dt, 1.0, 0, nullptr);
-    return launched(ctx);
+    return launched(ctx, launch_k_curl_e2f(ctx->tune[TUNE_k_curl_e2f], ctx->hot, s, F_Exi, F_RBxi,
+                                           update_b ? F_Bxi : -1, -1.0, ctx->dt, 1.0, 0, nullptr, 0));
 }
 
 int launch_update_u(mhd_ctx *ctx)
 {
     prof_begin(ctx, "k_update_u");
-    k_update_u<<<grid_kind(ctx, KIND_CELL0), kThreads, 0, ctx->stream>>>(ctx->dbv, ctx->dt);
-    return launched(ctx);
+    return launched(ctx, launch_k_update_u(ctx->hot, ctx->stream, ctx->dt));
 }
 
 
@@ -831,9 +798,8 @@ int launch_curl_rng(mhd_ctx *ctx, int fE0, int fR0, int fB0, double mult, int mu
     if (R.nreg_max == 0)
         return MHD_OK;
     prof_begin(ctx, "k_curl_e2f");
-    launch_k_curl_e2f(ctx->tune[TUNE_k_curl_e2f], dim3(grid_for(R.nreg_max), ctx->nblocks), ctx->stream, 
-        ctx->dbv, fE0, fR0, fB0, mult, ctx->dt, 1.0, mult_is_neg_dt, R.rng);
-    return launched(ctx);
+    return launched(ctx, launch_k_curl_e2f(ctx->tune[TUNE_k_curl_e2f], ctx->hot, ctx->stream, fE0, fR0, fB0, mult,
+                                           ctx->dt, 1.0, mult_is_neg_dt, R.rng, R.nreg_max));
 }
 
 int launch_jedge_rng(mhd_ctx *ctx, int fB0, int fJ0)
@@ -842,8 +808,7 @@ int launch_jedge_rng(mhd_ctx *ctx, int fB0, int fJ0)
     if (R.nreg_max == 0)
         return MHD_OK;
     prof_begin(ctx, "k_jedge");
-    k_jedge<<<dim3(grid_for(R.nreg_max), ctx->nblocks), kThreads, 0, ctx->stream>>>(ctx->dbv, fB0, fJ0, 1.0, R.rng);
-    return launched(ctx);
+    return launched(ctx, launch_k_jedge(ctx->hot, ctx->stream, fB0, fJ0, R.rng, R.nreg_max));
 }
 
 // UnpackVecToImplicitEres_: Eres[unknowns] <- x (column *jdev of x0 when
@@ -1204,34 +1169,27 @@ int launch_step_c(mhd_ctx *ctx)
 // regulates Eres_eta on the pole rings.
 int launch_resistive_explicit(mhd_ctx *ctx)
 {
-    const int nb = ctx->nblocks;
     cudaStream_t s = ctx->stream;
-    const unsigned gs = grid_for(max_stagger(ctx));
     for (int q = 0; q < ctx->res_nsub; ++q)
     {
         RUN(run_sync(ctx, "Bface"));
         prof_begin(ctx, "k_bcell");
-        launch_k_bcell(false, dim3(grid_for(max_box(ctx, LOC_CELL, 0)), nb), s, ctx->dbv);
-        RUN(launched(ctx));
+        RUN(launched(ctx, launch_k_bcell(ctx->hot, s)));
         RUN(run_sync(ctx, "B_cell"));
         RUN(launch_pole(ctx, POLE_BZETA));
         prof_begin(ctx, "k_jedge");
-        k_jedge<<<dim3(gs, nb), kThreads, 0, s>>>(ctx->dbv, F_Bxi, F_Jxi, 1.0, nullptr);
-        RUN(launched(ctx));
+        RUN(launched(ctx, launch_k_jedge(ctx->hot, s, F_Bxi, F_Jxi, nullptr, 0)));
         RUN(run_sync(ctx, "Jedge"));
         prof_begin(ctx, "k_jcell");
-        k_jcell<<<dim3(grid_for(max_box(ctx, LOC_CELL, 0)), nb), kThreads, 0, s>>>(ctx->dbv);
-        RUN(launched(ctx));
+        RUN(launched(ctx, launch_k_jcell(false, ctx->hot, s)));
         RUN(launch_pole(ctx, POLE_JCELL));
         RUN(run_sync(ctx, "J_cell"));
         prof_begin(ctx, "k_eres_explicit");
-        k_eres_explicit<<<dim3(gs, nb), kThreads, 0, s>>>(ctx->dbv, ctx->res_inver_Rem);
-        RUN(launched(ctx));
+        RUN(launched(ctx, launch_k_eres_explicit(ctx->hot, s, ctx->res_inver_Rem)));
         RUN(run_sync(ctx, "Eres"));
         prof_begin(ctx, "k_curl_e2f");
-        launch_k_curl_e2f(ctx->tune[TUNE_k_curl_e2f], dim3(gs, nb), s, ctx->dbv, F_Eresxi, F_RBresxi, F_Bxi, -1.0, ctx->dt,
-                                                     double(ctx->res_nsub), 0, nullptr);
-        RUN(launched(ctx));
+        RUN(launched(ctx, launch_k_curl_e2f(ctx->tune[TUNE_k_curl_e2f], ctx->hot, s, F_Eresxi, F_RBresxi, F_Bxi, -1.0,
+                                            ctx->dt, double(ctx->res_nsub), 0, nullptr, 0)));
         RUN(run_sync(ctx, "Bface"));
     }
     return MHD_OK;
@@ -1321,24 +1279,18 @@ int hall_copy_b(mhd_ctx *ctx, bool snapshot)
 // touches neither input).
 int hall_emf_from_current_b(mhd_ctx *ctx)
 {
-    const int nb = ctx->nblocks;
     cudaStream_t s = ctx->stream;
     prof_begin(ctx, "k_bcell_jedge");
-    launch_k_bcell_jedge(ctx->tune[TUNE_k_bcell_jedge], false, grid_kind(ctx, KIND_STAG), s, ctx->dbv);
-    RUN(launched(ctx));
+    RUN(launched(ctx, launch_k_bcell_jedge(ctx->tune[TUNE_k_bcell_jedge], false, ctx->hot, s)));
     RUN(run_sync(ctx, "B_cell", true));
     RUN(run_sync(ctx, "Jedge"));
     prof_begin(ctx, "k_jcell");
-    k_jcell<<<dim3(grid_for(max_box(ctx, LOC_CELL, 0)), nb), kThreads, 0, s>>>(ctx->dbv);
-    RUN(launched(ctx));
+    RUN(launched(ctx, launch_k_jcell(false, ctx->hot, s)));
     RUN(run_sync(ctx, "J_cell", true));
     prof_begin(ctx, "k_hall_cell");
-    k_hall_cell<<<dim3(grid_for(max_box(ctx, LOC_CELL, ctx->G)), nb), kThreads, 0, s>>>(ctx->dbv, ctx->c,
-                                                                                        ctx->hall_coef);
-    RUN(launched(ctx));
+    RUN(launched(ctx, launch_k_hall_cell(ctx->hot, s, ctx->c, ctx->hall_coef)));
     prof_begin(ctx, "k_hall_edge");
-    launch_k_hall_edge(ctx->tune[TUNE_k_hall_edge], grid_kind(ctx, KIND_STAG), s, ctx->dbv, ctx->hall_zb, ctx->hall_nzb);
-    return launched(ctx);
+    return launched(ctx, launch_k_hall_edge(ctx->tune[TUNE_k_hall_edge], ctx->hot, s, ctx->hall_zb, ctx->hall_nzb));
 }
 
 // the trial B of the Ehall unknowns in the pool (UnpackVecToEhallField_:
@@ -1353,13 +1305,8 @@ int hall_trial_b(mhd_ctx *ctx)
         LAUNCHN(k_alias_copy, H.nalias, ctx->pool, H.alias, H.owner, H.sign, H.nalias);
     RUN(run_sync(ctx, "Ehall", true));
     prof_begin(ctx, "k_curl_e2f");
-    if (H.from_snapshot)
-        k_curl_from_snapshot<<<grid_kind(ctx, KIND_STAG), kThreads, 0, ctx->stream>>>(ctx->dbv, F_Ehxi, F_RBxi, F_Bxi,
-                                                                                      -1.0, ctx->dt, H.bs);
-    else
-        launch_k_curl_e2f(ctx->tune[TUNE_k_curl_e2f], dim3(grid_for(max_stagger(ctx)), ctx->nblocks), ctx->stream,
-                          ctx->dbv, F_Ehxi, F_RBxi, F_Bxi, -1.0, ctx->dt, 1.0, 0, nullptr);
-    RUN(launched(ctx));
+    RUN(launched(ctx, launch_k_curl_e2f(ctx->tune[TUNE_k_curl_e2f], ctx->hot, ctx->stream, F_Ehxi, F_RBxi, F_Bxi, -1.0,
+                                        ctx->dt, 1.0, 0, nullptr, 0, H.from_snapshot ? H.bs : nullptr)));
     return run_sync(ctx, "Bface");
 }
 
@@ -1515,8 +1462,7 @@ int launch_resistive_part(mhd_ctx *ctx)
 int launch_rk2(mhd_ctx *ctx, int save)
 {
     prof_begin(ctx, "k_rk2");
-    k_rk2<<<grid_kind(ctx, KIND_STAG), kThreads, 0, ctx->stream>>>(ctx->dbv, save);
-    return launched(ctx);
+    return launched(ctx, launch_k_rk2(ctx->hot, ctx->stream, save));
 }
 
 // One SSP-RK2 step (Shu and Osher, 1988) from two of StepOnce's Euler stages
@@ -1691,6 +1637,52 @@ extern "C" {
 
 namespace
 {
+// the hot kernels' launch arguments from the blocks' views
+void build_hot(mhd_ctx *ctx)
+{
+    ctx->hot.G = ctx->G;
+    ctx->hot.chunks.clear();
+    for (int b0 = 0; b0 < ctx->nblocks; b0 += kHotMax)
+    {
+        HotChunk c{};
+        c.args.n = std::min(ctx->nblocks - b0, kHotMax);
+        c.args.flat = ctx->nruns > 1 ? 1 : 0;
+        for (int q = 0; q < c.args.n; ++q)
+        {
+            const BlockView &v = ctx->hbv[size_t(b0 + q)];
+            HotBlock &h = c.args.v[q];
+            h.p0 = v.f[0];
+            h.p32 = v.g32;
+            h.rk = v.rk;
+            h.qref = v.qref;
+            h.vol = uint32_t(v.vol);
+            h.si = uint32_t(v.NJ) * uint32_t(v.NK);
+            h.sj = uint32_t(v.NK);
+            h.o = uint32_t(pidx(v, 0, 0, 0));
+            h.ni = v.ni;
+            h.nj = v.nj;
+            h.nk = v.nk;
+            h.run = v.run;
+            h.blk = b0 + q;
+            const int e[3] = {0, 2, 1}; // KIND_CELL0, KIND_CELL1, KIND_STAG
+            for (int kind = 0; kind < 3; ++kind)
+            {
+                h.dk[kind] = fast_div(uint32_t(v.nk + e[kind]));
+                h.dj[kind] = fast_div(uint32_t(v.nj + e[kind]));
+                const uint32_t n = grid_for(kind_points(v, kind));
+                h.cta0[kind] = int(c.ctas[kind]);
+                c.ctas[kind] = c.args.flat ? c.ctas[kind] + n : std::max(c.ctas[kind], n);
+            }
+            c.padded = std::max(c.padded, int64_t(v.ni + 2 * v.G) * (v.nj + 2 * v.G) * (v.nk + 2 * v.G));
+        }
+        c.few.n = c.args.n;
+        c.few.flat = c.args.flat;
+        for (int q = 0; q < std::min(c.args.n, kHotFew); ++q)
+            c.few.v[q] = c.args.v[q];
+        ctx->hot.chunks.push_back(c);
+    }
+}
+
 int create_ctx(const mhd_block_desc *blocks, int32_t nblocks, const int32_t *run_of_block, int32_t nruns,
                const mhd_params *params, mhd_ctx **out)
 {
@@ -1751,13 +1743,17 @@ int create_ctx(const mhd_block_desc *blocks, int32_t nblocks, const int32_t *run
         const int NI = v.ni + 1 + 2 * v.G;
         v.NJ = v.nj + 1 + 2 * v.G;
         v.NK = v.nk + 1 + 2 * v.G;
-        v.vol = int64_t(NI) * v.NJ * v.NK;
+        v.vol = (int64_t(NI) * v.NJ * v.NK + 31) & ~int64_t(31); // 256-byte aligned planes
+        if (v.vol > INT32_MAX)
+        {
+            delete ctx;
+            return MHD_ENOMEM; // (more than any device holds)
+        }
         ctx->max_cells = std::max<int64_t>(ctx->max_cells, int64_t(v.ni) * v.nj * v.nk);
         for (int f = 0; f < NFIELD; ++f)
         {
             ctx->base[size_t(f)][size_t(b)] = off;
             off += size_t(kFields[f].ncomp) * size_t(v.vol);
-            off = (off + 31) & ~size_t(31); // 256-byte aligned planes
         }
     }
     ctx->pool_n = off;
@@ -1827,34 +1823,29 @@ int create_ctx(const mhd_block_desc *blocks, int32_t nblocks, const int32_t *run
     }
     for (int b = 0; b < nblocks; ++b)
         ctx->hbv[size_t(b)].qref = ctx->qref + 6 * size_t(run[size_t(b)]);
-    // flattened launches when the batch holds several runs
+    // a batch of several runs launches one grid row of every block's CTAs: the
+    // block of each CTA of the face-tiled kernels (the hot kernels search
+    // their launch arguments instead)
     if (nruns > 1)
     {
         std::vector<int> tab;
-        int64_t first[NKIND] = {};
-        for (int kind = 0; kind < NKIND; ++kind)
+        for (int b = 0; b < nblocks; ++b)
         {
-            first[kind] = int64_t(tab.size());
-            for (int b = 0; b < nblocks; ++b)
-            {
-                BlockView &v = ctx->hbv[size_t(b)];
-                const int64_t n = grid_for(kind_points(v, kind));
-                v.cta0[kind] = int(int64_t(tab.size()) - first[kind]);
-                tab.insert(tab.end(), size_t(n), b);
-            }
-            ctx->cta_total[kind] = int64_t(tab.size()) - first[kind];
-            if (ctx->cta_total[kind] > INT_MAX)
-                return bail(MHD_EINVAL);
+            BlockView &v = ctx->hbv[size_t(b)];
+            v.tile0 = int(tab.size());
+            tab.insert(tab.end(), size_t(grid_for(kind_points(v, KIND_TILE1))), b);
         }
+        if (tab.size() > size_t(INT_MAX))
+            return bail(MHD_EINVAL);
+        ctx->tiles = int64_t(tab.size());
         if (cudaMalloc(&ctx->cta_tab, tab.size() * sizeof(int)) != cudaSuccess)
             return bail(MHD_ENOMEM);
         if (cudaMemcpy(ctx->cta_tab, tab.data(), tab.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess)
             return bail(MHD_ECUDA);
         for (auto &v : ctx->hbv)
-            for (int kind = 0; kind < NKIND; ++kind)
-                v.cta_blk[kind] = ctx->cta_tab + first[kind];
-        ctx->flat = true;
+            v.tile_blk = ctx->cta_tab;
     }
+    build_hot(ctx);
     if (cudaMalloc(&ctx->dbv, sizeof(BlockView) * size_t(nblocks)) != cudaSuccess)
         return bail(MHD_ENOMEM);
     if (cudaMemcpy(ctx->dbv, ctx->hbv.data(), sizeof(BlockView) * size_t(nblocks), cudaMemcpyHostToDevice) !=
@@ -2443,9 +2434,7 @@ static int materialise_pv(mhd_ctx *ctx)
     RUN(materialise_group(ctx, "Ucell"));
     RUN(ensure_geom(ctx));
     prof_begin(ctx, "k_pv_uplus_dt");
-    launch_k_pv_uplus_dt(ctx->tune[TUNE_k_pv_uplus_dt], false, dim3(grid_for(max_box(ctx, LOC_CELL, ctx->G)), ctx->nblocks),
-                         ctx->stream, ctx->dbv, ctx->c, nullptr, ctx->G, 0);
-    RUN(launched(ctx));
+    RUN(launched(ctx, launch_k_pv_all(ctx->hot, ctx->stream, ctx->c)));
     RUN(run_sync(ctx, "Uplus", true));
     ctx->pv_dirty = false;
     return MHD_OK;
@@ -3506,6 +3495,7 @@ int mhd_set_integrator(mhd_ctx *ctx, int32_t integrator)
                 v.rk = ctx->rk + o;
                 o += 8 * size_t(v.vol);
             }
+            build_hot(ctx);
             CK(ctx, cudaMemcpyAsync(ctx->dbv, ctx->hbv.data(), sizeof(BlockView) * ctx->hbv.size(),
                                     cudaMemcpyHostToDevice, ctx->stream));
             CK(ctx, cudaStreamSynchronize(ctx->stream));
@@ -3727,7 +3717,7 @@ int mhd_stage(mhd_ctx *ctx, int32_t stage_id)
         RUN(launched(ctx));
         break;
     case MHD_STAGE_FLUID_RHS:
-        RUN(launch_fluid_rhs(ctx));
+        RUN(launch_fluid_ucontra(ctx));
         break;
     case MHD_STAGE_INDUCTION:
         RUN(launch_induction(ctx, false));
@@ -3736,9 +3726,8 @@ int mhd_stage(mhd_ctx *ctx, int32_t stage_id)
         RUN(launch_update_u(ctx));
         {
             prof_begin(ctx, "k_curl_e2f");
-            launch_k_curl_e2f(ctx->tune[TUNE_k_curl_e2f], grid_kind(ctx, KIND_STAG), ctx->stream, ctx->dbv, F_Exi, -1, F_Bxi, -1.0,
-                                                                                ctx->dt, 1.0, 0, nullptr);
-            RUN(launched(ctx));
+            RUN(launched(ctx, launch_k_curl_e2f(ctx->tune[TUNE_k_curl_e2f], ctx->hot, ctx->stream, F_Exi, -1, F_Bxi,
+                                                -1.0, ctx->dt, 1.0, 0, nullptr, 0)));
         }
         break;
     case MHD_STAGE_HALL_EMF:
@@ -3746,13 +3735,10 @@ int mhd_stage(mhd_ctx *ctx, int32_t stage_id)
         RUN(materialise_group(ctx, "B_cell"));
         RUN(materialise_group(ctx, "J_cell"));
         prof_begin(ctx, "k_hall_cell");
-        k_hall_cell<<<dim3(grid_for(max_box(ctx, LOC_CELL, ctx->G)), ctx->nblocks), kThreads, 0, ctx->stream>>>(
-            ctx->dbv, ctx->c, ctx->hall_coef);
-        RUN(launched(ctx));
+        RUN(launched(ctx, launch_k_hall_cell(ctx->hot, ctx->stream, ctx->c, ctx->hall_coef)));
         prof_begin(ctx, "k_hall_edge");
-        launch_k_hall_edge(ctx->tune[TUNE_k_hall_edge], grid_kind(ctx, KIND_STAG), ctx->stream, ctx->dbv,
-                           ctx->hall_zb, ctx->hall_nzb);
-        RUN(launched(ctx));
+        RUN(launched(ctx, launch_k_hall_edge(ctx->tune[TUNE_k_hall_edge], ctx->hot, ctx->stream, ctx->hall_zb,
+                                             ctx->hall_nzb)));
         break;
     case MHD_STAGE_HALL_SOLVE:
         // one implicit Hall solve at the current dt, then calc_Bcell (as StepOnce)
@@ -3760,8 +3746,7 @@ int mhd_stage(mhd_ctx *ctx, int32_t stage_id)
             return fail(ctx, MHD_ESTATE, "the implicit Hall solve is not set up");
         RUN(launch_hall_implicit(ctx));
         prof_begin(ctx, "k_bcell");
-        launch_k_bcell(false, dim3(grid_for(max_box(ctx, LOC_CELL, 0)), ctx->nblocks), ctx->stream, ctx->dbv);
-        RUN(launched(ctx));
+        RUN(launched(ctx, launch_k_bcell(ctx->hot, ctx->stream)));
         RUN(run_sync(ctx, "B_cell"));
         break;
     case MHD_STAGE_DIVB:

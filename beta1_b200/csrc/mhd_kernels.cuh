@@ -2,6 +2,7 @@
 #pragma once
 
 #include "mhd_layout.cuh"
+#include "mhd_hot.cuh"
 #include "mhd_pole.cuh"
 #include "mhd_geom.cuh"
 #include "mhd_output.cuh"
@@ -22,35 +23,11 @@ struct Consts
     double ne_floor;
 };
 
-__global__ void k_fluid_rhs(const BlockView *bvs, Consts c, int64_t maxpts);
 __global__ void k_ucontra(const BlockView *bvs);
 __global__ void k_face_normals(const BlockView *bvs);
-// Face / edge kernels run one thread per staggered point (i, j, k) in
-// [0, n + 1)^3 and handle all three axes there.  rng (may be null): per
-// block a region box lo[3], hi[3]; only points inside it are processed.
-__global__ void k_update_u(const BlockView *bvs, const double *dtp);
 __global__ void k_divb(const BlockView *bvs);
 // mixed precision (mhd_kernels_mixed.cu)
 __global__ void k_geom32(const BlockView *bvs);
-__global__ void k_rk2(const BlockView *bvs, int save);
-__global__ void k_hall_cell(const BlockView *bvs, Consts c, double hall_coef);
-// the Hall edge EMF, variant 0: per-edge cell reads (no launch bounds), 1: the
-// seven cells of a staggered point read once (at least 2 CTAs per SM); the
-// same bits
-int launch_k_hall_edge(int variant, dim3 grid, cudaStream_t st, const BlockView *bvs, const int *zb, int nzb);
-__global__ void k_eres_explicit(const BlockView *bvs, double inver_Rem);
-// calc_Bcell on the inner cells (2-D launch, one grid row per block); w32:
-// from the FP32 weight copies (mixed form)
-void launch_k_bcell(bool w32, dim3 grid, cudaStream_t st, const BlockView *bvs);
-__global__ void k_jedge(const BlockView *bvs, int fB0, int fJ0, double mult, const int *rng);
-__global__ void k_jcell(const BlockView *bvs);
-// RHS = mult curl E and B = B* + dt RHS on the inner faces, B* from a snapshot
-// (bs[3 * block + axis]: the snapshot's B arrays of each block, pool layout)
-__global__ void k_curl_from_snapshot(const BlockView *bvs, int fE0, int fR0, int fB0, double mult, const double *dtp,
-                                     const double *const *bs);
-// J_cell on the inner cells over the flattened KIND_CELL0 grid (w32: FP32 weights)
-void launch_k_jcell(bool w32, dim3 grid, cudaStream_t st, const BlockView *bvs);
-
 // Pole handlers and repairs on eta Poles (mhd_pole.cuh): per Pole a
 // (block, direction) pair in `poles`, one grid row per Pole
 __global__ void k_pole(const BlockView *bvs, const int *poles, int op);
@@ -276,27 +253,44 @@ __global__ void k_hall_take(double *X, const double *Xt, double *F, const double
 __global__ void k_copy_segments(double *dst, const double *src, const int64_t *seg, int nseg);
 
 
-// Hot stencil kernels in register / occupancy variants (the same code under
-// different __launch_bounds__ minimum CTAs per SM; 0 = no launch bounds, the
-// compiler's own allocation); variant 0 is the default.  Returns -1 for an
-// unknown variant.
-// k_pv_uplus_dt: minimum CTAs per SM 4, 0, 5, and variant 3: at 4 without
-// J_cell, which launch_k_jcell computes in a pass of its own before it; w32:
-// J_cell from the FP32 weight copies (mixed form)
-int launch_k_pv_uplus_dt(int variant, bool w32, dim3 grid, cudaStream_t st, const BlockView *bvs, Consts c,
-                         unsigned long long *dt_key, int depth, int with_jcell);
-// k_fluid_ucontra: minimum CTAs per SM 0, 3
-int launch_k_fluid_ucontra(int variant, dim3 grid, cudaStream_t st, const BlockView *bvs, Consts c);
-// k_bcell_jedge: minimum CTAs per SM 0, 6; w32 as above
-int launch_k_bcell_jedge(int variant, bool w32, dim3 grid, cudaStream_t st, const BlockView *bvs);
-// k_eface: minimum CTAs per SM 0, 6
-int launch_k_eface(int variant, dim3 grid, cudaStream_t st, const BlockView *bvs);
-// k_curl_e2f: minimum CTAs per SM 0, 6
-int launch_k_curl_e2f(int variant, dim3 grid, cudaStream_t st, const BlockView *bvs, int fE0, int fR0, int fB0,
-                      double mult, const double *dtp, double dtdiv, int mult_is_neg_dt, const int *rng);
-// k_eedge: minimum CTAs per SM 0, 8
-int launch_k_eedge(int variant, dim3 grid, cudaStream_t st, const BlockView *bvs);
-// k_fluid_mixed: minimum CTAs per SM 3, 0, 2
-int launch_k_fluid_mixed(int variant, dim3 grid, cudaStream_t st, const BlockView *bvs, Consts c);
+// Hot stencil kernels of a step (mhd_kernels_step.cu, mhd_kernels_mixed.cu).
+// Each launcher returns its number of launches (one per chunk of blocks, see
+// HotGrid) or -1 for an unknown variant; variants are register / occupancy
+// forms of the same code (minimum CTAs per SM of the launch bounds) with the
+// same bits, variant 0 the default.
+// k_pv_uplus_dt (KIND_CELL1): minimum CTAs per SM 4, 1, 5, and variant 3: at 4
+// without J_cell, which launch_k_jcell computes in a pass of its own before
+// it; w32: J_cell from the FP32 weight copies (mixed form)
+int launch_k_pv_uplus_dt(int variant, bool w32, const HotGrid &h, cudaStream_t st, Consts c, unsigned long long *dt_key);
+// PV_H, U_plus and the face states on the whole array
+int launch_k_pv_all(const HotGrid &h, cudaStream_t st, Consts c);
+// fluid RHS and contravariant velocities: minimum CTAs per SM 2, 3
+int launch_k_fluid_ucontra(int variant, const HotGrid &h, cudaStream_t st, Consts c);
+// B_cell with the J edges: minimum CTAs per SM 2, 6; w32 as above
+int launch_k_bcell_jedge(int variant, bool w32, const HotGrid &h, cudaStream_t st);
+// B_cell alone, the J edges of (fB0, fJ0) alone (rng: per block a region box
+// lo[3], hi[3] of at most nreg points; null: every inner edge), J_cell alone
+int launch_k_bcell(const HotGrid &h, cudaStream_t st);
+int launch_k_jedge(const HotGrid &h, cudaStream_t st, int fB0, int fJ0, const int *rng, int64_t nreg);
+int launch_k_jcell(bool w32, const HotGrid &h, cudaStream_t st);
+// face EMF: minimum CTAs per SM 2, 6; edge EMF: 3, 8
+int launch_k_eface(int variant, const HotGrid &h, cudaStream_t st);
+int launch_k_eedge(int variant, const HotGrid &h, cudaStream_t st);
+// RHS = mult curl E and B += dt / dtdiv RHS on the inner faces (fR0, fB0 < 0:
+// not written; rng, nreg as above): minimum CTAs per SM 1, 6.  bs (may be
+// null): B = B* + dt RHS with B* from a snapshot (bs[3 block + axis]: the
+// snapshot's B arrays of each block, pool layout)
+int launch_k_curl_e2f(int variant, const HotGrid &h, cudaStream_t st, int fE0, int fR0, int fB0, double mult,
+                      const double *dtp, double dtdiv, int mult_is_neg_dt, const int *rng, int64_t nreg,
+                      const double *const *bs = nullptr);
+int launch_k_update_u(const HotGrid &h, cudaStream_t st, const double *dtp);
+int launch_k_rk2(const HotGrid &h, cudaStream_t st, int save);
+int launch_k_eres_explicit(const HotGrid &h, cudaStream_t st, double inver_Rem);
+int launch_k_hall_cell(const HotGrid &h, cudaStream_t st, Consts c, double hall_coef);
+// Hall edge EMF (zb: boxes of zeroed edges): minimum CTAs per SM 4, 2
+int launch_k_hall_edge(int variant, const HotGrid &h, cudaStream_t st, const int *zb, int nzb);
+// k_fluid_mixed: minimum CTAs per SM 3, 1, 2; variants 3 and 4 are the
+// face-tiled kernels (on `tiles`, the KIND_TILE1 grid of bvs)
+int launch_k_fluid_mixed(int variant, const HotGrid &h, dim3 tiles, cudaStream_t st, const BlockView *bvs, Consts c);
 
 } // namespace mhd

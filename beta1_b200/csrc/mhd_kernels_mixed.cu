@@ -15,6 +15,7 @@
 // FP64 round-off.  Compiled without contracted multiply-adds, so that the
 // per-cell and the face-tiled flux kernels give the same bits.
 #include "mhd_kernels.cuh"
+#include "mhd_hot_launch.cuh"
 
 namespace mhd
 {
@@ -119,84 +120,79 @@ __device__ __forceinline__ void rusanov_dev32(const BlockView &b, const Ref32 &r
 // divergence of the reference-state flux Phi0(S) (S the sum of the cell's
 // signed face vectors), the FP64 J x B force with the Hall_Num_Limiter weight
 // and its work, over the FP64 cell volume
-__device__ __forceinline__ void mixed_rhs(const BlockView &b, const Consts &c, int64_t p, double jac,
-                                          const double S[3], const float r[5])
+__device__ __forceinline__ void mixed_rhs(const double *q0, const Consts &c, const double U[4], const double J[3],
+                                          const double B[3], double jac, const double S[3], const float r[5],
+                                          double R[5])
 {
-    const int64_t v = b.vol;
-    const double *q0 = b.qref;
     const double US = S[0] * q0[1] + S[1] * q0[2] + S[2] * q0[3];
     const double mS = q0[0] * US;
     const double phi[5] = {mS, mS * q0[1] + S[0] * q0[4], mS * q0[2] + S[1] * q0[4], mS * q0[3] + S[2] * q0[4],
                            US * (q0[5] + q0[4])};
-    const double rho = b.f[F_U][p];
+    const double rho = U[0];
     const double n_true = ((rho < 0.0) ? 0.0 : rho) / c.M_H * c.M_ref;
     const double fc = c.mom_hall * (n_true / sqrt(n_true * n_true + c.ne_floor * c.ne_floor));
-    const double *J = b.f[F_Jcell], *B = b.f[F_Bcell], *U = b.f[F_U];
-    const double jx = J[p], jy = J[v + p], jz = J[2 * v + p];
-    const double bx = B[p], by = B[v + p], bz = B[2 * v + p];
-    const double fx = jy * bz - jz * by, fy = jz * bx - jx * bz, fz = jx * by - jy * bx;
+    const double fx = J[1] * B[2] - J[2] * B[1], fy = J[2] * B[0] - J[0] * B[2], fz = J[0] * B[1] - J[1] * B[0];
     const double invJ = 1.0 / jac;
     // the work uses calc_PV's velocities U_m / max(rho, 1e-12) (the mixed
     // form's derived pass leaves PV_H to read-out), as one quotient
     const double rho_pv = (rho < 1e-12) ? 1e-12 : rho;
-    const double fU = fx * U[v + p] + fy * U[2 * v + p] + fz * U[3 * v + p];
-    double *R = b.f[F_RHS];
-    R[p] = -(double(r[0]) + phi[0]) * invJ;
-    R[v + p] = -(double(r[1]) + phi[1]) * invJ + fc * fx;
-    R[2 * v + p] = -(double(r[2]) + phi[2]) * invJ + fc * fy;
-    R[3 * v + p] = -(double(r[3]) + phi[3]) * invJ + fc * fz;
-    R[4 * v + p] = -(double(r[4]) + phi[4]) * invJ + fc * (fU / rho_pv);
+    const double fU = fx * U[1] + fy * U[2] + fz * U[3];
+    R[0] = -(double(r[0]) + phi[0]) * invJ;
+    R[1] = -(double(r[1]) + phi[1]) * invJ + fc * fx;
+    R[2] = -(double(r[2]) + phi[2]) * invJ + fc * fy;
+    R[3] = -(double(r[3]) + phi[3]) * invJ + fc * fz;
+    R[4] = -(double(r[4]) + phi[4]) * invJ + fc * (fU / rho_pv);
 }
 
 // Fluid RHS of the inner cells (FP32 flux divergence, FP64 J x B source) and
 // the FP64 contravariant velocities of the cells within one ghost layer; the
-// FP64 face metric read for the velocities is the one the fluxes round.
-// variants: at least 3 CTAs per SM (80 registers; the default: 1.73 -> 1.52 ms
-// per step on the shell sweep against 2 CTAs per SM), uncapped (96
-// registers), at least 2
-__device__ __forceinline__ void k_fluid_mixed_body(const BlockView *__restrict__ bvs, Consts c)
+// FP64 face metric read for the velocities is the one the fluxes round.  All
+// stores are at the end, so that the loads of one axis do not wait for the
+// results of the axis before.
+// variants: at least 3 CTAs per SM (80 registers; the default), the
+// compiler's own allocation, at least 2
+struct QHot
 {
-    int64_t t;
-    const BlockView &b = bvs[cta_block(bvs, KIND_CELL1, t)];
-    const int lo = -1;
-    const int n0 = b.ni + 2, n1 = b.nj + 2, n2 = b.nk + 2;
-    if (t >= int64_t(n0) * n1 * n2)
+    const float *q;
+    uint64_t v;
+    __device__ __forceinline__ float operator()(int plane, int64_t c) const { return q[plane * v + c]; }
+};
+
+template <class A> __device__ __forceinline__ void k_fluid_mixed_body(const A &args, const Consts &c)
+{
+    uint32_t t, p;
+    const HotBlock &b = hot_block<KIND_CELL1>(args, t);
+    int i, j, k;
+    if (!hot_point<KIND_CELL1>(b, t, i, j, k, p))
         return;
-    const int k = lo + int(t % n2);
-    t /= n2;
-    const int j = lo + int(t % n1);
-    const int i = lo + int(t / n1);
-    const int64_t v = b.vol;
-    const int64_t p = pidx(b, i, j, k);
-    const double jac = b.f[F_Jac][p];
-    const bool inner = i >= 0 && j >= 0 && k >= 0 && i < b.ni && j < b.nj && k < b.nk;
+    const uint64_t v = b.vol;
+    const bool inner = hot_inner(b, i, j, k);
+    const double jac = *hot_at(b, p, F_Jac);
     // contravariant velocities (cell_u_contra): (k-bar . U_plus) / (|Jac| + 1e-30)
-    const double *Up = b.f[F_Uplus];
-    const double ux = Up[p], uy = Up[v + p], uz = Up[2 * v + p];
+    const double *Up = hot_at(b, p, F_Uplus);
+    const double ux = Up[0], uy = Up[v], uz = Up[2 * v];
     const double inv_jac = 1.0 / (fabs(jac) + 1.0e-30);
-    double *UC = b.f[F_UC];
-    const float *g = b.g32;
     const double *q0 = b.qref;
     const Ref32 r0 = {float(q0[0]), {float(q0[1]), float(q0[2]), float(q0[3])}, float(q0[5] + q0[4])};
-    // one axis at a time: its face metric at the low (p) and high (pp) face,
-    // the cell's velocity along it, its share of the FP64 sum of signed face
-    // vectors, and (inner cells) its two FP32 face fluxes -- the same
-    // operations in the same order as forming all three axes first, with a
-    // third of the metric live at once
+    const QHot q{hot_plane32(b, p, kPlane32Q), v};
+    // one axis at a time: its face metric at the low and high face, the
+    // cell's velocity along it, its share of the FP64 sum of signed face
+    // vectors, and (inner cells) its two FP32 face fluxes
     double S[3] = {0.0, 0.0, 0.0};
     float r[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+    double uc[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a)
     {
-        const int64_t pp = a == 0 ? pidx(b, i + 1, j, k) : a == 1 ? pidx(b, i, j + 1, k) : pidx(b, i, j, k + 1);
-        const double *M = b.f[F_JDxi + a];
+        const int s = a == 0 ? int(b.si) : a == 1 ? int(b.sj) : 1;
+        const double *M = hot_at(b, p, F_JDxi + a);
         double m_[3], p_[3];
         float km[3], kp[3];
 #pragma unroll
         for (int d = 0; d < 3; ++d)
         {
-            m_[d] = M[d * v + p];
-            p_[d] = M[d * v + pp];
+            m_[d] = M[d * v];
+            p_[d] = M[d * v + s];
             km[d] = float(m_[d]);
             kp[d] = float(p_[d]);
             S[d] += p_[d] - m_[d];
@@ -204,31 +200,40 @@ __device__ __forceinline__ void k_fluid_mixed_body(const BlockView *__restrict__
         const double kx = 0.5 * (m_[0] + p_[0]);
         const double ky = 0.5 * (m_[1] + p_[1]);
         const double kz = 0.5 * (m_[2] + p_[2]);
-        UC[a * v + p] = (kx * ux + ky * uy + kz * uz) * inv_jac;
+        uc[a] = (kx * ux + ky * uy + kz * uz) * inv_jac;
         if (inner)
         {
-            const int64_t pm = a == 0 ? pidx(b, i - 1, j, k) : a == 1 ? pidx(b, i, j - 1, k) : pidx(b, i, j, k - 1);
+            const float *g = hot_plane32(b, p, G32_AREA + a);
             float Fm[5], Fp[5];
-            rusanov_dev32(b, r0, km[0], km[1], km[2], g[(G32_AREA + a) * v + p], p, pm, Fm);
-            rusanov_dev32(b, r0, kp[0], kp[1], kp[2], g[(G32_AREA + a) * v + pp], pp, p, Fp);
+            rusanov_dev32q(q, r0, km[0], km[1], km[2], g[0], 0, -s, Fm);
+            rusanov_dev32q(q, r0, kp[0], kp[1], kp[2], g[s], s, 0, Fp);
 #pragma unroll
             for (int m = 0; m < 5; ++m)
                 r[m] += Fp[m] - Fm[m];
         }
     }
     if (inner)
-        mixed_rhs(b, c, p, jac, S, r);
+    {
+        const double *U = hot_at(b, p, F_U), *J = hot_at(b, p, F_Jcell), *B = hot_at(b, p, F_Bcell);
+        const double u[4] = {U[0], U[v], U[2 * v], U[3 * v]};
+        const double Jc[3] = {J[0], J[v], J[2 * v]}, Bc[3] = {B[0], B[v], B[2 * v]};
+        double R[5];
+        mixed_rhs(q0, c, u, Jc, Bc, jac, S, r, R);
+        double *out = hot_at(b, p, F_RHS);
+#pragma unroll
+        for (int m = 0; m < 5; ++m)
+            out[m * v] = R[m];
+    }
+    double *UC = hot_at(b, p, F_UC);
+    UC[0] = uc[0];
+    UC[v] = uc[1];
+    UC[2 * v] = uc[2];
 }
 
-template <int MINB>
-__global__ void __launch_bounds__(256, MINB) k_fluid_mixed_t(const BlockView *__restrict__ bvs, Consts c)
+template <class A, int MINB>
+__global__ void __launch_bounds__(256, MINB) k_fluid_mixed_t(const __grid_constant__ A a, Consts c)
 {
-    k_fluid_mixed_body(bvs, c);
-}
-// the compiler's own register allocation (no launch bounds)
-__global__ void k_fluid_mixed_free(const BlockView *__restrict__ bvs, Consts c)
-{
-    k_fluid_mixed_body(bvs, c);
+    k_fluid_mixed_body(a, c);
 }
 
 
@@ -266,10 +271,9 @@ template <bool STAGED> __device__ __forceinline__ void k_fluid_mixed_tile_body(c
     __shared__ float Fy[TILE_I][TILE_J + 1][TILE_K][5];
     __shared__ float Fz[TILE_I][TILE_J][TILE_K + 1][5];
     __shared__ float qs[STAGED ? 7 * QS_N : 1];
-    int64_t t;
-    const BlockView &b = bvs[cta_block(bvs, KIND_TILE1, t)];
+    int64_t tile;
+    const BlockView &b = bvs[tile_block(bvs, tile)];
     const int ntj = (b.nj + 2 + TILE_J - 1) / TILE_J, ntk = (b.nk + 2 + TILE_K - 1) / TILE_K;
-    const int64_t tile = t / 256;
     if (tile >= int64_t((b.ni + 2 + TILE_I - 1) / TILE_I) * ntj * ntk)
         return; // the whole CTA
     const int i0 = -1 + int(tile / (int64_t(ntj) * ntk)) * TILE_I;
@@ -407,7 +411,14 @@ template <bool STAGED> __device__ __forceinline__ void k_fluid_mixed_tile_body(c
         for (int m = 0; m < 5; ++m)
             r[m] += Fp[m] - Fm[m];
     }
-    mixed_rhs(b, c, p, jac, S, r);
+    const double *U = b.f[F_U], *J = b.f[F_Jcell], *B = b.f[F_Bcell];
+    const double u[4] = {U[p], U[v + p], U[2 * v + p], U[3 * v + p]};
+    const double Jc[3] = {J[p], J[v + p], J[2 * v + p]}, Bc[3] = {B[p], B[v + p], B[2 * v + p]};
+    double R[5];
+    mixed_rhs(q0, c, u, Jc, Bc, jac, S, r, R);
+#pragma unroll
+    for (int m = 0; m < 5; ++m)
+        b.f[F_RHS][m * v + p] = R[m];
 }
 
 __global__ void __launch_bounds__(256, 2) k_fluid_mixed_tile(const BlockView *__restrict__ bvs, Consts c)
@@ -423,29 +434,27 @@ __global__ void __launch_bounds__(256, 2) k_fluid_mixed_staged(const BlockView *
 // launchers of the register / occupancy variants (tuned by mhd_autotune);
 // variant 3 is the face-tiled kernel, 4 the same with the staged face states
 // (both on the KIND_TILE1 grid)
-int launch_k_fluid_mixed(int variant, dim3 grid, cudaStream_t st, const BlockView *bvs, Consts c)
+int launch_k_fluid_mixed(int variant, const HotGrid &h, dim3 tiles, cudaStream_t st, const BlockView *bvs, Consts c)
 {
-    switch (variant)
-    {
-    case 3:
-        k_fluid_mixed_tile<<<grid, 256, 0, st>>>(bvs, c);
-        break;
-    case 4:
-        k_fluid_mixed_staged<<<grid, 256, 0, st>>>(bvs, c);
-        break;
-    case 0:
-        k_fluid_mixed_t<3><<<grid, 256, 0, st>>>(bvs, c);
-        break;
-    case 1:
-        k_fluid_mixed_free<<<grid, 256, 0, st>>>(bvs, c);
-        break;
-    case 2:
-        k_fluid_mixed_t<2><<<grid, 256, 0, st>>>(bvs, c);
-        break;
-    default:
+    if (variant < 0 || variant > 4)
         return -1;
+    if (variant >= 3)
+    {
+        if (variant == 3)
+            k_fluid_mixed_tile<<<tiles, 256, 0, st>>>(bvs, c);
+        else
+            k_fluid_mixed_staged<<<tiles, 256, 0, st>>>(bvs, c);
+        return 1;
     }
-    return 0;
+    return hot_for(h, KIND_CELL1, [&](const auto &a, dim3 g) {
+        using A = std::decay_t<decltype(a)>;
+        if (variant == 0)
+            hot_launch(k_fluid_mixed_t<A, 3>, g, st, a, c);
+        else if (variant == 1)
+            hot_launch(k_fluid_mixed_t<A, 1>, g, st, a, c);
+        else
+            hot_launch(k_fluid_mixed_t<A, 2>, g, st, a, c);
+    });
 }
 
 } // namespace mhd

@@ -139,39 +139,37 @@ struct BlockView
     // reference state of the mixed-precision flux (rho, u, v, w, p, E)
     int run;
     const double *qref;
-    // flattened launches over blocks of uneven sizes: per launch kind the
-    // block of every CTA (same table in every view; null = 2-D launches with
-    // one grid row per block) and this block's first CTA
-    const int *cta_blk[4];
-    int cta0[4];
+    // face-tiled kernels in one grid row over blocks of uneven sizes: the
+    // block of every CTA (same table in every view; null = one grid row per
+    // block) and this block's first CTA
+    const int *tile_blk;
+    int tile0;
 };
 
-// launch kinds of the flattened grids: cells with depth 0, cells with depth
-// 1, the staggered box [0, n + 1)^3 of the face / edge kernels, and tiles of
-// TILE_I x TILE_J x TILE_K cells over the depth-1 box (one CTA each)
+// launch kinds: cells with depth 0, cells with depth 1, the staggered box
+// [0, n + 1)^3 of the face / edge kernels, and tiles of TILE_I x TILE_J x
+// TILE_K cells over the depth-1 box (one CTA each)
 enum : int
 {
     KIND_CELL0 = 0,
     KIND_CELL1 = 1,
     KIND_STAG = 2,
-    KIND_TILE1 = 3,
-    NKIND = 4
+    KIND_TILE1 = 3
 };
 constexpr int TILE_I = 2, TILE_J = 4, TILE_K = 32; // TILE_I * TILE_J * TILE_K = 256 threads
 
 #ifdef __CUDACC__
-// Block and thread-in-block of the calling thread: flattened launches (one
-// grid row) look the block up per CTA, 2-D launches take blockIdx.y.
-__device__ __forceinline__ int cta_block(const BlockView *bvs, int kind, int64_t &t)
+// block of the calling CTA of a face-tiled kernel and its tile
+__device__ __forceinline__ int tile_block(const BlockView *bvs, int64_t &tile)
 {
-    const int *tab = bvs[0].cta_blk[kind];
+    const int *tab = bvs[0].tile_blk;
     if (tab && gridDim.y == 1)
     {
         const int bi = tab[blockIdx.x];
-        t = int64_t(blockIdx.x - bvs[bi].cta0[kind]) * blockDim.x + threadIdx.x;
+        tile = int64_t(blockIdx.x) - bvs[bi].tile0;
         return bi;
     }
-    t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    tile = blockIdx.x;
     return int(blockIdx.y);
 }
 #endif
