@@ -7,6 +7,8 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <bitset>
+#include <initializer_list>
 #include <climits>
 #include <cmath>
 #include <cstdint>
@@ -76,9 +78,37 @@ struct CopyList
     uint64_t *src = nullptr;
     double *tmp = nullptr; // non-null when a source is also a destination
     int64_t n = 0;
-    // the same copies with 32-bit offsets, when the pool has fewer than 2^32
-    // points and no copy is staged (a quarter less traffic per copy)
-    uint32_t *dst32 = nullptr, *src32 = nullptr;
+};
+
+// One pass of a step's Syncs: copies and fixed values that depend on no other
+// of the pass, with 32-bit pool offsets where the pool has fewer than 2^32
+// points (24 instead of 32 bytes moved per copy).
+struct SyncPass
+{
+    uint64_t *dst = nullptr, *src = nullptr, *cdst = nullptr;
+    uint32_t *dst32 = nullptr, *src32 = nullptr, *cdst32 = nullptr;
+    double *cval = nullptr;
+    int64_t n = 0, nconst = 0;
+};
+// The Syncs of consecutive groups as passes: one, or (wall handlers in a
+// Pole context) one before and one after them.
+struct StepSync
+{
+    SyncPass a, b;
+    bool usable = false; // else the groups' own lists run one by one
+};
+
+// A group's hot part resolved on the host to independent copies and fixed
+// values: a, and in a Pole context with wall handlers b after them.
+struct Resolved
+{
+    struct Part
+    {
+        std::vector<uint64_t> d, s, cd;
+        std::vector<double> cv;
+    } a, b;
+    std::bitset<NFIELD> fields; // fields it writes or reads
+    bool usable = false;
 };
 
 // One sync group.  The full tables are what the reference's Sync writes.
@@ -98,6 +128,7 @@ struct SyncMap
     bool staged = false;
     bool built = false; // device lists match the host tables
     CopyList full, hot, post;
+    Resolved res, res_full; // of the hot and of the full lists
     // Pole contexts: the copies and fixed values a step leaves for read-out
     // (cold), written then without the rings, walls and post-wall copies
     CopyList cold;
@@ -196,6 +227,7 @@ struct mhd_ctx
     int *cta_tab = nullptr; // block of every CTA of the face-tiled kernels (batches)
     int64_t tiles = 0;      // those CTAs
     std::map<std::string, SyncMap> syncs;
+    std::map<std::string, StepSync> step_syncs; // by the groups' names joined with '+'
     // eta Poles: (block, direction) pairs; a context with Poles runs every
     // sync in the topology order of the Pole shell
     std::vector<int> poles;
@@ -323,12 +355,14 @@ struct mhd_ctx
 static void free_resistive(mhd_ctx *ctx);
 static int resistive_region(mhd_ctx *ctx, const std::vector<uint64_t> &seed);
 static void free_list(CopyList &m);
+static void free_step_syncs(mhd_ctx *ctx);
 static int build_all_syncs(mhd_ctx *ctx);
 static int materialise_field(mhd_ctx *ctx, int f);
 static int materialise_group(mhd_ctx *ctx, const std::string &group);
 static int materialise_all(mhd_ctx *ctx);
 static void mark_dirty(mhd_ctx *ctx);
 int build_sync(mhd_ctx *ctx, const std::string &group, SyncMap &m);
+static int step_sync(mhd_ctx *ctx, std::initializer_list<const char *> groups, unsigned full, StepSync **out);
 
 namespace
 {
@@ -483,41 +517,48 @@ int gather_map(mhd_ctx *ctx, const CopyList &s)
         return launched(ctx);
     }
     prof_begin(ctx, "k_gather");
-    if (s.dst32)
-        k_gather32<<<grid_for(s.n), kThreads, 0, ctx->stream>>>(ctx->pool, s.dst32, s.src32, s.n);
-    else
-        k_gather<<<grid_for(s.n), kThreads, 0, ctx->stream>>>(ctx->pool, s.dst, s.src, s.n);
+    k_gather<<<grid_for(s.n), kThreads, 0, ctx->stream>>>(ctx->pool, s.dst, s.src, s.n);
+    return launched(ctx);
+}
+
+int set_consts(mhd_ctx *ctx, const CopyList &l)
+{
+    if (l.nconst == 0)
+        return MHD_OK;
+    prof_begin(ctx, "k_set_consts");
+    k_set_consts<<<grid_for(l.nconst), kThreads, 0, ctx->stream>>>(ctx->pool, l.cdst, l.cval, l.nconst);
     return launched(ctx);
 }
 
 // fixed values then copies of a list (no wall handlers)
 int apply_list(mhd_ctx *ctx, const CopyList &l)
 {
-    if (l.nconst > 0)
-    {
-        prof_begin(ctx, "k_set_consts");
-        k_set_consts<<<grid_for(l.nconst), kThreads, 0, ctx->stream>>>(ctx->pool, l.cdst, l.cval, l.nconst);
-        RUN(launched(ctx));
-    }
+    RUN(set_consts(ctx, l));
     return gather_map(ctx, l);
 }
 
-// one Pole operation on every Pole of the context
-int launch_pole(mhd_ctx *ctx, int op)
+// Pole operations that touch different points, on every Pole of the context in one launch
+int launch_pole(mhd_ctx *ctx, std::initializer_list<int> list, int jeta_ring = 1)
 {
     const int np = int(ctx->poles.size() / 2);
-    if (np == 0)
+    if (np == 0 || list.size() == 0)
         return MHD_OK;
-    int64_t w = 0;
+    int ni = 0, nk = 0;
     for (int q = 0; q < np; ++q)
     {
         const BlockView &v = ctx->hbv[size_t(ctx->poles[size_t(2 * q)])];
-        w = std::max(w, pole_work(op, v.ni, v.nk));
+        ni = std::max(ni, v.ni);
+        nk = std::max(nk, v.nk);
     }
+    PoleOps ops{};
+    for (int op : list)
+        ops.op[ops.n++] = op;
+    ops.jeta_ring = jeta_ring;
     prof_begin(ctx, "k_pole");
-    launch_pole_op(op, w, np, ctx->stream, ctx->dbv, ctx->dpoles, ctx->pole_cache, ctx->pole_stride, 0);
+    launch_pole_ops(ops, ni, nk, np, ctx->stream, ctx->dbv, ctx->dpoles, ctx->pole_cache, ctx->pole_stride);
     return launched(ctx);
 }
+int launch_pole(mhd_ctx *ctx, int op) { return launch_pole(ctx, {op}); }
 
 // the values the Pole handlers of a group compute on the pole rings
 // (Z4_Lunar/src/boundary/Boundary_Build.cpp:61-269)
@@ -529,16 +570,35 @@ int pole_rings(mhd_ctx *ctx, const std::string &group)
         return launch_pole(ctx, POLE_RING_BXI);
     if (group == "B_cell")
         return launch_pole(ctx, POLE_BCELL);
-    if (group == "Eedge")
-    {
-        RUN(launch_pole(ctx, POLE_EXI_AXIS));
-        return launch_pole(ctx, POLE_EETA_REG);
-    }
+    if (group == "Eedge") // E_xi on the pole line, E_eta on the ring
+        return launch_pole(ctx, {POLE_EXI_AXIS, POLE_EETA_REG});
     if (group == "Jedge")
         return launch_pole(ctx, POLE_JETA);
     if (group == "Eres" || group == "Eres1form")
         return launch_pole(ctx, POLE_ERES_REG);
     return MHD_OK;
+}
+
+int run_pass(mhd_ctx *ctx, const SyncPass &p)
+{
+    if (p.n + p.nconst == 0)
+        return MHD_OK;
+    prof_begin(ctx, "k_gather");
+    if (p.dst32 || p.cdst32)
+        launch_k_sync(ctx->stream, ctx->pool, p.dst32, p.src32, p.n, p.cdst32, p.cval, p.nconst);
+    else
+        launch_k_sync(ctx->stream, ctx->pool, p.dst, p.src, p.n, p.cdst, p.cval, p.nconst);
+    return launched(ctx);
+}
+
+int run_walls(mhd_ctx *ctx, const SyncMap &m)
+{
+    if (m.walls.empty())
+        return MHD_OK;
+    prof_begin(ctx, "k_wall_u_all");
+    launch_k_wall_u(dim3(grid_for(m.wall_cols), unsigned(m.walls.size())), ctx->stream, ctx->dbv, m.dwalls,
+                    ctx->c.gamma);
+    return launched(ctx);
 }
 
 // LunarBoundary::Sync(group): phase A (fixed values, wall handlers), then
@@ -547,7 +607,7 @@ int pole_rings(mhd_ctx *ctx, const std::string &group)
 // read before the wall handlers, the wall handlers, the copies of what they
 // wrote, then the fixed values -- always with the full lists (the Pole
 // repairs of the derived-field pass change sources of earlier syncs).
-int run_sync(mhd_ctx *ctx, const char *group, bool full = false)
+int run_sync(mhd_ctx *ctx, const char *group, bool full = false, bool rings = true)
 {
     auto it = ctx->syncs.find(group);
     if (it == ctx->syncs.end())
@@ -559,46 +619,60 @@ int run_sync(mhd_ctx *ctx, const char *group, bool full = false)
             return fail(ctx, MHD_ESTATE, "sync group %s changed during capture", group);
         RUN(build_sync(ctx, it->first, m));
     }
+    const CopyList &l = full ? m.full : m.hot;
     if (!ctx->poles.empty())
     {
         // the hot lists in a step: the cold rest is written at read-out
-        const CopyList &l = full ? m.full : m.hot;
-        RUN(pole_rings(ctx, it->first));
+        if (rings)
+            RUN(pole_rings(ctx, it->first));
         RUN(gather_map(ctx, l));
-        if (!m.walls.empty())
-        {
-            prof_begin(ctx, "k_wall_u_all");
-            k_wall_u_all<<<dim3(grid_for(m.wall_cols), unsigned(m.walls.size())), kThreads, 0, ctx->stream>>>(
-                ctx->dbv, m.dwalls, ctx->c.gamma);
-            RUN(launched(ctx));
-        }
+        RUN(run_walls(ctx, m));
         RUN(gather_map(ctx, m.post));
-        if (l.nconst > 0)
-        {
-            prof_begin(ctx, "k_set_consts");
-            k_set_consts<<<grid_for(l.nconst), kThreads, 0, ctx->stream>>>(ctx->pool, l.cdst, l.cval, l.nconst);
-            RUN(launched(ctx));
-        }
+        RUN(set_consts(ctx, l));
         ctx->dirty[it->first] = !full && (m.cold.n > 0 || m.cold.nconst > 0);
         return MHD_OK;
     }
-    const CopyList &l = full ? m.full : m.hot;
-    if (l.nconst > 0)
-    {
-        prof_begin(ctx, "k_set_consts");
-        k_set_consts<<<grid_for(l.nconst), kThreads, 0, ctx->stream>>>(ctx->pool, l.cdst, l.cval, l.nconst);
-        RUN(launched(ctx));
-    }
-    if (!m.walls.empty())
-    {
-        prof_begin(ctx, "k_wall_u_all");
-        k_wall_u_all<<<dim3(grid_for(m.wall_cols), unsigned(m.walls.size())), kThreads, 0, ctx->stream>>>(
-            ctx->dbv, m.dwalls, ctx->c.gamma);
-        RUN(launched(ctx));
-    }
+    RUN(set_consts(ctx, l));
+    RUN(run_walls(ctx, m));
     RUN(gather_map(ctx, l));
     ctx->dirty[it->first] = !full && (m.hot.n != m.full.n || m.hot.nconst != m.full.nconst);
     return MHD_OK;
+}
+
+// The Syncs of consecutive groups of a step (hot lists; full[q]: the full list
+// of group q) in as few passes as their dependences allow: wall handlers, if
+// any, and one pass of all copies and fixed values (build_step_sync resolves
+// them); one by one where they cannot be resolved.
+int run_syncs(mhd_ctx *ctx, std::initializer_list<const char *> groups, bool rings = true, unsigned full = 0)
+{
+    StepSync *s = nullptr;
+    RUN(step_sync(ctx, groups, full, &s));
+    unsigned q = 0;
+    if (!s->usable)
+    {
+        for (const char *g : groups)
+            RUN(run_sync(ctx, g, ((full >> q++) & 1) != 0, rings));
+        return MHD_OK;
+    }
+    const bool poles = !ctx->poles.empty();
+    if (poles && rings)
+        for (const char *g : groups)
+            if (ctx->syncs.count(g))
+                RUN(pole_rings(ctx, g));
+    if (poles)
+        RUN(run_pass(ctx, s->a));
+    for (const char *g : groups)
+    {
+        const bool f = ((full >> q++) & 1) != 0;
+        const auto it = ctx->syncs.find(g);
+        if (it == ctx->syncs.end())
+            continue;
+        const SyncMap &m = it->second;
+        RUN(run_walls(ctx, m));
+        ctx->dirty[it->first] = poles ? !f && (m.cold.n > 0 || m.cold.nconst > 0)
+                                      : !f && (m.hot.n != m.full.n || m.hot.nconst != m.full.nconst);
+    }
+    return run_pass(ctx, poles ? s->b : s->a);
 }
 
 // face areas and unit normals from the uploaded JD (eager, outside graphs)
@@ -639,14 +713,15 @@ int ensure_geom(mhd_ctx *ctx)
         }
         for (int op : {int(POLE_BCELL), int(POLE_EETA_REG), int(POLE_JCELL)})
         {
-            int64_t w = 0;
+            int ni = 0, nk = 0;
             for (int q = 0; q < np; ++q)
             {
                 const BlockView &v = ctx->hbv[size_t(ctx->poles[size_t(2 * q)])];
-                w = std::max(w, pole_work(op, v.ni, v.nk));
+                ni = std::max(ni, v.ni);
+                nk = std::max(nk, v.nk);
             }
             prof_begin(ctx, "k_pole");
-            launch_pole_op(op, w, np, ctx->stream, ctx->dbv, ctx->dpoles, ctx->pole_cache, ctx->pole_stride, 1);
+            launch_pole_build(op, ni, nk, np, ctx->stream, ctx->dbv, ctx->dpoles, ctx->pole_cache, ctx->pole_stride);
             RUN(launched(ctx));
         }
     }
@@ -670,29 +745,33 @@ int launch_jcell_split(mhd_ctx *ctx)
     return launched(ctx, launch_k_jcell(ctx->pool32 != nullptr, ctx->hot, ctx->stream));
 }
 
-int launch_update_derived(mhd_ctx *ctx)
+int launch_arm_dt(mhd_ctx *ctx)
 {
+    prof_begin(ctx, "k_arm_dt");
+    k_arm_dt<<<1, 128, 0, ctx->stream>>>(ctx->dt_key, ctx->nruns);
+    return launched(ctx);
+}
+
+// armed: the dt reductions are (the step's update arms them)
+int launch_update_derived(mhd_ctx *ctx, bool armed)
+{
+    if (!armed)
+        RUN(launch_arm_dt(ctx));
     if (!ctx->poles.empty())
         return launch_update_derived_pole(ctx);
     cudaStream_t s = ctx->stream;
     prof_begin(ctx, "k_bcell_jedge");
     RUN(launched(ctx, launch_k_bcell_jedge(ctx->tune[TUNE_k_bcell_jedge], ctx->pool32 != nullptr, ctx->hot, s)));
-    RUN(run_sync(ctx, "B_cell"));
-    RUN(run_sync(ctx, "Jedge"));
-    // arm the dt reduction, then J_cell, PV / U_plus and the CFL bound of the next step
-    prof_begin(ctx, "k_arm_dt");
-    k_arm_dt<<<1, 128, 0, s>>>(ctx->dt_key, ctx->nruns);
-    RUN(launched(ctx));
-    // first ghost layer only: deeper PV / U_plus ghosts are read by no kernel
-    // of the step and are filled when read out (materialise_pv)
+    RUN(run_syncs(ctx, {"B_cell", "Jedge"}));
+    // J_cell, PV / U_plus and the CFL bound of the next step; the first ghost
+    // layer only: deeper PV / U_plus ghosts are read by no kernel of the step
+    // and are filled when read out (materialise_pv)
     RUN(launch_jcell_split(ctx));
     prof_begin(ctx, "k_pv_uplus_dt");
     ctx->pv_dirty = true;
     RUN(launched(ctx, launch_k_pv_uplus_dt(ctx->tune[TUNE_k_pv_uplus_dt], ctx->pool32 != nullptr, ctx->hot, s, ctx->c,
                                            ctx->dt_key)));
-    RUN(run_sync(ctx, "J_cell"));
-    RUN(run_sync(ctx, "Uplus"));
-    return MHD_OK;
+    return run_syncs(ctx, {"J_cell", "Uplus"});
 }
 
 // UpdateDerivedFields_ with Poles, in the reference's order: calc_Bcell and
@@ -700,57 +779,68 @@ int launch_update_derived(mhd_ctx *ctx)
 // (which the J edges then read), Calc_J_Edge and Sync("Jedge"), then J_cell
 // (with PV / U_plus / the CFL bound), its pole-shell repair, and the syncs.
 // B_cell and the J edges run as one pass before the rewrite; the few J edges
-// that read a rewritten face are formed again after it (k_pole_jedge).
+// that read a rewritten face are formed again after it (POLE_JEDGE), with the
+// ring of Sync("Jedge") in the same launch.
 int launch_update_derived_pole(mhd_ctx *ctx)
 {
     cudaStream_t s = ctx->stream;
     prof_begin(ctx, "k_bcell_jedge");
     RUN(launched(ctx, launch_k_bcell_jedge(ctx->tune[TUNE_k_bcell_jedge], ctx->pool32 != nullptr, ctx->hot, s)));
-    RUN(run_sync(ctx, "B_cell"));
+    RUN(run_syncs(ctx, {"B_cell"}));
     RUN(launch_pole(ctx, POLE_BZETA));
-    {
-        const int np = int(ctx->poles.size() / 2);
-        int64_t w = 0;
-        for (int q = 0; q < np; ++q)
-        {
-            const BlockView &v = ctx->hbv[size_t(ctx->poles[size_t(2 * q)])];
-            w = std::max<int64_t>(w, int64_t(v.ni + 1) * 2 * (v.nk + 1));
-        }
-        prof_begin(ctx, "k_jedge");
-        k_pole_jedge<<<dim3(grid_for(w), unsigned(np)), kThreads, 0, s>>>(ctx->dbv, ctx->dpoles);
-        RUN(launched(ctx));
-    }
-    RUN(run_sync(ctx, "Jedge"));
-    prof_begin(ctx, "k_arm_dt");
-    k_arm_dt<<<1, 128, 0, s>>>(ctx->dt_key, ctx->nruns);
-    RUN(launched(ctx));
+    if (ctx->syncs.count("Jedge"))
+        RUN(launch_pole(ctx, {POLE_JEDGE, POLE_JETA}, 0));
+    else
+        RUN(launch_pole(ctx, POLE_JEDGE));
+    RUN(run_syncs(ctx, {"Jedge"}, false));
     RUN(launch_jcell_split(ctx));
     prof_begin(ctx, "k_pv_uplus_dt");
     ctx->pv_dirty = true;
     RUN(launched(ctx, launch_k_pv_uplus_dt(ctx->tune[TUNE_k_pv_uplus_dt], ctx->pool32 != nullptr, ctx->hot, s, ctx->c,
                                            ctx->dt_key)));
     RUN(launch_pole(ctx, POLE_JCELL));
-    RUN(run_sync(ctx, "J_cell"));
-    RUN(run_sync(ctx, "Uplus"));
-    return MHD_OK;
+    return run_syncs(ctx, {"J_cell", "Uplus"});
+}
+
+// the runs' clocks, for the kernel that starts or ends a step
+RunClock run_clock(const mhd_ctx *ctx)
+{
+    return RunClock{ctx->dt_key, ctx->dt, ctx->time, ctx->step, ctx->err, ctx->prm.dt_abort, ctx->nruns};
+}
+
+// Sync("Ucell") and Sync("Bface") in one
+int sync_state(mhd_ctx *ctx)
+{
+    if (!ctx->poles.empty() && ctx->syncs.count("Ucell") && ctx->syncs.count("Bface"))
+    {
+        // both groups' rings in one launch
+        StepSync *s = nullptr;
+        RUN(step_sync(ctx, {"Ucell", "Bface"}, 0, &s));
+        if (s->usable)
+        {
+            RUN(launch_pole(ctx, {POLE_RING_U, POLE_RING_BXI}));
+            return run_syncs(ctx, {"Ucell", "Bface"}, false);
+        }
+    }
+    return run_syncs(ctx, {"Ucell", "Bface"});
 }
 
 // fluid RHS together with the contravariant velocities of the EMF stencils
-int launch_fluid_ucontra(mhd_ctx *ctx)
+int launch_fluid_ucontra(mhd_ctx *ctx, const RunClock &rc = RunClock{})
 {
     if (ctx->pool32)
     {
         prof_begin(ctx, "k_fluid_mixed");
         const int var = ctx->tune[TUNE_k_fluid_mixed];
         return launched(ctx, launch_k_fluid_mixed(var, ctx->hot, grid_tiles(ctx), ctx->stream, ctx->dbv,
-                                                  ctx->c));
+                                                  ctx->c, rc));
     }
     prof_begin(ctx, "k_fluid_ucontra");
-    return launched(ctx, launch_k_fluid_ucontra(ctx->tune[TUNE_k_fluid_ucontra], ctx->hot, ctx->stream, ctx->c));
+    return launched(ctx, launch_k_fluid_ucontra(ctx->tune[TUNE_k_fluid_ucontra], ctx->hot, ctx->stream, ctx->c, rc));
 }
 
-// AssembleRHS_Induction_CT_; with_ucontra unless the fluid pass computed them
-int launch_induction(mhd_ctx *ctx, bool update_b, bool with_ucontra = true)
+// AssembleRHS_Induction_CT_ up to the edge EMF; with_ucontra unless the fluid pass computed them
+int launch_edge_emf(mhd_ctx *ctx, bool with_ucontra)
 {
     const int nb = ctx->nblocks;
     cudaStream_t s = ctx->stream;
@@ -762,21 +852,29 @@ int launch_induction(mhd_ctx *ctx, bool update_b, bool with_ucontra = true)
     }
     prof_begin(ctx, "k_eface");
     RUN(launched(ctx, launch_k_eface(ctx->tune[TUNE_k_eface], ctx->hot, s)));
-    RUN(run_sync(ctx, "Eface"));
+    RUN(run_syncs(ctx, {"Eface"}));
     // inner edges; ghost edges keep their zero of AssembleRHS_Induction_CT_
     // except where the Eedge sync writes them
     prof_begin(ctx, "k_eedge");
     RUN(launched(ctx, launch_k_eedge(ctx->tune[TUNE_k_eedge], ctx->hot, s)));
-    RUN(run_sync(ctx, "Eedge"));
-    prof_begin(ctx, "k_curl_e2f");
-    return launched(ctx, launch_k_curl_e2f(ctx->tune[TUNE_k_curl_e2f], ctx->hot, s, F_Exi, F_RBxi,
-                                           update_b ? F_Bxi : -1, -1.0, ctx->dt, 1.0, 0, nullptr, 0));
+    return run_syncs(ctx, {"Eedge"});
 }
 
-int launch_update_u(mhd_ctx *ctx)
+// AssembleRHS_Induction_CT_ without the update (a stage)
+int launch_induction(mhd_ctx *ctx)
+{
+    RUN(launch_edge_emf(ctx, true));
+    prof_begin(ctx, "k_curl_e2f");
+    return launched(ctx, launch_k_curl_e2f(ctx->tune[TUNE_k_curl_e2f], ctx->hot, ctx->stream, F_Exi, F_RBxi, -1, -1.0,
+                                           ctx->dt, 1.0, 0, nullptr, 0));
+}
+
+// ApplyUpdate_Euler_ of cells and faces (rhs_b: RHS_B is stored)
+int launch_update(mhd_ctx *ctx, bool rhs_b, const RunClock &rc)
 {
     prof_begin(ctx, "k_update_u");
-    return launched(ctx, launch_k_update_u(ctx->hot, ctx->stream, ctx->dt));
+    return launched(ctx, launch_k_update(ctx->tune[TUNE_k_curl_e2f], ctx->hot, ctx->stream, rhs_b ? F_RBxi : -1,
+                                         ctx->dt, rc));
 }
 
 
@@ -1130,34 +1228,25 @@ int launch_resistive(mhd_ctx *ctx)
     return launch_curl_rng(ctx, F_Eresxi, F_RBresxi, F_Bxi, -1.0, 0);
 }
 
-// the Euler stage at the current dt: fluid RHS, CT induction with the
-// face-B update, cell update.  (The cell update stays a pass of its own: in
-// the latency-bound mixed flux pass it ran slower than alone.)
-int launch_euler_core(mhd_ctx *ctx)
+// The Euler stage: fluid RHS, CT induction, cell and face update.  first: the
+// step's start (dt from the CFL minima), in the flux pass; last: its end (run
+// data, dt reductions armed), in the update.  (The cell update stays out of
+// the flux pass: in that latency-bound pass it ran slower than alone.)
+int launch_euler_core(mhd_ctx *ctx, bool first, bool last)
 {
-    RUN(launch_fluid_ucontra(ctx));
-    RUN(launch_induction(ctx, /*update_b=*/true, /*with_ucontra=*/false));
-    return launch_update_u(ctx);
+    RUN(launch_fluid_ucontra(ctx, first ? run_clock(ctx) : RunClock{}));
+    RUN(launch_edge_emf(ctx, /*with_ucontra=*/false));
+    return launch_update(ctx, true, last ? run_clock(ctx) : RunClock{});
 }
 
 // one LunarSolver::StepOnce, explicit part: dt, fluid RHS, CT induction, update
-int launch_step_a(mhd_ctx *ctx)
-{
-    prof_begin(ctx, "k_begin_step");
-    k_begin_step<<<1, 128, 0, ctx->stream>>>(ctx->dt_key, ctx->dt, ctx->err, ctx->prm.dt_abort, ctx->nruns);
-    RUN(launched(ctx));
-    return launch_euler_core(ctx);
-}
+int launch_step_a(mhd_ctx *ctx) { return launch_euler_core(ctx, true, true); }
 
-// ... and its closing part: run data, Sync("Ucell"), Sync("Bface"), derived fields
+// ... and its closing part: Sync("Ucell"), Sync("Bface"), derived fields
 int launch_step_c(mhd_ctx *ctx)
 {
-    prof_begin(ctx, "k_end_step");
-    k_end_step<<<1, 128, 0, ctx->stream>>>(ctx->dt, ctx->time, ctx->step, ctx->nruns);
-    RUN(launched(ctx));
-    RUN(run_sync(ctx, "Ucell"));
-    RUN(run_sync(ctx, "Bface"));
-    return launch_update_derived(ctx);
+    RUN(sync_state(ctx));
+    return launch_update_derived(ctx, true);
 }
 
 // ResistiveDiffusionSubcycles_ (Z4_Lunar/src/physics/LunarSolver_MagneticRHS.cpp:53-115):
@@ -1172,25 +1261,25 @@ int launch_resistive_explicit(mhd_ctx *ctx)
     cudaStream_t s = ctx->stream;
     for (int q = 0; q < ctx->res_nsub; ++q)
     {
-        RUN(run_sync(ctx, "Bface"));
+        RUN(run_syncs(ctx, {"Bface"}));
         prof_begin(ctx, "k_bcell");
         RUN(launched(ctx, launch_k_bcell(ctx->hot, s)));
-        RUN(run_sync(ctx, "B_cell"));
+        RUN(run_syncs(ctx, {"B_cell"}));
         RUN(launch_pole(ctx, POLE_BZETA));
         prof_begin(ctx, "k_jedge");
         RUN(launched(ctx, launch_k_jedge(ctx->hot, s, F_Bxi, F_Jxi, nullptr, 0)));
-        RUN(run_sync(ctx, "Jedge"));
+        RUN(run_syncs(ctx, {"Jedge"}));
         prof_begin(ctx, "k_jcell");
         RUN(launched(ctx, launch_k_jcell(false, ctx->hot, s)));
         RUN(launch_pole(ctx, POLE_JCELL));
-        RUN(run_sync(ctx, "J_cell"));
+        RUN(run_syncs(ctx, {"J_cell"}));
         prof_begin(ctx, "k_eres_explicit");
         RUN(launched(ctx, launch_k_eres_explicit(ctx->hot, s, ctx->res_inver_Rem)));
-        RUN(run_sync(ctx, "Eres"));
+        RUN(run_syncs(ctx, {"Eres"}));
         prof_begin(ctx, "k_curl_e2f");
         RUN(launched(ctx, launch_k_curl_e2f(ctx->tune[TUNE_k_curl_e2f], ctx->hot, s, F_Eresxi, F_RBresxi, F_Bxi, -1.0,
                                             ctx->dt, double(ctx->res_nsub), 0, nullptr, 0)));
-        RUN(run_sync(ctx, "Bface"));
+        RUN(run_syncs(ctx, {"Bface"}));
     }
     return MHD_OK;
 }
@@ -1474,12 +1563,13 @@ int launch_rk2(mhd_ctx *ctx, int save)
 int launch_step_rk2(mhd_ctx *ctx)
 {
     RUN(launch_rk2(ctx, 1));
-    RUN(launch_step_a(ctx));
+    RUN(launch_euler_core(ctx, true, false));
     RUN(launch_resistive_part(ctx));
-    RUN(run_sync(ctx, "Ucell"));
-    RUN(run_sync(ctx, "Bface"));
-    RUN(launch_update_derived(ctx));
-    RUN(launch_euler_core(ctx));
+    RUN(sync_state(ctx));
+    // (this stage's CFL bounds are not used: the reductions are armed again by
+    // the second stage's update, for the ones of the step's end)
+    RUN(launch_update_derived(ctx, true));
+    RUN(launch_euler_core(ctx, false, true));
     RUN(launch_resistive_part(ctx));
     RUN(launch_rk2(ctx, 0));
     return launch_step_c(ctx);
@@ -1885,6 +1975,7 @@ int mhd_ctx_destroy(mhd_ctx *ctx)
         free_list(kv.second.cold);
         cudaFree(kv.second.dwalls);
     }
+    free_step_syncs(ctx);
     cudaFree(ctx->dpoles);
     cudaFree(ctx->pole_cache);
     cudaFree(ctx->diag_keys);
@@ -2098,8 +2189,6 @@ static void free_list(CopyList &m)
 {
     cudaFree(m.dst);
     cudaFree(m.src);
-    cudaFree(m.dst32);
-    cudaFree(m.src32);
     cudaFree(m.tmp);
     cudaFree(m.cdst);
     cudaFree(m.cval);
@@ -2124,17 +2213,21 @@ static void free_resistive(mhd_ctx *ctx)
     R.graph_loops = loops;
 }
 
-// pool offset -> (block, i, j, k) of the point (component dropped)
+// pool offset -> (field, block, i, j, k) of the point (component dropped); the
+// pool holds the blocks one after another, each kPoolPlanes planes
 struct PoolDecoder
 {
-    std::vector<std::pair<uint64_t, int>> starts; // (base offset, field * nblocks + block), sorted
     const mhd_ctx *ctx;
+    int field_of[kPoolPlanes];
+    std::vector<uint64_t> start; // first offset of each block, then the pool's end
     explicit PoolDecoder(const mhd_ctx *c) : ctx(c)
     {
         for (int f = 0; f < NFIELD; ++f)
-            for (int b = 0; b < c->nblocks; ++b)
-                starts.push_back({uint64_t(c->base[size_t(f)][size_t(b)]), f * c->nblocks + b});
-        std::sort(starts.begin(), starts.end());
+            for (int m = 0; m < kFields[f].ncomp; ++m)
+                field_of[plane_of(f) + m] = f;
+        for (int b = 0; b < c->nblocks; ++b)
+            start.push_back(uint64_t(c->base[0][size_t(b)]));
+        start.push_back(uint64_t(c->pool_n));
     }
     bool operator()(uint64_t off, int &b, int &i, int &j, int &k) const
     {
@@ -2143,22 +2236,38 @@ struct PoolDecoder
     }
     bool decode(uint64_t off, int &f, int &b, int &i, int &j, int &k) const
     {
-        auto it = std::upper_bound(starts.begin(), starts.end(), std::make_pair(off, INT32_MAX));
-        if (it == starts.begin())
+        if (off >= start.back())
             return false;
-        --it;
-        f = it->second / ctx->nblocks;
-        b = it->second % ctx->nblocks;
+        b = int(std::upper_bound(start.begin(), start.end() - 1, off) - start.begin()) - 1;
         const BlockView &v = ctx->hbv[size_t(b)];
-        const uint64_t rel = off - it->first;
-        if (rel >= uint64_t(v.vol) * uint64_t(kFields[f].ncomp))
-            return false;
-        const int64_t p = int64_t(rel % uint64_t(v.vol));
-        k = int(p % v.NK) - v.G;
-        j = int((p / v.NK) % v.NJ) - v.G;
-        i = int(p / (int64_t(v.NK) * v.NJ)) - v.G;
+        const uint64_t rel = off - start[size_t(b)];
+        const uint32_t q = uint32_t(rel / uint64_t(v.vol)), p = uint32_t(rel - q * uint64_t(v.vol));
+        f = field_of[q];
+        const uint32_t ij = p / uint32_t(v.NK);
+        k = int(p - ij * uint32_t(v.NK)) - v.G;
+        const uint32_t ii = ij / uint32_t(v.NJ);
+        j = int(ij - ii * uint32_t(v.NJ)) - v.G;
+        i = int(ii) - v.G;
         return true;
     }
+};
+
+// a set of offsets as a sorted list, with a mark per entry
+struct OffsetSet
+{
+    std::vector<uint64_t> v;
+    std::vector<char> mark;
+    explicit OffsetSet(std::vector<uint64_t> x) : v(std::move(x))
+    {
+        std::sort(v.begin(), v.end());
+        mark.assign(v.size(), 0);
+    }
+    int64_t find(uint64_t o) const
+    {
+        const auto it = std::lower_bound(v.begin(), v.end(), o);
+        return it != v.end() && *it == o ? it - v.begin() : -1;
+    }
+    bool has(uint64_t o) const { return find(o) >= 0; }
 };
 
 struct IBox
@@ -2210,13 +2319,33 @@ static int upload_list(mhd_ctx *ctx, CopyList &l, const std::vector<uint64_t> &c
     l.n = int64_t(d.size());
     if (staged && l.n > 0)
         CK(ctx, cudaMalloc(&l.tmp, size_t(l.n) * 8));
-    if (!staged && l.n > 0 && ctx->pool_n < (size_t(1) << 32))
-    {
-        const std::vector<uint32_t> d32(d.begin(), d.end()), s32(s2.begin(), s2.end());
-        RUN(upload_vec(ctx, d32, &l.dst32));
-        RUN(upload_vec(ctx, s32, &l.src32));
-    }
     return MHD_OK;
+}
+
+static void free_step_syncs(mhd_ctx *ctx)
+{
+    for (auto &kv : ctx->step_syncs)
+        for (SyncPass *p : {&kv.second.a, &kv.second.b})
+            for (void *q : {(void *)p->dst, (void *)p->src, (void *)p->cdst, (void *)p->dst32, (void *)p->src32,
+                            (void *)p->cdst32, (void *)p->cval})
+                cudaFree(q);
+    ctx->step_syncs.clear();
+}
+
+static int upload_pass(mhd_ctx *ctx, const Resolved::Part &r, SyncPass &p)
+{
+    p.n = int64_t(r.d.size());
+    p.nconst = int64_t(r.cd.size());
+    RUN(upload_vec(ctx, r.cv, &p.cval));
+    if (ctx->pool_n < (size_t(1) << 32))
+    {
+        RUN(upload_vec(ctx, std::vector<uint32_t>(r.d.begin(), r.d.end()), &p.dst32));
+        RUN(upload_vec(ctx, std::vector<uint32_t>(r.s.begin(), r.s.end()), &p.src32));
+        return upload_vec(ctx, std::vector<uint32_t>(r.cd.begin(), r.cd.end()), &p.cdst32);
+    }
+    RUN(upload_vec(ctx, r.d, &p.dst));
+    RUN(upload_vec(ctx, r.s, &p.src));
+    return upload_vec(ctx, r.cd, &p.cdst);
 }
 
 // Ghost depth of each field that a kernel of the step reads: the face,
@@ -2262,16 +2391,134 @@ static int hot_depth(const mhd_ctx *ctx, int f)
     }
 }
 
-static bool hot_point(const mhd_ctx *ctx, const PoolDecoder &dec, uint64_t off)
+// hot points, with the depth of every field looked up once
+struct HotPoints
+{
+    const PoolDecoder &dec;
+    int depth[NFIELD];
+    HotPoints(const mhd_ctx *ctx, const PoolDecoder &d) : dec(d)
+    {
+        for (int f = 0; f < NFIELD; ++f)
+            depth[f] = hot_depth(ctx, f);
+    }
+    // f: the point's field (-1: not a field point, hot)
+    bool operator()(uint64_t off, int &f) const
+    {
+        int b, i, j, k;
+        if (!dec.decode(off, f, b, i, j, k))
+        {
+            f = -1;
+            return true;
+        }
+        const int d = depth[f];
+        const BlockView &v = dec.ctx->hbv[size_t(b)];
+        int pl[3];
+        loc_plus(kFields[f].loc, pl[0], pl[1], pl[2]);
+        return i >= -d && j >= -d && k >= -d && i < v.ni + pl[0] + d && j < v.nj + pl[1] + d && k < v.nk + pl[2] + d;
+    }
+};
+
+// Is the point one the wall handlers of the group write (the boundary cell
+// layer and the ghost layers beyond it on the wall's face) or, with reach = 1,
+// read (one layer further inside)?
+static bool wall_point(const mhd_ctx *ctx, const SyncMap &m, const PoolDecoder &dec, uint64_t off, int reach)
 {
     int f, b, i, j, k;
-    if (!dec.decode(off, f, b, i, j, k))
+    if (m.walls.empty() || !dec.decode(off, f, b, i, j, k))
+        return false;
+    for (const auto &w : m.walls)
+    {
+        if (w.first != b)
+            continue;
+        const BlockView &v = ctx->hbv[size_t(b)];
+        const int ax = std::abs(w.second) - 1;
+        const int p[3] = {i, j, k}, n[3] = {v.ni, v.nj, v.nk};
+        if ((w.second < 0 && p[ax] <= reach) || (w.second > 0 && p[ax] >= n[ax] - 1 - reach))
+            return true;
+    }
+    return false;
+}
+
+// A group's lists as independent copies and fixed values (Resolved), by the
+// order its Sync runs them in:
+// * without Poles: fixed values, wall handlers, copies.  A copy from a fixed
+//   value is that value; a fixed value a copy overwrites is left out; the
+//   wall handlers run first, so they may touch no fixed value.
+// * with Poles: copies, wall handlers, post-wall copies, fixed values.  A copy
+//   a fixed value overwrites in the same pass is left out; a post-wall copy
+//   may read no fixed value's point.
+// In either case no source is a destination (a staged list is not resolved).
+static void resolve_lists(const mhd_ctx *ctx, const SyncMap &m, const PoolDecoder &dec, const std::vector<uint64_t> &d,
+                          const std::vector<uint64_t> &s, const std::vector<uint64_t> &cd,
+                          const std::vector<double> &cv, Resolved &r)
+{
+    r = Resolved();
+    if (m.staged)
+        return;
+    std::vector<std::pair<uint64_t, double>> cs(cd.size());
+    for (size_t t = 0; t < cd.size(); ++t)
+        cs[t] = {cd[t], cv[t]};
+    std::stable_sort(cs.begin(), cs.end(), [](const auto &x, const auto &y) { return x.first < y.first; });
+    std::vector<uint64_t> co(cs.size());
+    for (size_t t = 0; t < cs.size(); ++t)
+    {
+        co[t] = cs[t].first;
+        if (t > 0 && co[t] == co[t - 1])
+            return; // two values for one point
+    }
+    OffsetSet consts(std::move(co));
+    const bool poles = !ctx->poles.empty();
+    // a second pass after the wall handlers, or for the fixed values where a
+    // copy reads one's point (it reads what the point held before)
+    bool two = poles && (!m.walls.empty() || !m.hd2.empty());
+    for (size_t t = 0; poles && !two && t < s.size(); ++t)
+        two = consts.has(s[t]);
+    if (!poles)
+        for (uint64_t o : cd)
+            if (wall_point(ctx, m, dec, o, 1))
+                return;
+    auto part = [&](const std::vector<uint64_t> &pd, const std::vector<uint64_t> &ps, bool with_consts,
+                    Resolved::Part &out) {
+        for (size_t t = 0; t < pd.size(); ++t)
+        {
+            const int64_t at = with_consts ? consts.find(pd[t]) : -1, from = with_consts ? consts.find(ps[t]) : -1;
+            if (poles && at >= 0)
+                continue; // overwritten by the fixed value
+            if (poles && from >= 0)
+                return false;
+            if (at >= 0)
+                consts.mark[size_t(at)] = 1;
+            if (from >= 0)
+            {
+                out.cd.push_back(pd[t]);
+                out.cv.push_back(cs[size_t(from)].second);
+                continue;
+            }
+            out.d.push_back(pd[t]);
+            out.s.push_back(ps[t]);
+        }
+        if (with_consts)
+            for (size_t t = 0; t < cs.size(); ++t)
+                if (!consts.mark[t])
+                {
+                    out.cd.push_back(cs[t].first);
+                    out.cv.push_back(cs[t].second);
+                }
         return true;
-    const int d = hot_depth(ctx, f);
-    const BlockView &v = ctx->hbv[size_t(b)];
-    int pl[3];
-    loc_plus(kFields[f].loc, pl[0], pl[1], pl[2]);
-    return i >= -d && j >= -d && k >= -d && i < v.ni + pl[0] + d && j < v.nj + pl[1] + d && k < v.nk + pl[2] + d;
+    };
+    if (!part(d, s, !two, r.a) || (two && !part(m.hd2, m.hs2, true, r.b)))
+    {
+        r = Resolved();
+        return;
+    }
+    for (const auto *tab : {&r.a.d, &r.a.s, &r.a.cd, &r.b.d, &r.b.s, &r.b.cd})
+        for (uint64_t off : *tab)
+        {
+            int f, b, i, j, k;
+            if (dec.decode(off, f, b, i, j, k))
+                r.fields.set(size_t(f));
+        }
+    r.usable = true;
 }
 
 // Hot and cold lists of a Pole context's group.  Its Sync runs the rings,
@@ -2290,51 +2537,39 @@ static int build_sync_pole(mhd_ctx *ctx, const std::string &group, SyncMap &m, c
     std::vector<uint64_t> d, s2, cd, dc, sc, cdc;
     std::vector<double> cv, cvc;
     const bool all_hot = (group == "Bface");
-    std::unordered_set<uint64_t> later(m.hcd.begin(), m.hcd.end());
-    later.insert(m.hd2.begin(), m.hd2.end());
-    // points the wall handlers write: the boundary cell layer and the ghost
-    // layers beyond it on the wall's face
-    auto wall_point = [&](uint64_t off) {
-        int f, b, i, j, k;
-        if (m.walls.empty() || !dec.decode(off, f, b, i, j, k))
-            return false;
-        for (const auto &w : m.walls)
-        {
-            if (w.first != b)
-                continue;
-            const BlockView &v = ctx->hbv[size_t(b)];
-            const int ax = std::abs(w.second) - 1;
-            const int p[3] = {i, j, k}, n[3] = {v.ni, v.nj, v.nk};
-            if ((w.second < 0 && p[ax] <= 0) || (w.second > 0 && p[ax] >= n[ax] - 1))
-                return true;
-        }
-        return false;
-    };
-    std::unordered_set<uint64_t> hot_dst, post_dst(m.hd2.begin(), m.hd2.end());
+    const HotPoints hot_at_point(ctx, dec);
+    OffsetSet consts(m.hcd); // marked: at the destination of a hot copy
+    const OffsetSet post(m.hd2);
+    int f;
     for (size_t t = 0; t < m.hd.size(); ++t)
     {
         // a copy the wall handlers or the post-wall copies overwrite in the
         // same Sync must run before them, in the step
-        const bool hot = all_hot || hot_point(ctx, dec, m.hd[t]) || later.count(m.hs[t]) || wall_point(m.hs[t]) ||
-                         wall_point(m.hd[t]) || post_dst.count(m.hd[t]);
+        const bool at = hot_at_point(m.hd[t], f);
+        if (f >= 0 && ctx->field_group[size_t(f)] != group)
+            ctx->field_group[size_t(f)] = group;
+        const bool hot = all_hot || at || consts.has(m.hs[t]) || post.has(m.hs[t]) ||
+                         wall_point(ctx, m, dec, m.hs[t], 0) || wall_point(ctx, m, dec, m.hd[t], 0) ||
+                         post.has(m.hd[t]);
         (hot ? d : dc).push_back(m.hd[t]);
         (hot ? s2 : sc).push_back(m.hs[t]);
-        if (hot)
-            hot_dst.insert(m.hd[t]);
+        const int64_t c = hot ? consts.find(m.hd[t]) : -1;
+        if (c >= 0)
+            consts.mark[size_t(c)] = 1;
     }
     for (size_t t = 0; t < m.hcd.size(); ++t)
     {
-        const bool hot = all_hot || hot_point(ctx, dec, m.hcd[t]) || hot_dst.count(m.hcd[t]);
+        const bool at = hot_at_point(m.hcd[t], f);
+        if (f >= 0 && ctx->field_group[size_t(f)] != group)
+            ctx->field_group[size_t(f)] = group;
+        const int64_t c = consts.find(m.hcd[t]);
+        const bool hot = all_hot || at || consts.mark[size_t(c)];
         (hot ? cd : cdc).push_back(m.hcd[t]);
         (hot ? cv : cvc).push_back(m.hcv[t]);
     }
     RUN(upload_list(ctx, m.hot, cd, cv, d, s2, m.staged));
     RUN(upload_list(ctx, m.cold, cdc, cvc, dc, sc, m.staged));
-    int f, b, i, j, k;
-    for (const auto *tab : {&m.hd, &m.hcd})
-        for (uint64_t off : *tab)
-            if (dec.decode(off, f, b, i, j, k))
-                ctx->field_group[size_t(f)] = group;
+    resolve_lists(ctx, m, dec, d, s2, cd, cv, m.res);
     m.built = true;
     return MHD_OK;
 }
@@ -2363,36 +2598,126 @@ int build_sync(mhd_ctx *ctx, const std::string &group, SyncMap &m)
     const PoolDecoder dec(ctx);
     std::vector<uint64_t> d, s2, cd;
     std::vector<double> cv;
+    free_step_syncs(ctx);
+    m.res_full = Resolved();
     if (!ctx->poles.empty())
         return build_sync_pole(ctx, group, m, dec);
+    const HotPoints hot_at_point(ctx, dec);
+    OffsetSet consts(m.hcd); // marked: the source of a hot copy
+    int f;
     for (size_t t = 0; t < m.hd.size(); ++t)
-        if (hot_point(ctx, dec, m.hd[t]))
-        {
-            d.push_back(m.hd[t]);
-            s2.push_back(m.hs[t]);
-        }
-    std::unordered_set<uint64_t> srcs(s2.begin(), s2.end());
+    {
+        const bool at = hot_at_point(m.hd[t], f);
+        if (f >= 0 && ctx->field_group[size_t(f)] != group)
+            ctx->field_group[size_t(f)] = group;
+        if (!at)
+            continue;
+        d.push_back(m.hd[t]);
+        s2.push_back(m.hs[t]);
+        const int64_t c = consts.find(m.hs[t]);
+        if (c >= 0)
+            consts.mark[size_t(c)] = 1;
+    }
     for (size_t t = 0; t < m.hcd.size(); ++t)
-        if (hot_point(ctx, dec, m.hcd[t]) || srcs.count(m.hcd[t]))
+    {
+        const bool at = hot_at_point(m.hcd[t], f);
+        if (f >= 0 && ctx->field_group[size_t(f)] != group)
+            ctx->field_group[size_t(f)] = group;
+        if (at || consts.mark[size_t(consts.find(m.hcd[t]))])
         {
             cd.push_back(m.hcd[t]);
             cv.push_back(m.hcv[t]);
         }
+    }
     RUN(upload_list(ctx, m.hot, cd, cv, d, s2, m.staged));
-    int f, b, i, j, k;
-    for (const auto *tab : {&m.hd, &m.hcd})
-        for (uint64_t off : *tab)
-            if (dec.decode(off, f, b, i, j, k))
-                ctx->field_group[size_t(f)] = group;
+    resolve_lists(ctx, m, dec, d, s2, cd, cv, m.res);
     m.built = true;
     return MHD_OK;
 }
 
+// The passes of consecutive groups' Syncs (built on first use; full: bit q for
+// the full list of group q).  Groups go together when they touch different
+// fields; a group that cannot be resolved makes the whole entry unusable.
+static int step_sync(mhd_ctx *ctx, std::initializer_list<const char *> groups, unsigned full, StepSync **out)
+{
+    std::string key = std::to_string(full);
+    for (const char *g : groups)
+        key += std::string("+") + g;
+    for (const char *g : groups)
+    {
+        const auto it = ctx->syncs.find(g);
+        if (it == ctx->syncs.end() || it->second.built)
+            continue;
+        if (ctx->capturing)
+            return fail(ctx, MHD_ESTATE, "sync group %s changed during capture", g);
+        RUN(build_sync(ctx, it->first, it->second));
+    }
+    auto found = ctx->step_syncs.find(key);
+    if (found == ctx->step_syncs.end())
+    {
+        if (ctx->capturing)
+            return fail(ctx, MHD_ESTATE, "sync groups %s not prepared before capture", key.c_str());
+        StepSync s;
+        Resolved all;
+        std::bitset<NFIELD> seen;
+        s.usable = true;
+        unsigned q = 0;
+        for (const char *g : groups)
+        {
+            const bool f = ((full >> q++) & 1) != 0;
+            const auto it = ctx->syncs.find(g);
+            if (it == ctx->syncs.end())
+                continue;
+            SyncMap &m = it->second;
+            if (f && !m.res_full.usable)
+                resolve_lists(ctx, m, PoolDecoder(ctx), m.hd, m.hs, m.hcd, m.hcv, m.res_full);
+            const Resolved &r = f ? m.res_full : m.res;
+            s.usable = s.usable && r.usable && (seen & r.fields).none();
+            if (!s.usable)
+                break;
+            seen |= r.fields;
+            for (auto part : {&Resolved::a, &Resolved::b})
+            {
+                Resolved::Part &t = all.*part;
+                const Resolved::Part &x = r.*part;
+                t.d.insert(t.d.end(), x.d.begin(), x.d.end());
+                t.s.insert(t.s.end(), x.s.begin(), x.s.end());
+                t.cd.insert(t.cd.end(), x.cd.begin(), x.cd.end());
+                t.cv.insert(t.cv.end(), x.cv.begin(), x.cv.end());
+            }
+        }
+        if (s.usable)
+        {
+            RUN(upload_pass(ctx, all.a, s.a));
+            RUN(upload_pass(ctx, all.b, s.b));
+        }
+        found = ctx->step_syncs.emplace(key, s).first;
+    }
+    *out = &found->second;
+    return MHD_OK;
+}
+
+// every group's lists and the passes of the step (before a capture)
 static int build_all_syncs(mhd_ctx *ctx)
 {
     for (auto &kv : ctx->syncs)
         if (!kv.second.built)
             RUN(build_sync(ctx, kv.first, kv.second));
+    StepSync *s = nullptr;
+    RUN(step_sync(ctx, {"Eface"}, 0, &s));
+    RUN(step_sync(ctx, {"Eedge"}, 0, &s));
+    RUN(step_sync(ctx, {"Ucell", "Bface"}, 0, &s));
+    RUN(step_sync(ctx, {"J_cell", "Uplus"}, 0, &s));
+    if (ctx->poles.empty())
+        RUN(step_sync(ctx, {"B_cell", "Jedge"}, 0, &s));
+    if (!ctx->poles.empty() || ctx->res_nsub > 0)
+    {
+        RUN(step_sync(ctx, {"B_cell"}, 0, &s));
+        RUN(step_sync(ctx, {"Jedge"}, 0, &s));
+    }
+    if (ctx->res_nsub > 0)
+        for (const char *g : {"Bface", "J_cell", "Eres"})
+            RUN(step_sync(ctx, {g}, 0, &s));
     return MHD_OK;
 }
 
@@ -2931,6 +3256,7 @@ int mhd_set_sync_wall(mhd_ctx *ctx, const char *group, int32_t block, int32_t di
     if (!ctx || !group || block < 0 || block >= ctx->nblocks || direction == 0 || direction < -3 || direction > 3)
         return fail(ctx, MHD_EINVAL, "bad wall handler arguments");
     ctx->syncs[group].walls.emplace_back(block, direction);
+    ctx->syncs[group].built = false;
     drop_graph(ctx);
     return MHD_OK;
 }
@@ -3340,7 +3666,7 @@ int mhd_autotune(mhd_ctx *ctx, int32_t reps, int32_t *min_ctas, int32_t n)
                                 save ? static_cast<const void *>(ctx->dt_key) : static_cast<const void *>(clk),
                                 clock_bytes, cudaMemcpyDeviceToDevice, s));
         if (!save)
-            RUN(launch_update_derived(ctx)); // derived fields of the restored state
+            RUN(launch_update_derived(ctx, false)); // derived fields of the restored state
         return MHD_OK;
     };
     cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -3542,7 +3868,7 @@ int mhd_update_derived(mhd_ctx *ctx)
     if (!ctx)
         return MHD_EINVAL;
     RUN(ensure_geom(ctx));
-    RUN(launch_update_derived(ctx));
+    RUN(launch_update_derived(ctx, false));
     CK(ctx, cudaStreamSynchronize(ctx->stream));
     return MHD_OK;
 }
@@ -3635,9 +3961,8 @@ int step_host(mhd_ctx *ctx, int32_t nsteps, const double *state_in, double *stat
             off += n;
         }
     RUN(ensure_geom(ctx));
-    RUN(run_sync(ctx, "Ucell"));
-    RUN(run_sync(ctx, "Bface"));
-    RUN(launch_update_derived(ctx));
+    RUN(sync_state(ctx));
+    RUN(launch_update_derived(ctx, false));
     RUN(run_steps(ctx, nsteps));
     for (int f : {int(F_U), int(F_Bxi)})
         RUN(materialise_field(ctx, f));
@@ -3713,22 +4038,17 @@ int mhd_stage(mhd_ctx *ctx, int32_t stage_id)
     {
     case MHD_STAGE_TIMESTEP:
         prof_begin(ctx, "k_begin_step");
-        k_begin_step<<<1, 128, 0, ctx->stream>>>(ctx->dt_key, ctx->dt, ctx->err, ctx->prm.dt_abort, ctx->nruns);
+        k_begin_step<<<1, 128, 0, ctx->stream>>>(run_clock(ctx));
         RUN(launched(ctx));
         break;
     case MHD_STAGE_FLUID_RHS:
         RUN(launch_fluid_ucontra(ctx));
         break;
     case MHD_STAGE_INDUCTION:
-        RUN(launch_induction(ctx, false));
+        RUN(launch_induction(ctx));
         break;
     case MHD_STAGE_UPDATE:
-        RUN(launch_update_u(ctx));
-        {
-            prof_begin(ctx, "k_curl_e2f");
-            RUN(launched(ctx, launch_k_curl_e2f(ctx->tune[TUNE_k_curl_e2f], ctx->hot, ctx->stream, F_Exi, -1, F_Bxi,
-                                                -1.0, ctx->dt, 1.0, 0, nullptr, 0)));
-        }
+        RUN(launch_update(ctx, false, RunClock{}));
         break;
     case MHD_STAGE_HALL_EMF:
         // the edge stencils read B_cell / J_cell one ghost layer deep

@@ -35,6 +35,7 @@ __host__ __device__ constexpr int plane_of(int f)
 #undef MHD_PLANE
     return q;
 }
+constexpr int kPoolPlanes = plane_of(NFIELD);
 // planes of the mixed form's FP32 range: face geometry, face states, weights
 constexpr int kPlane32Q = G32_N, kPlane32W = G32_N + Q32_N;
 
@@ -100,6 +101,16 @@ struct HotGrid
 };
 
 #ifdef __CUDACC__
+
+// Programmatic dependent launch: a kernel launched with the attribute may start
+// while the kernel before it drains; what it does before pdl_wait() must read
+// nothing an earlier kernel writes.  Every kernel of the step waits, so a
+// kernel that has finished implies all before it have.
+__device__ __forceinline__ void pdl_wait()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 
 // block of the calling CTA and the thread's index among the block's threads
 template <int KIND, class A> __device__ __forceinline__ const HotBlock &hot_block(const A &a, uint32_t &t)

@@ -11,14 +11,30 @@ namespace mhd
 
 constexpr unsigned kHotCta = 256;
 
+// A launch that may start while the kernel before it on the stream drains
+// (the kernel waits before it reads what others write, pdl_wait): about 1 us
+// less from kernel to kernel inside the step's graph.
 template <class... P, class... Q>
-inline void hot_launch(void (*kernel)(P...), dim3 grid, cudaStream_t st, Q &&...args)
+inline void pdl_launch(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st,
+                       Q &&...args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
-    cfg.blockDim = dim3(kHotCta);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, kernel, std::forward<Q>(args)...);
+}
+
+template <class... P, class... Q>
+inline void hot_launch(void (*kernel)(P...), dim3 grid, cudaStream_t st, Q &&...args)
+{
+    pdl_launch(kernel, grid, kHotCta, 0, st, std::forward<Q>(args)...);
 }
 
 // f(arguments, grid) for every chunk of blocks over a kind's points, or, with

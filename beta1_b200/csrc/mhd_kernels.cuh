@@ -23,38 +23,74 @@ struct Consts
     double ne_floor;
 };
 
+// The runs' clocks (dt_key null: nothing to do)
+struct RunClock
+{
+    unsigned long long *dt_key; // CFL minima in their order-preserving form
+    double *dt, *time;
+    long long *step;
+    int *err;
+    double dt_abort;
+    int nruns;
+};
+#ifdef __CUDACC__
+__device__ __forceinline__ void begin_run(const RunClock &rc, int r)
+{
+    const double d = __longlong_as_double((long long)rc.dt_key[r]);
+    rc.dt[r] = d;
+    if (!isfinite(d) || d < rc.dt_abort)
+        rc.err[0] = MHD_EDT;
+}
+__device__ __forceinline__ void end_run(const RunClock &rc, int r)
+{
+    rc.time[r] += rc.dt[r];
+    rc.step[r] += 1;
+    rc.dt_key[r] = (unsigned long long)__double_as_longlong(1e100); // dt_local's initial bound
+}
+#endif
+
 __global__ void k_ucontra(const BlockView *bvs);
 __global__ void k_face_normals(const BlockView *bvs);
 __global__ void k_divb(const BlockView *bvs);
 // mixed precision (mhd_kernels_mixed.cu)
 __global__ void k_geom32(const BlockView *bvs);
-// Pole handlers and repairs on eta Poles (mhd_pole.cuh): per Pole a
-// (block, direction) pair in `poles`, one grid row per Pole
-__global__ void k_pole(const BlockView *bvs, const int *poles, int op);
-// Calc_J_Edge again on the J_xi / J_eta edges that read the B_zeta faces
-// POLE_BZETA rewrote (staggered layers jc, jc + 1 of each Pole; grid.y: Poles)
-__global__ void k_pole_jedge(const BlockView *bvs, const int *poles);
-// one Pole operation over every Pole (work items per Pole: pole_work); the
-// ring least squares run one warp per ring, with their geometry-only normal
-// matrices in `cache` (per Pole, per least-squares operation, `stride`
-// rings, 10 values each), which build = 1 fills (after every geometry change)
-void launch_pole_op(int op, int64_t work, int npoles, cudaStream_t st, const BlockView *bvs, const int *poles,
-                    double *cache, int stride, int build);
+// Pole operations (mhd_pole.cuh) over every Pole in one launch: up to four
+// that touch different points; POLE_JEDGE: Calc_J_Edge again on the J_xi /
+// J_eta edges that read the B_zeta faces POLE_BZETA rewrote (staggered layers
+// jc, jc + 1 of each Pole; jeta_ring = 0: the ring POLE_JETA writes left out).
+// The ring sums run one warp per ring; the least squares' geometry-only normal
+// matrices are in `cache` (per Pole, per least-squares operation, `stride`
+// rings, 10 values each), which launch_pole_build fills after every geometry
+// change.  ni, nk: the largest of the Poles' blocks.
+constexpr int POLE_JEDGE = NPOLE_OP;
+struct PoleOps
+{
+    int n;
+    int op[4];
+    int cta0[5]; // first CTA of each operation; the grid's size last
+    int jeta_ring;
+};
+void launch_pole_ops(PoleOps ops, int ni, int nk, int npoles, cudaStream_t st, const BlockView *bvs, const int *poles,
+                     double *cache, int stride);
+void launch_pole_build(int op, int ni, int nk, int npoles, cudaStream_t st, const BlockView *bvs, const int *poles,
+                       double *cache, int stride);
 __global__ void k_geometry(const BlockView *bvs, int blk, NodeMesh m, int G, int group0, double b0, double b1,
                            double b2);
 // output-step minima / maxima over the inner cells of a run's blocks (run < 0:
 // every block); keys[0..DIAG_NMIN) minima, keys[DIAG_NMIN..DIAG_NMIN + DIAG_NQ) maxima
 __global__ void k_diag_init(unsigned long long *keys);
 __global__ void k_diag(const BlockView *bvs, int run, unsigned long long *keys);
-__global__ void k_begin_step(const unsigned long long *dt_key, double *dt, int *err, double dt_abort, int nruns);
+__global__ void k_begin_step(RunClock rc);
 __global__ void k_arm_dt(unsigned long long *dt_key, int nruns);
-__global__ void k_end_step(const double *dt, double *time, long long *step, int nruns);
 __global__ void k_gather(double *pool, const uint64_t *dst, const uint64_t *src, int64_t n);
-// the same with 32-bit pool offsets (pools of fewer than 2^32 points)
-__global__ void k_gather32(double *pool, const uint32_t *dst, const uint32_t *src, int64_t n);
+// copies and fixed values of one or more Syncs, independent of one another,
+// with 64-bit or (pools of fewer than 2^32 points) 32-bit pool offsets
+void launch_k_sync(cudaStream_t st, double *pool, const uint64_t *dst, const uint64_t *src, int64_t n,
+                   const uint64_t *cdst, const double *cval, int64_t nconst);
+void launch_k_sync(cudaStream_t st, double *pool, const uint32_t *dst, const uint32_t *src, int64_t n,
+                   const uint32_t *cdst, const double *cval, int64_t nconst);
 __global__ void k_set_consts(double *pool, const uint64_t *dst, const double *val, int64_t n);
-__global__ void k_wall_u(const BlockView *bvs, int blk, int dir, double gamma);
-__global__ void k_wall_u_all(const BlockView *bvs, const int *walls, double gamma);
+void launch_k_wall_u(dim3 grid, cudaStream_t st, const BlockView *bvs, const int *walls, double gamma);
 __global__ void k_gather_stage(double *tmp, const double *pool, const uint64_t *src, int64_t n);
 __global__ void k_scatter_stage(double *pool, const double *tmp, const uint64_t *dst, int64_t n);
 __global__ void k_aos_to_soa(const BlockView *bvs, int blk, int fid, int ncomp, int lo0, int lo1, int lo2, int n0,
@@ -265,7 +301,8 @@ int launch_k_pv_uplus_dt(int variant, bool w32, const HotGrid &h, cudaStream_t s
 // PV_H, U_plus and the face states on the whole array
 int launch_k_pv_all(const HotGrid &h, cudaStream_t st, Consts c);
 // fluid RHS and contravariant velocities: minimum CTAs per SM 2, 3
-int launch_k_fluid_ucontra(int variant, const HotGrid &h, cudaStream_t st, Consts c);
+// (rc: the start of the step's run clocks, in the same launch)
+int launch_k_fluid_ucontra(int variant, const HotGrid &h, cudaStream_t st, Consts c, RunClock rc);
 // B_cell with the J edges: minimum CTAs per SM 2, 6; w32 as above
 int launch_k_bcell_jedge(int variant, bool w32, const HotGrid &h, cudaStream_t st);
 // B_cell alone, the J edges of (fB0, fJ0) alone (rng: per block a region box
@@ -277,13 +314,16 @@ int launch_k_jcell(bool w32, const HotGrid &h, cudaStream_t st);
 int launch_k_eface(int variant, const HotGrid &h, cudaStream_t st);
 int launch_k_eedge(int variant, const HotGrid &h, cudaStream_t st);
 // RHS = mult curl E and B += dt / dtdiv RHS on the inner faces (fR0, fB0 < 0:
-// not written; rng, nreg as above): minimum CTAs per SM 1, 6.  bs (may be
+// not written; rng, nreg as above): minimum CTAs per SM 4, 6.  bs (may be
 // null): B = B* + dt RHS with B* from a snapshot (bs[3 block + axis]: the
 // snapshot's B arrays of each block, pool layout)
 int launch_k_curl_e2f(int variant, const HotGrid &h, cudaStream_t st, int fE0, int fR0, int fB0, double mult,
                       const double *dtp, double dtdiv, int mult_is_neg_dt, const int *rng, int64_t nreg,
                       const double *const *bs = nullptr);
-int launch_k_update_u(const HotGrid &h, cudaStream_t st, const double *dtp);
+// the Euler update of the inner cells and faces in one pass, U += dt RHS_H and
+// RHS_B = -curl E (stored in fR0 when >= 0), B += dt RHS_B; rc: the end of the
+// step's run clocks.  Variants of k_curl_e2f.
+int launch_k_update(int variant, const HotGrid &h, cudaStream_t st, int fR0, const double *dtp, RunClock rc);
 int launch_k_rk2(const HotGrid &h, cudaStream_t st, int save);
 int launch_k_eres_explicit(const HotGrid &h, cudaStream_t st, double inver_Rem);
 int launch_k_hall_cell(const HotGrid &h, cudaStream_t st, Consts c, double hall_coef);
@@ -291,6 +331,7 @@ int launch_k_hall_cell(const HotGrid &h, cudaStream_t st, Consts c, double hall_
 int launch_k_hall_edge(int variant, const HotGrid &h, cudaStream_t st, const int *zb, int nzb);
 // k_fluid_mixed: minimum CTAs per SM 3, 1, 2; variants 3 and 4 are the
 // face-tiled kernels (on `tiles`, the KIND_TILE1 grid of bvs)
-int launch_k_fluid_mixed(int variant, const HotGrid &h, dim3 tiles, cudaStream_t st, const BlockView *bvs, Consts c);
+int launch_k_fluid_mixed(int variant, const HotGrid &h, dim3 tiles, cudaStream_t st, const BlockView *bvs, Consts c,
+                         RunClock rc);
 
 } // namespace mhd

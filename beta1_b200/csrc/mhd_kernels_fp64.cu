@@ -7,6 +7,7 @@
 // that no multiply-add is contracted, and the results agree with the
 // reference bit for bit.
 #include "mhd_kernels.cuh"
+#include "mhd_hot_launch.cuh"
 
 #include <cfloat>
 #include <cmath>
@@ -204,17 +205,12 @@ __device__ __forceinline__ void jedge_one(const BlockView &b, int ea, int i, int
     b.f[fJ0 + ea][c0] = J * b.f[F_alphaxi + ea][c0];
 }
 
-// Start of StepOnce: dt = global minimum of the CFL bounds, abort check
-// (dt < dt_abort or NaN sets the error word, LunarSolver_Timestep.cpp:128-139).
-__global__ void k_begin_step(const unsigned long long *dt_key, double *dt, int *err, double dt_abort, int nruns)
+// Start of StepOnce in a launch of its own (a stage; the step's flux kernel
+// does it in its first CTA)
+__global__ void k_begin_step(RunClock rc)
 {
-    for (int r = threadIdx.x; r < nruns; r += blockDim.x)
-    {
-        const double d = __longlong_as_double((long long)dt_key[r]);
-        dt[r] = d;
-        if (!isfinite(d) || d < dt_abort)
-            err[0] = MHD_EDT;
-    }
+    for (int r = threadIdx.x; r < rc.nruns; r += blockDim.x)
+        begin_run(rc, r);
 }
 
 __device__ __forceinline__ unsigned long long dbl_key(double x)
@@ -230,16 +226,6 @@ __global__ void k_arm_dt(unsigned long long *dt_key, int nruns)
         dt_key[r] = dbl_key(1e100);
 }
 
-// End of StepOnce: run-data counters (Z4_Lunar/src/LunarSolver_Driver.cpp:75-79)
-__global__ void k_end_step(const double *dt, double *time, long long *step, int nruns)
-{
-    for (int r = threadIdx.x; r < nruns; r += blockDim.x)
-    {
-        time[r] += dt[r];
-        step[r] += 1;
-    }
-}
-
 // ---------------------------------------------------------------------------
 // compiled Sync: dst <- src over the field pool
 // ---------------------------------------------------------------------------
@@ -251,12 +237,44 @@ __global__ void k_gather(double *__restrict__ pool, const uint64_t *__restrict__
         pool[dst[t]] = pool[src[t]];
 }
 
-__global__ void k_gather32(double *__restrict__ pool, const uint32_t *__restrict__ dst,
-                           const uint32_t *__restrict__ src, int64_t n)
+// Copies and fixed values of one or more Syncs in one pass: no destination is
+// another's source, so their order does not matter.  The lists are read
+// before the wait for the kernel that writes the sources (they never change
+// inside a step).
+template <typename I>
+__global__ void k_sync(double *__restrict__ pool, const I *__restrict__ dst, const I *__restrict__ src, int64_t n,
+                       const I *__restrict__ cdst, const double *__restrict__ cval, int64_t nconst)
 {
     const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t < n)
-        pool[dst[t]] = pool[src[t]];
+    {
+        const I d = dst[t], s = src[t];
+        pdl_wait();
+        pool[d] = pool[s];
+    }
+    else if (t - n < nconst)
+    {
+        const I d = cdst[t - n];
+        const double v = cval[t - n];
+        pdl_wait();
+        pool[d] = v;
+    }
+}
+template <typename I>
+static void sync_launch(cudaStream_t st, double *pool, const I *dst, const I *src, int64_t n, const I *cdst,
+                        const double *cval, int64_t nconst)
+{
+    pdl_launch(k_sync<I>, dim3(unsigned((n + nconst + 255) / 256)), 256, 0, st, pool, dst, src, n, cdst, cval, nconst);
+}
+void launch_k_sync(cudaStream_t st, double *pool, const uint64_t *dst, const uint64_t *src, int64_t n,
+                   const uint64_t *cdst, const double *cval, int64_t nconst)
+{
+    sync_launch(st, pool, dst, src, n, cdst, cval, nconst);
+}
+void launch_k_sync(cudaStream_t st, double *pool, const uint32_t *dst, const uint32_t *src, int64_t n,
+                   const uint32_t *cdst, const double *cval, int64_t nconst)
+{
+    sync_launch(st, pool, dst, src, n, cdst, cval, nconst);
 }
 
 // phase A of a Sync: points set to fixed values by physical handlers
@@ -276,17 +294,18 @@ __global__ void k_set_consts(double *__restrict__ pool, const uint64_t *__restri
 // layer's state.  One thread per boundary cell column; dir = +-1, +-2, +-3.
 __device__ __forceinline__ void wall_u_one(const BlockView &b, int dir, double gamma, int64_t t);
 
-__global__ void k_wall_u(const BlockView *__restrict__ bvs, int blk, int dir, double gamma)
-{
-    wall_u_one(bvs[blk], dir, gamma, int64_t(blockIdx.x) * blockDim.x + threadIdx.x);
-}
-
 // all Solid_Surface handlers of a sync in one launch: walls[2 q] = block,
 // walls[2 q + 1] = direction of handler q = blockIdx.y
 __global__ void k_wall_u_all(const BlockView *__restrict__ bvs, const int *__restrict__ walls, double gamma)
 {
     const int q = blockIdx.y;
+    pdl_wait();
     wall_u_one(bvs[walls[2 * q]], walls[2 * q + 1], gamma, int64_t(blockIdx.x) * blockDim.x + threadIdx.x);
+}
+
+void launch_k_wall_u(dim3 grid, cudaStream_t st, const BlockView *bvs, const int *walls, double gamma)
+{
+    pdl_launch(k_wall_u_all, grid, 256, 0, st, bvs, walls, gamma);
 }
 
 __device__ __forceinline__ void wall_u_one(const BlockView &b, int dir, double gamma, int64_t t)
@@ -911,14 +930,6 @@ __global__ void k_diag(const BlockView *__restrict__ bvs, int run, unsigned long
     }
 }
 
-// Pole handlers and repairs: one thread per pole_one work item (mhd_pole.cuh)
-__global__ void k_pole(const BlockView *__restrict__ bvs, const int *__restrict__ poles, int op)
-{
-    const BlockView &b = bvs[poles[2 * blockIdx.y]];
-    const int side = poles[2 * blockIdx.y + 1] > 0 ? 1 : -1;
-    pole_one(b, side, op, int64_t(blockIdx.x) * blockDim.x + threadIdx.x);
-}
-
 // The J edges that read a B_zeta face the Pole rewrite changed (POLE_BZETA
 // writes the first cell layer jc at each Pole: J_xi at j = jc, jc + 1 and
 // J_eta at j = jc read it): Calc_J_Edge again on the staggered points
@@ -926,64 +937,122 @@ __global__ void k_pole(const BlockView *__restrict__ bvs, const int *__restrict_
 // formed before the rewrite, in the fused B_cell / J-edge pass, from the
 // same faces, so the J edges are those of the reference's order (calc_Bcell
 // with the rewrite, then Calc_J_Edge) bit for bit.  Work items per Pole:
-// (ni + 1) x 2 x (nk + 1).
-__global__ void k_pole_jedge(const BlockView *__restrict__ bvs, const int *__restrict__ poles)
+// (ni + 1) x 2 x (nk + 1).  jeta_ring = 0: without the J_eta ring at jc, which
+// POLE_JETA in the same launch overwrites in the reference's order.
+__host__ __device__ inline int64_t pole_items(int op, int ni, int nk)
 {
-    const BlockView &b = bvs[poles[2 * blockIdx.y]];
-    const int side = poles[2 * blockIdx.y + 1] > 0 ? 1 : -1;
+    return op == POLE_JEDGE ? int64_t(ni + 1) * 2 * (nk + 1) : pole_work(op, ni, nk);
+}
+__device__ __forceinline__ void pole_jedge_one(const BlockView &b, int side, int64_t t, int jeta_ring)
+{
     const int jc = side < 0 ? 0 : b.nj - 1;
-    const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (t >= int64_t(b.ni + 1) * 2 * (b.nk + 1))
+    if (t >= pole_items(POLE_JEDGE, b.ni, b.nk))
         return;
     const int k = int(t % (b.nk + 1)), j = jc + int((t / (b.nk + 1)) % 2), i = int(t / (2 * int64_t(b.nk + 1)));
 #pragma unroll
     for (int ea = 0; ea < 2; ++ea)
-        if (inner_of(b, 1, ea, i, j, k))
+        if (inner_of(b, 1, ea, i, j, k) && (ea == 0 || j != jc || jeta_ring))
             jedge_one(b, ea, i, j, k, F_Bxi, F_Jxi, 1.0);
 }
 
 // ---------------------------------------------------------------------------
-// The ring least squares of POLE_BCELL, POLE_EETA_REG and POLE_JCELL with one
-// warp per ring.  The lanes form the pushed vectors and values of 32 k at a
+// The ring sums (POLE_RING_U, POLE_RING_BXI) and ring least squares
+// (POLE_BCELL, POLE_EETA_REG / POLE_ERES_REG, POLE_JCELL) with one warp per
+// ring.  The lanes form the pushed vectors, values and products of 32 k at a
 // time (square roots and divisions in parallel, the same operations as
 // pole_one).  Each sum then runs in one lane over the pushes in the
 // reference's order (k, then the handler's order within k), so it equals the
-// one-thread ring sum bit for bit: the normal matrix A and the count depend
-// on the geometry only and are summed once per geometry (build), nine lanes
-// one entry each; every application sums the right-hand side, three lanes
-// one component each, and lane 0 regularises, solves and broadcasts.
+// one-thread ring sum bit for bit: a skipped push adds +0, which changes no
+// sum that starts at +0.  The normal matrix A and the count depend on the
+// geometry only and are summed once per geometry (build), nine lanes one entry
+// each; every application sums the right-hand side, three lanes one component
+// each, and lane 0 regularises, solves and broadcasts.
+// What bounds them: the chain of dependent adds (8 nk for J_cell) and two
+// rounds of loads.  With the products formed by all lanes and the sums
+// unrolled over shared memory the chain is adds alone; before, each step read
+// the flag, the value and the vector and branched.
 // ---------------------------------------------------------------------------
 constexpr int kPoleWarps = 4; // warps (rings) per CTA
 constexpr int kPoleTerms = 8; // at most 8 pushes per k (J_cell)
 
-struct PoleTerm
+// One chunk of pushes of a warp in shared memory: products (apply: phi s[a] in
+// row a; build: s[a] s[c] in row 3 a + c), 0 for a push that is skipped, and
+// its use flag.  Push q of lane l sits at 32 q + l (no bank conflicts for the
+// lanes' writes); a row is 2 doubles longer than its pushes, so that the
+// lanes that sum read different banks.
+constexpr int kPoleRow = 32 * kPoleTerms + 2;
+struct PoleChunk
 {
-    double s[3], phi;
-    int ok;
+    double *p;
+    int *ok;
 };
+__host__ __device__ constexpr size_t pole_chunk_bytes(bool build)
+{
+    return (build ? 9 : 3) * size_t(kPoleRow) * sizeof(double) + 32 * kPoleTerms * sizeof(int);
+}
 
-// one chunk of pushes: build: lane q < 9 sums s[q / 3] s[q % 3] (A), lane 9
-// counts; apply: lane a < 3 sums phi s[a]
-__device__ __forceinline__ void pole_accumulate(const PoleTerm *sh, int nterm, bool build, double &acc, int &cnt)
+__device__ __forceinline__ void pole_term(const PoleChunk &sh, int q, bool build, bool ok, const double s[3],
+                                          double phi)
+{
+    const int e = 32 * q + (threadIdx.x & 31);
+    sh.ok[e] = ok ? 1 : 0;
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+    {
+        if (!build)
+            sh.p[a * kPoleRow + e] = ok ? phi * s[a] : 0.0;
+        else
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+                sh.p[(3 * a + c) * kPoleRow + e] = ok ? s[a] * s[c] : 0.0;
+    }
+}
+
+// the chunk's pushes in order (lane, then the lane's NQ pushes)
+template <int NQ> __device__ __forceinline__ void pole_accumulate(const PoleChunk &sh, bool build, double &acc, int &cnt)
 {
     const int lane = threadIdx.x & 31;
-    if (build)
+    if (lane < (build ? 9 : 3))
     {
-        if (lane < 9)
+        const double *x = sh.p + lane * kPoleRow;
+#pragma unroll
+        for (int l = 0; l < 32; l += 8 / (NQ > 4 ? 8 : NQ > 1 ? 4 : 1))
         {
-            const int a = lane / 3, c = lane % 3;
-            for (int q = 0; q < nterm; ++q)
-                if (sh[q].ok)
-                    acc += sh[q].s[a] * sh[q].s[c];
+            constexpr int L = 8 / (NQ > 4 ? 8 : NQ > 1 ? 4 : 1);
+            double y[L * NQ];
+#pragma unroll
+            for (int e = 0; e < L * NQ; ++e)
+                y[e] = x[32 * (e % NQ) + l + e / NQ];
+#pragma unroll
+            for (int e = 0; e < L * NQ; ++e)
+                acc += y[e];
         }
-        else if (lane == 9)
-            for (int q = 0; q < nterm; ++q)
-                cnt += sh[q].ok ? 1 : 0;
     }
-    else if (lane < 3)
-        for (int q = 0; q < nterm; ++q)
-            if (sh[q].ok)
-                acc += sh[q].phi * sh[q].s[lane];
+    else if (build && lane == 9)
+        for (int q = 0; q < 32 * NQ; ++q)
+            cnt += sh.ok[q];
+}
+
+// k average of a ring (pole_one's POLE_RING_U / POLE_RING_BXI)
+__device__ __forceinline__ void pole_ring_warp(const BlockView &b, int side, int op, int64_t t, const PoleChunk &sh)
+{
+    const int lane = threadIdx.x & 31;
+    const bool u = op == POLE_RING_U;
+    const int i = u ? int(t / 5) : int(t), m = u ? int(t % 5) : 0, jc = side < 0 ? 0 : b.nj - 1;
+    double *F = b.f[u ? F_U : F_Bxi] + int64_t(m) * b.vol + pidx(b, i, jc, 0);
+    double acc = 0.0;
+    int cnt = 0;
+    for (int k0 = 0; k0 < b.nk; k0 += 32)
+    {
+        sh.p[lane] = k0 + lane < b.nk ? F[k0 + lane] : 0.0;
+        __syncwarp();
+        if (lane == 0)
+            pole_accumulate<1>(sh, false, acc, cnt);
+        __syncwarp();
+    }
+    const double avg = __shfl_sync(0xffffffffu, acc, 0) / double(b.nk);
+    for (int k = lane; k < b.nk; k += 32)
+        F[k] = avg;
 }
 
 // build: store the ring's A and count (cache[0..8], cache[9]); apply: lane 0
@@ -1029,7 +1098,7 @@ __device__ bool pole_finish(double acc, int cnt, bool build, double *cache, bool
     return status == 0;
 }
 
-__device__ void pole_bcell_warp(const BlockView &b, int side, int64_t t, PoleTerm *sh, double *cache, bool build)
+__device__ void pole_bcell_warp(const BlockView &b, int side, int64_t t, const PoleChunk &sh, double *cache, bool build)
 {
     const int lane = threadIdx.x & 31;
     const int nj = b.nj, nk = b.nk;
@@ -1043,6 +1112,7 @@ __device__ void pole_bcell_warp(const BlockView &b, int side, int64_t t, PoleTer
     const double sn = side < 0 ? 1.0 : -1.0;
     const double *Aet = b.f[F_JDeta], *Axi = b.f[F_JDxi];
     const double *Bet = b.f[F_Beta], *Bxi = b.f[F_Bxi], *Aadd = b.f[F_Baddeta], *Xadd = b.f[F_Baddxi];
+    const double zero[3] = {0.0, 0.0, 0.0};
     double acc = 0.0;
     int cnt = 0;
     for (int k0 = 0; k0 < nk; k0 += 32)
@@ -1051,27 +1121,27 @@ __device__ void pole_bcell_warp(const BlockView &b, int side, int64_t t, PoleTer
         if (k < nk)
         {
             const int64_t pn = pidx(b, i, jn, k), p0 = pidx(b, i, jc, k), p1 = pidx(b, i + 1, jc, k);
-            PoleTerm *o = sh + 3 * lane;
-            double f = Bet[pn];
+            double f[3] = {Bet[pn], Bxi[p0], Bxi[p1]};
             if (total)
-                f += Aadd[pn];
-            o[0] = PoleTerm{{sn * Aet[pn], sn * Aet[v + pn], sn * Aet[2 * v + pn]}, sn * f, 0};
-            f = Bxi[p0];
-            if (total)
-                f += Xadd[p0];
-            o[1] = PoleTerm{{-Axi[p0], -Axi[v + p0], -Axi[2 * v + p0]}, -f, 0};
-            f = Bxi[p1];
-            if (total)
-                f += Xadd[p1];
-            o[2] = PoleTerm{{Axi[p1], Axi[v + p1], Axi[2 * v + p1]}, f, 0};
-            for (int q = 0; q < 3; ++q)
             {
-                const double *S = o[q].s;
-                o[q].ok = !((S[0] * S[0] + S[1] * S[1] + S[2] * S[2]) <= 1.0e-300);
+                f[0] += Aadd[pn];
+                f[1] += Xadd[p0];
+                f[2] += Xadd[p1];
             }
+            const double S[3][3] = {{sn * Aet[pn], sn * Aet[v + pn], sn * Aet[2 * v + pn]},
+                                    {-Axi[p0], -Axi[v + p0], -Axi[2 * v + p0]},
+                                    {Axi[p1], Axi[v + p1], Axi[2 * v + p1]}};
+            const double phi[3] = {sn * f[0], -f[1], f[2]};
+#pragma unroll
+            for (int q = 0; q < 3; ++q)
+                pole_term(sh, q, build,
+                          !((S[q][0] * S[q][0] + S[q][1] * S[q][1] + S[q][2] * S[q][2]) <= 1.0e-300), S[q], phi[q]);
         }
+        else
+            for (int q = 0; q < 3; ++q)
+                pole_term(sh, q, build, false, zero, 0.0);
         __syncwarp();
-        pole_accumulate(sh, 3 * min(32, nk - k0), build, acc, cnt);
+        pole_accumulate<3>(sh, build, acc, cnt);
         __syncwarp();
     }
     // BC_Pole_Bcell_Collapse_ solves whenever the regularised system is regular
@@ -1091,7 +1161,7 @@ __device__ void pole_bcell_warp(const BlockView &b, int side, int64_t t, PoleTer
 
 // the regulation of E_eta (field F_Eeta) or Eres_eta (F_Ereseta): both are
 // eta edges of the same ring, so their normal matrices (from dr_eta) are one
-__device__ void pole_eeta_warp(const BlockView &b, int side, int64_t t, PoleTerm *sh, double *cache, bool build,
+__device__ void pole_eeta_warp(const BlockView &b, int side, int64_t t, const PoleChunk &sh, double *cache, bool build,
                                int field)
 {
     const int lane = threadIdx.x & 31;
@@ -1106,24 +1176,24 @@ __device__ void pole_eeta_warp(const BlockView &b, int side, int64_t t, PoleTerm
     for (int k0 = 0; k0 < nk; k0 += 32) // k = n_k is the same edge as k = 0
     {
         const int k = k0 + lane;
+        double s[3] = {0.0, 0.0, 0.0}, phi = 0.0;
+        bool ok = false;
         if (k < nk)
         {
             const int64_t p = pidx(b, i, jc, k);
             const double d0 = dr[p], d1 = dr[v + p], d2 = dr[2 * v + p];
+            const double e = build ? 0.0 : E[p];
             const double L = sqrt(d0 * d0 + d1 * d1 + d2 * d2);
-            PoleTerm &o = sh[lane];
-            o.ok = !(L < 1.0e-14);
-            if (o.ok)
-            {
-                const double invL = 1.0 / L;
-                o.s[0] = d0 * invL;
-                o.s[1] = d1 * invL;
-                o.s[2] = d2 * invL;
-                o.phi = build ? 0.0 : E[p] * invL;
-            }
+            ok = !(L < 1.0e-14);
+            const double invL = 1.0 / L;
+            s[0] = d0 * invL;
+            s[1] = d1 * invL;
+            s[2] = d2 * invL;
+            phi = e * invL;
         }
+        pole_term(sh, 0, build, ok, s, phi);
         __syncwarp();
-        pole_accumulate(sh, min(32, nk - k0), build, acc, cnt);
+        pole_accumulate<1>(sh, build, acc, cnt);
         __syncwarp();
     }
     double Ev[3];
@@ -1160,7 +1230,7 @@ __device__ void pole_eeta_warp(const BlockView &b, int side, int64_t t, PoleTerm
         E[pidx(b, i, jc, k)] = avg;
 }
 
-__device__ void pole_jcell_warp(const BlockView &b, int side, int64_t t, PoleTerm *sh, double *cache, bool build)
+__device__ void pole_jcell_warp(const BlockView &b, int side, int64_t t, const PoleChunk &sh, double *cache, bool build)
 {
     const int lane = threadIdx.x & 31;
     const int nj = b.nj, nk = b.nk;
@@ -1178,28 +1248,28 @@ __device__ void pole_jcell_warp(const BlockView &b, int side, int64_t t, PoleTer
     for (int k0 = 0; k0 < nk; k0 += 32)
     {
         const int k = k0 + lane;
-        if (k < nk)
-        {
 #pragma unroll
-            for (int q = 0; q < 8; ++q)
+        for (int q = 0; q < 8; ++q)
+        {
+            double s[3] = {0.0, 0.0, 0.0}, phi = 0.0;
+            bool ok = false;
+            if (k < nk)
             {
                 const int64_t p = pidx(b, i + di[q], q < 4 ? jc : jt, k + dk[q]);
                 const double *dr = b.f[fd[q]];
                 const double dx = dr[p], dy = dr[v + p], dz = dr[2 * v + p];
+                const double J = build ? 0.0 : b.f[fj[q]][p];
                 const double L = sqrt(dx * dx + dy * dy + dz * dz);
-                PoleTerm &o = sh[8 * lane + q];
-                o.ok = !(L < 1.0e-14);
-                if (o.ok)
-                {
-                    o.s[0] = dx / L;
-                    o.s[1] = dy / L;
-                    o.s[2] = dz / L;
-                    o.phi = build ? 0.0 : b.f[fj[q]][p] / L;
-                }
+                ok = !(L < 1.0e-14);
+                s[0] = dx / L;
+                s[1] = dy / L;
+                s[2] = dz / L;
+                phi = J / L;
             }
+            pole_term(sh, q, build, ok, s, phi);
         }
         __syncwarp();
-        pole_accumulate(sh, 8 * min(32, nk - k0), build, acc, cnt);
+        pole_accumulate<8>(sh, build, acc, cnt);
         __syncwarp();
     }
     double Jp[3];
@@ -1222,37 +1292,93 @@ __host__ __device__ inline int pole_lsq_slot(int op)
     return op == POLE_BCELL ? 0 : (op == POLE_EETA_REG || op == POLE_ERES_REG) ? 1 : op == POLE_JCELL ? 2 : -1;
 }
 
-// cache: per Pole, per least-squares operation, per ring i (stride rings):
-// A (9 values) and the push count
-__global__ void __launch_bounds__(32 * kPoleWarps) k_pole_warp(const BlockView *__restrict__ bvs,
-                                                               const int *__restrict__ poles, int op,
-                                                               double *__restrict__ cache, int stride, int build)
+__host__ __device__ inline bool pole_ring_op(int op)
 {
-    __shared__ PoleTerm sh[kPoleWarps][32 * kPoleTerms];
-    const BlockView &b = bvs[poles[2 * blockIdx.y]];
-    const int side = poles[2 * blockIdx.y + 1] > 0 ? 1 : -1;
-    const int warp = threadIdx.x >> 5;
-    const int64_t t = int64_t(blockIdx.x) * kPoleWarps + warp;
-    if (t >= pole_work(op, b.ni, b.nk))
-        return; // the whole warp leaves together
-    const int ring = (op == POLE_BCELL) ? int(t >> 1) : int(t);
-    double *c = cache + ((int64_t(blockIdx.y) * 3 + pole_lsq_slot(op)) * stride + ring) * 10;
-    if (op == POLE_BCELL)
-        pole_bcell_warp(b, side, t, sh[warp], c, build != 0);
-    else if (op == POLE_EETA_REG || op == POLE_ERES_REG)
-        pole_eeta_warp(b, side, t, sh[warp], c, build != 0, op == POLE_ERES_REG ? F_Ereseta : F_Eeta);
-    else
-        pole_jcell_warp(b, side, t, sh[warp], c, build != 0);
+    return op == POLE_RING_U || op == POLE_RING_BXI || pole_lsq_slot(op) >= 0;
 }
 
-void launch_pole_op(int op, int64_t work, int npoles, cudaStream_t st, const BlockView *bvs, const int *poles,
-                    double *cache, int stride, int build)
+// cache: per Pole, per least-squares operation, per ring i (stride rings):
+// A (9 values) and the push count
+__device__ __forceinline__ void pole_warp_item(const BlockView &b, int side, int pole, int op, int64_t t,
+                                               const PoleChunk &sh,                                               double *cache, int stride, bool build)
 {
-    if (pole_lsq_slot(op) >= 0)
-        k_pole_warp<<<dim3(unsigned((work + kPoleWarps - 1) / kPoleWarps), unsigned(npoles)), 32 * kPoleWarps, 0,
-                      st>>>(bvs, poles, op, cache, stride, build);
-    else if (!build)
-        k_pole<<<dim3(unsigned((work + 255) / 256), unsigned(npoles)), 256, 0, st>>>(bvs, poles, op);
+    if (t >= pole_work(op, b.ni, b.nk))
+        return; // the whole warp leaves together
+    if (pole_lsq_slot(op) < 0)
+    {
+        pole_ring_warp(b, side, op, t, sh);
+        return;
+    }
+    const int ring = (op == POLE_BCELL) ? int(t >> 1) : int(t);
+    double *c = cache + ((int64_t(pole) * 3 + pole_lsq_slot(op)) * stride + ring) * 10;
+    if (op == POLE_BCELL)
+        pole_bcell_warp(b, side, t, sh, c, build);
+    else if (op == POLE_EETA_REG || op == POLE_ERES_REG)
+        pole_eeta_warp(b, side, t, sh, c, build, op == POLE_ERES_REG ? F_Ereseta : F_Eeta);
+    else
+        pole_jcell_warp(b, side, t, sh, c, build);
+}
+
+// up to four operations on every Pole (grid row): rings one warp each, the
+// others one thread per work item
+__global__ void __launch_bounds__(32 * kPoleWarps) k_pole(const BlockView *__restrict__ bvs,
+                                                          const int *__restrict__ poles, PoleOps ops,
+                                                          double *__restrict__ cache, int stride, int build)
+{
+    extern __shared__ __align__(16) unsigned char pole_smem[];
+    unsigned char *mine = pole_smem + (threadIdx.x >> 5) * pole_chunk_bytes(build != 0);
+    const PoleChunk sh{reinterpret_cast<double *>(mine),
+                       reinterpret_cast<int *>(mine + (build ? 9 : 3) * size_t(kPoleRow) * sizeof(double))};
+    int q = 0;
+    while (q + 1 < ops.n && int(blockIdx.x) >= ops.cta0[q + 1])
+        ++q;
+    const int op = ops.op[q];
+    const int64_t cta = int(blockIdx.x) - ops.cta0[q];
+    const BlockView &b = bvs[poles[2 * blockIdx.y]];
+    const int side = poles[2 * blockIdx.y + 1] > 0 ? 1 : -1;
+    pdl_wait();
+    if (pole_ring_op(op))
+    {
+        const int warp = threadIdx.x >> 5;
+        pole_warp_item(b, side, int(blockIdx.y), op, cta * kPoleWarps + warp, sh, cache, stride, build != 0);
+    }
+    else if (op == POLE_JEDGE)
+        pole_jedge_one(b, side, cta * blockDim.x + threadIdx.x, ops.jeta_ring);
+    else
+        pole_one(b, side, op, cta * blockDim.x + threadIdx.x);
+}
+
+static void pole_launch(PoleOps ops, int ni, int nk, int npoles, cudaStream_t st, const BlockView *bvs,
+                        const int *poles, double *cache, int stride, int build)
+{
+    int x = 0;
+    for (int q = 0; q < ops.n; ++q)
+    {
+        ops.cta0[q] = x;
+        const int64_t w = pole_items(ops.op[q], ni, nk), per = pole_ring_op(ops.op[q]) ? kPoleWarps : 32 * kPoleWarps;
+        x += int((w + per - 1) / per);
+    }
+    ops.cta0[ops.n] = x;
+    const size_t smem = pole_chunk_bytes(build != 0) * kPoleWarps;
+    if (build)
+        cudaFuncSetAttribute(k_pole, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    pdl_launch(k_pole, dim3(unsigned(x), unsigned(npoles)), 32 * kPoleWarps, smem, st, bvs, poles, ops, cache,
+               stride, build);
+}
+
+void launch_pole_ops(PoleOps ops, int ni, int nk, int npoles, cudaStream_t st, const BlockView *bvs, const int *poles,
+                     double *cache, int stride)
+{
+    pole_launch(ops, ni, nk, npoles, st, bvs, poles, cache, stride, 0);
+}
+
+void launch_pole_build(int op, int ni, int nk, int npoles, cudaStream_t st, const BlockView *bvs, const int *poles,
+                       double *cache, int stride)
+{
+    PoleOps ops{};
+    ops.n = 1;
+    ops.op[0] = op;
+    pole_launch(ops, ni, nk, npoles, st, bvs, poles, cache, stride, 1);
 }
 
 } // namespace mhd

@@ -158,12 +158,17 @@ struct QHot
     __device__ __forceinline__ float operator()(int plane, int64_t c) const { return q[plane * v + c]; }
 };
 
-template <class A> __device__ __forceinline__ void k_fluid_mixed_body(const A &args, const Consts &c)
+template <class A> __device__ __forceinline__ void k_fluid_mixed_body(const A &args, const Consts &c, const RunClock &rc)
 {
     uint32_t t, p;
     const HotBlock &b = hot_block<KIND_CELL1>(args, t);
     int i, j, k;
-    if (!hot_point<KIND_CELL1>(b, t, i, j, k, p))
+    const bool in_box = hot_point<KIND_CELL1>(b, t, i, j, k, p);
+    pdl_wait();
+    if (rc.dt_key && blockIdx.x == 0 && blockIdx.y == 0) // start of the step (see k_fluid_ucontra_t)
+        for (int r = threadIdx.x; r < rc.nruns; r += blockDim.x)
+            begin_run(rc, r);
+    if (!in_box)
         return;
     const uint64_t v = b.vol;
     const bool inner = hot_inner(b, i, j, k);
@@ -231,9 +236,9 @@ template <class A> __device__ __forceinline__ void k_fluid_mixed_body(const A &a
 }
 
 template <class A, int MINB>
-__global__ void __launch_bounds__(256, MINB) k_fluid_mixed_t(const __grid_constant__ A a, Consts c)
+__global__ void __launch_bounds__(256, MINB) k_fluid_mixed_t(const __grid_constant__ A a, Consts c, RunClock rc)
 {
-    k_fluid_mixed_body(a, c);
+    k_fluid_mixed_body(a, c, rc);
 }
 
 
@@ -434,26 +439,30 @@ __global__ void __launch_bounds__(256, 2) k_fluid_mixed_staged(const BlockView *
 // launchers of the register / occupancy variants (tuned by mhd_autotune);
 // variant 3 is the face-tiled kernel, 4 the same with the staged face states
 // (both on the KIND_TILE1 grid)
-int launch_k_fluid_mixed(int variant, const HotGrid &h, dim3 tiles, cudaStream_t st, const BlockView *bvs, Consts c)
+int launch_k_fluid_mixed(int variant, const HotGrid &h, dim3 tiles, cudaStream_t st, const BlockView *bvs, Consts c,
+                         RunClock rc)
 {
     if (variant < 0 || variant > 4)
         return -1;
     if (variant >= 3)
     {
+        if (rc.dt_key)
+            k_begin_step<<<1, 128, 0, st>>>(rc);
         if (variant == 3)
             k_fluid_mixed_tile<<<tiles, 256, 0, st>>>(bvs, c);
         else
             k_fluid_mixed_staged<<<tiles, 256, 0, st>>>(bvs, c);
-        return 1;
+        return rc.dt_key ? 2 : 1;
     }
     return hot_for(h, KIND_CELL1, [&](const auto &a, dim3 g) {
         using A = std::decay_t<decltype(a)>;
         if (variant == 0)
-            hot_launch(k_fluid_mixed_t<A, 3>, g, st, a, c);
+            hot_launch(k_fluid_mixed_t<A, 3>, g, st, a, c, rc);
         else if (variant == 1)
-            hot_launch(k_fluid_mixed_t<A, 1>, g, st, a, c);
+            hot_launch(k_fluid_mixed_t<A, 1>, g, st, a, c, rc);
         else
-            hot_launch(k_fluid_mixed_t<A, 2>, g, st, a, c);
+            hot_launch(k_fluid_mixed_t<A, 2>, g, st, a, c, rc);
+        rc = RunClock{}; // the first launch only
     });
 }
 

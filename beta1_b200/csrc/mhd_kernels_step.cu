@@ -35,6 +35,27 @@ __device__ __forceinline__ double smax(double a, double b) { return (a < b) ? b 
 
 constexpr int kHotThreads = 256;
 
+// Start of StepOnce, in the first CTA of the step's first kernel (no kernel of
+// the step before the update reads dt): dt = global minimum of the CFL bounds,
+// abort check (dt < dt_abort or NaN sets the error word,
+// LunarSolver_Timestep.cpp:128-139).
+__device__ __forceinline__ void run_begin(const RunClock &rc)
+{
+    if (rc.dt_key && blockIdx.x == 0 && blockIdx.y == 0)
+        for (int r = threadIdx.x; r < rc.nruns; r += blockDim.x)
+            begin_run(rc, r);
+}
+
+// The run data of StepOnce's end (Z4_Lunar/src/LunarSolver_Driver.cpp:75-79)
+// and the arming of the dt reductions, in the first CTA of the update (the
+// next reduction runs in the derived-field pass after it)
+__device__ __forceinline__ void run_end(const RunClock &rc)
+{
+    if (rc.dt_key && blockIdx.x == 0 && blockIdx.y == 0)
+        for (int r = threadIdx.x; r < rc.nruns; r += blockDim.x)
+            end_run(rc, r);
+}
+
 // the strides of one axis
 __device__ __forceinline__ int hot_stride(const HotBlock &b, int a)
 {
@@ -103,12 +124,15 @@ __device__ __forceinline__ void rusanov(const FaceState &L, const FaceState &R, 
 // Fluid RHS of the inner cells and contravariant velocities (cell_u_contra,
 // LunarSolver_MagExplicit_Ideal.cpp:95-115) of the cells within one ghost
 // layer, one axis at a time: both read the axis's face vectors at p and p + 1.
-template <class A> __device__ __forceinline__ void fluid_ucontra_body(const A &a, const Consts &c)
+template <class A> __device__ __forceinline__ void fluid_ucontra_body(const A &a, const Consts &c, const RunClock &rc)
 {
     uint32_t t, p;
     const HotBlock &b = hot_block<KIND_CELL1>(a, t);
     int i, j, k;
-    if (!hot_point<KIND_CELL1>(b, t, i, j, k, p))
+    const bool in_box = hot_point<KIND_CELL1>(b, t, i, j, k, p);
+    pdl_wait();
+    run_begin(rc);
+    if (!in_box)
         return;
     const uint64_t v = b.vol;
     const bool inner = hot_inner(b, i, j, k);
@@ -177,9 +201,9 @@ template <class A> __device__ __forceinline__ void fluid_ucontra_body(const A &a
 }
 
 template <class A, int MINB>
-__global__ void __launch_bounds__(kHotThreads, MINB) k_fluid_ucontra_t(const __grid_constant__ A a, Consts c)
+__global__ void __launch_bounds__(kHotThreads, MINB) k_fluid_ucontra_t(const __grid_constant__ A a, Consts c, RunClock rc)
 {
-    fluid_ucontra_body(a, c);
+    fluid_ucontra_body(a, c, rc);
 }
 
 // ---------------------------------------------------------------------------
@@ -203,7 +227,9 @@ template <class A> __device__ __forceinline__ void eface_body(const A &a)
     uint32_t t, p;
     const HotBlock &b = hot_block<KIND_STAG>(a, t);
     int i, j, k;
-    if (!hot_point<KIND_STAG>(b, t, i, j, k, p))
+    const bool in_box = hot_point<KIND_STAG>(b, t, i, j, k, p);
+    pdl_wait();
+    if (!in_box)
         return;
     const uint64_t v = b.vol;
     const int st[3] = {int(b.si), int(b.sj), 1};
@@ -289,7 +315,9 @@ template <class A> __device__ __forceinline__ void eedge_body(const A &a)
     uint32_t t, p;
     const HotBlock &b = hot_block<KIND_STAG>(a, t);
     int i, j, k;
-    if (!hot_point<KIND_STAG>(b, t, i, j, k, p))
+    const bool in_box = hot_point<KIND_STAG>(b, t, i, j, k, p);
+    pdl_wait();
+    if (!in_box)
         return;
     const uint64_t v = b.vol;
     const int si = int(b.si), sj = int(b.sj);
@@ -365,71 +393,79 @@ __device__ __forceinline__ void point_curl(const HotBlock &b, uint32_t p, int qE
 // a snapshot, B = bs + dt RHS (bs[3 block + axis], in the pool's point layout).
 // The snapshot form is the implicit Hall trial's update: the same operands and
 // operations as restoring B first, so the same bits, without the copy.
-template <class A>
-__device__ __forceinline__ void curl_body(const A &a, int qE, int qR, int qB, double mult, const double *dtp,
-                                          double dtdiv, int mult_is_neg_dt, const int *rng, const double *const *bs)
+// CELLS: the whole Euler update in one pass, also the cell part (U += dt * RHS_H
+// on the inner cells, LunarSolver_Advance.cpp:82-93); one launch instead of two
+// and twice the loads in flight.
+struct CurlArgs
+{
+    int qE, qR, qB;
+    double mult;
+    const double *dtp;
+    double dtdiv;
+    int mult_is_neg_dt;
+    const int *rng;
+    const double *const *bs;
+};
+template <bool CELLS, class A>
+__device__ __forceinline__ void curl_body(const A &a, const CurlArgs &x, const RunClock &rc)
 {
     uint32_t t, p;
     const HotBlock &b = hot_block<KIND_STAG>(a, t);
     int i, j, k;
-    if (!hot_stagger(b, rng, t, i, j, k, p))
+    const bool in_box = hot_stagger(b, x.rng, t, i, j, k, p);
+    pdl_wait();
+    if (CELLS)
+        run_end(rc);
+    if (!in_box)
         return;
+    const uint64_t v = b.vol;
+    const double mult = x.mult_is_neg_dt ? -x.dtp[b.run] : x.mult;
     double dtB = 0.0;
-    if (mult_is_neg_dt)
-        mult = -dtp[b.run];
-    if (qB >= 0)
-        dtB = dtp[b.run] / dtdiv;
-    double curl[3], B[3];
-    point_curl(b, p, qE, curl);
-    if (qB >= 0)
+    if (x.qB >= 0)
+        dtB = x.dtp[b.run] / x.dtdiv;
+    double curl[3], B[3], u[5], r[5];
+    point_curl(b, p, x.qE, curl);
+    if (x.qB >= 0)
     {
 #pragma unroll
         for (int fa = 0; fa < 3; ++fa)
-            B[fa] = bs ? bs[3 * b.blk + fa][p] : *hot_plane(b, p, qB + fa);
+            B[fa] = x.bs ? x.bs[3 * b.blk + fa][p] : *hot_plane(b, p, x.qB + fa);
+    }
+    const bool cell = CELLS && hot_inner(b, i, j, k);
+    if (cell)
+    {
+        const double *U = hot_at(b, p, F_U), *R = hot_at(b, p, F_RHS);
+#pragma unroll
+        for (int m = 0; m < 5; ++m)
+        {
+            u[m] = U[m * v];
+            r[m] = R[m * v];
+        }
     }
 #pragma unroll
     for (int fa = 0; fa < 3; ++fa)
         if (hot_face(b, fa, i, j, k))
         {
             const double rhs = mult * curl[fa];
-            if (qR >= 0)
-                *hot_plane(b, p, qR + fa) = rhs;
-            if (qB >= 0)
-                *hot_plane(b, p, qB + fa) = B[fa] + dtB * rhs;
+            if (x.qR >= 0)
+                *hot_plane(b, p, x.qR + fa) = rhs;
+            if (x.qB >= 0)
+                *hot_plane(b, p, x.qB + fa) = B[fa] + dtB * rhs;
         }
-}
-
-template <class A, int MINB>
-__global__ void __launch_bounds__(kHotThreads, MINB)
-    k_curl_e2f_t(const __grid_constant__ A a, int qE, int qR, int qB, double mult, const double *dtp, double dtdiv,
-                 int mult_is_neg_dt, const int *rng, const double *const *bs)
-{
-    curl_body(a, qE, qR, qB, mult, dtp, dtdiv, mult_is_neg_dt, rng, bs);
-}
-
-// cell part of ApplyUpdate_Euler_ (LunarSolver_Advance.cpp:82-93): U += dt*RHS_H
-template <class A>
-__global__ void __launch_bounds__(kHotThreads) k_update_u_t(const __grid_constant__ A a, const double *dtp)
-{
-    uint32_t t, p;
-    const HotBlock &b = hot_block<KIND_CELL0>(a, t);
-    int i, j, k;
-    if (!hot_point<KIND_CELL0>(b, t, i, j, k, p))
-        return;
-    const double dt = dtp[b.run];
-    const uint64_t v = b.vol;
-    double *U = hot_at(b, p, F_U);
-    const double *R = hot_at(b, p, F_RHS);
-    double u[5], r[5];
-#pragma unroll
-    for (int m = 0; m < 5; ++m)
+    if (cell)
     {
-        u[m] = U[m * v];
-        r[m] = R[m * v];
-    }
+        double *U = hot_at(b, p, F_U);
 #pragma unroll
-    for (int m = 0; m < 5; ++m)
-        U[m * v] = u[m] + dt * r[m];
+        for (int m = 0; m < 5; ++m)
+            U[m * v] = u[m] + dtB * r[m];
+    }
+}
+
+template <bool CELLS, class A, int MINB>
+__global__ void __launch_bounds__(kHotThreads, MINB)
+    k_curl_e2f_t(const __grid_constant__ A a, const __grid_constant__ CurlArgs x, RunClock rc)
+{
+    curl_body<CELLS>(a, x, rc);
 }
 
 // SSP-RK2 (Shu and Osher, 1988) from two Euler stages at one dt: the state
@@ -441,7 +477,9 @@ template <class A> __global__ void __launch_bounds__(kHotThreads) k_rk2_t(const 
     uint32_t t, p;
     const HotBlock &b = hot_block<KIND_STAG>(a, t);
     int i, j, k;
-    if (!hot_point<KIND_STAG>(b, t, i, j, k, p))
+    const bool in_box = hot_point<KIND_STAG>(b, t, i, j, k, p);
+    pdl_wait();
+    if (!in_box)
         return;
     const uint64_t v = b.vol;
     double *r = b.rk + p;
@@ -497,7 +535,9 @@ template <typename WT, bool EDGES, class A> __device__ __forceinline__ void bcel
     uint32_t t, p;
     const HotBlock &b = hot_block<KIND>(a, t);
     int i, j, k;
-    if (!hot_point<KIND>(b, t, i, j, k, p))
+    const bool in_box = hot_point<KIND>(b, t, i, j, k, p);
+    pdl_wait();
+    if (!in_box)
         return;
     const uint64_t v = b.vol;
     const int st[3] = {int(b.si), int(b.sj), 1};
@@ -580,7 +620,9 @@ __global__ void __launch_bounds__(kHotThreads) k_jedge_t(const __grid_constant__
     uint32_t t, p;
     const HotBlock &b = hot_block<KIND_STAG>(a, t);
     int i, j, k;
-    if (!hot_stagger(b, rng, t, i, j, k, p))
+    const bool in_box = hot_stagger(b, rng, t, i, j, k, p);
+    pdl_wait();
+    if (!in_box)
         return;
     const int st[3] = {int(b.si), int(b.sj), 1};
     double h0[3], hm[3][3], al[3];
@@ -631,7 +673,9 @@ template <typename WT, class A> __global__ void __launch_bounds__(kHotThreads) k
     uint32_t t, p;
     const HotBlock &b = hot_block<KIND_CELL0>(a, t);
     int i, j, k;
-    if (!hot_point<KIND_CELL0>(b, t, i, j, k, p))
+    const bool in_box = hot_point<KIND_CELL0>(b, t, i, j, k, p);
+    pdl_wait();
+    if (!in_box)
         return;
     double jx, jy, jz;
     jcell_sum<WT>(b, p, jx, jy, jz);
@@ -797,7 +841,9 @@ __device__ __forceinline__ void pv_uplus_dt_body(const A &a, const Consts &c, un
     const HotBlock &b = hot_block<KIND_CELL1>(a, t);
     int i, j, k;
     double dtc = 1e100;
-    if (hot_point<KIND_CELL1>(b, t, i, j, k, p))
+    const bool in_box = hot_point<KIND_CELL1>(b, t, i, j, k, p);
+    pdl_wait();
+    if (in_box)
     {
         const uint64_t v = b.vol;
         const bool inner = hot_inner(b, i, j, k);
@@ -878,6 +924,7 @@ template <class A> __global__ void __launch_bounds__(kHotThreads) k_pv_all_t(con
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t n2 = uint32_t(b.nk + 2 * G), n1 = uint32_t(b.nj + 2 * G);
     const uint32_t q = t / n2, ii = q / n1;
+    pdl_wait();
     if (ii >= uint32_t(b.ni + 2 * G))
         return;
     const int i = int(ii) - G, j = int(q - ii * n1) - G, k = int(t - q * n2) - G;
@@ -900,7 +947,9 @@ __global__ void __launch_bounds__(kHotThreads) k_eres_explicit_t(const __grid_co
     uint32_t t, p;
     const HotBlock &b = hot_block<KIND_STAG>(a, t);
     int i, j, k;
-    if (!hot_point<KIND_STAG>(b, t, i, j, k, p))
+    const bool in_box = hot_point<KIND_STAG>(b, t, i, j, k, p);
+    pdl_wait();
+    if (!in_box)
         return;
     const uint64_t v = b.vol;
     const double *Jc = hot_at(b, p, F_Jcell);
@@ -950,6 +999,7 @@ __global__ void __launch_bounds__(kHotThreads)
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t n2 = uint32_t(b.nk + 2 * G), n1 = uint32_t(b.nj + 2 * G);
     const uint32_t q = t / n2, ii = q / n1;
+    pdl_wait();
     if (ii >= uint32_t(b.ni + 2 * G))
         return;
     const int i = int(ii) - G, j = int(q - ii * n1) - G, k = int(t - q * n2) - G;
@@ -1024,7 +1074,9 @@ __global__ void __launch_bounds__(kHotThreads, MINB)
     uint32_t t, p;
     const HotBlock &b = hot_block<KIND_STAG>(a, t);
     int i, j, k;
-    if (!hot_point<KIND_STAG>(b, t, i, j, k, p))
+    const bool in_box = hot_point<KIND_STAG>(b, t, i, j, k, p);
+    pdl_wait();
+    if (!in_box)
         return;
     const uint64_t v = b.vol;
     const int si = int(b.si), sj = int(b.sj);
@@ -1100,16 +1152,17 @@ int launch_k_pv_all(const HotGrid &h, cudaStream_t st, Consts c)
     });
 }
 
-int launch_k_fluid_ucontra(int variant, const HotGrid &h, cudaStream_t st, Consts c)
+int launch_k_fluid_ucontra(int variant, const HotGrid &h, cudaStream_t st, Consts c, RunClock rc)
 {
     if (variant < 0 || variant > 1)
         return -1;
     return hot_for(h, KIND_CELL1, [&](const auto &a, dim3 g) {
         using A = std::decay_t<decltype(a)>;
         if (variant == 0)
-            hot_launch(k_fluid_ucontra_t<A, 2>, g, st, a, c);
+            hot_launch(k_fluid_ucontra_t<A, 2>, g, st, a, c, rc);
         else
-            hot_launch(k_fluid_ucontra_t<A, 3>, g, st, a, c);
+            hot_launch(k_fluid_ucontra_t<A, 3>, g, st, a, c, rc);
+        rc = RunClock{}; // the first launch only
     });
 }
 
@@ -1185,23 +1238,33 @@ int launch_k_curl_e2f(int variant, const HotGrid &h, cudaStream_t st, int fE0, i
 {
     if (variant < 0 || variant > 1)
         return -1;
-    const int qE = plane_of(fE0), qR = fR0 >= 0 ? plane_of(fR0) : -1, qB = fB0 >= 0 ? plane_of(fB0) : -1;
+    const CurlArgs x{plane_of(fE0), fR0 >= 0 ? plane_of(fR0) : -1, fB0 >= 0 ? plane_of(fB0) : -1, mult, dtp, dtdiv,
+                     mult_is_neg_dt, rng, bs};
     return hot_for(
         h, KIND_STAG,
         [&](const auto &a, dim3 g) {
             using A = std::decay_t<decltype(a)>;
             if (variant == 0)
-                hot_launch(k_curl_e2f_t<A, 1>, g, st, a, qE, qR, qB, mult, dtp, dtdiv, mult_is_neg_dt, rng, bs);
+                hot_launch(k_curl_e2f_t<false, A, 4>, g, st, a, x, RunClock{});
             else
-                hot_launch(k_curl_e2f_t<A, 6>, g, st, a, qE, qR, qB, mult, dtp, dtdiv, mult_is_neg_dt, rng, bs);
+                hot_launch(k_curl_e2f_t<false, A, 6>, g, st, a, x, RunClock{});
         },
         nreg);
 }
 
-int launch_k_update_u(const HotGrid &h, cudaStream_t st, const double *dtp)
+int launch_k_update(int variant, const HotGrid &h, cudaStream_t st, int fR0, const double *dtp, RunClock rc)
 {
-    return hot_for(h, KIND_CELL0, [&](const auto &a, dim3 g) {
-        hot_launch(k_update_u_t<std::decay_t<decltype(a)>>, g, st, a, dtp);
+    if (variant < 0 || variant > 1)
+        return -1;
+    const CurlArgs x{plane_of(F_Exi), fR0 >= 0 ? plane_of(fR0) : -1, plane_of(F_Bxi), -1.0, dtp, 1.0, 0, nullptr,
+                     nullptr};
+    return hot_for(h, KIND_STAG, [&](const auto &a, dim3 g) {
+        using A = std::decay_t<decltype(a)>;
+        if (variant == 0)
+            hot_launch(k_curl_e2f_t<true, A, 4>, g, st, a, x, rc);
+        else
+            hot_launch(k_curl_e2f_t<true, A, 6>, g, st, a, x, rc);
+        rc = RunClock{}; // the first launch only
     });
 }
 
