@@ -3,6 +3,7 @@
 // and the per-step launch sequence replayed as a CUDA graph.
 #include "mhd_device_scope.h"
 #include "mhd_kernels.cuh"
+#include "mhd_hot_launch.cuh"
 
 #include <cuda_runtime.h>
 
@@ -97,6 +98,15 @@ struct StepSync
     SyncPass a, b;
     bool usable = false; // else the groups' own lists run one by one
 };
+// which part of a group's lists: the step's hot one, all of it, or (contexts
+// without Poles) what a Hall residual reads: the hot one, with the first ghost
+// layer of B_cell and J_cell and without Bind_cell
+enum SyncPart
+{
+    SYNC_HOT,
+    SYNC_FULL,
+    SYNC_HALL
+};
 
 // A group's hot part resolved on the host to independent copies and fixed
 // values: a, and in a Pole context with wall handlers b after them.
@@ -128,7 +138,7 @@ struct SyncMap
     bool staged = false;
     bool built = false; // device lists match the host tables
     CopyList full, hot, post;
-    Resolved res, res_full; // of the hot and of the full lists
+    Resolved res; // of the hot lists
     // Pole contexts: the copies and fixed values a step leaves for read-out
     // (cold), written then without the rings, walls and post-wall copies
     CopyList cold;
@@ -149,7 +159,7 @@ const char *const kKernelNames[] = {
     "k_bcell_jedge",  "k_fluid_ucontra", "k_wall_u_all",   "k_hall_cell",    "k_hall_edge",
     "k_pack_vec",     "k_geom32",       "k_fluid_mixed",  "k_gmres_resist", "k_pole",
     "k_geometry",     "k_diag_init",   "k_diag",        "k_rk2",          "k_hall_begin",    "k_hall_step_begin",
-    "k_hall_gmres_init", "k_hall_cycle_prep", "k_hall_ls_begin", "k_hall_ls_check", "k_hall_accept", "k_hall_column",
+    "k_hall_gmres_init", "k_hall_cycle_prep", "k_hall_ls_begin", "k_hall_ls_check", "k_hall_accept",
     "k_hall_trial",   "k_hall_jv_dots", "k_hall_proj_dots", "k_hall_next",  "k_hall_res_dots", "k_hall_restart_r",
     "k_hall_gmres_prologue", "k_norm2", "k_hall_take",    "k_copy_segments"};
 constexpr int kNumKernelNames = int(sizeof(kKernelNames) / sizeof(kKernelNames[0]));
@@ -318,6 +328,13 @@ struct mhd_ctx
         // (no staged copies, no wall handler), so the points neither the curl
         // nor the sync writes keep B*
         bool from_snapshot = false;
+        // host copies of the unknowns and aliases, and the points beside the
+        // unknowns a trial writes (aliases and Sync("Ehall")) in one list;
+        // without it (fused = false) the passes run one by one
+        std::vector<uint64_t> he, ha, ho;
+        std::vector<double> hs;
+        HallList list{};
+        bool fused = false, list_built = false;
         double *X = nullptr, *F = nullptr, *Xt = nullptr, *Ft = nullptr, *dx = nullptr, *b = nullptr, *r = nullptr;
         double *V = nullptr, *w = nullptr, *partial = nullptr, *dots = nullptr;
         unsigned *done = nullptr;                  // CTAs finished in a reduction pass
@@ -356,13 +373,15 @@ static void free_resistive(mhd_ctx *ctx);
 static int resistive_region(mhd_ctx *ctx, const std::vector<uint64_t> &seed);
 static void free_list(CopyList &m);
 static void free_step_syncs(mhd_ctx *ctx);
+static void free_hall_list(mhd_ctx *ctx);
 static int build_all_syncs(mhd_ctx *ctx);
+static int build_hall_list(mhd_ctx *ctx);
 static int materialise_field(mhd_ctx *ctx, int f);
 static int materialise_group(mhd_ctx *ctx, const std::string &group);
 static int materialise_all(mhd_ctx *ctx);
 static void mark_dirty(mhd_ctx *ctx);
 int build_sync(mhd_ctx *ctx, const std::string &group, SyncMap &m);
-static int step_sync(mhd_ctx *ctx, std::initializer_list<const char *> groups, unsigned full, StepSync **out);
+static int step_sync(mhd_ctx *ctx, std::initializer_list<const char *> groups, SyncPart part, StepSync **out);
 
 namespace
 {
@@ -639,19 +658,18 @@ int run_sync(mhd_ctx *ctx, const char *group, bool full = false, bool rings = tr
     return MHD_OK;
 }
 
-// The Syncs of consecutive groups of a step (hot lists; full[q]: the full list
-// of group q) in as few passes as their dependences allow: wall handlers, if
-// any, and one pass of all copies and fixed values (build_step_sync resolves
-// them); one by one where they cannot be resolved.
-int run_syncs(mhd_ctx *ctx, std::initializer_list<const char *> groups, bool rings = true, unsigned full = 0)
+// The Syncs of consecutive groups of a step (per group its hot list, or the
+// part mode names) in as few passes as their dependences allow: wall
+// handlers, if any, and one pass of all copies and fixed values (step_sync
+// resolves them); one by one where they cannot be resolved.
+int run_syncs(mhd_ctx *ctx, std::initializer_list<const char *> groups, bool rings = true, SyncPart part = SYNC_HOT)
 {
     StepSync *s = nullptr;
-    RUN(step_sync(ctx, groups, full, &s));
-    unsigned q = 0;
+    RUN(step_sync(ctx, groups, part, &s));
     if (!s->usable)
     {
         for (const char *g : groups)
-            RUN(run_sync(ctx, g, ((full >> q++) & 1) != 0, rings));
+            RUN(run_sync(ctx, g, part != SYNC_HOT, rings));
         return MHD_OK;
     }
     const bool poles = !ctx->poles.empty();
@@ -663,7 +681,7 @@ int run_syncs(mhd_ctx *ctx, std::initializer_list<const char *> groups, bool rin
         RUN(run_pass(ctx, s->a));
     for (const char *g : groups)
     {
-        const bool f = ((full >> q++) & 1) != 0;
+        const bool f = part == SYNC_FULL;
         const auto it = ctx->syncs.find(g);
         if (it == ctx->syncs.end())
             continue;
@@ -815,7 +833,7 @@ int sync_state(mhd_ctx *ctx)
     {
         // both groups' rings in one launch
         StepSync *s = nullptr;
-        RUN(step_sync(ctx, {"Ucell", "Bface"}, 0, &s));
+        RUN(step_sync(ctx, {"Ucell", "Bface"}, SYNC_HOT, &s));
         if (s->usable)
         {
             RUN(launch_pole(ctx, {POLE_RING_U, POLE_RING_BXI}));
@@ -959,14 +977,14 @@ int dots(mhd_ctx *ctx, const double *V, int nvec, const int *jdev, const double 
     do                                                            \
     {                                                             \
         prof_begin(ctx, #name);                                   \
-        name<<<1, 1, 0, ctx->stream>>>(__VA_ARGS__);              \
+        pdl_launch(name, dim3(1), 1, 0, ctx->stream, __VA_ARGS__); \
         RUN(launched(ctx));                                       \
     } while (0)
 #define LAUNCHN(name, n, ...)                                     \
     do                                                            \
     {                                                             \
         prof_begin(ctx, #name);                                   \
-        name<<<grid_for(n), kThreads, 0, ctx->stream>>>(__VA_ARGS__); \
+        pdl_launch(name, dim3(grid_for(n)), kThreads, 0, ctx->stream, __VA_ARGS__); \
         RUN(launched(ctx));                                       \
     } while (0)
 
@@ -1212,7 +1230,7 @@ int launch_gmres_persistent(mhd_ctx *ctx)
 int launch_resistive(mhd_ctx *ctx)
 {
     auto &R = ctx->res;
-    RUN(run_sync(ctx, "Bface"));
+    RUN(run_syncs(ctx, {"Bface"}));
     RUN(launch_jedge_rng(ctx, F_Bxi, F_Jxi));
     if (R.n > 0 && R.pgrid > 0)
         RUN(launch_gmres_persistent(ctx));
@@ -1343,7 +1361,7 @@ int hall_cond(mhd_ctx *ctx, cudaGraphConditionalNodeType type, cudaGraphConditio
     do                                                                       \
     {                                                                        \
         prof_begin(ctx, #name);                                              \
-        name<<<ctx->hall.ngroups, 256, 0, ctx->stream>>>(__VA_ARGS__);       \
+        pdl_launch(name, dim3(unsigned(ctx->hall.ngroups)), 256, 0, ctx->stream, __VA_ARGS__); \
         RUN(launched(ctx));                                                  \
     } while (0)
 
@@ -1362,41 +1380,51 @@ int hall_copy_b(mhd_ctx *ctx, bool snapshot)
     return launched(ctx);
 }
 
-// UpdateMagneticDerivedFields_ with the B_cell / J_cell ghosts the Hall
-// stencils read, then the Hall edge EMF.  B_cell and the J edges in one pass
+// UpdateMagneticDerivedFields_ with the B_cell / J_cell ghost layer the Hall
+// stencils read (the deeper ones once, after the solve; Bind_cell by the
+// derived pass of the step's end), then the Hall edge EMF.  B_cell and the J edges in one pass
 // (both read only the face B; the B_cell sync between them in the reference
 // touches neither input).
 int hall_emf_from_current_b(mhd_ctx *ctx)
 {
     cudaStream_t s = ctx->stream;
     prof_begin(ctx, "k_bcell_jedge");
-    RUN(launched(ctx, launch_k_bcell_jedge(ctx->tune[TUNE_k_bcell_jedge], false, ctx->hot, s)));
-    RUN(run_sync(ctx, "B_cell", true));
-    RUN(run_sync(ctx, "Jedge"));
+    RUN(launched(ctx, launch_k_bcell_jedge(ctx->tune[TUNE_k_bcell_jedge], false, ctx->hot, s, false)));
+    RUN(run_syncs(ctx, {"B_cell", "Jedge"}, true, SYNC_HALL));
     prof_begin(ctx, "k_jcell");
     RUN(launched(ctx, launch_k_jcell(false, ctx->hot, s)));
-    RUN(run_sync(ctx, "J_cell", true));
+    RUN(run_syncs(ctx, {"J_cell"}, true, SYNC_HALL));
     prof_begin(ctx, "k_hall_cell");
-    RUN(launched(ctx, launch_k_hall_cell(ctx->hot, s, ctx->c, ctx->hall_coef)));
+    RUN(launched(ctx, launch_k_hall_cell(ctx->hot, s, ctx->c, ctx->hall_coef, false)));
     prof_begin(ctx, "k_hall_edge");
     return launched(ctx, launch_k_hall_edge(ctx->tune[TUNE_k_hall_edge], ctx->hot, s, ctx->hall_zb, ctx->hall_nzb));
 }
 
-// the trial B of the Ehall unknowns in the pool (UnpackVecToEhallField_:
-// owners already written, then their aliases), Sync("Ehall"), B = B* + dt
-// (-curl Ehall) on inner faces (theta = 1), Sync("Bface")
+// The trial Ehall = X + (*a) v in the pool (a null: X): its unknowns, their
+// aliases and Sync("Ehall") (UnpackVecToEhallField_), the vector kept in Xt
+// (may be null); jd: v is column *jd of v0
+int hall_trial(mhd_ctx *ctx, const double *a, const double *v0, int64_t ldv, const int *jd, double *Xt)
+{
+    auto &H = ctx->hall;
+    const HallList l = H.fused ? H.list : HallList{};
+    LAUNCHN(k_hall_trial, H.n + l.n1 + l.n2 + l.n3, ctx->pool, H.e, H.X, a, v0, ldv, jd, Xt, H.n, l);
+    if (H.fused)
+        return MHD_OK;
+    if (H.nalias > 0)
+        LAUNCHN(k_alias_copy, H.nalias, ctx->pool, H.alias, H.owner, H.sign, H.nalias);
+    return run_sync(ctx, "Ehall", true);
+}
+
+// B = B* + dt (-curl Ehall) on inner faces (theta = 1), Sync("Bface")
 int hall_trial_b(mhd_ctx *ctx)
 {
     auto &H = ctx->hall;
     if (!H.from_snapshot)
         RUN(hall_copy_b(ctx, false));
-    if (H.nalias > 0)
-        LAUNCHN(k_alias_copy, H.nalias, ctx->pool, H.alias, H.owner, H.sign, H.nalias);
-    RUN(run_sync(ctx, "Ehall", true));
     prof_begin(ctx, "k_curl_e2f");
     RUN(launched(ctx, launch_k_curl_e2f(ctx->tune[TUNE_k_curl_e2f], ctx->hot, ctx->stream, F_Ehxi, F_RBxi, F_Bxi, -1.0,
                                         ctx->dt, 1.0, 0, nullptr, 0, H.from_snapshot ? H.bs : nullptr)));
-    return run_sync(ctx, "Bface");
+    return run_syncs(ctx, {"Bface"});
 }
 
 // FormFunction_ up to the predicted Hall EMF of the trial in the pool
@@ -1413,14 +1441,12 @@ int hall_arnoldi(mhd_ctx *ctx, cudaGraphConditionalHandle hin)
 {
     auto &H = ctx->hall;
     const int *jd = &H.st->j;
-    LAUNCHN(k_hall_trial, H.n, ctx->pool, H.e, H.X, &H.ctl->h, H.V, H.n, jd, H.Xt, H.n);
+    RUN(hall_trial(ctx, &H.ctl->h, H.V, H.n, jd, H.Xt));
     RUN(hall_chain(ctx));
     HALL_RED(k_hall_jv_dots, ctx->pool, H.e, H.Xt, H.F, &H.ctl->h, H.w, H.V, H.n, H.st, H.n, H.partial, H.st->hcol,
              H.done);
-    HALL_RED(k_hall_proj_dots, H.V, H.n, H.st, H.w, H.n, H.partial, H.dots, H.done);
-    LAUNCH1(k_hall_column, H.st, H.dots);
+    HALL_RED(k_hall_proj_dots, H.V, H.n, H.st, H.w, H.n, H.partial, H.dots, H.done, hin, hall_use(ctx));
     LAUNCHN(k_hall_next, H.n, H.V, H.n, H.w, H.st, H.dots, H.n);
-    LAUNCH1(k_inner_check, H.st, hin, hall_use(ctx));
     return MHD_OK;
 }
 
@@ -1428,7 +1454,7 @@ int hall_arnoldi(mhd_ctx *ctx, cudaGraphConditionalHandle hin)
 int hall_restart_product(mhd_ctx *ctx, cudaGraphConditionalHandle)
 {
     auto &H = ctx->hall;
-    LAUNCHN(k_hall_trial, H.n, ctx->pool, H.e, H.X, &H.ctl->hdx, H.dx, 0, nullptr, H.Xt, H.n);
+    RUN(hall_trial(ctx, &H.ctl->hdx, H.dx, 0, nullptr, H.Xt));
     RUN(hall_chain(ctx));
     LAUNCHN(k_hall_restart_r, H.n, ctx->pool, H.e, H.Xt, H.F, &H.ctl->hdx, H.b, H.r, H.n);
     return MHD_OK;
@@ -1462,7 +1488,7 @@ int hall_cycle(mhd_ctx *ctx, cudaGraphConditionalHandle hout)
 int hall_ls_trial(mhd_ctx *ctx, cudaGraphConditionalHandle hls)
 {
     auto &H = ctx->hall;
-    LAUNCHN(k_hall_trial, H.n, ctx->pool, H.e, H.X, &H.ctl->lambda, H.dx, 0, nullptr, H.Xt, H.n);
+    RUN(hall_trial(ctx, &H.ctl->lambda, H.dx, 0, nullptr, H.Xt));
     RUN(hall_chain(ctx));
     HALL_RED(k_hall_res_dots, ctx->pool, H.e, H.Xt, H.Ft, H.n, H.partial, H.dots + 48, H.done);
     LAUNCH1(k_hall_ls_check, H.ctl, H.dots + 48, hls, hall_use(ctx));
@@ -1508,7 +1534,8 @@ int launch_hall_implicit(mhd_ctx *ctx)
     }
     RUN(hall_copy_b(ctx, true));
     LAUNCHN(k_pack_vec, H.n, ctx->pool, H.e, H.X, H.n);
-    // F of the initial guess (the unknowns in the pool are X already)
+    // F of the initial guess
+    RUN(hall_trial(ctx, nullptr, nullptr, 0, nullptr, nullptr));
     RUN(hall_chain(ctx));
     HALL_RED(k_hall_res_dots, ctx->pool, H.e, H.X, H.F, H.n, H.partial, H.dots + 60, H.done);
     cudaGraphConditionalHandle hn;
@@ -1523,8 +1550,15 @@ int launch_hall_implicit(mhd_ctx *ctx)
         H.kb_nested = H.kb[HALL_KB_NEWTON];
         H.kb[HALL_KB_NEWTON] -= (H.kb[HALL_KB_CYCLE] + H.kb[HALL_KB_INNER] + H.kb[HALL_KB_RESTART]) + H.kb[HALL_KB_LS];
     }
-    // the final update with the converged Hall EMF
-    LAUNCHN(k_hall_trial, H.n, ctx->pool, H.e, H.X, nullptr, nullptr, 0, nullptr, nullptr, H.n);
+    // the ghost layers beyond the first of B_cell, J_cell and the Hall cell
+    // EMF, as the last residual leaves them
+    RUN(run_syncs(ctx, {"B_cell", "J_cell"}, true, SYNC_FULL));
+    prof_begin(ctx, "k_hall_cell");
+    RUN(launched(ctx, launch_k_hall_cell(ctx->hot, ctx->stream, ctx->c, ctx->hall_coef, true)));
+    // the final update with the converged Hall EMF, every ghost edge written
+    RUN(hall_trial(ctx, nullptr, nullptr, 0, nullptr, nullptr));
+    if (H.fused)
+        RUN(run_sync(ctx, "Ehall", true));
     return hall_trial_b(ctx);
 }
 
@@ -2599,7 +2633,8 @@ int build_sync(mhd_ctx *ctx, const std::string &group, SyncMap &m)
     std::vector<uint64_t> d, s2, cd;
     std::vector<double> cv;
     free_step_syncs(ctx);
-    m.res_full = Resolved();
+    if (group == "Ehall")
+        ctx->hall.list_built = false;
     if (!ctx->poles.empty())
         return build_sync_pole(ctx, group, m, dec);
     const HotPoints hot_at_point(ctx, dec);
@@ -2635,12 +2670,46 @@ int build_sync(mhd_ctx *ctx, const std::string &group, SyncMap &m)
     return MHD_OK;
 }
 
-// The passes of consecutive groups' Syncs (built on first use; full: bit q for
-// the full list of group q).  Groups go together when they touch different
-// fields; a group that cannot be resolved makes the whole entry unusable.
-static int step_sync(mhd_ctx *ctx, std::initializer_list<const char *> groups, unsigned full, StepSync **out)
+// the lists of a part of a group other than its hot one (no Poles)
+static void resolve_part(const mhd_ctx *ctx, const SyncMap &m, SyncPart part, Resolved &r)
 {
-    std::string key = std::to_string(full);
+    const PoolDecoder dec(ctx);
+    if (part == SYNC_FULL)
+    {
+        resolve_lists(ctx, m, dec, m.hd, m.hs, m.hcd, m.hcv, r);
+        return;
+    }
+    HotPoints near(ctx, dec);
+    near.depth[F_Bcell] = near.depth[F_Jcell] = 1;
+    near.depth[F_Bind] = -(1 << 20);
+    OffsetSet consts(m.hcd); // marked: the source of a copy
+    std::vector<uint64_t> d, s, cd;
+    std::vector<double> cv;
+    int f;
+    for (size_t t = 0; t < m.hd.size(); ++t)
+        if (near(m.hd[t], f))
+        {
+            d.push_back(m.hd[t]);
+            s.push_back(m.hs[t]);
+            const int64_t c = consts.find(m.hs[t]);
+            if (c >= 0)
+                consts.mark[size_t(c)] = 1;
+        }
+    for (size_t t = 0; t < m.hcd.size(); ++t)
+        if (near(m.hcd[t], f) || consts.mark[size_t(consts.find(m.hcd[t]))])
+        {
+            cd.push_back(m.hcd[t]);
+            cv.push_back(m.hcv[t]);
+        }
+    resolve_lists(ctx, m, dec, d, s, cd, cv, r);
+}
+
+// The passes of consecutive groups' Syncs, built on first use.  Groups go
+// together when they touch different fields; a group that cannot be resolved
+// makes the whole entry unusable.
+static int step_sync(mhd_ctx *ctx, std::initializer_list<const char *> groups, SyncPart part, StepSync **out)
+{
+    std::string key = std::to_string(int(part));
     for (const char *g : groups)
         key += std::string("+") + g;
     for (const char *g : groups)
@@ -2661,25 +2730,23 @@ static int step_sync(mhd_ctx *ctx, std::initializer_list<const char *> groups, u
         Resolved all;
         std::bitset<NFIELD> seen;
         s.usable = true;
-        unsigned q = 0;
         for (const char *g : groups)
         {
-            const bool f = ((full >> q++) & 1) != 0;
             const auto it = ctx->syncs.find(g);
             if (it == ctx->syncs.end())
                 continue;
-            SyncMap &m = it->second;
-            if (f && !m.res_full.usable)
-                resolve_lists(ctx, m, PoolDecoder(ctx), m.hd, m.hs, m.hcd, m.hcv, m.res_full);
-            const Resolved &r = f ? m.res_full : m.res;
+            Resolved own;
+            if (part != SYNC_HOT)
+                resolve_part(ctx, it->second, part, own);
+            const Resolved &r = part != SYNC_HOT ? own : it->second.res;
             s.usable = s.usable && r.usable && (seen & r.fields).none();
             if (!s.usable)
                 break;
             seen |= r.fields;
-            for (auto part : {&Resolved::a, &Resolved::b})
+            for (auto piece : {&Resolved::a, &Resolved::b})
             {
-                Resolved::Part &t = all.*part;
-                const Resolved::Part &x = r.*part;
+                Resolved::Part &t = all.*piece;
+                const Resolved::Part &x = r.*piece;
                 t.d.insert(t.d.end(), x.d.begin(), x.d.end());
                 t.s.insert(t.s.end(), x.s.begin(), x.s.end());
                 t.cd.insert(t.cd.end(), x.cd.begin(), x.cd.end());
@@ -2697,6 +2764,147 @@ static int step_sync(mhd_ctx *ctx, std::initializer_list<const char *> groups, u
     return MHD_OK;
 }
 
+static void free_hall_list(mhd_ctx *ctx)
+{
+    HallList &l = ctx->hall.list;
+    for (const void *p : {(const void *)l.d1, (const void *)l.idx, (const void *)l.sign, (const void *)l.d2,
+                          (const void *)l.s2, (const void *)l.d3, (const void *)l.val})
+        cudaFree(const_cast<void *>(p));
+    l = HallList{};
+    ctx->hall.fused = ctx->hall.list_built = false;
+}
+
+// What a trial writes beside its unknowns, in the order of the passes it
+// replaces (aliases, then Sync("Ehall")'s fixed values, then its copies; the
+// inner edges only, as deep as the curl reads): each point's value as an
+// expression of the unknowns, a fixed value or a point no trial writes.  Not
+// fused (the passes run one by one) when Sync("Ehall") is staged or has wall
+// handlers, an alias's owner is no unknown, or one of the three writes an
+// unknown's point.
+static int build_hall_list(mhd_ctx *ctx)
+{
+    auto &H = ctx->hall;
+    if (H.list_built)
+        return MHD_OK;
+    free_hall_list(ctx);
+    H.list_built = true;
+    const auto it = ctx->syncs.find("Ehall");
+    if (it == ctx->syncs.end() || it->second.staged || !it->second.walls.empty() || !ctx->poles.empty())
+        return MHD_OK;
+    const SyncMap &m = it->second;
+    const PoolDecoder dec(ctx);
+    HotPoints inner(ctx, dec);
+    for (int &d : inner.depth)
+        d = 0;
+    struct Expr
+    {
+        uint64_t off;
+        int64_t idx; // >= 0: sign * unknown; -1: the fixed value `sign`
+        double sign;
+    };
+    std::vector<Expr> known;
+    auto sorted = [&]() {
+        std::stable_sort(known.begin(), known.end(), [](const Expr &x, const Expr &y) { return x.off < y.off; });
+    };
+    auto find = [&](uint64_t off) -> const Expr * {
+        const auto p = std::lower_bound(known.begin(), known.end(), off,
+                                        [](const Expr &x, uint64_t o) { return x.off < o; });
+        return p != known.end() && p->off == off ? &*p : nullptr;
+    };
+    for (size_t t = 0; t < H.he.size(); ++t)
+        known.push_back({H.he[t], int64_t(t), 1.0});
+    sorted();
+    std::vector<Expr> points; // written beside the unknowns before the copies
+    for (size_t q = 0; q < H.ha.size(); ++q)
+    {
+        const Expr *o = find(H.ho[q]);
+        if (!o || find(H.ha[q]))
+            return MHD_OK;
+        points.push_back({H.ha[q], o->idx, H.hs[q]});
+    }
+    const OffsetSet consts(m.hcd), alias(H.ha);
+    for (size_t q = 0; q < m.hcd.size(); ++q)
+        if (find(m.hcd[q]))
+            return MHD_OK;
+    points.erase(std::remove_if(points.begin(), points.end(), [&](const Expr &x) { return consts.has(x.off); }),
+                 points.end());
+    std::vector<Expr> fixed;
+    for (size_t q = 0; q < m.hcd.size(); ++q)
+        fixed.push_back({m.hcd[q], -1, m.hcv[q]});
+    for (const Expr &x : points)
+        known.push_back(x);
+    for (const Expr &x : fixed)
+        known.push_back(x);
+    sorted();
+    std::vector<uint64_t> d1, d2, s2, d3;
+    std::vector<int64_t> idx;
+    std::vector<double> sign, val;
+    int f;
+    std::vector<uint64_t> copied;
+    for (size_t t = 0; t < m.hd.size(); ++t)
+    {
+        if (!inner(m.hd[t], f))
+            continue;
+        const Expr *at = find(m.hd[t]), *from = find(m.hs[t]);
+        if (at && at->idx >= 0 && !alias.has(m.hd[t]))
+            return MHD_OK; // an unknown's own point
+        copied.push_back(m.hd[t]);
+        if (!from)
+        {
+            d2.push_back(m.hd[t]);
+            s2.push_back(m.hs[t]);
+        }
+        else if (from->idx >= 0)
+        {
+            d1.push_back(m.hd[t]);
+            idx.push_back(from->idx);
+            sign.push_back(from->sign);
+        }
+        else
+        {
+            d3.push_back(m.hd[t]);
+            val.push_back(from->sign);
+        }
+    }
+    const OffsetSet over(std::move(copied));
+    for (const Expr &x : points)
+        if (!over.has(x.off))
+        {
+            d1.push_back(x.off);
+            idx.push_back(x.idx);
+            sign.push_back(x.sign);
+        }
+    for (const Expr &x : fixed)
+        if (!over.has(x.off) && inner(x.off, f))
+        {
+            d3.push_back(x.off);
+            val.push_back(x.sign);
+        }
+    HallList &l = H.list;
+    uint64_t *u = nullptr;
+    int64_t *iv = nullptr;
+    double *dv = nullptr;
+    RUN(upload_vec(ctx, d1, &u));
+    l.d1 = u;
+    RUN(upload_vec(ctx, idx, &iv));
+    l.idx = iv;
+    RUN(upload_vec(ctx, sign, &dv));
+    l.sign = dv;
+    RUN(upload_vec(ctx, d2, &u));
+    l.d2 = u;
+    RUN(upload_vec(ctx, s2, &u));
+    l.s2 = u;
+    RUN(upload_vec(ctx, d3, &u));
+    l.d3 = u;
+    RUN(upload_vec(ctx, val, &dv));
+    l.val = dv;
+    l.n1 = int64_t(d1.size());
+    l.n2 = int64_t(d2.size());
+    l.n3 = int64_t(d3.size());
+    H.fused = true;
+    return MHD_OK;
+}
+
 // every group's lists and the passes of the step (before a capture)
 static int build_all_syncs(mhd_ctx *ctx)
 {
@@ -2704,20 +2912,29 @@ static int build_all_syncs(mhd_ctx *ctx)
         if (!kv.second.built)
             RUN(build_sync(ctx, kv.first, kv.second));
     StepSync *s = nullptr;
-    RUN(step_sync(ctx, {"Eface"}, 0, &s));
-    RUN(step_sync(ctx, {"Eedge"}, 0, &s));
-    RUN(step_sync(ctx, {"Ucell", "Bface"}, 0, &s));
-    RUN(step_sync(ctx, {"J_cell", "Uplus"}, 0, &s));
+    RUN(step_sync(ctx, {"Eface"}, SYNC_HOT, &s));
+    RUN(step_sync(ctx, {"Eedge"}, SYNC_HOT, &s));
+    RUN(step_sync(ctx, {"Ucell", "Bface"}, SYNC_HOT, &s));
+    RUN(step_sync(ctx, {"J_cell", "Uplus"}, SYNC_HOT, &s));
     if (ctx->poles.empty())
-        RUN(step_sync(ctx, {"B_cell", "Jedge"}, 0, &s));
+        RUN(step_sync(ctx, {"B_cell", "Jedge"}, SYNC_HOT, &s));
     if (!ctx->poles.empty() || ctx->res_nsub > 0)
     {
-        RUN(step_sync(ctx, {"B_cell"}, 0, &s));
-        RUN(step_sync(ctx, {"Jedge"}, 0, &s));
+        RUN(step_sync(ctx, {"B_cell"}, SYNC_HOT, &s));
+        RUN(step_sync(ctx, {"Jedge"}, SYNC_HOT, &s));
     }
+    if (ctx->res_nsub > 0 || ctx->res.on || ctx->hall.on)
+        RUN(step_sync(ctx, {"Bface"}, SYNC_HOT, &s));
     if (ctx->res_nsub > 0)
-        for (const char *g : {"Bface", "J_cell", "Eres"})
-            RUN(step_sync(ctx, {g}, 0, &s));
+        for (const char *g : {"J_cell", "Eres"})
+            RUN(step_sync(ctx, {g}, SYNC_HOT, &s));
+    if (ctx->hall.on)
+    {
+        RUN(step_sync(ctx, {"J_cell"}, SYNC_HALL, &s));
+        RUN(step_sync(ctx, {"B_cell", "Jedge"}, SYNC_HALL, &s));
+        RUN(step_sync(ctx, {"B_cell", "J_cell"}, SYNC_FULL, &s));
+        RUN(build_hall_list(ctx));
+    }
     return MHD_OK;
 }
 
@@ -3476,6 +3693,7 @@ int mhd_set_hall_implicit(mhd_ctx *ctx, int64_t n, const int64_t *unknowns, int6
                     (void *)H.w, (void *)H.partial, (void *)H.dots, (void *)H.st, (void *)H.ctl, (void *)H.done,
                     (void *)H.seg_snap, (void *)H.seg_restore, (void *)H.bs})
         cudaFree(p);
+    free_hall_list(ctx);
     H = mhd_ctx::HallImplicit();
     drop_graph(ctx);
     if (n == 0)
@@ -3499,8 +3717,11 @@ int mhd_set_hall_implicit(mhd_ctx *ctx, int64_t n, const int64_t *unknowns, int6
     RUN(upload_vec(ctx, he, &H.e));
     RUN(upload_vec(ctx, ha, &H.alias));
     RUN(upload_vec(ctx, ho, &H.owner));
-    std::vector<double> hs(sign, sign + nalias);
-    RUN(upload_vec(ctx, hs, &H.sign));
+    H.hs.assign(sign, sign + nalias);
+    RUN(upload_vec(ctx, H.hs, &H.sign));
+    H.he = he;
+    H.ha = ha;
+    H.ho = ho;
     H.n = n;
     H.nalias = nalias;
     H.rtol = rtol;
@@ -4055,7 +4276,7 @@ int mhd_stage(mhd_ctx *ctx, int32_t stage_id)
         RUN(materialise_group(ctx, "B_cell"));
         RUN(materialise_group(ctx, "J_cell"));
         prof_begin(ctx, "k_hall_cell");
-        RUN(launched(ctx, launch_k_hall_cell(ctx->hot, ctx->stream, ctx->c, ctx->hall_coef)));
+        RUN(launched(ctx, launch_k_hall_cell(ctx->hot, ctx->stream, ctx->c, ctx->hall_coef, true)));
         prof_begin(ctx, "k_hall_edge");
         RUN(launched(ctx, launch_k_hall_edge(ctx->tune[TUNE_k_hall_edge], ctx->hot, ctx->stream, ctx->hall_zb,
                                              ctx->hall_nzb)));

@@ -187,6 +187,70 @@ __device__ __forceinline__ float *hot_plane32(const HotBlock &b, uint32_t p, int
     return b.p32 + (uint64_t(b.vol) * uint32_t(q) + p);
 }
 
+// L2 prefetch of what a later CTA of the launch reads: the CTA kAhead CTAs on
+// (x fastest, then y), its points' range of each listed plane, one bulk
+// prefetch per plane by one lane.  planes: pool planes, or ~q for plane q of
+// the FP32 range.  For the flux passes, whose 80 to 124 registers leave 16 to
+// 24 warps per SM to hide DRAM latency: FP64 84 -> 71 us on 0.76 M cells, mixed
+// 221 -> 199 us on 2.27 M.  37 to 148 CTAs ahead are the same, 296 and more
+// slower.  The passes with more warps or a weight stream got slower (PV 96 ->
+// 110 us, B_cell 50 -> 52) and do not use it.
+constexpr uint32_t kAhead = 74;
+template <int KIND, int N, class A>
+__device__ __forceinline__ void hot_prefetch(const A &a, const int16_t (&planes)[N])
+{
+    static_assert(N <= 32, "one warp");
+    if (threadIdx.x >= N)
+        return;
+    uint32_t cta = blockIdx.x + kAhead;
+    int bi = int(blockIdx.y);
+    if (a.flat)
+    {
+        if (cta >= gridDim.x)
+            return;
+        int lo = 0, hi = a.n;
+        while (hi - lo > 1)
+        {
+            const int mid = (lo + hi) >> 1;
+            if (uint32_t(a.v[mid].cta0[KIND]) <= cta)
+                lo = mid;
+            else
+                hi = mid;
+        }
+        bi = lo;
+        cta -= uint32_t(a.v[lo].cta0[KIND]);
+    }
+    else if (cta >= gridDim.x)
+    {
+        cta -= gridDim.x;
+        if (++bi >= a.n || cta >= gridDim.x)
+            return;
+    }
+    const HotBlock &b = a.v[bi];
+    int i, j, k;
+    uint32_t p0, p1;
+    if (!hot_point<KIND>(b, cta * blockDim.x, i, j, k, p0))
+        return;
+    if (!hot_point<KIND>(b, cta * blockDim.x + blockDim.x - 1, i, j, k, p1))
+        p1 = p0 + blockDim.x < b.vol ? p0 + blockDim.x : b.vol - 1;
+    const int q = planes[threadIdx.x];
+    const char *at;
+    uint32_t bytes;
+    if (q >= 0)
+    {
+        p0 &= ~1u;
+        at = reinterpret_cast<const char *>(b.p0 + (uint64_t(b.vol) * uint32_t(q) + p0));
+        bytes = (p1 - p0 + 2) / 2 * 16;
+    }
+    else
+    {
+        p0 &= ~3u;
+        at = reinterpret_cast<const char *>(b.p32 + (uint64_t(b.vol) * uint32_t(~q) + p0));
+        bytes = (p1 - p0 + 4) / 4 * 16;
+    }
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(at), "r"(bytes) : "memory");
+}
+
 // inner cell
 __device__ __forceinline__ bool hot_inner(const HotBlock &b, int i, int j, int k)
 {

@@ -258,18 +258,32 @@ __global__ void k_hall_cycle_prep(HallCtl *c, const double *dx2, cudaGraphCondit
 __global__ void k_hall_ls_begin(HallCtl *c, cudaGraphConditionalHandle h, int use);
 __global__ void k_hall_ls_check(HallCtl *c, const double *ft2, cudaGraphConditionalHandle h, int use);
 __global__ void k_hall_accept(HallCtl *c, cudaGraphConditionalHandle h, int use);
-__global__ void k_hall_column(GmresState *st, const double *d);
+// what the points beside the unknowns take at a trial: n1 times sign x
+// unknown idx, n2 copies of points no trial writes, n3 fixed values
+struct HallList
+{
+    const uint64_t *d1;
+    const int64_t *idx;
+    const double *sign;
+    int64_t n1;
+    const uint64_t *d2, *s2;
+    int64_t n2;
+    const uint64_t *d3;
+    const double *val;
+    int64_t n3;
+};
 // Xt = X + (*a) v (v = v0 + (*jdev) ldv; Xt = X when a is null), written into the pool's unknowns
 __global__ void k_hall_trial(double *pool, const uint64_t *e, const double *X, const double *a, const double *v0,
-                             int64_t ldv, const int *jdev, double *Xt, int64_t n);
+                             int64_t ldv, const int *jdev, double *Xt, int64_t n, HallList l);
 // w = ((Xt - pool[e]) - F) / *h and out[c] = V_c . w for c <= j
 __global__ void k_hall_jv_dots(const double *pool, const uint64_t *e, const double *Xt, const double *F,
                                const double *h, double *w, const double *V, int64_t ldv, const GmresState *st,
                                int64_t n, double *partial, double *out, unsigned *done);
-// w -= sum_c hcol[c] V_c; out[c] = V_c . w (c <= j), out[j + 1] = w . w
-__global__ void k_hall_proj_dots(const double *V, int64_t ldv, const GmresState *st, double *w, int64_t n,
-                                 double *partial, double *out, unsigned *done);
-// V_{j+1} = (w - sum_c d[c] V_c) / hcol[j + 1]
+// w -= sum_c hcol[c] V_c; out[c] = V_c . w (c <= j), out[j + 1] = w . w; then,
+// in the last CTA, the Hessenberg column, the counters and the loop condition
+__global__ void k_hall_proj_dots(const double *V, int64_t ldv, GmresState *st, double *w, int64_t n, double *partial,
+                                 double *out, unsigned *done, cudaGraphConditionalHandle h, int use);
+// V_{j+1} = (w - sum_c d[c] V_c) / hcol[j + 1], j the column just counted
 __global__ void k_hall_next(double *V, int64_t ldv, const double *w, const GmresState *st, const double *d,
                             int64_t n);
 // Ft = Xt - pool[e]; out[0] = Ft . Ft
@@ -304,7 +318,8 @@ int launch_k_pv_all(const HotGrid &h, cudaStream_t st, Consts c);
 // (rc: the start of the step's run clocks, in the same launch)
 int launch_k_fluid_ucontra(int variant, const HotGrid &h, cudaStream_t st, Consts c, RunClock rc);
 // B_cell with the J edges: minimum CTAs per SM 2, 6; w32 as above
-int launch_k_bcell_jedge(int variant, bool w32, const HotGrid &h, cudaStream_t st);
+// (ind = false: without Bind_cell, FP64 weights; the Hall solve's trials)
+int launch_k_bcell_jedge(int variant, bool w32, const HotGrid &h, cudaStream_t st, bool ind = true);
 // B_cell alone, the J edges of (fB0, fJ0) alone (rng: per block a region box
 // lo[3], hi[3] of at most nreg points; null: every inner edge), J_cell alone
 int launch_k_bcell(const HotGrid &h, cudaStream_t st);
@@ -326,7 +341,8 @@ int launch_k_curl_e2f(int variant, const HotGrid &h, cudaStream_t st, int fE0, i
 int launch_k_update(int variant, const HotGrid &h, cudaStream_t st, int fR0, const double *dtp, RunClock rc);
 int launch_k_rk2(const HotGrid &h, cudaStream_t st, int save);
 int launch_k_eres_explicit(const HotGrid &h, cudaStream_t st, double inver_Rem);
-int launch_k_hall_cell(const HotGrid &h, cudaStream_t st, Consts c, double hall_coef);
+// Hall cell EMF on every ghost layer, or (all = false) one, as deep as the edge EMF reads
+int launch_k_hall_cell(const HotGrid &h, cudaStream_t st, Consts c, double hall_coef, bool all);
 // Hall edge EMF (zb: boxes of zeroed edges): minimum CTAs per SM 4, 2
 int launch_k_hall_edge(int variant, const HotGrid &h, cudaStream_t st, const int *zb, int nzb);
 // k_fluid_mixed: minimum CTAs per SM 3, 1, 2; variants 3 and 4 are the

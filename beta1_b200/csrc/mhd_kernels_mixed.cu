@@ -158,12 +158,26 @@ struct QHot
     __device__ __forceinline__ float operator()(int plane, int64_t c) const { return q[plane * v + c]; }
 };
 
+// planes of the L2 prefetch (hot_prefetch)
+__constant__ int16_t kPfMixed[] = {
+    int16_t(~(kPlane32Q + 0)), int16_t(~(kPlane32Q + 1)), int16_t(~(kPlane32Q + 2)), int16_t(~(kPlane32Q + 3)),
+    int16_t(~(kPlane32Q + 4)), int16_t(~(kPlane32Q + 5)), int16_t(~(kPlane32Q + 6)), int16_t(~(G32_AREA + 0)),
+    int16_t(~(G32_AREA + 1)), int16_t(~(G32_AREA + 2)), int16_t(plane_of(F_JDxi) + 0), int16_t(plane_of(F_JDxi) + 1),
+    int16_t(plane_of(F_JDxi) + 2), int16_t(plane_of(F_JDeta) + 0), int16_t(plane_of(F_JDeta) + 1),
+    int16_t(plane_of(F_JDeta) + 2), int16_t(plane_of(F_JDzeta) + 0), int16_t(plane_of(F_JDzeta) + 1),
+    int16_t(plane_of(F_JDzeta) + 2), int16_t(plane_of(F_Jac)), int16_t(plane_of(F_Uplus) + 0),
+    int16_t(plane_of(F_Uplus) + 1), int16_t(plane_of(F_Uplus) + 2), int16_t(plane_of(F_U) + 0),
+    int16_t(plane_of(F_U) + 1), int16_t(plane_of(F_U) + 2), int16_t(plane_of(F_U) + 3), int16_t(plane_of(F_Jcell) + 0),
+    int16_t(plane_of(F_Jcell) + 1), int16_t(plane_of(F_Jcell) + 2), int16_t(plane_of(F_Bcell) + 0),
+    int16_t(plane_of(F_Bcell) + 1)};
+
 template <class A> __device__ __forceinline__ void k_fluid_mixed_body(const A &args, const Consts &c, const RunClock &rc)
 {
     uint32_t t, p;
     const HotBlock &b = hot_block<KIND_CELL1>(args, t);
     int i, j, k;
     const bool in_box = hot_point<KIND_CELL1>(b, t, i, j, k, p);
+    hot_prefetch<KIND_CELL1>(args, kPfMixed);
     pdl_wait();
     if (rc.dt_key && blockIdx.x == 0 && blockIdx.y == 0) // start of the step (see k_fluid_ucontra_t)
         for (int r = threadIdx.x; r < rc.nruns; r += blockDim.x)

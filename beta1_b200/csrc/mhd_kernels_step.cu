@@ -56,6 +56,10 @@ __device__ __forceinline__ void run_end(const RunClock &rc)
             end_run(rc, r);
 }
 
+
+// planes of the kernels' L2 prefetch (hot_prefetch)
+__constant__ int16_t kPfFlux[] = {int16_t(plane_of(F_U)), int16_t(plane_of(F_PV) + 0), int16_t(plane_of(F_PV) + 1), int16_t(plane_of(F_PV) + 2), int16_t(plane_of(F_PV) + 3), int16_t(plane_of(F_RhoE)), int16_t(plane_of(F_Cs)), int16_t(plane_of(F_JDxi) + 0), int16_t(plane_of(F_JDxi) + 1), int16_t(plane_of(F_JDxi) + 2), int16_t(plane_of(F_JDeta) + 0), int16_t(plane_of(F_JDeta) + 1), int16_t(plane_of(F_JDeta) + 2), int16_t(plane_of(F_JDzeta) + 0), int16_t(plane_of(F_JDzeta) + 1), int16_t(plane_of(F_JDzeta) + 2), int16_t(plane_of(F_NAxi)), int16_t(plane_of(F_NAeta)), int16_t(plane_of(F_NAzeta)), int16_t(plane_of(F_Jac)), int16_t(plane_of(F_Uplus) + 0), int16_t(plane_of(F_Uplus) + 1), int16_t(plane_of(F_Uplus) + 2), int16_t(plane_of(F_Jcell) + 0), int16_t(plane_of(F_Jcell) + 1), int16_t(plane_of(F_Jcell) + 2), int16_t(plane_of(F_Bcell) + 0), int16_t(plane_of(F_Bcell) + 1), int16_t(plane_of(F_Bcell) + 2)};
+
 // the strides of one axis
 __device__ __forceinline__ int hot_stride(const HotBlock &b, int a)
 {
@@ -130,6 +134,7 @@ template <class A> __device__ __forceinline__ void fluid_ucontra_body(const A &a
     const HotBlock &b = hot_block<KIND_CELL1>(a, t);
     int i, j, k;
     const bool in_box = hot_point<KIND_CELL1>(b, t, i, j, k, p);
+    hot_prefetch<KIND_CELL1>(a, kPfFlux);
     pdl_wait();
     run_begin(rc);
     if (!in_box)
@@ -528,8 +533,8 @@ template <> __device__ __forceinline__ const float *hot_weights<float>(const Hot
 
 // WT: double (the reference's weights, FP64 form) or float (their FP32
 // copies, mixed form: the products and sums stay FP64); EDGES: with the J
-// edges (else B_cell alone)
-template <typename WT, bool EDGES, class A> __device__ __forceinline__ void bcell_jedge_body(const A &a)
+// edges (else B_cell alone); IND: with Bind_cell
+template <typename WT, bool EDGES, bool IND, class A> __device__ __forceinline__ void bcell_jedge_body(const A &a)
 {
     constexpr int KIND = EDGES ? KIND_STAG : KIND_CELL0;
     uint32_t t, p;
@@ -588,14 +593,16 @@ template <typename WT, bool EDGES, class A> __device__ __forceinline__ void bcel
             {
                 const double w = double(W[(6 * c + q) * v]);
                 bt[c] += w * tot[q];
-                bi[c] += w * ind[q];
+                if (IND)
+                    bi[c] += w * ind[q];
             }
         double *Bc = hot_at(b, p, F_Bcell), *Bi = hot_at(b, p, F_Bind);
 #pragma unroll
         for (int c = 0; c < 3; ++c)
         {
             Bc[c * v] = bt[c];
-            Bi[c * v] = bi[c];
+            if (IND)
+                Bi[c * v] = bi[c];
         }
     }
     if (EDGES)
@@ -607,10 +614,10 @@ template <typename WT, bool EDGES, class A> __device__ __forceinline__ void bcel
     }
 }
 
-template <typename WT, bool EDGES, class A, int MINB>
+template <typename WT, bool EDGES, class A, int MINB, bool IND = true>
 __global__ void __launch_bounds__(kHotThreads, MINB) k_bcell_jedge_t(const __grid_constant__ A a)
 {
-    bcell_jedge_body<WT, EDGES>(a);
+    bcell_jedge_body<WT, EDGES, IND>(a);
 }
 
 // the J edges alone: planes qB of the face field, qJ of the edge field
@@ -989,21 +996,10 @@ __global__ void __launch_bounds__(kHotThreads) k_eres_explicit_t(const __grid_co
 // (Z4_Lunar/src/physics/LunarSolver_MagExplicit_Hall.cpp:8-457)
 // ---------------------------------------------------------------------------
 
-// Ehc = alpha (J x B) and beta = |alpha| |B| on every cell of the array, with
-// alpha = hall_coef / ne_eff (Hall_Num_Limiter); 2-D launch, one grid row per block
-template <class A>
-__global__ void __launch_bounds__(kHotThreads)
-    k_hall_cell_t(const __grid_constant__ A a, Consts c, double hall_coef, int G)
+// Ehc = alpha (J x B) and beta = |alpha| |B|, with alpha = hall_coef / ne_eff
+// (Hall_Num_Limiter)
+__device__ __forceinline__ void hall_cell_one(const HotBlock &b, uint32_t p, const Consts &c, double hall_coef)
 {
-    const HotBlock &b = a.v[blockIdx.y];
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t n2 = uint32_t(b.nk + 2 * G), n1 = uint32_t(b.nj + 2 * G);
-    const uint32_t q = t / n2, ii = q / n1;
-    pdl_wait();
-    if (ii >= uint32_t(b.ni + 2 * G))
-        return;
-    const int i = int(ii) - G, j = int(q - ii * n1) - G, k = int(t - q * n2) - G;
-    const uint32_t p = b.o + uint32_t(i) * b.si + uint32_t(j) * b.sj + uint32_t(k);
     const uint64_t v = b.vol;
     const double rho = *hot_at(b, p, F_U);
     const double *J = hot_at(b, p, F_Jcell), *B = hot_at(b, p, F_Bcell);
@@ -1019,15 +1015,70 @@ __global__ void __launch_bounds__(kHotThreads)
     *hot_at(b, p, F_HallBeta) = fabs(alpha) * sqrt(Bx * Bx + By * By + Bz * Bz);
 }
 
-// zero box test of the Hall edge EMF (Solid_Surface layers and Pole edges):
-// zb[8 q ..]: block, edge axis, lo[3], hi[3]
-__device__ __forceinline__ bool hall_zeroed(const int *__restrict__ zb, int nzb, int bi, int ea, int i, int j, int k)
+// every cell of the array; 2-D launch, one grid row per block
+template <class A>
+__global__ void __launch_bounds__(kHotThreads)
+    k_hall_cell_all_t(const __grid_constant__ A a, Consts c, double hall_coef, int G)
+{
+    const HotBlock &b = a.v[blockIdx.y];
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t n2 = uint32_t(b.nk + 2 * G), n1 = uint32_t(b.nj + 2 * G);
+    const uint32_t q = t / n2, ii = q / n1;
+    pdl_wait();
+    if (ii >= uint32_t(b.ni + 2 * G))
+        return;
+    const int i = int(ii) - G, j = int(q - ii * n1) - G, k = int(t - q * n2) - G;
+    hall_cell_one(b, b.o + uint32_t(i) * b.si + uint32_t(j) * b.sj + uint32_t(k), c, hall_coef);
+}
+
+// the cells within one ghost layer
+template <class A>
+__global__ void __launch_bounds__(kHotThreads) k_hall_cell_t(const __grid_constant__ A a, Consts c, double hall_coef)
+{
+    uint32_t t, p;
+    const HotBlock &b = hot_block<KIND_CELL1>(a, t);
+    int i, j, k;
+    const bool in_box = hot_point<KIND_CELL1>(b, t, i, j, k, p);
+    pdl_wait();
+    if (in_box)
+        hall_cell_one(b, p, c, hall_coef);
+}
+
+// Zero boxes of the Hall edge EMF (Solid_Surface layers and Pole edges): zb[8 q
+// ..]: block, edge axis, lo[3], hi[3].  The CTA keeps its block's boxes in
+// shared memory (a grid of B blocks has about 3 B, three of them a block's; read
+// per edge from global memory they took 60 % of the kernel).
+constexpr int kHallBoxes = 24;
+struct HallBoxes
+{
+    int n;               // this block's boxes; more than kHallBoxes: read zb instead
+    int b[kHallBoxes][7]; // axis, lo, hi
+};
+__device__ __forceinline__ void hall_boxes(HallBoxes &s, const int *zb, int nzb, int blk)
+{
+    if (threadIdx.x == 0)
+        s.n = 0;
+    __syncthreads();
+    for (int q = int(threadIdx.x); q < nzb; q += kHotThreads)
+        if (zb[8 * q] == blk)
+        {
+            const int at = atomicAdd(&s.n, 1);
+            if (at < kHallBoxes)
+                for (int e = 0; e < 7; ++e)
+                    s.b[at][e] = zb[8 * q + 1 + e];
+        }
+    __syncthreads();
+}
+__device__ __forceinline__ bool hall_zeroed(const HallBoxes &s, const int *zb, int nzb, int blk, int ea, int i, int j,
+                                            int k)
 {
     bool zero = false;
-    for (int q = 0; q < nzb && !zero; ++q)
+    const bool own = s.n <= kHallBoxes;
+    for (int q = 0; q < (own ? s.n : nzb) && !zero; ++q)
     {
-        const int *z = zb + 8 * q;
-        zero = (z[0] == bi && z[1] == ea && i >= z[2] && j >= z[3] && k >= z[4] && i < z[5] && j < z[6] && k < z[7]);
+        const int *z = own ? s.b[q] : zb + 8 * q + 1;
+        zero = (own || z[-1] == blk) && z[0] == ea && i >= z[1] && j >= z[2] && k >= z[3] && i < z[4] && j < z[5] &&
+               k < z[6];
     }
     return zero;
 }
@@ -1071,10 +1122,12 @@ template <class A, int MINB>
 __global__ void __launch_bounds__(kHotThreads, MINB)
     k_hall_edge_t(const __grid_constant__ A a, const int *__restrict__ zb, int nzb)
 {
+    __shared__ HallBoxes boxes;
     uint32_t t, p;
     const HotBlock &b = hot_block<KIND_STAG>(a, t);
     int i, j, k;
     const bool in_box = hot_point<KIND_STAG>(b, t, i, j, k, p);
+    hall_boxes(boxes, zb, nzb, b.blk);
     pdl_wait();
     if (!in_box)
         return;
@@ -1092,7 +1145,7 @@ __global__ void __launch_bounds__(kHotThreads, MINB)
     for (int ea = 0; ea < 3; ++ea)
     {
         in[ea] = hot_edge(b, ea, i, j, k);
-        if (!in[ea] || hall_zeroed(zb, nzb, b.blk, ea, i, j, k))
+        if (!in[ea] || hall_zeroed(boxes, zb, nzb, b.blk, ea, i, j, k))
             continue;
         const double *r = hot_at(b, p, F_drxi + ea);
         const double dr[3] = {r[0], r[v], r[2 * v]};
@@ -1166,14 +1219,16 @@ int launch_k_fluid_ucontra(int variant, const HotGrid &h, cudaStream_t st, Const
     });
 }
 
-int launch_k_bcell_jedge(int variant, bool w32, const HotGrid &h, cudaStream_t st)
+int launch_k_bcell_jedge(int variant, bool w32, const HotGrid &h, cudaStream_t st, bool ind)
 {
     if (variant < 0 || variant > 1)
         return -1;
     return hot_for(h, KIND_STAG, [&](const auto &a, dim3 g) {
         using A = std::decay_t<decltype(a)>;
         auto go = [&](auto kernel) { hot_launch(kernel, g, st, a); };
-        if (variant == 0)
+        if (!ind)
+            variant == 0 ? go(k_bcell_jedge_t<double, true, A, 2, false>) : go(k_bcell_jedge_t<double, true, A, 6, false>);
+        else if (variant == 0)
             w32 ? go(k_bcell_jedge_t<float, true, A, 2>) : go(k_bcell_jedge_t<double, true, A, 2>);
         else
             w32 ? go(k_bcell_jedge_t<float, true, A, 6>) : go(k_bcell_jedge_t<double, true, A, 6>);
@@ -1281,10 +1336,14 @@ int launch_k_eres_explicit(const HotGrid &h, cudaStream_t st, double inver_Rem)
     });
 }
 
-int launch_k_hall_cell(const HotGrid &h, cudaStream_t st, Consts c, double hall_coef)
+int launch_k_hall_cell(const HotGrid &h, cudaStream_t st, Consts c, double hall_coef, bool all)
 {
-    return hot_for_padded(h, [&](const auto &a, dim3 g) {
-        hot_launch(k_hall_cell_t<std::decay_t<decltype(a)>>, g, st, a, c, hall_coef, h.G);
+    if (all)
+        return hot_for_padded(h, [&](const auto &a, dim3 g) {
+            hot_launch(k_hall_cell_all_t<std::decay_t<decltype(a)>>, g, st, a, c, hall_coef, h.G);
+        });
+    return hot_for(h, KIND_CELL1, [&](const auto &a, dim3 g) {
+        hot_launch(k_hall_cell_t<std::decay_t<decltype(a)>>, g, st, a, c, hall_coef);
     });
 }
 

@@ -17,6 +17,7 @@
 // the host reads the two loop flags instead.  Kernels that work on "column
 // j" read j from the state.
 #include "mhd_kernels.cuh"
+#include "mhd_hot_launch.cuh"
 
 namespace mhd
 {
@@ -27,6 +28,7 @@ __global__ void k_dots(const double *__restrict__ V, int64_t ldv, int nvec, cons
                        double *__restrict__ partial, const int *__restrict__ jdev, double *__restrict__ out,
                        unsigned int *__restrict__ done)
 {
+    pdl_wait();
     const int c = blockIdx.y;
     const int nv = jdev ? jdev[0] + 1 : nvec;
     if (c >= nv)
@@ -77,6 +79,7 @@ __global__ void k_dots(const double *__restrict__ V, int64_t ldv, int nvec, cons
 __global__ void k_sub_proj(const double *__restrict__ V, int64_t ldv, int nvec, const double *__restrict__ h,
                            double *__restrict__ w, int64_t n, const int *__restrict__ jdev)
 {
+    pdl_wait();
     const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t >= n)
         return;
@@ -90,6 +93,7 @@ __global__ void k_sub_proj(const double *__restrict__ V, int64_t ldv, int nvec, 
 // a[c] += b[c] for c <= j
 __global__ void k_add_small(double *__restrict__ a, const double *__restrict__ b, const int *__restrict__ jdev)
 {
+    pdl_wait();
     const int c = threadIdx.x;
     if (c <= jdev[0])
         a[c] += b[c];
@@ -99,6 +103,7 @@ __global__ void k_add_small(double *__restrict__ a, const double *__restrict__ b
 __global__ void k_div_guard(double *__restrict__ y, const double *__restrict__ x, const double *__restrict__ a,
                             int64_t n, const int *__restrict__ guard)
 {
+    pdl_wait();
     if (guard && guard[0] == 0)
         return;
     const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -110,6 +115,7 @@ __global__ void k_div_guard(double *__restrict__ y, const double *__restrict__ x
 __global__ void k_div_next(double *__restrict__ V, int64_t ldv, const double *__restrict__ w,
                            const GmresState *__restrict__ st, int64_t n)
 {
+    pdl_wait();
     if (st->breakdown)
         return;
     const int j = st->j;
@@ -137,6 +143,7 @@ __device__ __forceinline__ void gmres_init_state(GmresState *st, const double *_
 
 __global__ void k_gmres_init(GmresState *st, const double *__restrict__ b2, double rtol, double atol, int maxit, int m)
 {
+    pdl_wait();
     gmres_init_state(st, b2, rtol, atol, maxit, m);
 }
 
@@ -144,6 +151,7 @@ __global__ void k_gmres_init(GmresState *st, const double *__restrict__ b2, doub
 __global__ void k_cycle_start(GmresState *st, const double *__restrict__ beta2, cudaGraphConditionalHandle h,
                               int use_handle)
 {
+    pdl_wait();
     const double beta = sqrt(beta2[0]);
     st->beta = beta;
     for (int i = 0; i < 32; ++i)
@@ -196,12 +204,13 @@ __device__ __forceinline__ void gmres_rotate_column(GmresState *st)
 
 __global__ void k_gmres_column(GmresState *st, const double *__restrict__ wnorm2)
 {
+    pdl_wait();
     st->hcol[st->j + 1] = sqrt(wnorm2[0]);
     gmres_rotate_column(st);
 }
 
 // end of an Arnoldi step: counters and the inner loop condition
-__global__ void k_inner_check(GmresState *st, cudaGraphConditionalHandle h, int use_handle)
+__device__ __forceinline__ void inner_check(GmresState *st, cudaGraphConditionalHandle h, int use_handle)
 {
     st->its += 1;
     st->total_its += 1;
@@ -212,9 +221,16 @@ __global__ void k_inner_check(GmresState *st, cudaGraphConditionalHandle h, int 
         cudaGraphSetConditional(h, unsigned(go));
 }
 
+__global__ void k_inner_check(GmresState *st, cudaGraphConditionalHandle h, int use_handle)
+{
+    pdl_wait();
+    inner_check(st, h, use_handle);
+}
+
 // back substitution H y = g over the cycle's j columns
 __global__ void k_gmres_solve_y(GmresState *st)
 {
+    pdl_wait();
     const int m = st->j;
     for (int i = m - 1; i >= 0; --i)
     {
@@ -229,6 +245,7 @@ __global__ void k_gmres_solve_y(GmresState *st)
 __global__ void k_add_basis(const double *__restrict__ V, int64_t ldv, const GmresState *__restrict__ st,
                             double *__restrict__ x, int64_t n)
 {
+    pdl_wait();
     const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t >= n)
         return;
@@ -242,6 +259,7 @@ __global__ void k_add_basis(const double *__restrict__ V, int64_t ldv, const Gmr
 // end of a cycle: converged (PETSc's default test), out of iterations, or restart
 __global__ void k_outer_check(GmresState *st, cudaGraphConditionalHandle h, int use_handle)
 {
+    pdl_wait();
     st->total_cycles += 1;
     int go = 0;
     if (st->reason != 0)
@@ -259,6 +277,7 @@ __global__ void k_outer_check(GmresState *st, cudaGraphConditionalHandle h, int 
 
 __global__ void k_zero(double *__restrict__ x, int64_t n)
 {
+    pdl_wait();
     const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t < n)
         x[t] = 0.0;
@@ -268,6 +287,7 @@ __global__ void k_zero(double *__restrict__ x, int64_t n)
 __global__ void k_residual(const double *__restrict__ b, const double *__restrict__ y, double *__restrict__ r,
                            int64_t n)
 {
+    pdl_wait();
     const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t < n)
         r[t] = b[t] - y[t];
@@ -282,6 +302,7 @@ __global__ void k_residual(const double *__restrict__ b, const double *__restric
 __global__ void k_scatter_vec(double *__restrict__ pool, const uint64_t *__restrict__ dst,
                               const double *__restrict__ x0, int64_t ldx, const int *__restrict__ jdev, int64_t n)
 {
+    pdl_wait();
     const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t >= n)
         return;
@@ -294,6 +315,7 @@ __global__ void k_resist_out(const double *__restrict__ pool, const uint64_t *__
                              const uint64_t *__restrict__ dj, const double *__restrict__ eta, double *__restrict__ y,
                              int64_t n)
 {
+    pdl_wait();
     const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t < n)
         y[t] = pool[e[t]] - eta[t] * pool[dj[t]];
@@ -303,6 +325,7 @@ __global__ void k_resist_out(const double *__restrict__ pool, const uint64_t *__
 __global__ void k_resist_rhs(const double *__restrict__ pool, const uint64_t *__restrict__ j,
                              const double *__restrict__ eta, double *__restrict__ b, int64_t n)
 {
+    pdl_wait();
     const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t < n)
         b[t] = 0.0 + eta[t] * pool[j[t]];
@@ -312,6 +335,7 @@ __global__ void k_resist_rhs(const double *__restrict__ pool, const uint64_t *__
 __global__ void k_alias_copy(double *__restrict__ pool, const uint64_t *__restrict__ alias,
                              const uint64_t *__restrict__ owner, const double *__restrict__ sign, int64_t n)
 {
+    pdl_wait();
     const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t < n)
         pool[alias[t]] = sign[t] * pool[owner[t]];
@@ -327,6 +351,7 @@ __global__ void k_alias_copy(double *__restrict__ pool, const uint64_t *__restri
 __global__ void k_pack_vec(const double *__restrict__ pool, const uint64_t *__restrict__ src, double *__restrict__ x,
                            int64_t n)
 {
+    pdl_wait();
     const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t < n)
         x[t] = pool[src[t]];
@@ -403,8 +428,8 @@ __device__ __forceinline__ void block_partials(const double (&acc)[N], int c0, i
     __syncthreads();
 }
 
-// out[c] for c < nd from the CTAs' partials, by the last CTA to arrive
-__device__ void grid_finish(int nd, const double *__restrict__ partial, double *__restrict__ out,
+// out[c] for c < nd from the CTAs' partials, by the last CTA to arrive (true there)
+__device__ bool grid_finish(int nd, const double *__restrict__ partial, double *__restrict__ out,
                             unsigned *__restrict__ done)
 {
     constexpr int kWarps = kRedThreads / 32;
@@ -416,7 +441,7 @@ __device__ void grid_finish(int nd, const double *__restrict__ partial, double *
         last = (atomicAdd(done, 1u) == gridDim.x - 1);
     __syncthreads();
     if (!last)
-        return;
+        return false;
     __threadfence();
     for (int c = wid; c < nd; c += kWarps)
     {
@@ -430,12 +455,14 @@ __device__ void grid_finish(int nd, const double *__restrict__ partial, double *
     }
     if (threadIdx.x == 0)
         *done = 0u;
+    return true;
 }
 } // namespace
 
 __global__ void k_hall_begin(HallCtl *c, const double *__restrict__ f2, const GmresState *__restrict__ st, double rtol,
                              double atol, int maxit, cudaGraphConditionalHandle h, int use)
 {
+    pdl_wait();
     c->f = sqrt(f2[0]);
     c->f0 = c->f;
     c->rtol = rtol;
@@ -450,6 +477,7 @@ __global__ void k_hall_begin(HallCtl *c, const double *__restrict__ f2, const Gm
 // start of a Newton step: ||X|| and the difference step of unit vectors
 __global__ void k_hall_step_begin(HallCtl *c, const double *__restrict__ x2)
 {
+    pdl_wait();
     c->xnorm = sqrt(x2[0]);
     c->h = fd_scale() * (1.0 + c->xnorm) / 1.0;
     c->first = 1;
@@ -458,6 +486,7 @@ __global__ void k_hall_step_begin(HallCtl *c, const double *__restrict__ x2)
 __global__ void k_hall_gmres_init(GmresState *st, const double *__restrict__ b2, double rtol, double atol, int maxit,
                                   int m, cudaGraphConditionalHandle hout, int use)
 {
+    pdl_wait();
     gmres_init_state(st, b2, rtol, atol, maxit, m);
     set_cond(hout, use, 1);
 }
@@ -466,6 +495,7 @@ __global__ void k_hall_gmres_init(GmresState *st, const double *__restrict__ b2,
 // (none on the first cycle, where r = b, nor when dx = 0)
 __global__ void k_hall_cycle_prep(HallCtl *c, const double *__restrict__ dx2, cudaGraphConditionalHandle h, int use)
 {
+    pdl_wait();
     const double dn = sqrt(dx2[0]);
     const int go = !c->first && dn > 0.0;
     if (go)
@@ -480,6 +510,7 @@ __global__ void k_hall_cycle_prep(HallCtl *c, const double *__restrict__ dx2, cu
 
 __global__ void k_hall_ls_begin(HallCtl *c, cudaGraphConditionalHandle h, int use)
 {
+    pdl_wait();
     c->lambda = 1.0;
     c->cut = 0;
     c->ls = 1;
@@ -490,6 +521,7 @@ __global__ void k_hall_ls_begin(HallCtl *c, cudaGraphConditionalHandle h, int us
 // else halve lambda, at most 12 trials (the last one is taken regardless)
 __global__ void k_hall_ls_check(HallCtl *c, const double *__restrict__ ft2, cudaGraphConditionalHandle h, int use)
 {
+    pdl_wait();
     const double ft = sqrt(ft2[0]);
     c->ft = ft;
     c->pass[2] += 1;
@@ -506,6 +538,7 @@ __global__ void k_hall_ls_check(HallCtl *c, const double *__restrict__ ft2, cuda
 
 __global__ void k_hall_accept(HallCtl *c, cudaGraphConditionalHandle h, int use)
 {
+    pdl_wait();
     c->f = c->ft;
     c->it += 1;
     c->pass[0] += 1;
@@ -514,7 +547,7 @@ __global__ void k_hall_accept(HallCtl *c, cudaGraphConditionalHandle h, int use)
 
 // the column of a CGS2 step whose second pass gave d: h += d, and
 // ||w''||^2 = ||w'||^2 - ||d||^2 (w'' = w' - V d with V orthonormal)
-__global__ void k_hall_column(GmresState *st, const double *__restrict__ d)
+__device__ void hall_column(GmresState *st, const double *d)
 {
     const int j = st->j;
     double s2 = d[j + 1];
@@ -527,22 +560,39 @@ __global__ void k_hall_column(GmresState *st, const double *__restrict__ d)
     gmres_rotate_column(st);
 }
 
+// Xt = X + (*a) v into the pool's unknowns, their aliases and the points
+// Sync("Ehall") writes: what each of these takes is known from the vectors
+// (HallList), so the three dependent passes (unknowns, aliases, copies) are one.
 __global__ void k_hall_trial(double *__restrict__ pool, const uint64_t *__restrict__ e, const double *__restrict__ X,
                              const double *__restrict__ a, const double *__restrict__ v0, int64_t ldv,
-                             const int *__restrict__ jdev, double *__restrict__ Xt, int64_t n)
+                             const int *__restrict__ jdev, double *__restrict__ Xt, int64_t n, HallList l)
 {
     const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (t >= n)
-        return;
-    double x = X[t];
-    if (a)
+    pdl_wait();
+    if (t < n + l.n1)
     {
-        const double *v = jdev ? v0 + int64_t(jdev[0]) * ldv : v0;
-        x = x + a[0] * v[t];
+        const int64_t u = t < n ? t : l.idx[t - n];
+        double x = X[u];
+        if (a)
+        {
+            const double *v = jdev ? v0 + int64_t(jdev[0]) * ldv : v0;
+            x = x + a[0] * v[u];
+        }
+        if (t < n)
+        {
+            if (Xt)
+                Xt[t] = x;
+            pool[e[t]] = x;
+        }
+        else
+            pool[l.d1[t - n]] = l.sign[t - n] * x;
+        return;
     }
-    if (Xt)
-        Xt[t] = x;
-    pool[e[t]] = x;
+    int64_t q = t - n - l.n1;
+    if (q < l.n2)
+        pool[l.d2[q]] = pool[l.s2[q]];
+    else if ((q -= l.n2) < l.n3)
+        pool[l.d3[q]] = l.val[q];
 }
 
 __global__ void __launch_bounds__(kRedThreads) k_hall_jv_dots(const double *__restrict__ pool,
@@ -555,6 +605,7 @@ __global__ void __launch_bounds__(kRedThreads) k_hall_jv_dots(const double *__re
                                                               double *__restrict__ partial, double *__restrict__ out,
                                                               unsigned *__restrict__ done)
 {
+    pdl_wait();
     const int nv = st->j + 1;
     const double hh = h[0];
     const int64_t t0 = int64_t(blockIdx.x) * blockDim.x + threadIdx.x, ts = int64_t(gridDim.x) * blockDim.x;
@@ -585,11 +636,12 @@ __global__ void __launch_bounds__(kRedThreads) k_hall_jv_dots(const double *__re
 }
 
 __global__ void __launch_bounds__(kRedThreads) k_hall_proj_dots(const double *__restrict__ V, int64_t ldv,
-                                                                const GmresState *__restrict__ st,
-                                                                double *__restrict__ w, int64_t n,
-                                                                double *__restrict__ partial,
-                                                                double *__restrict__ out, unsigned *__restrict__ done)
+                                                                GmresState *st, double *__restrict__ w, int64_t n,
+                                                                double *__restrict__ partial, double *out,
+                                                                unsigned *__restrict__ done,
+                                                                cudaGraphConditionalHandle h, int use)
 {
+    pdl_wait();
     __shared__ double hs[kMdMax];
     const int nv = st->j + 1;
     if (int(threadIdx.x) < nv)
@@ -634,18 +686,28 @@ __global__ void __launch_bounds__(kRedThreads) k_hall_proj_dots(const double *__
         }
         block_partials(acc, c0, nv, partial);
     }
-    grid_finish(nv + 1, partial, out, done);
+    if (grid_finish(nv + 1, partial, out, done))
+    {
+        // the last CTA: the Hessenberg column and the loop test (neither reads V_{j+1})
+        __syncthreads();
+        if (threadIdx.x == 0)
+        {
+            hall_column(st, out);
+            inner_check(st, h, use);
+        }
+    }
 }
 
 __global__ void k_hall_next(double *__restrict__ V, int64_t ldv, const double *__restrict__ w,
                             const GmresState *__restrict__ st, const double *__restrict__ d, int64_t n)
 {
+    pdl_wait();
     if (st->breakdown)
         return;
     const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t >= n)
         return;
-    const int j = st->j;
+    const int j = st->j - 1; // (the column is counted already)
     double s = w[t];
     for (int c = 0; c <= j; ++c)
         s -= d[c] * V[int64_t(c) * ldv + t];
@@ -658,6 +720,7 @@ __global__ void __launch_bounds__(kRedThreads) k_hall_res_dots(const double *__r
                                                                int64_t n, double *__restrict__ partial,
                                                                double *__restrict__ out, unsigned *__restrict__ done)
 {
+    pdl_wait();
     double acc[1] = {0.0};
     for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < n; t += int64_t(gridDim.x) * blockDim.x)
     {
@@ -674,6 +737,7 @@ __global__ void k_hall_restart_r(const double *__restrict__ pool, const uint64_t
                                  const double *__restrict__ h, const double *__restrict__ b, double *__restrict__ r,
                                  int64_t n)
 {
+    pdl_wait();
     const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t < n)
         r[t] = b[t] - ((Xt[t] - pool[e[t]]) - F[t]) / h[0];
@@ -686,6 +750,7 @@ __global__ void __launch_bounds__(kRedThreads) k_hall_gmres_prologue(const doubl
                                                                      double *__restrict__ out,
                                                                      unsigned *__restrict__ done)
 {
+    pdl_wait();
     double acc[1] = {0.0};
     for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < n; t += int64_t(gridDim.x) * blockDim.x)
     {
@@ -703,6 +768,7 @@ __global__ void __launch_bounds__(kRedThreads) k_norm2(const double *__restrict_
                                                        double *__restrict__ partial, double *__restrict__ out,
                                                        unsigned *__restrict__ done)
 {
+    pdl_wait();
     double acc[1] = {0.0};
     for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < n; t += int64_t(gridDim.x) * blockDim.x)
         acc[0] += x[t] * x[t];
@@ -713,6 +779,7 @@ __global__ void __launch_bounds__(kRedThreads) k_norm2(const double *__restrict_
 __global__ void k_hall_take(double *__restrict__ X, const double *__restrict__ Xt, double *__restrict__ F,
                             const double *__restrict__ Ft, int64_t n)
 {
+    pdl_wait();
     const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t < n)
     {
@@ -724,6 +791,7 @@ __global__ void k_hall_take(double *__restrict__ X, const double *__restrict__ X
 __global__ void k_copy_segments(double *__restrict__ dst, const double *__restrict__ src,
                                 const int64_t *__restrict__ seg, int nseg)
 {
+    pdl_wait();
     const int s = blockIdx.y;
     if (s >= nseg)
         return;
