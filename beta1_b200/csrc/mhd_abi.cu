@@ -184,7 +184,8 @@ const char *const kTuneNames[NTUNE] = {"k_pv_uplus_dt", "k_fluid_ucontra", "k_bc
                                        "k_curl_e2f",    "k_eedge",         "k_fluid_mixed",  "k_gmres_resist",
                                        "k_hall_edge"};
 // per variant (variant 0, the default, first) the reported value: the minimum
-// CTAs per SM of its launch bounds (0: the default's own); 12 for the
+// CTAs per SM of its launch bounds (0: the default's own; 3 for the default
+// k_fluid_mixed, which now runs at 4); 12 for the
 // face-tiled k_fluid_mixed (2 CTAs per SM), 16 for the same with its face
 // states staged in shared memory, 14 for k_pv_uplus_dt with J_cell in a pass
 // of its own (the PV pass at 4); for the persistent k_gmres_resist the CTAs of
@@ -249,6 +250,7 @@ struct mhd_ctx
     // and PV / U_plus computed on the first ghost layer only
     std::map<std::string, bool> dirty;
     bool pv_dirty = false;
+    bool eface_zero = true; // the zero components of Eface hold zero on the inner faces
     bool geom_dirty = true; // face areas / normals to recompute from JD
     std::vector<std::string> field_group = std::vector<std::string>(NFIELD); // group that syncs a field
     double *staging = nullptr;
@@ -857,6 +859,15 @@ int launch_fluid_ucontra(mhd_ctx *ctx, const RunClock &rc = RunClock{})
     return launched(ctx, launch_k_fluid_ucontra(ctx->tune[TUNE_k_fluid_ucontra], ctx->hot, ctx->stream, ctx->c, rc));
 }
 
+int ensure_eface_zero(mhd_ctx *ctx)
+{
+    if (ctx->eface_zero)
+        return MHD_OK;
+    ctx->eface_zero = true;
+    prof_begin(ctx, "k_eface");
+    return launched(ctx, launch_k_eface_zero(ctx->hot, ctx->stream));
+}
+
 // AssembleRHS_Induction_CT_ up to the edge EMF; with_ucontra unless the fluid pass computed them
 int launch_edge_emf(mhd_ctx *ctx, bool with_ucontra)
 {
@@ -881,6 +892,7 @@ int launch_edge_emf(mhd_ctx *ctx, bool with_ucontra)
 // AssembleRHS_Induction_CT_ without the update (a stage)
 int launch_induction(mhd_ctx *ctx)
 {
+    RUN(ensure_eface_zero(ctx));
     RUN(launch_edge_emf(ctx, true));
     prof_begin(ctx, "k_curl_e2f");
     return launched(ctx, launch_k_curl_e2f(ctx->tune[TUNE_k_curl_e2f], ctx->hot, ctx->stream, F_Exi, F_RBxi, -1, -1.0,
@@ -1415,22 +1427,24 @@ int hall_trial(mhd_ctx *ctx, const double *a, const double *v0, int64_t ldv, con
     return run_sync(ctx, "Ehall", true);
 }
 
-// B = B* + dt (-curl Ehall) on inner faces (theta = 1), Sync("Bface")
-int hall_trial_b(mhd_ctx *ctx)
+// B = B* + dt (-curl Ehall) on inner faces (theta = 1), Sync("Bface"); last:
+// the solve's final update, which also leaves RHS_B
+int hall_trial_b(mhd_ctx *ctx, bool last)
 {
     auto &H = ctx->hall;
     if (!H.from_snapshot)
         RUN(hall_copy_b(ctx, false));
     prof_begin(ctx, "k_curl_e2f");
-    RUN(launched(ctx, launch_k_curl_e2f(ctx->tune[TUNE_k_curl_e2f], ctx->hot, ctx->stream, F_Ehxi, F_RBxi, F_Bxi, -1.0,
-                                        ctx->dt, 1.0, 0, nullptr, 0, H.from_snapshot ? H.bs : nullptr)));
+    RUN(launched(ctx, launch_k_curl_e2f(ctx->tune[TUNE_k_curl_e2f], ctx->hot, ctx->stream, F_Ehxi, last ? F_RBxi : -1,
+                                        F_Bxi, -1.0, ctx->dt, 1.0, 0, nullptr, 0,
+                                        H.from_snapshot ? H.bs : nullptr)));
     return run_syncs(ctx, {"Bface"});
 }
 
 // FormFunction_ up to the predicted Hall EMF of the trial in the pool
 int hall_chain(mhd_ctx *ctx)
 {
-    RUN(hall_trial_b(ctx));
+    RUN(hall_trial_b(ctx, false));
     return hall_emf_from_current_b(ctx);
 }
 
@@ -1559,7 +1573,7 @@ int launch_hall_implicit(mhd_ctx *ctx)
     RUN(hall_trial(ctx, nullptr, nullptr, 0, nullptr, nullptr));
     if (H.fused)
         RUN(run_sync(ctx, "Ehall", true));
-    return hall_trial_b(ctx);
+    return hall_trial_b(ctx, true);
 }
 
 // the part of a step before the eagerly driven solves: the explicit step,
@@ -1732,6 +1746,8 @@ int build_graph(mhd_ctx *ctx)
 int run_steps(mhd_ctx *ctx, int nsteps)
 {
     RUN(build_graph(ctx));
+    if (nsteps > 0)
+        RUN(ensure_eface_zero(ctx));
     for (int s = 0; s < nsteps; ++s)
     {
         if (ctx->gexec)
@@ -2082,6 +2098,8 @@ static int transfer(mhd_ctx *ctx, const char *name, int32_t block, const double 
     const int nc = kFields[f].ncomp;
     if (hin)
     {
+        if (f >= F_Efxi && f <= F_Efzeta)
+            ctx->eface_zero = false;
         if (f == F_JDxi || f == F_JDeta || f == F_JDzeta || f == F_WB || f == F_WJ || f == F_drxi || f == F_dreta ||
             f == F_drzeta)
             ctx->geom_dirty = true; // face normals, FP32 copies and Pole matrices follow
@@ -4398,6 +4416,7 @@ int mhd_profile_step(mhd_ctx *ctx, int32_t cap, int32_t *kernel_ids, float *ms, 
         return MHD_EINVAL;
     RUN(ensure_geom(ctx));
     RUN(build_all_syncs(ctx));
+    RUN(ensure_eface_zero(ctx));
     ctx->profiling = true;
     ctx->prof_ev.clear();
     ctx->prof_names.clear();

@@ -325,7 +325,8 @@ int launch_k_bcell_jedge(int variant, bool w32, const HotGrid &h, cudaStream_t s
 int launch_k_bcell(const HotGrid &h, cudaStream_t st);
 int launch_k_jedge(const HotGrid &h, cudaStream_t st, int fB0, int fJ0, const int *rng, int64_t nreg);
 int launch_k_jcell(bool w32, const HotGrid &h, cudaStream_t st);
-// face EMF: minimum CTAs per SM 2, 6; edge EMF: 3, 8
+// the components of Eface that are zero; face EMF (the others): minimum CTAs per SM 2, 6; edge EMF: 3, 8
+int launch_k_eface_zero(const HotGrid &h, cudaStream_t st);
 int launch_k_eface(int variant, const HotGrid &h, cudaStream_t st);
 int launch_k_eedge(int variant, const HotGrid &h, cudaStream_t st);
 // RHS = mult curl E and B += dt / dtdiv RHS on the inner faces (fR0, fB0 < 0:
@@ -345,7 +346,7 @@ int launch_k_eres_explicit(const HotGrid &h, cudaStream_t st, double inver_Rem);
 int launch_k_hall_cell(const HotGrid &h, cudaStream_t st, Consts c, double hall_coef, bool all);
 // Hall edge EMF (zb: boxes of zeroed edges): minimum CTAs per SM 4, 2
 int launch_k_hall_edge(int variant, const HotGrid &h, cudaStream_t st, const int *zb, int nzb);
-// k_fluid_mixed: minimum CTAs per SM 3, 1, 2; variants 3 and 4 are the
+// k_fluid_mixed: minimum CTAs per SM 4, 1, 2; variants 3 and 4 are the
 // face-tiled kernels (on `tiles`, the KIND_TILE1 grid of bvs)
 int launch_k_fluid_mixed(int variant, const HotGrid &h, dim3 tiles, cudaStream_t st, const BlockView *bvs, Consts c,
                          RunClock rc);

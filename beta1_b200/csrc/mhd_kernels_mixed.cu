@@ -146,11 +146,12 @@ __device__ __forceinline__ void mixed_rhs(const double *q0, const Consts &c, con
 
 // Fluid RHS of the inner cells (FP32 flux divergence, FP64 J x B source) and
 // the FP64 contravariant velocities of the cells within one ghost layer; the
-// FP64 face metric read for the velocities is the one the fluxes round.  All
-// stores are at the end, so that the loads of one axis do not wait for the
-// results of the axis before.
-// variants: at least 3 CTAs per SM (80 registers; the default), the
-// compiler's own allocation, at least 2
+// FP64 face metric read for the velocities is the one the fluxes round.  The
+// axes are a real loop: unrolled, the loads of the next axis cost registers
+// (3 CTAs per SM with 52 bytes of spills, 198 us on 2.27 M cells); rolled, 4
+// CTAs per SM fit (64 registers, 187 us), and the L2 prefetch covers the rest.
+// variants: at least 4 CTAs per SM (the default), the compiler's own
+// allocation, at least 2
 struct QHot
 {
     const float *q;
@@ -199,8 +200,7 @@ template <class A> __device__ __forceinline__ void k_fluid_mixed_body(const A &a
     // vectors, and (inner cells) its two FP32 face fluxes
     double S[3] = {0.0, 0.0, 0.0};
     float r[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-    double uc[3];
-#pragma unroll
+#pragma unroll 1
     for (int a = 0; a < 3; ++a)
     {
         const int s = a == 0 ? int(b.si) : a == 1 ? int(b.sj) : 1;
@@ -219,7 +219,7 @@ template <class A> __device__ __forceinline__ void k_fluid_mixed_body(const A &a
         const double kx = 0.5 * (m_[0] + p_[0]);
         const double ky = 0.5 * (m_[1] + p_[1]);
         const double kz = 0.5 * (m_[2] + p_[2]);
-        uc[a] = (kx * ux + ky * uy + kz * uz) * inv_jac;
+        hot_at(b, p, F_UC)[a * v] = (kx * ux + ky * uy + kz * uz) * inv_jac;
         if (inner)
         {
             const float *g = hot_plane32(b, p, G32_AREA + a);
@@ -243,10 +243,6 @@ template <class A> __device__ __forceinline__ void k_fluid_mixed_body(const A &a
         for (int m = 0; m < 5; ++m)
             out[m * v] = R[m];
     }
-    double *UC = hot_at(b, p, F_UC);
-    UC[0] = uc[0];
-    UC[v] = uc[1];
-    UC[2 * v] = uc[2];
 }
 
 template <class A, int MINB>
@@ -471,7 +467,7 @@ int launch_k_fluid_mixed(int variant, const HotGrid &h, dim3 tiles, cudaStream_t
     return hot_for(h, KIND_CELL1, [&](const auto &a, dim3 g) {
         using A = std::decay_t<decltype(a)>;
         if (variant == 0)
-            hot_launch(k_fluid_mixed_t<A, 3>, g, st, a, c, rc);
+            hot_launch(k_fluid_mixed_t<A, 4>, g, st, a, c, rc);
         else if (variant == 1)
             hot_launch(k_fluid_mixed_t<A, 1>, g, st, a, c, rc);
         else

@@ -281,15 +281,27 @@ template <class A> __device__ __forceinline__ void eface_body(const A &a)
                                        u0[b1], tot0[fa]);
             const double g2 = emf_flux(btm[fa][b2], bt0[b2], bim[fa][b2], bi0[b2], um[fa][fa], u0[fa], um[fa][b2],
                                        u0[b2], tot0[fa]);
-            double e[3];
-            e[fa] = 0.0;
-            e[b1] = g2;
-            e[b2] = -g1;
-            double *F = hot_at(b, p, F_Efxi + fa);
-            F[0] = e[0];
-            F[v] = e[1];
-            F[2 * v] = e[2];
+            // (component fa of face axis fa is zero and stays so, k_eface_zero_t)
+            *hot_at(b, p, F_Efxi + fa, b1) = g2;
+            *hot_at(b, p, F_Efxi + fa, b2) = -g1;
         }
+}
+
+// the zero components of Eface: zero in a new pool; written again after an
+// Eface field was uploaded
+template <class A> __global__ void __launch_bounds__(kHotThreads) k_eface_zero_t(const __grid_constant__ A a)
+{
+    uint32_t t, p;
+    const HotBlock &b = hot_block<KIND_STAG>(a, t);
+    int i, j, k;
+    const bool in_box = hot_point<KIND_STAG>(b, t, i, j, k, p);
+    pdl_wait();
+    if (!in_box)
+        return;
+#pragma unroll
+    for (int fa = 0; fa < 3; ++fa)
+        if (hot_face(b, fa, i, j, k))
+            *hot_at(b, p, F_Efxi + fa, fa) = 0.0;
 }
 
 template <class A, int MINB>
@@ -746,7 +758,7 @@ template <> __device__ __forceinline__ const float *hot_face_plane<float>(const 
 // primitive and face-state quantities of one cell (calc_PV, calc_Uplus)
 struct CellState
 {
-    double rho, u, v, w, pr, T, up[3], cs, rhoe;
+    double rho, u, v, w, pr, up[3], cs, rhoe;
 };
 __device__ __forceinline__ CellState cell_state(const double U[5], const Consts &c)
 {
@@ -761,7 +773,6 @@ __device__ __forceinline__ CellState cell_state(const double U[5], const Consts 
         eint = 0.0;
     s.pr = (c.gamma - 1.0) * eint;
     s.pr = smax(s.pr, 1e-12);
-    s.T = s.pr / (s.rho * c.state_coeff);
     const bool has_plasma = U[0] > 1e-20;
     s.up[0] = has_plasma ? s.u : 0.0;
     s.up[1] = has_plasma ? s.v : 0.0;
@@ -773,9 +784,10 @@ __device__ __forceinline__ CellState cell_state(const double U[5], const Consts 
     return s;
 }
 
-// WT double: PV_H, U_plus and the FP64 face states; float (mixed form): U_plus
-// (PV_H is left to read-out: the mixed flux reads the FP32 face states, its
-// J x B source the velocities from U).  In a mixed context also the FP32 face
+// WT double: PV_H without its temperature, U_plus and the FP64 face states;
+// float (mixed form): U_plus.  No kernel of a step reads the temperature, and
+// none of the mixed form PV_H (its flux reads the FP32 face states, its J x B
+// source the velocities from U); the read-out pass forms PV_H anew (k_pv_all).  In a mixed context also the FP32 face
 // states, deviations from the reference state (formed in FP64), sound speed.
 template <typename WT>
 __device__ __forceinline__ void store_cell_state(const HotBlock &b, uint32_t p, double U0, const CellState &s)
@@ -788,7 +800,6 @@ __device__ __forceinline__ void store_cell_state(const HotBlock &b, uint32_t p, 
         PV[v] = s.v;
         PV[2 * v] = s.w;
         PV[3 * v] = s.pr;
-        PV[4 * v] = s.T;
         *hot_at(b, p, F_Cs) = s.cs;
         *hot_at(b, p, F_RhoE) = s.rhoe;
     }
@@ -858,10 +869,18 @@ __device__ __forceinline__ void pv_uplus_dt_body(const A &a, const Consts &c, un
 #pragma unroll
         for (int m = 0; m < 5; ++m)
             U[m] = hot_at(b, p, F_U)[m * v];
+        // FP64: the cell state is stored before the CFL bound and J_cell comes
+        // last, so that no phase's results stay live over the next one's loads
+        // (12 instead of 88 bytes of spills at 64 registers; 95 -> 87 us on 0.76
+        // M cells).  Mixed form: J_cell's loads first, all stores last (195
+        // against 201 us on 2.27 M cells; its weights take half the registers).
+        constexpr bool kEarly = sizeof(WT) == sizeof(double);
         double jx, jy, jz;
-        if (JCELL && inner)
+        if (JCELL && inner && !kEarly)
             jcell_sum<WT>(b, p, jx, jy, jz);
         const CellState s = cell_state(U, c);
+        if (kEarly)
+            store_cell_state<WT>(b, p, U[0], s);
         if (inner)
         {
             const double V = fabs(*hot_at(b, p, F_Jac));
@@ -905,13 +924,16 @@ __device__ __forceinline__ void pv_uplus_dt_body(const A &a, const Consts &c, un
             }
             if (JCELL)
             {
+                if (kEarly)
+                    jcell_sum<WT>(b, p, jx, jy, jz);
                 double *Jc = hot_at(b, p, F_Jcell);
                 Jc[0] = jx;
                 Jc[v] = jy;
                 Jc[2 * v] = jz;
             }
         }
-        store_cell_state<WT>(b, p, U[0], s);
+        if (!kEarly)
+            store_cell_state<WT>(b, p, U[0], s);
     }
     reduce_key(dbl_key(dtc), dt_key + b.run);
 }
@@ -940,7 +962,9 @@ template <class A> __global__ void __launch_bounds__(kHotThreads) k_pv_all_t(con
 #pragma unroll
     for (int m = 0; m < 5; ++m)
         U[m] = hot_at(b, p, F_U)[m * uint64_t(b.vol)];
-    store_cell_state<double>(b, p, U[0], cell_state(U, c));
+    const CellState s = cell_state(U, c);
+    store_cell_state<double>(b, p, U[0], s);
+    *hot_at(b, p, F_PV, 4) = s.pr / (s.rho * c.state_coeff);
 }
 
 // Explicit resistive edge EMF, AddResistiveEdgeEMF_To_ on a zeroed Eres
@@ -1272,6 +1296,12 @@ int launch_k_eface(int variant, const HotGrid &h, cudaStream_t st)
         else
             hot_launch(k_eface_t<A, 6>, g, st, a);
     });
+}
+
+int launch_k_eface_zero(const HotGrid &h, cudaStream_t st)
+{
+    return hot_for(h, KIND_STAG,
+                   [&](const auto &a, dim3 g) { hot_launch(k_eface_zero_t<std::decay_t<decltype(a)>>, g, st, a); });
 }
 
 int launch_k_eedge(int variant, const HotGrid &h, cudaStream_t st)

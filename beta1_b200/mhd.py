@@ -27,7 +27,8 @@ PREC_FP64 = 0
 PREC_MIXED = 1
 
 # the default variant of each tunable kernel, in the values mhd_autotune
-# reports (minimum CTAs per SM of its launch bounds, 0: the default's own; 12: the
+# reports (minimum CTAs per SM of its launch bounds, 0: the default's own,
+# 3: k_fluid_mixed's default; 12: the
 # face-tiled k_fluid_mixed, 16: the same with staged face states; 14:
 # k_pv_uplus_dt with J_cell in its own pass;
 # k_gmres_resist: the CTAs of the persistent grid, 0: two per SM)

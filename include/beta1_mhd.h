@@ -310,7 +310,7 @@ int mhd_set_flux_reference_run(mhd_ctx *ctx, int32_t run, const double prim[5]);
    call does not advance the simulation.  Call it after the state is loaded.
    min_ctas[i] (i < n, at most MHD_NTUNE) receives the chosen minimum CTAs
    per SM of kernel mhd_tune_name(i) (0: the default form's own launch bounds;
-   12: the face-tiled k_fluid_mixed, 16: the same with
+   3: the default k_fluid_mixed; 12: the face-tiled k_fluid_mixed, 16: the same with
    its FP32 face states staged in shared memory; 14: k_pv_uplus_dt
    with J_cell in a pass of its own).  For the persistent k_gmres_resist the
    value is the CTAs of its grid (0: two per SM); its partial sums group

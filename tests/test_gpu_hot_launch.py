@@ -1,0 +1,72 @@
+"""The hot kernels' launch forms: batches past the blocks of one launch (65
+runs and more: two launches per kernel), grids past the small argument form
+(9 blocks and more), a batch of several runs against each run alone, and the
+components of Eface the face kernel leaves alone.  Every form runs the same
+arithmetic per point, so the fields agree bit for bit."""
+import numpy as np
+import pytest
+
+from conftest import load_golden, periodic_setup
+
+from beta1_b200 import case, solver
+
+pytestmark = pytest.mark.gpu
+
+FIELDS = ("U_H", "B_xi", "B_eta", "B_zeta", "PV_H", "J_cell", "E_xi", "Eface_eta", "RHS_H", "RHS_B_zeta")
+
+
+@pytest.mark.parametrize("nruns", [2, 9, 64, 65, 70])
+def test_batch_sizes(nruns):
+    """copies of the periodic fixture, one run each: the reference's step"""
+    g = load_golden("periodic_8x6x5_steps.npz")
+    spec, st = periodic_setup(g)
+    host = solver.host_setup(spec, "periodic", "device")
+    bt = solver.Batch([(spec, "periodic")] * nruns, host=iter([host] * nruns))
+    try:
+        bt.load_states([st] * nruns)
+        bt.step(1)
+        for r in sorted({0, 1, nruns // 2, nruns - 1}):
+            for f in FIELDS:
+                assert np.array_equal(bt.field(r, f), g["s1/" + f]), (r, f)
+    finally:
+        bt.ctx.close()
+
+
+def test_twelve_blocks_alone_and_in_a_batch():
+    """a 12-block slab (one launch of the large argument form) and the same
+    run beside another of other extents in a batch (flattened launches)"""
+    spec = case.slab_case(11, (5, 7), (3, 4))
+    other = case.slab_case(9, (4, 33), (1, 2))
+    st, st2 = case.inflow_state(spec, seed=3), case.inflow_state(other, seed=4)
+    s = solver.Solver(spec, topology="tiled", geometry_on="device")
+    bt = solver.Batch([(other, "tiled"), (spec, "tiled")], geometry_on="device")
+    try:
+        s.load_state(st)
+        bt.load_states([st2, st])
+        s.step(3)
+        bt.step(3)
+        for b in range(12):
+            for f in FIELDS:
+                assert np.array_equal(bt.field(1, f, b), s.field(f, b)), (b, f)
+    finally:
+        s.ctx.close()
+        bt.ctx.close()
+
+
+def test_uploaded_eface():
+    """the zero components of an uploaded Eface are zero after a step"""
+    g = load_golden("periodic_8x6x5_steps.npz")
+    spec, st = periodic_setup(g)
+    s = solver.Solver(spec)
+    try:
+        s.load_state(st)
+        for f in ("Eface_xi", "Eface_eta", "Eface_zeta"):
+            s.ctx.upload(f, 0, np.full_like(s.field(f), 3.0))
+            assert np.all(s.field(f) == 3.0)
+        s.step(1)
+        n = spec.blocks[0].ncell
+        for d, f in enumerate(("Eface_xi", "Eface_eta", "Eface_zeta")):
+            inner = tuple(slice(4, 4 + n[a] + (a == d)) for a in range(3))
+            assert np.array_equal(s.field(f)[inner], g["s1/" + f][inner]), f
+    finally:
+        s.ctx.close()
