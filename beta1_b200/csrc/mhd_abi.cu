@@ -223,6 +223,9 @@ struct mhd_ctx
     float *pool32 = nullptr; // FP32 planes of the mixed-precision form
     std::vector<std::vector<size_t>> base; // [field][block] offset in pool
     cudaStream_t stream = nullptr;
+    // beside the main stream inside a step: what only a later kernel needs
+    cudaStream_t side = nullptr;
+    cudaEvent_t fork_ev[3] = {nullptr, nullptr, nullptr};
     cudaGraph_t graph = nullptr, graph_a = nullptr, graph_c = nullptr;
     cudaGraphExec_t gexec = nullptr, gexec_a = nullptr, gexec_c = nullptr;
     int64_t graph_kernels = 0, graph_kernels_a = 0, graph_kernels_c = 0;
@@ -754,7 +757,8 @@ int ensure_geom(mhd_ctx *ctx)
 // stream beside PV's FP64 work).  Each sync runs after the pass that writes
 // its fields and before any pass that reads them; the reference's order
 // among these independent fields does not change any value.
-int launch_update_derived_pole(mhd_ctx *ctx);
+int launch_update_derived(mhd_ctx *ctx, bool armed, bool joined);
+int launch_update_derived_pole(mhd_ctx *ctx, bool joined);
 
 // J_cell's own pass when the derived-field pass runs split (k_pv_uplus_dt variant kPvSplit)
 int launch_jcell_split(mhd_ctx *ctx)
@@ -772,17 +776,79 @@ int launch_arm_dt(mhd_ctx *ctx)
     return launched(ctx);
 }
 
-// armed: the dt reductions are (the step's update arms them)
-int launch_update_derived(mhd_ctx *ctx, bool armed)
+// Work beside the main stream: fork() makes the side stream wait for the main
+// one so far, join(e) the main stream for the side one so far; between them
+// launches go to the side stream while a SideScope lives.  Eager profiling
+// times launches one by one on the main stream and does not fork.
+bool forks(const mhd_ctx *ctx) { return !ctx->profiling; }
+int fork_side(mhd_ctx *ctx, int e)
+{
+    CK(ctx, cudaEventRecord(ctx->fork_ev[e], ctx->stream));
+    CK(ctx, cudaStreamWaitEvent(ctx->side, ctx->fork_ev[e], 0));
+    return MHD_OK;
+}
+int mark_side(mhd_ctx *ctx, int e)
+{
+    CK(ctx, cudaEventRecord(ctx->fork_ev[e], ctx->side));
+    return MHD_OK;
+}
+int join_side(mhd_ctx *ctx, int e)
+{
+    CK(ctx, cudaStreamWaitEvent(ctx->stream, ctx->fork_ev[e], 0));
+    return MHD_OK;
+}
+struct SideScope
+{
+    mhd_ctx *ctx;
+    cudaStream_t saved;
+    explicit SideScope(mhd_ctx *c) : ctx(c), saved(c->stream) { c->stream = c->side; }
+    ~SideScope() { ctx->stream = saved; }
+};
+
+// Sync("Ucell") beside the chain from Sync("Bface") to the J edges, neither of
+// which reads the other's fields: where it has wall or Pole handlers, three to
+// four small launches that the B_cell pass hides (with the Pole J_cell beside the
+// PV pass: a 96 x 64 x 64 shell 230 -> 216 us a step, six shells 877 -> 859, a
+// 4-block slab 34.7 -> 32.6); a copy list alone goes with Sync("Bface")'s in one
+// pass.
+bool side_ucell(const mhd_ctx *ctx)
+{
+    const auto it = ctx->syncs.find("Ucell");
+    return forks(ctx) && it != ctx->syncs.end() && (!it->second.walls.empty() || !ctx->poles.empty());
+}
+
+// Sync("Ucell"), Sync("Bface"), then UpdateDerivedFields_.  armed: the dt
+// reductions are (the step's update arms them).
+int launch_sync_derived(mhd_ctx *ctx, bool armed)
+{
+    if (!side_ucell(ctx))
+    {
+        RUN(run_syncs(ctx, {"Ucell", "Bface"}));
+        return launch_update_derived(ctx, armed, false);
+    }
+    RUN(fork_side(ctx, 0));
+    {
+        SideScope s(ctx);
+        RUN(run_syncs(ctx, {"Ucell"}));
+        RUN(mark_side(ctx, 1));
+    }
+    RUN(run_syncs(ctx, {"Bface"}));
+    return launch_update_derived(ctx, armed, true);
+}
+
+// joined: Sync("Ucell") runs on the side stream (event 1)
+int launch_update_derived(mhd_ctx *ctx, bool armed, bool joined)
 {
     if (!armed)
         RUN(launch_arm_dt(ctx));
     if (!ctx->poles.empty())
-        return launch_update_derived_pole(ctx);
+        return launch_update_derived_pole(ctx, joined);
     cudaStream_t s = ctx->stream;
     prof_begin(ctx, "k_bcell_jedge");
     RUN(launched(ctx, launch_k_bcell_jedge(ctx->tune[TUNE_k_bcell_jedge], ctx->pool32 != nullptr, ctx->hot, s)));
     RUN(run_syncs(ctx, {"B_cell", "Jedge"}));
+    if (joined)
+        RUN(join_side(ctx, 1));
     // J_cell, PV / U_plus and the CFL bound of the next step; the first ghost
     // layer only: deeper PV / U_plus ghosts are read by no kernel of the step
     // and are filled when read out (materialise_pv)
@@ -800,8 +866,9 @@ int launch_update_derived(mhd_ctx *ctx, bool armed)
 // (with PV / U_plus / the CFL bound), its pole-shell repair, and the syncs.
 // B_cell and the J edges run as one pass before the rewrite; the few J edges
 // that read a rewritten face are formed again after it (POLE_JEDGE), with the
-// ring of Sync("Jedge") in the same launch.
-int launch_update_derived_pole(mhd_ctx *ctx)
+// ring of Sync("Jedge") in the same launch.  The pole shell's J_cell reads the
+// J edges only, so it runs beside the PV pass, which leaves those cells out.
+int launch_update_derived_pole(mhd_ctx *ctx, bool joined)
 {
     cudaStream_t s = ctx->stream;
     prof_begin(ctx, "k_bcell_jedge");
@@ -813,12 +880,25 @@ int launch_update_derived_pole(mhd_ctx *ctx)
     else
         RUN(launch_pole(ctx, POLE_JEDGE));
     RUN(run_syncs(ctx, {"Jedge"}, false));
+    const bool split = ctx->tune[TUNE_k_pv_uplus_dt] == kPvSplit, beside = forks(ctx) && !split;
+    if (joined)
+        RUN(join_side(ctx, 1));
+    if (beside)
+    {
+        RUN(fork_side(ctx, 0));
+        SideScope sc(ctx);
+        RUN(launch_pole(ctx, POLE_JCELL_FIRST));
+        RUN(mark_side(ctx, 2));
+    }
     RUN(launch_jcell_split(ctx));
     prof_begin(ctx, "k_pv_uplus_dt");
     ctx->pv_dirty = true;
     RUN(launched(ctx, launch_k_pv_uplus_dt(ctx->tune[TUNE_k_pv_uplus_dt], ctx->pool32 != nullptr, ctx->hot, s, ctx->c,
                                            ctx->dt_key)));
-    RUN(launch_pole(ctx, POLE_JCELL));
+    if (beside)
+        RUN(join_side(ctx, 2));
+    else
+        RUN(launch_pole(ctx, split ? int(POLE_JCELL) : POLE_JCELL_FIRST));
     return run_syncs(ctx, {"J_cell", "Uplus"});
 }
 
@@ -826,23 +906,6 @@ int launch_update_derived_pole(mhd_ctx *ctx)
 RunClock run_clock(const mhd_ctx *ctx)
 {
     return RunClock{ctx->dt_key, ctx->dt, ctx->time, ctx->step, ctx->err, ctx->prm.dt_abort, ctx->nruns};
-}
-
-// Sync("Ucell") and Sync("Bface") in one
-int sync_state(mhd_ctx *ctx)
-{
-    if (!ctx->poles.empty() && ctx->syncs.count("Ucell") && ctx->syncs.count("Bface"))
-    {
-        // both groups' rings in one launch
-        StepSync *s = nullptr;
-        RUN(step_sync(ctx, {"Ucell", "Bface"}, SYNC_HOT, &s));
-        if (s->usable)
-        {
-            RUN(launch_pole(ctx, {POLE_RING_U, POLE_RING_BXI}));
-            return run_syncs(ctx, {"Ucell", "Bface"}, false);
-        }
-    }
-    return run_syncs(ctx, {"Ucell", "Bface"});
 }
 
 // fluid RHS together with the contravariant velocities of the EMF stencils
@@ -1275,8 +1338,7 @@ int launch_step_a(mhd_ctx *ctx) { return launch_euler_core(ctx, true, true); }
 // ... and its closing part: Sync("Ucell"), Sync("Bface"), derived fields
 int launch_step_c(mhd_ctx *ctx)
 {
-    RUN(sync_state(ctx));
-    return launch_update_derived(ctx, true);
+    return launch_sync_derived(ctx, true);
 }
 
 // ResistiveDiffusionSubcycles_ (Z4_Lunar/src/physics/LunarSolver_MagneticRHS.cpp:53-115):
@@ -1613,10 +1675,9 @@ int launch_step_rk2(mhd_ctx *ctx)
     RUN(launch_rk2(ctx, 1));
     RUN(launch_euler_core(ctx, true, false));
     RUN(launch_resistive_part(ctx));
-    RUN(sync_state(ctx));
     // (this stage's CFL bounds are not used: the reductions are armed again by
     // the second stage's update, for the ones of the step's end)
-    RUN(launch_update_derived(ctx, true));
+    RUN(launch_sync_derived(ctx, true));
     RUN(launch_euler_core(ctx, false, true));
     RUN(launch_resistive_part(ctx));
     RUN(launch_rk2(ctx, 0));
@@ -1804,6 +1865,9 @@ void build_hot(mhd_ctx *ctx)
             h.nk = v.nk;
             h.run = v.run;
             h.blk = b0 + q;
+            for (size_t p = 0; p < ctx->poles.size(); p += 2)
+                if (ctx->poles[p] == h.blk)
+                    h.poles |= ctx->poles[p + 1] < 0 ? 1 : 2;
             const int e[3] = {0, 2, 1}; // KIND_CELL0, KIND_CELL1, KIND_STAG
             for (int kind = 0; kind < 3; ++kind)
             {
@@ -1901,8 +1965,12 @@ int create_ctx(const mhd_block_desc *blocks, int32_t nblocks, const int32_t *run
         mhd_ctx_destroy(ctx);
         return code;
     };
-    if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess)
+    if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking) != cudaSuccess)
         return bail(MHD_ECUDA);
+    for (auto &e : ctx->fork_ev)
+        if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess)
+            return bail(MHD_ECUDA);
     {
         void *p = nullptr;
         if (cudaGetSymbolAddress(&p, g_noalloc_staging) != cudaSuccess)
@@ -2043,6 +2111,11 @@ int mhd_ctx_destroy(mhd_ctx *ctx)
     cudaFree(ctx->dbv);
     cudaFree(ctx->pool);
     cudaFree(ctx->pool32);
+    for (auto &e : ctx->fork_ev)
+        if (e)
+            cudaEventDestroy(e);
+    if (ctx->side)
+        cudaStreamDestroy(ctx->side);
     if (ctx->stream)
         cudaStreamDestroy(ctx->stream);
     delete ctx;
@@ -2932,6 +3005,11 @@ static int build_all_syncs(mhd_ctx *ctx)
     StepSync *s = nullptr;
     RUN(step_sync(ctx, {"Eface"}, SYNC_HOT, &s));
     RUN(step_sync(ctx, {"Eedge"}, SYNC_HOT, &s));
+    if (ctx->syncs.count("Ucell") && (!ctx->syncs["Ucell"].walls.empty() || !ctx->poles.empty()))
+    {
+        RUN(step_sync(ctx, {"Ucell"}, SYNC_HOT, &s));
+        RUN(step_sync(ctx, {"Bface"}, SYNC_HOT, &s));
+    }
     RUN(step_sync(ctx, {"Ucell", "Bface"}, SYNC_HOT, &s));
     RUN(step_sync(ctx, {"J_cell", "Uplus"}, SYNC_HOT, &s));
     if (ctx->poles.empty())
@@ -3478,6 +3556,7 @@ int mhd_set_pole(mhd_ctx *ctx, int32_t block, int32_t direction)
     cudaFree(ctx->dpoles);
     ctx->dpoles = nullptr;
     RUN(upload_vec(ctx, ctx->poles, &ctx->dpoles));
+    build_hot(ctx);
     for (auto &kv : ctx->syncs)
         kv.second.built = false;
     ctx->geom_dirty = true; // the rings' normal matrices
@@ -3905,7 +3984,7 @@ int mhd_autotune(mhd_ctx *ctx, int32_t reps, int32_t *min_ctas, int32_t n)
                                 save ? static_cast<const void *>(ctx->dt_key) : static_cast<const void *>(clk),
                                 clock_bytes, cudaMemcpyDeviceToDevice, s));
         if (!save)
-            RUN(launch_update_derived(ctx, false)); // derived fields of the restored state
+            RUN(launch_update_derived(ctx, false, false)); // derived fields of the restored state
         return MHD_OK;
     };
     cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -4107,7 +4186,7 @@ int mhd_update_derived(mhd_ctx *ctx)
     if (!ctx)
         return MHD_EINVAL;
     RUN(ensure_geom(ctx));
-    RUN(launch_update_derived(ctx, false));
+    RUN(launch_update_derived(ctx, false, false));
     CK(ctx, cudaStreamSynchronize(ctx->stream));
     return MHD_OK;
 }
@@ -4200,8 +4279,7 @@ int step_host(mhd_ctx *ctx, int32_t nsteps, const double *state_in, double *stat
             off += n;
         }
     RUN(ensure_geom(ctx));
-    RUN(sync_state(ctx));
-    RUN(launch_update_derived(ctx, false));
+    RUN(launch_sync_derived(ctx, false));
     RUN(run_steps(ctx, nsteps));
     for (int f : {int(F_U), int(F_Bxi)})
         RUN(materialise_field(ctx, f));

@@ -68,6 +68,7 @@ struct HotBlock
     uint32_t o;         // offset of the point (0, 0, 0)
     int ni, nj, nk;
     int run, blk;
+    int poles;          // 1: a Pole at j = 0, 2: at j = n_j
     int cta0[3];        // flattened launches: first CTA per kind, within this launch
     // quotients by n_k + e and n_j + e: e = 0 (KIND_CELL0), 2 (KIND_CELL1), 1 (KIND_STAG)
     FastDiv dk[3], dj[3];

@@ -58,11 +58,12 @@ __global__ void k_geom32(const BlockView *bvs);
 // that touch different points; POLE_JEDGE: Calc_J_Edge again on the J_xi /
 // J_eta edges that read the B_zeta faces POLE_BZETA rewrote (staggered layers
 // jc, jc + 1 of each Pole; jeta_ring = 0: the ring POLE_JETA writes left out).
-// The ring sums run one warp per ring; the least squares' geometry-only normal
+// POLE_JCELL_FIRST: POLE_JCELL beside a derived pass that leaves the rings'
+// J_cell out.  The ring sums run a warp or a CTA per ring; the least squares' geometry-only normal
 // matrices are in `cache` (per Pole, per least-squares operation, `stride`
 // rings, 10 values each), which launch_pole_build fills after every geometry
 // change.  ni, nk: the largest of the Poles' blocks.
-constexpr int POLE_JEDGE = NPOLE_OP;
+constexpr int POLE_JEDGE = NPOLE_OP, POLE_JCELL_FIRST = NPOLE_OP + 1;
 struct PoleOps
 {
     int n;

@@ -10,6 +10,7 @@
 #include "mhd_hot_launch.cuh"
 
 #include <cfloat>
+#include <algorithm>
 #include <cmath>
 
 namespace mhd
@@ -941,7 +942,7 @@ __global__ void k_diag(const BlockView *__restrict__ bvs, int run, unsigned long
 // POLE_JETA in the same launch overwrites in the reference's order.
 __host__ __device__ inline int64_t pole_items(int op, int ni, int nk)
 {
-    return op == POLE_JEDGE ? int64_t(ni + 1) * 2 * (nk + 1) : pole_work(op, ni, nk);
+    return op == POLE_JEDGE ? int64_t(ni + 1) * 2 * (nk + 1) : pole_work(op == POLE_JCELL_FIRST ? POLE_JCELL : op, ni, nk);
 }
 __device__ __forceinline__ void pole_jedge_one(const BlockView &b, int side, int64_t t, int jeta_ring)
 {
@@ -957,150 +958,182 @@ __device__ __forceinline__ void pole_jedge_one(const BlockView &b, int side, int
 
 // ---------------------------------------------------------------------------
 // The ring sums (POLE_RING_U, POLE_RING_BXI) and ring least squares
-// (POLE_BCELL, POLE_EETA_REG / POLE_ERES_REG, POLE_JCELL) with one warp per
-// ring.  The lanes form the pushed vectors, values and products of 32 k at a
-// time (square roots and divisions in parallel, the same operations as
-// pole_one).  Each sum then runs in one lane over the pushes in the
-// reference's order (k, then the handler's order within k), so it equals the
-// one-thread ring sum bit for bit: a skipped push adds +0, which changes no
-// sum that starts at +0.  The normal matrix A and the count depend on the
-// geometry only and are summed once per geometry (build), nine lanes one entry
-// each; every application sums the right-hand side, three lanes one component
-// each, and lane 0 regularises, solves and broadcasts.
+// (POLE_BCELL, POLE_EETA_REG / POLE_ERES_REG, POLE_JCELL), a group of threads
+// per ring.  The threads form the products of a chunk of k (square roots and
+// divisions in parallel, the same operations as pole_one).  Each sum then runs
+// in one lane over the pushes in the reference's order (k, then the handler's
+// order within k), so it equals the one-thread ring sum bit for bit: a skipped
+// push adds +0, which changes no sum that starts at +0.  The normal matrix A
+// and the count depend on the geometry only and are summed once per geometry
+// (build), nine lanes one entry each; every application sums the right-hand
+// side, three lanes one component each, and one lane regularises, solves and
+// broadcasts.
 // What bounds them: the chain of dependent adds (8 nk for J_cell) and two
-// rounds of loads.  With the products formed by all lanes and the sums
-// unrolled over shared memory the chain is adds alone; before, each step read
-// the flag, the value and the vector and branched.
+// rounds of loads.  J_cell's 8 pushes per k, a square root and four divisions
+// each, take a CTA of 128 threads (a warp: 39 us on six shells of 30 to 100
+// rings per Pole, the CTA 29); the others, 1 or 3 pushes per k, a warp (U_H and
+// B_xi rings 12 us against 25 with a CTA each).
 // ---------------------------------------------------------------------------
-constexpr int kPoleWarps = 4; // warps (rings) per CTA
-constexpr int kPoleTerms = 8; // at most 8 pushes per k (J_cell)
+constexpr int kPoleThreads = 128;
+// a ring's group: T threads, K values of k per chunk, at most NQ pushes per k
+template <int T> struct PoleGroup
+{
+    static constexpr int K = T == 32 ? 32 : 64, NQ = T == 32 ? 3 : 8;
+    // a row of products is 2 doubles longer than its pushes, so that the lanes
+    // that sum read different banks
+    static constexpr int ROW = K * NQ + 2;
+    static __host__ __device__ constexpr size_t bytes(bool build)
+    {
+        return ((build ? 9 : 3) * size_t(ROW) + 4) * sizeof(double) + size_t(K) * NQ * sizeof(int);
+    }
+    static __device__ __forceinline__ int tid() { return int(threadIdx.x) % T; }
+    static __device__ __forceinline__ void sync()
+    {
+        if (T == 32)
+            __syncwarp();
+        else
+            __syncthreads();
+    }
+};
 
-// One chunk of pushes of a warp in shared memory: products (apply: phi s[a] in
-// row a; build: s[a] s[c] in row 3 a + c), 0 for a push that is skipped, and
-// its use flag.  Push q of lane l sits at 32 q + l (no bank conflicts for the
-// lanes' writes); a row is 2 doubles longer than its pushes, so that the
-// lanes that sum read different banks.
-constexpr int kPoleRow = 32 * kPoleTerms + 2;
+// One chunk of pushes in shared memory: products (apply: phi s[a] in row a;
+// build: s[a] s[c] in row 3 a + c), 0 for a push that is skipped, and its use
+// flag.  Push q of k sits at K q + k.
 struct PoleChunk
 {
     double *p;
     int *ok;
+    double *x;   // the solution, three values
+    int *status; // 0 solved, 1 no usable push, 2 singular
 };
-__host__ __device__ constexpr size_t pole_chunk_bytes(bool build)
-{
-    return (build ? 9 : 3) * size_t(kPoleRow) * sizeof(double) + 32 * kPoleTerms * sizeof(int);
-}
 
-__device__ __forceinline__ void pole_term(const PoleChunk &sh, int q, bool build, bool ok, const double s[3],
-                                          double phi)
+struct PolePush
 {
-    const int e = 32 * q + (threadIdx.x & 31);
-    sh.ok[e] = ok ? 1 : 0;
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-    {
-        if (!build)
-            sh.p[a * kPoleRow + e] = ok ? phi * s[a] : 0.0;
-        else
-#pragma unroll
-            for (int c = 0; c < 3; ++c)
-                sh.p[(3 * a + c) * kPoleRow + e] = ok ? s[a] * s[c] : 0.0;
-    }
-}
+    double s[3], phi;
+    bool ok;
+};
 
-// the chunk's pushes in order (lane, then the lane's NQ pushes)
-template <int NQ> __device__ __forceinline__ void pole_accumulate(const PoleChunk &sh, bool build, double &acc, int &cnt)
+// the sums of a ring's pushes push(q, k), q < NQ, in order (k, then q): the
+// group's lanes < 3 (build: < 9, and lane 9 the count) return them in acc
+template <int T, int NQ, class Push>
+__device__ __forceinline__ void pole_sum(const PoleChunk &sh, bool build, int nk, Push push, double &acc, int &cnt)
 {
-    const int lane = threadIdx.x & 31;
-    if (lane < (build ? 9 : 3))
+    using G = PoleGroup<T>;
+    constexpr int K = G::K;
+    const int tid = G::tid();
+    for (int k0 = 0; k0 < nk; k0 += K)
     {
-        const double *x = sh.p + lane * kPoleRow;
+        const int nl = min(K, (nk - k0 + 7) & ~7); // whole groups of 8; the tail adds zeros
 #pragma unroll
-        for (int l = 0; l < 32; l += 8 / (NQ > 4 ? 8 : NQ > 1 ? 4 : 1))
+        for (int e = tid; e < K * NQ; e += T)
         {
-            constexpr int L = 8 / (NQ > 4 ? 8 : NQ > 1 ? 4 : 1);
-            double y[L * NQ];
+            const int q = e / K, k = k0 + e % K;
+            PolePush t{{0.0, 0.0, 0.0}, 0.0, false};
+            if (k < nk)
+                t = push(q, k);
+            sh.ok[e] = t.ok ? 1 : 0;
 #pragma unroll
-            for (int e = 0; e < L * NQ; ++e)
-                y[e] = x[32 * (e % NQ) + l + e / NQ];
+            for (int a = 0; a < 3; ++a)
+            {
+                if (!build)
+                    sh.p[a * G::ROW + e] = t.ok ? t.phi * t.s[a] : 0.0;
+                else
 #pragma unroll
-            for (int e = 0; e < L * NQ; ++e)
-                acc += y[e];
+                    for (int c = 0; c < 3; ++c)
+                        sh.p[(3 * a + c) * G::ROW + e] = t.ok ? t.s[a] * t.s[c] : 0.0;
+            }
         }
+        G::sync();
+        if (tid < (build ? 9 : 3))
+        {
+            const double *x = sh.p + tid * G::ROW;
+            constexpr int L = NQ >= 8 ? 1 : NQ >= 3 ? 4 : 8; // k per unrolled group
+            for (int l = 0; l < nl; l += L)
+            {
+                double y[L * NQ];
+#pragma unroll
+                for (int e = 0; e < L * NQ; ++e)
+                    y[e] = x[K * (e % NQ) + l + e / NQ];
+#pragma unroll
+                for (int e = 0; e < L * NQ; ++e)
+                    acc += y[e];
+            }
+        }
+        else if (build && tid == 9)
+            for (int e = 0; e < K * NQ; ++e)
+                cnt += sh.ok[e];
+        G::sync();
     }
-    else if (build && lane == 9)
-        for (int q = 0; q < 32 * NQ; ++q)
-            cnt += sh.ok[q];
 }
 
 // k average of a ring (pole_one's POLE_RING_U / POLE_RING_BXI)
-__device__ __forceinline__ void pole_ring_warp(const BlockView &b, int side, int op, int64_t t, const PoleChunk &sh)
+__device__ __forceinline__ void pole_ring(const BlockView &b, int side, int op, int64_t t, const PoleChunk &sh)
 {
-    const int lane = threadIdx.x & 31;
     const bool u = op == POLE_RING_U;
     const int i = u ? int(t / 5) : int(t), m = u ? int(t % 5) : 0, jc = side < 0 ? 0 : b.nj - 1;
     double *F = b.f[u ? F_U : F_Bxi] + int64_t(m) * b.vol + pidx(b, i, jc, 0);
     double acc = 0.0;
     int cnt = 0;
-    for (int k0 = 0; k0 < b.nk; k0 += 32)
-    {
-        sh.p[lane] = k0 + lane < b.nk ? F[k0 + lane] : 0.0;
-        __syncwarp();
-        if (lane == 0)
-            pole_accumulate<1>(sh, false, acc, cnt);
-        __syncwarp();
-    }
+    // phi s = F 1: the value itself
+    pole_sum<32, 1>(sh, false, b.nk, [&](int, int k) { return PolePush{{1.0, 0.0, 0.0}, F[k], true}; }, acc, cnt);
     const double avg = __shfl_sync(0xffffffffu, acc, 0) / double(b.nk);
-    for (int k = lane; k < b.nk; k += 32)
+    for (int k = threadIdx.x & 31; k < b.nk; k += 32)
         F[k] = avg;
 }
 
-// build: store the ring's A and count (cache[0..8], cache[9]); apply: lane 0
-// loads them, regularises (trace of |A_aa| or of A_aa), solves and
-// broadcasts x.  status: 0 solved, 1 no usable push (count_guard), 2 singular
-__device__ bool pole_finish(double acc, int cnt, bool build, double *cache, bool trace_abs, bool count_guard,
-                            double x[3], int &status)
+// build: store the ring's A and count (cache[0..8], cache[9]) and return
+// false; apply: regularise (trace of |A_aa| or of A_aa), solve, leave x and
+// the status in shared memory; true when solved
+template <int T>
+__device__ bool pole_finish(const PoleChunk &sh, double acc, int cnt, bool build, double *cache, bool trace_abs,
+                            bool count_guard)
 {
-    const int lane = threadIdx.x & 31;
+    const int tid = PoleGroup<T>::tid();
     if (build)
     {
-        if (lane < 9)
-            cache[lane] = acc;
-        else if (lane == 9)
+        if (tid < 9)
+            cache[tid] = acc;
+        else if (tid == 9)
             cache[9] = double(cnt);
-        status = 3;
+        if (tid == 0)
+            *sh.status = 3;
+        PoleGroup<T>::sync();
         return false;
     }
-    const double r0 = __shfl_sync(0xffffffffu, acc, 0), r1 = __shfl_sync(0xffffffffu, acc, 1),
-                 r2 = __shfl_sync(0xffffffffu, acc, 2);
-    int st = 0;
-    double xs[3] = {0.0, 0.0, 0.0};
-    if (lane == 0)
+    if (tid < 32)
     {
-        if (count_guard && int(cache[9]) <= 0)
-            st = 1;
-        else
+        const double r0 = __shfl_sync(0xffffffffu, acc, 0), r1 = __shfl_sync(0xffffffffu, acc, 1),
+                     r2 = __shfl_sync(0xffffffffu, acc, 2);
+        if (tid == 0)
         {
-            double A[3][3] = {{cache[0], cache[1], cache[2]}, {cache[3], cache[4], cache[5]}, {cache[6], cache[7], cache[8]}};
-            const double rhs[3] = {r0, r1, r2};
-            const double tr = trace_abs ? fabs(A[0][0]) + fabs(A[1][1]) + fabs(A[2][2]) : A[0][0] + A[1][1] + A[2][2];
-            const double reg = 1.0e-12 * pole_max1(tr);
-            A[0][0] += reg;
-            A[1][1] += reg;
-            A[2][2] += reg;
-            st = pole_solve3(A, rhs, xs) ? 0 : 2;
+            int st = 0;
+            double xs[3] = {0.0, 0.0, 0.0};
+            if (count_guard && int(cache[9]) <= 0)
+                st = 1;
+            else
+            {
+                double A[3][3] = {
+                    {cache[0], cache[1], cache[2]}, {cache[3], cache[4], cache[5]}, {cache[6], cache[7], cache[8]}};
+                const double rhs[3] = {r0, r1, r2};
+                const double tr =
+                    trace_abs ? fabs(A[0][0]) + fabs(A[1][1]) + fabs(A[2][2]) : A[0][0] + A[1][1] + A[2][2];
+                const double reg = 1.0e-12 * pole_max1(tr);
+                A[0][0] += reg;
+                A[1][1] += reg;
+                A[2][2] += reg;
+                st = pole_solve3(A, rhs, xs) ? 0 : 2;
+            }
+            *sh.status = st;
+            for (int c = 0; c < 3; ++c)
+                sh.x[c] = xs[c];
         }
     }
-    status = __shfl_sync(0xffffffffu, st, 0);
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-        x[c] = __shfl_sync(0xffffffffu, xs[c], 0);
-    return status == 0;
+    PoleGroup<T>::sync();
+    return *sh.status == 0;
 }
 
-__device__ void pole_bcell_warp(const BlockView &b, int side, int64_t t, const PoleChunk &sh, double *cache, bool build)
+__device__ void pole_bcell(const BlockView &b, int side, int64_t t, const PoleChunk &sh, double *cache, bool build)
 {
-    const int lane = threadIdx.x & 31;
     const int nj = b.nj, nk = b.nk;
     const int64_t v = b.vol;
     const int i = int(t >> 1);
@@ -1112,60 +1145,46 @@ __device__ void pole_bcell_warp(const BlockView &b, int side, int64_t t, const P
     const double sn = side < 0 ? 1.0 : -1.0;
     const double *Aet = b.f[F_JDeta], *Axi = b.f[F_JDxi];
     const double *Bet = b.f[F_Beta], *Bxi = b.f[F_Bxi], *Aadd = b.f[F_Baddeta], *Xadd = b.f[F_Baddxi];
-    const double zero[3] = {0.0, 0.0, 0.0};
     double acc = 0.0;
     int cnt = 0;
-    for (int k0 = 0; k0 < nk; k0 += 32)
-    {
-        const int k = k0 + lane;
-        if (k < nk)
-        {
-            const int64_t pn = pidx(b, i, jn, k), p0 = pidx(b, i, jc, k), p1 = pidx(b, i + 1, jc, k);
-            double f[3] = {Bet[pn], Bxi[p0], Bxi[p1]};
+    // outer eta face, low and high xi face of each cell of the ring
+    pole_sum<32, 3>(
+        sh, build, nk,
+        [&](int q, int k) {
+            const int64_t p = q == 0 ? pidx(b, i, jn, k) : q == 1 ? pidx(b, i, jc, k) : pidx(b, i + 1, jc, k);
+            const double *A = q == 0 ? Aet : Axi;
+            const double a0 = A[p], a1 = A[v + p], a2 = A[2 * v + p];
+            double f = q == 0 ? Bet[p] : Bxi[p];
             if (total)
-            {
-                f[0] += Aadd[pn];
-                f[1] += Xadd[p0];
-                f[2] += Xadd[p1];
-            }
-            const double S[3][3] = {{sn * Aet[pn], sn * Aet[v + pn], sn * Aet[2 * v + pn]},
-                                    {-Axi[p0], -Axi[v + p0], -Axi[2 * v + p0]},
-                                    {Axi[p1], Axi[v + p1], Axi[2 * v + p1]}};
-            const double phi[3] = {sn * f[0], -f[1], f[2]};
-#pragma unroll
-            for (int q = 0; q < 3; ++q)
-                pole_term(sh, q, build,
-                          !((S[q][0] * S[q][0] + S[q][1] * S[q][1] + S[q][2] * S[q][2]) <= 1.0e-300), S[q], phi[q]);
-        }
-        else
-            for (int q = 0; q < 3; ++q)
-                pole_term(sh, q, build, false, zero, 0.0);
-        __syncwarp();
-        pole_accumulate<3>(sh, build, acc, cnt);
-        __syncwarp();
-    }
+                f += q == 0 ? Aadd[p] : Xadd[p];
+            PolePush o;
+            o.s[0] = q == 0 ? sn * a0 : q == 1 ? -a0 : a0;
+            o.s[1] = q == 0 ? sn * a1 : q == 1 ? -a1 : a1;
+            o.s[2] = q == 0 ? sn * a2 : q == 1 ? -a2 : a2;
+            o.phi = q == 0 ? sn * f : q == 1 ? -f : f;
+            o.ok = !((o.s[0] * o.s[0] + o.s[1] * o.s[1] + o.s[2] * o.s[2]) <= 1.0e-300);
+            return o;
+        },
+        acc, cnt);
     // BC_Pole_Bcell_Collapse_ solves whenever the regularised system is regular
-    double Bp[3];
-    int st;
-    if (!pole_finish(acc, cnt, build, cache, true, false, Bp, st))
+    if (!pole_finish<32>(sh, acc, cnt, build, cache, true, false))
         return;
     double *Out = b.f[total ? F_Bcell : F_Bind];
-    for (int k = lane; k < nk; k += 32)
+    for (int k = threadIdx.x & 31; k < nk; k += 32)
     {
         const int64_t p = pidx(b, i, jc, k);
-        Out[p] = Bp[0];
-        Out[v + p] = Bp[1];
-        Out[2 * v + p] = Bp[2];
+        Out[p] = sh.x[0];
+        Out[v + p] = sh.x[1];
+        Out[2 * v + p] = sh.x[2];
     }
 }
 
 // the regulation of E_eta (field F_Eeta) or Eres_eta (F_Ereseta): both are
 // eta edges of the same ring, so their normal matrices (from dr_eta) are one
-__device__ void pole_eeta_warp(const BlockView &b, int side, int64_t t, const PoleChunk &sh, double *cache, bool build,
-                               int field)
+__device__ void pole_eeta(const BlockView &b, int side, int64_t t, const PoleChunk &sh, double *cache, bool build,
+                          int field)
 {
-    const int lane = threadIdx.x & 31;
-    const int nj = b.nj, nk = b.nk;
+    const int nj = b.nj, nk = b.nk, tid = threadIdx.x & 31;
     const int64_t v = b.vol;
     const int i = int(t);
     const int jc = side < 0 ? 0 : nj - 1;
@@ -1173,197 +1192,200 @@ __device__ void pole_eeta_warp(const BlockView &b, int side, int64_t t, const Po
     const double *dr = b.f[F_dreta];
     double acc = 0.0;
     int cnt = 0;
-    for (int k0 = 0; k0 < nk; k0 += 32) // k = n_k is the same edge as k = 0
-    {
-        const int k = k0 + lane;
-        double s[3] = {0.0, 0.0, 0.0}, phi = 0.0;
-        bool ok = false;
-        if (k < nk)
-        {
+    // k = n_k is the same edge as k = 0
+    pole_sum<32, 1>(
+        sh, build, nk,
+        [&](int, int k) {
             const int64_t p = pidx(b, i, jc, k);
             const double d0 = dr[p], d1 = dr[v + p], d2 = dr[2 * v + p];
             const double e = build ? 0.0 : E[p];
             const double L = sqrt(d0 * d0 + d1 * d1 + d2 * d2);
-            ok = !(L < 1.0e-14);
             const double invL = 1.0 / L;
-            s[0] = d0 * invL;
-            s[1] = d1 * invL;
-            s[2] = d2 * invL;
-            phi = e * invL;
-        }
-        pole_term(sh, 0, build, ok, s, phi);
-        __syncwarp();
-        pole_accumulate<1>(sh, build, acc, cnt);
-        __syncwarp();
-    }
-    double Ev[3];
-    int st;
-    if (pole_finish(acc, cnt, build, cache, false, true, Ev, st))
+            return PolePush{{d0 * invL, d1 * invL, d2 * invL}, e * invL, !(L < 1.0e-14)};
+        },
+        acc, cnt);
+    if (pole_finish<32>(sh, acc, cnt, build, cache, false, true))
     {
-        for (int k = lane; k <= nk; k += 32)
+        for (int k = tid; k <= nk; k += 32)
         {
             const int64_t p = pidx(b, i, jc, k);
             const double d0 = dr[p], d1 = dr[v + p], d2 = dr[2 * v + p];
             const double L = sqrt(d0 * d0 + d1 * d1 + d2 * d2);
-            E[p] = (L < 1.0e-14) ? 0.0 : Ev[0] * d0 + Ev[1] * d1 + Ev[2] * d2;
+            E[p] = (L < 1.0e-14) ? 0.0 : sh.x[0] * d0 + sh.x[1] * d1 + sh.x[2] * d2;
         }
         return;
     }
-    if (st == 1) // no usable edge
+    if (*sh.status == 1) // no usable edge
     {
-        for (int k = lane; k <= nk; k += 32)
+        for (int k = tid; k <= nk; k += 32)
             E[pidx(b, i, jc, k)] = 0.0;
         return;
     }
-    if (st != 2)
+    if (*sh.status != 2)
         return; // build
-    // singular system: the ring average, summed in k order by lane 0
-    double avg = 0.0;
-    if (lane == 0)
+    // singular system: the ring average, summed in k order by one thread
+    if (tid == 0)
     {
+        double avg = 0.0;
         for (int k = 0; k <= nk; ++k)
             avg += E[pidx(b, i, jc, k)];
-        avg /= double(nk + 1);
+        sh.x[0] = avg / double(nk + 1);
     }
-    avg = __shfl_sync(0xffffffffu, avg, 0);
-    for (int k = lane; k <= nk; k += 32)
-        E[pidx(b, i, jc, k)] = avg;
+    __syncwarp();
+    for (int k = tid; k <= nk; k += 32)
+        E[pidx(b, i, jc, k)] = sh.x[0];
 }
 
-__device__ void pole_jcell_warp(const BlockView &b, int side, int64_t t, const PoleChunk &sh, double *cache, bool build)
+// calc_Jcell of one cell (LunarSolver_Tools.cpp:837-892), with the weights the
+// derived pass uses
+__device__ void jcell_plain(const BlockView &b, int i, int j, int k)
 {
-    const int lane = threadIdx.x & 31;
+    const double *Jx = b.f[F_Jxi], *Je = b.f[F_Jeta], *Jz = b.f[F_Jzeta];
+    const double s[12] = {Jx[pidx(b, i, j, k)],         Jx[pidx(b, i, j + 1, k)],     Jx[pidx(b, i, j, k + 1)],
+                          Jx[pidx(b, i, j + 1, k + 1)], Je[pidx(b, i, j, k)],         Je[pidx(b, i + 1, j, k)],
+                          Je[pidx(b, i, j, k + 1)],     Je[pidx(b, i + 1, j, k + 1)], Jz[pidx(b, i, j, k)],
+                          Jz[pidx(b, i + 1, j, k)],     Jz[pidx(b, i, j + 1, k)],     Jz[pidx(b, i + 1, j + 1, k)]};
+    const int64_t p = pidx(b, i, j, k), v = b.vol;
+    for (int c = 0; c < 3; ++c)
+    {
+        double J = 0.0;
+        for (int q = 0; q < 12; ++q)
+        {
+            const int64_t w = (12 * c + q) * v + p;
+            J += (b.w32 ? double(b.w32[W32_J * v + w]) : b.f[F_WJ][w]) * s[q];
+        }
+        b.f[F_Jcell][c * v + p] = J;
+    }
+}
+
+// first: the derived pass leaves the ring out, so a ring without a solution
+// takes calc_Jcell's values here (else it holds them already)
+__device__ void pole_jcell(const BlockView &b, int side, int64_t t, const PoleChunk &sh, double *cache, bool build,
+                           bool first)
+{
     const int nj = b.nj, nk = b.nk;
     const int64_t v = b.vol;
     const int i = int(t);
     const int jc = side < 0 ? 0 : nj - 1;
     const int jt = side < 0 ? jc + 1 : jc; // node plane one layer away from the Pole
-    // the 8 pushes of each k, in the order of the reference's loop
-    const int di[8] = {0, 1, 0, 1, 0, 0, 0, 1};
-    const int dk[8] = {0, 0, 1, 1, 0, 1, 0, 0};
-    const int fj[8] = {F_Jeta, F_Jeta, F_Jeta, F_Jeta, F_Jxi, F_Jxi, F_Jzeta, F_Jzeta};
-    const int fd[8] = {F_dreta, F_dreta, F_dreta, F_dreta, F_drxi, F_drxi, F_drzeta, F_drzeta};
     double acc = 0.0;
     int cnt = 0;
-    for (int k0 = 0; k0 < nk; k0 += 32)
-    {
-        const int k = k0 + lane;
-#pragma unroll
-        for (int q = 0; q < 8; ++q)
-        {
-            double s[3] = {0.0, 0.0, 0.0}, phi = 0.0;
-            bool ok = false;
-            if (k < nk)
-            {
-                const int64_t p = pidx(b, i + di[q], q < 4 ? jc : jt, k + dk[q]);
-                const double *dr = b.f[fd[q]];
-                const double dx = dr[p], dy = dr[v + p], dz = dr[2 * v + p];
-                const double J = build ? 0.0 : b.f[fj[q]][p];
-                const double L = sqrt(dx * dx + dy * dy + dz * dz);
-                ok = !(L < 1.0e-14);
-                s[0] = dx / L;
-                s[1] = dy / L;
-                s[2] = dz / L;
-                phi = J / L;
-            }
-            pole_term(sh, q, build, ok, s, phi);
-        }
-        __syncwarp();
-        pole_accumulate<8>(sh, build, acc, cnt);
-        __syncwarp();
-    }
-    double Jp[3];
-    int st;
-    if (!pole_finish(acc, cnt, build, cache, false, true, Jp, st))
+    // the 8 pushes of each k, in the order of the reference's loop: the four
+    // eta edges of the ring's cell, then two xi and two zeta edges at jt
+    pole_sum<kPoleThreads, 8>(
+        sh, build, nk,
+        [&](int q, int k) {
+            const int fa = q < 4 ? 1 : q < 6 ? 0 : 2;
+            const int di = q < 4 ? (q & 1) : q == 7, dk = q < 4 ? (q >> 1) : q == 5;
+            const int64_t p = pidx(b, i + di, fa == 1 ? jc : jt, k + dk);
+            const double *dr = b.f[F_drxi + fa];
+            const double dx = dr[p], dy = dr[v + p], dz = dr[2 * v + p];
+            const double J = build ? 0.0 : b.f[F_Jxi + fa][p];
+            const double L = sqrt(dx * dx + dy * dy + dz * dz);
+            return PolePush{{dx / L, dy / L, dz / L}, J / L, !(L < 1.0e-14)};
+        },
+        acc, cnt);
+    const bool solved = pole_finish<kPoleThreads>(sh, acc, cnt, build, cache, false, true);
+    if (build || (!solved && !first))
         return;
     double *Jc = b.f[F_Jcell];
-    for (int k = lane; k < nk; k += 32)
+    for (int k = threadIdx.x; k < nk; k += kPoleThreads)
     {
+        if (!solved)
+        {
+            jcell_plain(b, i, jc, k);
+            continue;
+        }
         const int64_t p = pidx(b, i, jc, k);
-        Jc[p] = Jp[0];
-        Jc[v + p] = Jp[1];
-        Jc[2 * v + p] = Jp[2];
+        Jc[p] = sh.x[0];
+        Jc[v + p] = sh.x[1];
+        Jc[2 * v + p] = sh.x[2];
     }
 }
 
 // which of the three least-squares operations (cache slot), -1 otherwise
 __host__ __device__ inline int pole_lsq_slot(int op)
 {
-    return op == POLE_BCELL ? 0 : (op == POLE_EETA_REG || op == POLE_ERES_REG) ? 1 : op == POLE_JCELL ? 2 : -1;
+    return op == POLE_BCELL                                  ? 0
+           : (op == POLE_EETA_REG || op == POLE_ERES_REG)    ? 1
+           : (op == POLE_JCELL || op == POLE_JCELL_FIRST)    ? 2
+                                                             : -1;
 }
 
-__host__ __device__ inline bool pole_ring_op(int op)
+// work items of an operation per CTA: rings by a CTA, rings by a warp, items by a thread
+__host__ __device__ inline int pole_per_cta(int op)
 {
-    return op == POLE_RING_U || op == POLE_RING_BXI || pole_lsq_slot(op) >= 0;
+    return pole_lsq_slot(op) == 2                                                      ? 1
+           : (op == POLE_RING_U || op == POLE_RING_BXI || pole_lsq_slot(op) >= 0) ? kPoleThreads / 32
+                                                                                  : kPoleThreads;
 }
 
-// cache: per Pole, per least-squares operation, per ring i (stride rings):
-// A (9 values) and the push count
-__device__ __forceinline__ void pole_warp_item(const BlockView &b, int side, int pole, int op, int64_t t,
-                                               const PoleChunk &sh,                                               double *cache, int stride, bool build)
-{
-    if (t >= pole_work(op, b.ni, b.nk))
-        return; // the whole warp leaves together
-    if (pole_lsq_slot(op) < 0)
-    {
-        pole_ring_warp(b, side, op, t, sh);
-        return;
-    }
-    const int ring = (op == POLE_BCELL) ? int(t >> 1) : int(t);
-    double *c = cache + ((int64_t(pole) * 3 + pole_lsq_slot(op)) * stride + ring) * 10;
-    if (op == POLE_BCELL)
-        pole_bcell_warp(b, side, t, sh, c, build);
-    else if (op == POLE_EETA_REG || op == POLE_ERES_REG)
-        pole_eeta_warp(b, side, t, sh, c, build, op == POLE_ERES_REG ? F_Ereseta : F_Eeta);
-    else
-        pole_jcell_warp(b, side, t, sh, c, build);
-}
-
-// up to four operations on every Pole (grid row): rings one warp each, the
-// others one thread per work item
-__global__ void __launch_bounds__(32 * kPoleWarps) k_pole(const BlockView *__restrict__ bvs,
-                                                          const int *__restrict__ poles, PoleOps ops,
-                                                          double *__restrict__ cache, int stride, int build)
+// up to four operations on every Pole (grid row).  cache: per Pole, per
+// least-squares operation, per ring i (stride rings): A (9 values) and the
+// push count
+__global__ void __launch_bounds__(kPoleThreads) k_pole(const BlockView *__restrict__ bvs, const int *__restrict__ poles,
+                                                       PoleOps ops, double *__restrict__ cache, int stride, int build)
 {
     extern __shared__ __align__(16) unsigned char pole_smem[];
-    unsigned char *mine = pole_smem + (threadIdx.x >> 5) * pole_chunk_bytes(build != 0);
-    const PoleChunk sh{reinterpret_cast<double *>(mine),
-                       reinterpret_cast<int *>(mine + (build ? 9 : 3) * size_t(kPoleRow) * sizeof(double))};
     int q = 0;
     while (q + 1 < ops.n && int(blockIdx.x) >= ops.cta0[q + 1])
         ++q;
-    const int op = ops.op[q];
+    const int op = ops.op[q], per = pole_per_cta(op);
     const int64_t cta = int(blockIdx.x) - ops.cta0[q];
     const BlockView &b = bvs[poles[2 * blockIdx.y]];
     const int side = poles[2 * blockIdx.y + 1] > 0 ? 1 : -1;
     pdl_wait();
-    if (pole_ring_op(op))
+    if (per == kPoleThreads)
     {
-        const int warp = threadIdx.x >> 5;
-        pole_warp_item(b, side, int(blockIdx.y), op, cta * kPoleWarps + warp, sh, cache, stride, build != 0);
+        const int64_t t = cta * kPoleThreads + threadIdx.x;
+        if (op == POLE_JEDGE)
+            pole_jedge_one(b, side, t, ops.jeta_ring);
+        else
+            pole_one(b, side, op, t);
+        return;
     }
-    else if (op == POLE_JEDGE)
-        pole_jedge_one(b, side, cta * blockDim.x + threadIdx.x, ops.jeta_ring);
+    const int warp = threadIdx.x >> 5;
+    const int64_t t = per == 1 ? cta : cta * per + warp;
+    if (t >= pole_items(op, b.ni, b.nk))
+        return; // the whole group leaves together
+    // the group's chunk: products, solution and status, use flags
+    unsigned char *mine = pole_smem + (per == 1 ? 0 : warp * PoleGroup<32>::bytes(build != 0));
+    const int rows = build ? 9 : 3, row = per == 1 ? PoleGroup<kPoleThreads>::ROW : PoleGroup<32>::ROW;
+    double *sp = reinterpret_cast<double *>(mine) + rows * row;
+    const PoleChunk sh{reinterpret_cast<double *>(mine), reinterpret_cast<int *>(sp + 4), sp,
+                       reinterpret_cast<int *>(sp + 3)};
+    if (pole_lsq_slot(op) < 0)
+    {
+        pole_ring(b, side, op, t, sh);
+        return;
+    }
+    const int ring = op == POLE_BCELL ? int(t >> 1) : int(t);
+    double *c = cache + ((int64_t(blockIdx.y) * 3 + pole_lsq_slot(op)) * stride + ring) * 10;
+    if (op == POLE_BCELL)
+        pole_bcell(b, side, t, sh, c, build != 0);
+    else if (op == POLE_EETA_REG || op == POLE_ERES_REG)
+        pole_eeta(b, side, t, sh, c, build != 0, op == POLE_ERES_REG ? F_Ereseta : F_Eeta);
     else
-        pole_one(b, side, op, cta * blockDim.x + threadIdx.x);
+        pole_jcell(b, side, t, sh, c, build != 0, op == POLE_JCELL_FIRST);
 }
 
 static void pole_launch(PoleOps ops, int ni, int nk, int npoles, cudaStream_t st, const BlockView *bvs,
                         const int *poles, double *cache, int stride, int build)
 {
     int x = 0;
+    size_t smem = 0;
     for (int q = 0; q < ops.n; ++q)
     {
+        const int per = pole_per_cta(ops.op[q]);
         ops.cta0[q] = x;
-        const int64_t w = pole_items(ops.op[q], ni, nk), per = pole_ring_op(ops.op[q]) ? kPoleWarps : 32 * kPoleWarps;
-        x += int((w + per - 1) / per);
+        x += int((pole_items(ops.op[q], ni, nk) + per - 1) / per);
+        smem = std::max(smem, per == 1              ? PoleGroup<kPoleThreads>::bytes(build != 0)
+                              : per < kPoleThreads ? per * PoleGroup<32>::bytes(build != 0)
+                                                   : size_t(0));
     }
     ops.cta0[ops.n] = x;
-    const size_t smem = pole_chunk_bytes(build != 0) * kPoleWarps;
-    if (build)
-        cudaFuncSetAttribute(k_pole, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-    pdl_launch(k_pole, dim3(unsigned(x), unsigned(npoles)), 32 * kPoleWarps, smem, st, bvs, poles, ops, cache,
-               stride, build);
+    pdl_launch(k_pole, dim3(unsigned(x), unsigned(npoles)), kPoleThreads, smem, st, bvs, poles, ops, cache, stride,
+               build);
 }
 
 void launch_pole_ops(PoleOps ops, int ni, int nk, int npoles, cudaStream_t st, const BlockView *bvs, const int *poles,

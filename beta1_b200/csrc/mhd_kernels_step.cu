@@ -865,6 +865,8 @@ __device__ __forceinline__ void pv_uplus_dt_body(const A &a, const Consts &c, un
     {
         const uint64_t v = b.vol;
         const bool inner = hot_inner(b, i, j, k);
+        // the Pole rings' J_cell is the least squares beside this pass (POLE_JCELL_FIRST)
+        const bool jc = JCELL && inner && !((b.poles & 1) && j == 0) && !((b.poles & 2) && j == b.nj - 1);
         double U[5];
 #pragma unroll
         for (int m = 0; m < 5; ++m)
@@ -876,7 +878,7 @@ __device__ __forceinline__ void pv_uplus_dt_body(const A &a, const Consts &c, un
         // against 201 us on 2.27 M cells; its weights take half the registers).
         constexpr bool kEarly = sizeof(WT) == sizeof(double);
         double jx, jy, jz;
-        if (JCELL && inner && !kEarly)
+        if (jc && !kEarly)
             jcell_sum<WT>(b, p, jx, jy, jz);
         const CellState s = cell_state(U, c);
         if (kEarly)
@@ -922,7 +924,7 @@ __device__ __forceinline__ void pv_uplus_dt_body(const A &a, const Consts &c, un
                 if (denom > 0.0)
                     dtc = c.cfl * V / denom;
             }
-            if (JCELL)
+            if (jc)
             {
                 if (kEarly)
                     jcell_sum<WT>(b, p, jx, jy, jz);
