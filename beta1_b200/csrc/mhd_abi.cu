@@ -237,6 +237,12 @@ struct mhd_ctx
     double *time = nullptr;
     long long *step = nullptr;
     int *err = nullptr;
+    // mapped host memory the step's kernels leave dt, time [nruns] and the
+    // error word in, and its device addresses
+    volatile double *h_mirror = nullptr;
+    volatile int *h_err = nullptr;
+    double *d_mirror = nullptr;
+    int *d_err = nullptr;
     double *qref = nullptr; // [nruns][6]
     int *cta_tab = nullptr; // block of every CTA of the face-tiled kernels (batches)
     int64_t tiles = 0;      // those CTAs
@@ -905,7 +911,8 @@ int launch_update_derived_pole(mhd_ctx *ctx, bool joined)
 // the runs' clocks, for the kernel that starts or ends a step
 RunClock run_clock(const mhd_ctx *ctx)
 {
-    return RunClock{ctx->dt_key, ctx->dt, ctx->time, ctx->step, ctx->err, ctx->prm.dt_abort, ctx->nruns};
+    return RunClock{ctx->dt_key, ctx->dt, ctx->time, ctx->step, ctx->err, ctx->prm.dt_abort, ctx->nruns,
+                    ctx->d_err, ctx->d_mirror, ctx->d_mirror + ctx->nruns};
 }
 
 // fluid RHS together with the contravariant velocities of the EMF stencils
@@ -1284,6 +1291,7 @@ int launch_gmres_persistent(mhd_ctx *ctx)
     a.atol = R.atol;
     a.bar = R.bar;
     a.err = ctx->err;
+    a.h_err = ctx->d_err;
     a.fa = FusedList{R.fa.dst, R.fa.kind, R.fa.idx, R.fa.val, R.fa.blk, R.fa.n};
     a.fb = FusedList{R.fb.dst, R.fb.kind, R.fb.idx, R.fb.val, R.fb.blk, R.fb.n};
     cudaLaunchConfig_t cfg = {};
@@ -1699,9 +1707,12 @@ int launch_step(mhd_ctx *ctx)
 
 int check_err(mhd_ctx *ctx)
 {
-    int e = 0;
-    CK(ctx, cudaMemcpyAsync(&e, ctx->err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     CK(ctx, cudaStreamSynchronize(ctx->stream));
+    if (*ctx->h_err == 0)
+        return MHD_OK;
+    *ctx->h_err = 0;
+    int e = 0;
+    CK(ctx, cudaMemcpy(&e, ctx->err, sizeof(int), cudaMemcpyDeviceToHost));
     if (e == MHD_EDT)
     {
         double d = 0.0;
@@ -1717,6 +1728,27 @@ int check_err(mhd_ctx *ctx)
         if (ctx->res.bar)
             cudaMemset(ctx->res.bar, 0, 4 * sizeof(unsigned));
         return fail(ctx, MHD_EKRYLOV, "persistent Krylov solve: a grid barrier wait gave up");
+    }
+    return MHD_OK;
+}
+
+// dt and time of the first nr runs after nsteps steps and check_err(): from
+// the host memory the steps left them in, or, without a step, from the device
+int read_clock(mhd_ctx *ctx, int nsteps, size_t nr, double *dt_out, double *time_out)
+{
+    for (size_t r = 0; nsteps > 0 && r < nr; ++r)
+    {
+        if (dt_out)
+            dt_out[r] = ctx->h_mirror[r];
+        if (time_out)
+            time_out[r] = ctx->h_mirror[size_t(ctx->nruns) + r];
+    }
+    if (nsteps == 0 && nr > 0)
+    {
+        if (dt_out)
+            CK(ctx, cudaMemcpy(dt_out, ctx->dt, 8 * nr, cudaMemcpyDeviceToHost));
+        if (time_out)
+            CK(ctx, cudaMemcpy(time_out, ctx->time, 8 * nr, cudaMemcpyDeviceToHost));
     }
     return MHD_OK;
 }
@@ -2029,6 +2061,16 @@ int create_ctx(const mhd_block_desc *blocks, int32_t nblocks, const int32_t *run
         if (cudaMemcpy(ctx->dt_key, keys.data(), 8 * nr, cudaMemcpyHostToDevice) != cudaSuccess)
             return bail(MHD_ECUDA);
     }
+    void *hm = nullptr, *dm = nullptr;
+    if (cudaHostAlloc(&hm, 16 * nr + 8, cudaHostAllocMapped) != cudaSuccess)
+        return bail(MHD_ENOMEM);
+    std::memset(hm, 0, 16 * nr + 8);
+    ctx->h_mirror = static_cast<volatile double *>(hm);
+    ctx->h_err = reinterpret_cast<volatile int *>(static_cast<char *>(hm) + 16 * nr);
+    if (cudaHostGetDevicePointer(&dm, hm, 0) != cudaSuccess)
+        return bail(MHD_ECUDA);
+    ctx->d_mirror = static_cast<double *>(dm);
+    ctx->d_err = reinterpret_cast<int *>(static_cast<char *>(dm) + 16 * nr);
     for (int b = 0; b < nblocks; ++b)
         ctx->hbv[size_t(b)].qref = ctx->qref + 6 * size_t(run[size_t(b)]);
     // a batch of several runs launches one grid row of every block's CTAs: the
@@ -2105,6 +2147,8 @@ int mhd_ctx_destroy(mhd_ctx *ctx)
             cudaStreamDestroy(sp);
     if (ctx->dt_key)
         cudaFree(ctx->dt_key);
+    if (ctx->h_mirror)
+        cudaFreeHost(const_cast<double *>(ctx->h_mirror));
     cudaFree(ctx->cta_tab);
     cudaFree(ctx->rk);
     cudaFree(ctx->staging);
@@ -2182,6 +2226,11 @@ static int transfer(mhd_ctx *ctx, const char *name, int32_t block, const double 
                                                                 hi[0] - lo[0], hi[1] - lo[1], hi[2] - lo[2],
                                                                 ctx->staging);
         RUN(launched(ctx));
+        // a copy from pageable memory has read its source when it returns
+        cudaPointerAttributes at{};
+        if (cudaPointerGetAttributes(&at, hin) == cudaSuccess && at.type == cudaMemoryTypeUnregistered)
+            return MHD_OK;
+        cudaGetLastError();
     }
     else
     {
@@ -4198,11 +4247,7 @@ int mhd_step(mhd_ctx *ctx, int32_t nsteps, double *dt_out, double *time_out)
         return MHD_EINVAL;
     RUN(run_steps(ctx, nsteps));
     RUN(check_err(ctx));
-    if (dt_out)
-        CK(ctx, cudaMemcpy(dt_out, ctx->dt, 8, cudaMemcpyDeviceToHost));
-    if (time_out)
-        CK(ctx, cudaMemcpy(time_out, ctx->time, 8, cudaMemcpyDeviceToHost));
-    return MHD_OK;
+    return read_clock(ctx, nsteps, 1, dt_out, time_out);
 }
 
 int mhd_batch_step(mhd_ctx *ctx, int32_t nsteps, double *dt_out, double *time_out, int32_t nruns)
@@ -4214,12 +4259,7 @@ int mhd_batch_step(mhd_ctx *ctx, int32_t nsteps, double *dt_out, double *time_ou
         return fail(ctx, MHD_EINVAL, "the context holds %d runs, not %d", ctx->nruns, nruns);
     RUN(run_steps(ctx, nsteps));
     RUN(check_err(ctx));
-    const size_t nr = size_t(nruns);
-    if (dt_out && nr)
-        CK(ctx, cudaMemcpy(dt_out, ctx->dt, 8 * nr, cudaMemcpyDeviceToHost));
-    if (time_out && nr)
-        CK(ctx, cudaMemcpy(time_out, ctx->time, 8 * nr, cudaMemcpyDeviceToHost));
-    return MHD_OK;
+    return read_clock(ctx, nsteps, size_t(nruns), dt_out, time_out);
 }
 
 namespace
@@ -4299,9 +4339,7 @@ int step_host(mhd_ctx *ctx, int32_t nsteps, const double *state_in, double *stat
         }
     CK(ctx, cudaMemcpyAsync(state_out, ctx->staging, size_t(count) * 8, cudaMemcpyDeviceToHost, ctx->stream));
     RUN(check_err(ctx));
-    if (dt_out)
-        CK(ctx, cudaMemcpy(dt_out, ctx->dt, 8, cudaMemcpyDeviceToHost));
-    return MHD_OK;
+    return read_clock(ctx, nsteps, 1, dt_out, nullptr);
 }
 } // namespace
 

@@ -32,18 +32,28 @@ struct RunClock
     int *err;
     double dt_abort;
     int nruns;
+    // the host's copy of error word, dt and time (mapped host memory): read
+    // after a stream synchronisation, so a step needs no copies back
+    volatile int *h_err;
+    volatile double *h_dt, *h_time;
 };
 #ifdef __CUDACC__
 __device__ __forceinline__ void begin_run(const RunClock &rc, int r)
 {
     const double d = __longlong_as_double((long long)rc.dt_key[r]);
     rc.dt[r] = d;
+    rc.h_dt[r] = d;
     if (!isfinite(d) || d < rc.dt_abort)
+    {
         rc.err[0] = MHD_EDT;
+        *rc.h_err = MHD_EDT;
+    }
 }
 __device__ __forceinline__ void end_run(const RunClock &rc, int r)
 {
-    rc.time[r] += rc.dt[r];
+    const double t = rc.time[r] + rc.dt[r];
+    rc.time[r] = t;
+    rc.h_time[r] = t;
     rc.step[r] += 1;
     rc.dt_key[r] = (unsigned long long)__double_as_longlong(1e100); // dt_local's initial bound
 }
@@ -190,6 +200,7 @@ struct ResistSolve
     double rtol, atol;
     unsigned *bar; // arrival count, generation
     int *err;      // set to MHD_EKRYLOV when a barrier wait gives up
+    volatile int *h_err; // ... and its copy in host memory
     // fused operator phases (n < 0: not fused, the copy-list phases run):
     // A: every Eres point the unknowns' writes and Sync("Eres1form") set,
     // each as one expression of the basis vector; B: the Sync("dB") copies,

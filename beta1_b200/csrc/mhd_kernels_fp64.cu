@@ -443,7 +443,7 @@ constexpr long long kBarrierSpins = 1ll << 22; // about a second of polling
 // bar[0]: arrival count, bar[1]: generation, bar[2]: polling limit of every
 // wait (0: kBarrierSpins; a smaller limit is set only by the failure-
 // detection hook mhd_test_stall_barrier, and the host clears it after use)
-__device__ __forceinline__ bool grid_barrier(unsigned *bar, int *err)
+__device__ __forceinline__ bool grid_barrier(unsigned *bar, int *err, volatile int *h_err)
 {
     __shared__ int ok; // one decision for the whole CTA
     __syncthreads();
@@ -468,6 +468,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned *bar, int *err)
                 if (++spins > limit)
                 {
                     atomicExch(err, MHD_EKRYLOV);
+                    *h_err = MHD_EKRYLOV;
                     break;
                 }
                 __nanosleep(64);
@@ -526,7 +527,7 @@ __device__ bool grid_dots(const ResistSolve &a, const double *V, int nv, const d
         }
         __syncthreads();
     }
-    if (!grid_barrier(a.bar, a.err))
+    if (!grid_barrier(a.bar, a.err, a.h_err))
         return false;
     for (int c = warp; c < nd; c += int(blockDim.x >> 5))
     {
@@ -550,7 +551,7 @@ __device__ bool grid_apply(const ResistSolve &a, const DevCopy &l, bool consts_d
     {
         for (int64_t t = t0; t < l.nconst; t += ts)
             a.pool[l.cdst[t]] = l.cval[t];
-        if (!grid_barrier(a.bar, a.err))
+        if (!grid_barrier(a.bar, a.err, a.h_err))
             return false;
     }
     if (l.n == 0)
@@ -559,7 +560,7 @@ __device__ bool grid_apply(const ResistSolve &a, const DevCopy &l, bool consts_d
     {
         for (int64_t t = t0; t < l.n; t += ts)
             l.tmp[t] = a.pool[l.src[t]];
-        if (!grid_barrier(a.bar, a.err))
+        if (!grid_barrier(a.bar, a.err, a.h_err))
             return false;
         for (int64_t t = t0; t < l.n; t += ts)
             a.pool[l.dst[t]] = __ldcg(&l.tmp[t]);
@@ -567,7 +568,7 @@ __device__ bool grid_apply(const ResistSolve &a, const DevCopy &l, bool consts_d
     else
         for (int64_t t = t0; t < l.n; t += ts)
             a.pool[l.dst[t]] = a.pool[l.src[t]];
-    return grid_barrier(a.bar, a.err);
+    return grid_barrier(a.bar, a.err, a.h_err);
 }
 
 // y = A (src / div) (MatMultImplicitResistive_): Eres at the unknowns and
@@ -580,7 +581,7 @@ __device__ bool grid_apply(const ResistSolve &a, const DevCopy &l, bool consts_d
 __device__ bool grid_matvec(const ResistSolve &a, const double *src, double div, bool first_barrier, double *y)
 {
     const int64_t t0 = int64_t(blockIdx.x) * blockDim.x + threadIdx.x, ts = int64_t(gridDim.x) * blockDim.x;
-    if (first_barrier && !grid_barrier(a.bar, a.err))
+    if (first_barrier && !grid_barrier(a.bar, a.err, a.h_err))
         return false;
     const double mdt = -a.dtp[0];
     if (a.fa.n >= 0)
@@ -601,7 +602,7 @@ __device__ bool grid_matvec(const ResistSolve &a, const double *src, double div,
                 v = a.pool[ix];
             a.pool[a.fa.dst[q]] = v;
         }
-        if (!grid_barrier(a.bar, a.err))
+        if (!grid_barrier(a.bar, a.err, a.h_err))
             return false;
     }
     else
@@ -613,7 +614,7 @@ __device__ bool grid_matvec(const ResistSolve &a, const double *src, double div,
         if (a.merge1)
             for (int64_t t = t0; t < a.eres1form.nconst; t += ts)
                 a.pool[a.eres1form.cdst[t]] = a.eres1form.cval[t];
-        if (!grid_barrier(a.bar, a.err))
+        if (!grid_barrier(a.bar, a.err, a.h_err))
             return false;
         if (!grid_apply(a, a.eres1form, a.merge1 != 0))
             return false;
@@ -651,12 +652,12 @@ __device__ bool grid_matvec(const ResistSolve &a, const double *src, double div,
                 v = a.pool[ix];
             a.pool[a.fb.dst[q]] = v;
         }
-        if (!grid_barrier(a.bar, a.err))
+        if (!grid_barrier(a.bar, a.err, a.h_err))
             return false;
     }
     else
     {
-        if (!grid_barrier(a.bar, a.err))
+        if (!grid_barrier(a.bar, a.err, a.h_err))
             return false;
         if (!grid_apply(a, a.db, a.merge2 != 0))
             return false;
