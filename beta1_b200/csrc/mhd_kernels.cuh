@@ -159,6 +159,14 @@ struct FusedList
     const double *val;
     const int *blk;
     int64_t n;
+    int64_t dyn; // the first dyn depend on the basis vector; the rest stay for the whole solve
+};
+// The region's faces the curl writes, per staggered point block, offset within
+// a plane, face mask (n < 0: the whole region boxes); dyn as above
+struct RegionList
+{
+    const uint32_t *pt;
+    int64_t n, dyn;
 };
 enum : int
 {
@@ -174,9 +182,10 @@ __host__ __device__ inline int64_t fuse_pack(int fa, int i, int j, int k)
     return ((int64_t(fa) * 4096 + (i + 64)) * 4096 + (j + 64)) * 4096 + (k + 64);
 }
 
+constexpr int kResistBlocks = 24; // blocks the solve keeps in shared memory
 struct ResistSolve
 {
-    const BlockView *bvs;
+    const HotBlock *hb; // every block (in shared memory up to kResistBlocks)
     double *pool;
     int nblocks;
     const uint64_t *e, *dj, *j; // unknowns' offsets in Eres, dJ and J
@@ -198,7 +207,7 @@ struct ResistSolve
     GmresState *st;
     int m, maxit;
     double rtol, atol;
-    unsigned *bar; // arrival count, generation
+    unsigned *bar; // arrival count, count at the start, polling limit
     int *err;      // set to MHD_EKRYLOV when a barrier wait gives up
     volatile int *h_err; // ... and its copy in host memory
     // fused operator phases (n < 0: not fused, the copy-list phases run):
@@ -206,6 +215,7 @@ struct ResistSolve
     // each as one expression of the basis vector; B: the Sync("dB") copies,
     // each as the curl at its source (or a fixed or unchanged value)
     FusedList fa, fb;
+    RegionList reg;
 };
 __global__ void k_gmres_resist(ResistSolve a);
 

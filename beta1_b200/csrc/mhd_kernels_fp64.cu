@@ -107,54 +107,12 @@ __global__ void k_ucontra(const BlockView *__restrict__ bvs)
     UC[2 * b.vol + p] = u_contra(b, 2, i, j, k);
 }
 
-// Staggered points (i, j, k) of a block in [0, n + 1) per axis, one thread
-// each, or in the box rng[6 * block] (lo[3], hi[3], within [0, n + 1)^3)
-// when a region table is given.
-__device__ __forceinline__ bool stagger_point(const BlockView &b, const int *rng, int blk, int64_t t, int &i, int &j,
-                                              int &k)
-{
-    int lo[3] = {0, 0, 0};
-    int n[3] = {b.ni + 1, b.nj + 1, b.nk + 1};
-    if (rng)
-    {
-        const int *r = rng + 6 * blk;
-        for (int a = 0; a < 3; ++a)
-        {
-            lo[a] = r[a];
-            n[a] = r[3 + a] - r[a];
-        }
-    }
-    return box_point(lo, n, t, i, j, k);
-}
-
 // is (i, j, k) an inner point of the face (kind 0) or edge (kind 1) axis a
 __device__ __forceinline__ bool inner_of(const BlockView &b, int kind, int a, int i, int j, int k)
 {
     int pl[3];
     loc_plus((kind == 0 ? LOC_FXI : LOC_EXI) + a, pl[0], pl[1], pl[2]);
     return i < b.ni + pl[0] && j < b.nj + pl[1] && k < b.nk + pl[2];
-}
-
-// the discrete curl of the edge field fE0 on face axis fa at (i, j, k)
-__device__ __forceinline__ double face_curl(const BlockView &b, int fE0, int fa, int i, int j, int k)
-{
-    const double *Ex = b.f[fE0], *Ee = b.f[fE0 + 1], *Ez = b.f[fE0 + 2];
-    const int64_t p = pidx(b, i, j, k);
-    if (fa == 0)
-        return (Ee[p] - Ee[pidx(b, i, j, k + 1)]) + (Ez[pidx(b, i, j + 1, k)] - Ez[p]);
-    if (fa == 1)
-        return (Ex[pidx(b, i, j, k + 1)] - Ex[p]) + (Ez[p] - Ez[pidx(b, i + 1, j, k)]);
-    return (Ex[p] - Ex[pidx(b, i, j + 1, k)]) + (Ee[pidx(b, i + 1, j, k)] - Ee[p]);
-}
-
-// the three inner faces at staggered point (i, j, k): fR0 = mult * curl fE0
-__device__ __forceinline__ void curl_point(const BlockView &b, int fE0, int fR0, double mult, int i, int j, int k)
-{
-    const int64_t p = pidx(b, i, j, k);
-#pragma unroll
-    for (int fa = 0; fa < 3; ++fa)
-        if (inner_of(b, 0, fa, i, j, k))
-            b.f[fR0 + fa][p] = mult * face_curl(b, fE0, fa, i, j, k);
 }
 
 // calc_divB on inner cells (Z4_Lunar/src/physics/LunarSolver_Tools.cpp:685-775;
@@ -440,42 +398,62 @@ __global__ void k_soa_to_aos(const BlockView *__restrict__ bvs, int blk, int fid
 
 constexpr long long kBarrierSpins = 1ll << 22; // about a second of polling
 
-// bar[0]: arrival count, bar[1]: generation, bar[2]: polling limit of every
-// wait (0: kBarrierSpins; a smaller limit is set only by the failure-
-// detection hook mhd_test_stall_barrier, and the host clears it after use)
-__device__ __forceinline__ bool grid_barrier(unsigned *bar, int *err, volatile int *h_err)
+// Grid barrier on a count that only grows: bar[0] arrivals, bar[1] the count
+// at which the launch starts (CTA 0 leaves the next launch's when the solve
+// ends; every CTA has read it before its first arrival, which CTA 0's exit
+// implies), bar[2] the polling limit of every wait (0: kBarrierSpins; a smaller
+// limit is set only by the failure-detection hook mhd_test_stall_barrier, and
+// the host clears all four words after a solve that gave up).  A CTA arrives
+// once per barrier and waits for the count of all, so the last arrival itself
+// releases the others: one round trip to L2 less per barrier than a count that
+// is reset behind a generation number, and no sleep between polls.  A CTA that
+// gives up arrives at no later barrier, so the others give up in turn; they
+// look at the error word while they wait.
+struct GridBar
+{
+    unsigned *bar;
+    int *err;
+    volatile int *h_err;
+    unsigned target, limit; // thread 0's
+};
+__device__ __forceinline__ GridBar grid_bar(unsigned *bar, int *err, volatile int *h_err)
+{
+    GridBar g{bar, err, h_err, 0u, 0u};
+    if (threadIdx.x == 0)
+    {
+        g.target = *(volatile unsigned *)(bar + 1);
+        g.limit = *(volatile unsigned *)(bar + 2);
+    }
+    return g;
+}
+__device__ __forceinline__ bool grid_barrier(GridBar &g)
 {
     __shared__ int ok; // one decision for the whole CTA
     __syncthreads();
     if (threadIdx.x == 0)
     {
-        volatile unsigned *gen = bar + 1;
-        const unsigned g = *gen;
-        const unsigned lim = *(volatile unsigned *)(bar + 2);
-        const long long limit = lim ? (long long)lim : kBarrierSpins;
-        __threadfence();
-        if (atomicAdd(bar, 1u) + 1u == gridDim.x)
+        const long long limit = g.limit ? (long long)g.limit : kBarrierSpins;
+        g.target += gridDim.x;
+        ok = 1;
+        long long spins = 0;
+        // release: what the CTA wrote before (cumulative through the barrier
+        // above); acquire: what the others wrote before their arrivals
+        asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(g.bar), "r"(1u) : "memory");
+        for (;;)
         {
-            atomicExch(bar, 0u);
-            __threadfence();
-            atomicAdd(bar + 1, 1u);
-        }
-        else
-        {
-            long long spins = 0;
-            while (*gen == g)
+            unsigned count;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(count) : "l"(g.bar) : "memory");
+            if (int(count - g.target) >= 0)
+                break;
+            ++spins;
+            if (spins > limit || ((spins & 255) == 0 && *(volatile int *)g.err == MHD_EKRYLOV))
             {
-                if (++spins > limit)
-                {
-                    atomicExch(err, MHD_EKRYLOV);
-                    *h_err = MHD_EKRYLOV;
-                    break;
-                }
-                __nanosleep(64);
+                atomicExch(g.err, MHD_EKRYLOV);
+                *g.h_err = MHD_EKRYLOV;
+                ok = 0;
+                break;
             }
         }
-        __threadfence();
-        ok = *(volatile int *)err != MHD_EKRYLOV;
     }
     __syncthreads();
     return ok != 0;
@@ -491,49 +469,64 @@ struct GmresScalars
 // out[c] = V_c . w for c < nv, or out[0] = w . w (V null); with_self also
 // out[nv] = w . w in the same reduction; every CTA ends with the same values
 // in out (shared memory)
-__device__ bool grid_dots(const ResistSolve &a, const double *V, int nv, const double *w, double *out, int &pbuf,
-                          bool with_self = false)
+__device__ bool grid_dots(const ResistSolve &a, GridBar &gb, const double *V, int nv, const double *w, double *out,
+                          int &pbuf, bool with_self = false)
 {
     __shared__ double wred[8][8];
     const int G = gridDim.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // CTAs past the vector's end hold no element: their partial sums are +0,
+    // which changes no sum that starts at +0, so they write none
+    const int Gn = int(min(int64_t(G), (a.n + int64_t(blockDim.x) - 1) / int64_t(blockDim.x)));
     double *part = a.partial + int64_t(pbuf) * 32 * G;
     pbuf ^= 1;
     const int nd = nv + (with_self ? 1 : 0);
-    for (int c0 = 0; c0 < nd; c0 += 8)
-    {
-        double acc[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-        for (int64_t t = int64_t(blockIdx.x) * blockDim.x + tid; t < a.n; t += int64_t(G) * blockDim.x)
+    if (int(blockIdx.x) < Gn)
+        for (int c0 = 0; c0 < nd; c0 += 8)
         {
-            const double wt = w[t];
+            double acc[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+            for (int64_t t = int64_t(blockIdx.x) * blockDim.x + tid; t < a.n; t += int64_t(G) * blockDim.x)
+            {
+                const double wt = w[t];
+#pragma unroll
+                for (int q = 0; q < 8; ++q)
+                    if (c0 + q < nd)
+                        acc[q] += ((V && c0 + q < nv) ? V[int64_t(c0 + q) * a.n + t] : wt) * wt;
+            }
 #pragma unroll
             for (int q = 0; q < 8; ++q)
                 if (c0 + q < nd)
-                    acc[q] += ((V && c0 + q < nv) ? V[int64_t(c0 + q) * a.n + t] : wt) * wt;
+                {
+                    for (int off = 16; off > 0; off >>= 1)
+                        acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], off);
+                    if (lane == 0)
+                        wred[warp][q] = acc[q];
+                }
+            __syncthreads();
+            if (tid < 8 && c0 + tid < nd)
+            {
+                double sum = 0.0;
+                for (int wp = 0; wp < int(blockDim.x >> 5); ++wp)
+                    sum += wred[wp][tid];
+                part[int64_t(c0 + tid) * G + blockIdx.x] = sum;
+            }
+            __syncthreads();
         }
-#pragma unroll
-        for (int q = 0; q < 8; ++q)
-            for (int off = 16; off > 0; off >>= 1)
-                acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], off);
-        if (lane == 0)
-            for (int q = 0; q < 8; ++q)
-                wred[warp][q] = acc[q];
-        __syncthreads();
-        if (tid < 8 && c0 + tid < nd)
-        {
-            double sum = 0.0;
-            for (int wp = 0; wp < int(blockDim.x >> 5); ++wp)
-                sum += wred[wp][tid];
-            part[int64_t(c0 + tid) * G + blockIdx.x] = sum;
-        }
-        __syncthreads();
-    }
-    if (!grid_barrier(a.bar, a.err, a.h_err))
+    if (!grid_barrier(gb))
         return false;
     for (int c = warp; c < nd; c += int(blockDim.x >> 5))
     {
         double sum = 0.0;
-        for (int g = lane; g < G; g += 32)
-            sum += __ldcg(&part[int64_t(c) * G + g]);
+        // (loads of a batch in flight together, added in CTA order)
+        for (int g = lane; g < Gn; g += 128)
+        {
+            double y[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                y[e] = g + 32 * e < Gn ? __ldcg(&part[int64_t(c) * G + g + 32 * e]) : 0.0;
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                sum += y[e];
+        }
         for (int off = 16; off > 0; off >>= 1)
             sum += __shfl_xor_sync(0xffffffffu, sum, off);
         if (lane == 0)
@@ -544,14 +537,14 @@ __device__ bool grid_dots(const ResistSolve &a, const double *V, int nv, const d
 }
 
 // fixed values (unless already written) then copies of a point list
-__device__ bool grid_apply(const ResistSolve &a, const DevCopy &l, bool consts_done)
+__device__ bool grid_apply(const ResistSolve &a, GridBar &gb, const DevCopy &l, bool consts_done)
 {
     const int64_t t0 = int64_t(blockIdx.x) * blockDim.x + threadIdx.x, ts = int64_t(gridDim.x) * blockDim.x;
     if (l.nconst > 0 && !consts_done)
     {
         for (int64_t t = t0; t < l.nconst; t += ts)
             a.pool[l.cdst[t]] = l.cval[t];
-        if (!grid_barrier(a.bar, a.err, a.h_err))
+        if (!grid_barrier(gb))
             return false;
     }
     if (l.n == 0)
@@ -560,7 +553,7 @@ __device__ bool grid_apply(const ResistSolve &a, const DevCopy &l, bool consts_d
     {
         for (int64_t t = t0; t < l.n; t += ts)
             l.tmp[t] = a.pool[l.src[t]];
-        if (!grid_barrier(a.bar, a.err, a.h_err))
+        if (!grid_barrier(gb))
             return false;
         for (int64_t t = t0; t < l.n; t += ts)
             a.pool[l.dst[t]] = __ldcg(&l.tmp[t]);
@@ -568,8 +561,137 @@ __device__ bool grid_apply(const ResistSolve &a, const DevCopy &l, bool consts_d
     else
         for (int64_t t = t0; t < l.n; t += ts)
             a.pool[l.dst[t]] = a.pool[l.src[t]];
-    return grid_barrier(a.bar, a.err, a.h_err);
+    return grid_barrier(gb);
 }
+
+// discrete curl of the edge planes qE on face axis fa of the point
+__device__ __forceinline__ double hot_curl(const HotBlock &b, uint32_t p, int qE, int fa)
+{
+    const int si = int(b.si), sj = int(b.sj);
+    const double *Ex = hot_plane(b, p, qE), *Ee = hot_plane(b, p, qE + 1), *Ez = hot_plane(b, p, qE + 2);
+    if (fa == 0)
+        return (Ee[0] - Ee[1]) + (Ez[sj] - Ez[0]);
+    if (fa == 1)
+        return (Ex[1] - Ex[0]) + (Ez[0] - Ez[si]);
+    return (Ex[0] - Ex[sj]) + (Ee[si] - Ee[0]);
+}
+
+// What a thread's first item of each phase's list needs that no phase writes:
+// read once at the start of the solve, because the fence of every barrier
+// drops the L1 lines a second read would hit.  The lists hold at most a few
+// items per thread, usually one.
+struct PreUnknown // an unknown's edge: its point, axis, resistivity, edge and face scales
+{
+    const HotBlock *b;
+    uint32_t p;
+    int ea;
+    uint64_t e;
+    double eta, alpha, beta[4];
+};
+struct PreFused // an item of a fused list; a curl's point and axis decoded
+{
+    uint64_t dst;
+    int kind, fa;
+    int64_t idx;
+    double val;
+    const HotBlock *b;
+    uint32_t p;
+};
+struct PreRegion // a staggered point of the region and its inner faces
+{
+    const HotBlock *b;
+    uint32_t p;
+    int faces;
+};
+
+// the other component and offset of each term of the edge circulation of axis
+// ea (CTOperators.cpp:58-110): (h1[o1] - h1[0]) + (h2[0] - h2[o2]) for ea = 0 ...
+__device__ __forceinline__ void edge_terms(const HotBlock &b, int ea, int &f1, int &o1, int &f2, int &o2)
+{
+    f1 = ea == 0 ? 1 : 0;
+    f2 = ea == 2 ? 1 : 2;
+    o1 = ea == 2 ? -int(b.sj) : -1;
+    o2 = ea == 0 ? -int(b.sj) : -int(b.si);
+}
+__device__ __forceinline__ PreUnknown load_unknown(const ResistSolve &a, const HotBlock *hb, int64_t t)
+{
+    PreUnknown u;
+    const int *l = a.uloc + 5 * t;
+    u.b = hb + l[0];
+    u.ea = l[1];
+    u.p = u.b->o + uint32_t(l[2]) * u.b->si + uint32_t(l[3]) * u.b->sj + uint32_t(l[4]);
+    u.e = a.e[t];
+    u.eta = a.eta[t];
+    int f1, o1, f2, o2;
+    edge_terms(*u.b, u.ea, f1, o1, f2, o2);
+    const double *b1 = hot_at(*u.b, u.p, F_betaxi) + uint64_t(f1) * u.b->vol;
+    const double *b2 = hot_at(*u.b, u.p, F_betaxi) + uint64_t(f2) * u.b->vol;
+    u.alpha = hot_at(*u.b, u.p, F_alphaxi)[uint64_t(u.ea) * u.b->vol];
+    u.beta[0] = b1[0];
+    u.beta[1] = b1[o1];
+    u.beta[2] = b2[0];
+    u.beta[3] = b2[o2];
+    return u;
+}
+// dJ at the unknown's edge (jedge_one's operations), stored; y = Eres - eta dJ
+__device__ __forceinline__ double unknown_value(const ResistSolve &a, const PreUnknown &u)
+{
+    int f1, o1, f2, o2;
+    edge_terms(*u.b, u.ea, f1, o1, f2, o2);
+    const double *F1 = hot_at(*u.b, u.p, F_dBxi) + uint64_t(f1) * u.b->vol;
+    const double *F2 = hot_at(*u.b, u.p, F_dBxi) + uint64_t(f2) * u.b->vol;
+    const double h1 = u.beta[0] * F1[0], m1 = u.beta[1] * F1[o1], h2 = u.beta[2] * F2[0], m2 = u.beta[3] * F2[o2];
+    const double E = a.pool[u.e];
+    const double val = u.ea == 1 ? (h1 - m1) + (m2 - h2) : (m1 - h1) + (h2 - m2);
+    const double dJ = val * u.alpha;
+    hot_at(*u.b, u.p, F_dJxi)[uint64_t(u.ea) * u.b->vol] = dJ;
+    return E - u.eta * dJ;
+}
+__device__ __forceinline__ PreFused load_fused(const FusedList &l, const HotBlock *hb, int64_t q)
+{
+    PreFused x;
+    x.dst = l.dst[q];
+    x.kind = l.kind[q];
+    x.idx = l.idx[q];
+    x.val = l.val[q];
+    x.fa = 0;
+    x.b = hb;
+    x.p = 0;
+    if (x.kind == FUSE_CURL)
+    {
+        const int k = int(x.idx % 4096) - 64, j = int((x.idx / 4096) % 4096) - 64;
+        const int i = int((x.idx / (int64_t(4096) * 4096)) % 4096) - 64;
+        x.fa = int(x.idx / (int64_t(4096) * 4096 * 4096));
+        x.b = hb + l.blk[q];
+        x.p = x.b->o + uint32_t(i) * x.b->si + uint32_t(j) * x.b->sj + uint32_t(k);
+    }
+    return x;
+}
+__device__ __forceinline__ PreRegion load_region(const ResistSolve &a, const HotBlock *hb, int64_t q)
+{
+    PreRegion r{hb, 0u, 0};
+    if (a.reg.n >= 0)
+    {
+        r.b = hb + a.reg.pt[3 * q];
+        r.p = a.reg.pt[3 * q + 1];
+        r.faces = int(a.reg.pt[3 * q + 2]);
+        return r;
+    }
+    const uint32_t blk = uint32_t(q) / uint32_t(a.nreg);
+    r.b = hb + blk;
+    int i, j, k;
+    if (hot_stagger(*r.b, a.rng, uint32_t(q) - blk * uint32_t(a.nreg), i, j, k, r.p))
+        for (int fa = 0; fa < 3; ++fa)
+            r.faces |= hot_face(*r.b, fa, i, j, k) ? 1 << fa : 0;
+    return r;
+}
+
+struct PreItems
+{
+    PreUnknown u;
+    PreFused fa, fb;
+    PreRegion r;
+};
 
 // y = A (src / div) (MatMultImplicitResistive_): Eres at the unknowns and
 // their aliases, Sync("Eres1form"), dB = -dt curl Eres on the region,
@@ -577,32 +699,33 @@ __device__ bool grid_apply(const ResistSolve &a, const DevCopy &l, bool consts_d
 // y = Eres - eta dJ.  src must be complete at entry unless first_barrier:
 // the aliases read other threads' elements.  src / div is the stored basis
 // vector bit for bit (the same division), so the basis vector itself need
-// not be complete.
-__device__ bool grid_matvec(const ResistSolve &a, const double *src, double div, bool first_barrier, double *y)
+// not be complete.  first: the solve's first product, which also writes the
+// points whose value no later one changes (the static tails of the lists).
+__device__ bool grid_matvec(const ResistSolve &a, GridBar &gb, const HotBlock *hb, const PreItems &pre,
+                            const double *src, double div, bool first_barrier, bool first, double *y)
 {
     const int64_t t0 = int64_t(blockIdx.x) * blockDim.x + threadIdx.x, ts = int64_t(gridDim.x) * blockDim.x;
-    if (first_barrier && !grid_barrier(a.bar, a.err, a.h_err))
+    if (first_barrier && !grid_barrier(gb))
         return false;
     const double mdt = -a.dtp[0];
     if (a.fa.n >= 0)
     {
         // one phase: every Eres point the unknowns, aliases and Sync("Eres1form") set
-        for (int64_t q = t0; q < a.fa.n; q += ts)
+        for (int64_t q = t0; q < (first ? a.fa.n : a.fa.dyn); q += ts)
         {
-            const int kd = a.fa.kind[q];
-            const int64_t ix = a.fa.idx[q];
+            const PreFused x = q == t0 ? pre.fa : load_fused(a.fa, hb, q);
             double v;
-            if (kd == FUSE_UNKNOWN)
-                v = src[ix] / div;
-            else if (kd == FUSE_ALIAS)
-                v = a.fa.val[q] * (src[ix] / div);
-            else if (kd == FUSE_CONST)
-                v = a.fa.val[q];
+            if (x.kind == FUSE_UNKNOWN)
+                v = src[x.idx] / div;
+            else if (x.kind == FUSE_ALIAS)
+                v = x.val * (src[x.idx] / div);
+            else if (x.kind == FUSE_CONST)
+                v = x.val;
             else
-                v = a.pool[ix];
-            a.pool[a.fa.dst[q]] = v;
+                v = a.pool[x.idx];
+            a.pool[x.dst] = v;
         }
-        if (!grid_barrier(a.bar, a.err, a.h_err))
+        if (!grid_barrier(gb))
             return false;
     }
     else
@@ -614,78 +737,97 @@ __device__ bool grid_matvec(const ResistSolve &a, const double *src, double div,
         if (a.merge1)
             for (int64_t t = t0; t < a.eres1form.nconst; t += ts)
                 a.pool[a.eres1form.cdst[t]] = a.eres1form.cval[t];
-        if (!grid_barrier(a.bar, a.err, a.h_err))
+        if (!grid_barrier(gb))
             return false;
-        if (!grid_apply(a, a.eres1form, a.merge1 != 0))
+        if (!grid_apply(a, gb, a.eres1form, a.merge1 != 0))
             return false;
     }
-    const int64_t np = int64_t(a.nblocks) * a.nreg;
+    const int64_t np = a.reg.n >= 0 ? (first ? a.reg.n : a.reg.dyn) : int64_t(a.nblocks) * a.nreg;
     for (int64_t q = t0; q < np; q += ts)
     {
-        const int blk = int(q / a.nreg);
-        const BlockView &b = a.bvs[blk];
-        int i, j, k;
-        if (stagger_point(b, a.rng, blk, q % a.nreg, i, j, k))
-            curl_point(b, F_Eresxi, F_dBxi, mdt, i, j, k);
+        const PreRegion r = q == t0 ? pre.r : load_region(a, hb, q);
+#pragma unroll
+        for (int fa = 0; fa < 3; ++fa)
+            if (r.faces & (1 << fa))
+                *hot_at(*r.b, r.p, F_dBxi + fa) = mdt * hot_curl(*r.b, r.p, plane_of(F_Eresxi), fa);
     }
-    if (a.merge2)
+    if (a.merge2 && (first || a.fb.n < 0))
         for (int64_t t = t0; t < a.db.nconst; t += ts)
             a.pool[a.db.cdst[t]] = a.db.cval[t];
     if (a.fb.n >= 0)
     {
         // the Sync("dB") copies in the same phase: each destination takes
         // the curl at its source directly (fixed values were written above)
-        for (int64_t q = t0; q < a.fb.n; q += ts)
+        for (int64_t q = t0; q < (first ? a.fb.n : a.fb.dyn); q += ts)
         {
-            const int kd = a.fb.kind[q];
-            const int64_t ix = a.fb.idx[q];
+            const PreFused x = q == t0 ? pre.fb : load_fused(a.fb, hb, q);
             double v;
-            if (kd == FUSE_CURL)
-            {
-                const int k = int(ix % 4096) - 64, j = int((ix / 4096) % 4096) - 64;
-                const int i = int((ix / (int64_t(4096) * 4096)) % 4096) - 64, fa = int(ix / (int64_t(4096) * 4096 * 4096));
-                v = mdt * face_curl(a.bvs[a.fb.blk[q]], F_Eresxi, fa, i, j, k);
-            }
-            else if (kd == FUSE_CONST)
-                v = a.fb.val[q];
+            if (x.kind == FUSE_CURL)
+                v = mdt * hot_curl(*x.b, x.p, plane_of(F_Eresxi), x.fa);
+            else if (x.kind == FUSE_CONST)
+                v = x.val;
             else
-                v = a.pool[ix];
-            a.pool[a.fb.dst[q]] = v;
+                v = a.pool[x.idx];
+            a.pool[x.dst] = v;
         }
-        if (!grid_barrier(a.bar, a.err, a.h_err))
+        if (!grid_barrier(gb))
             return false;
     }
     else
     {
-        if (!grid_barrier(a.bar, a.err, a.h_err))
+        if (!grid_barrier(gb))
             return false;
-        if (!grid_apply(a, a.db, a.merge2 != 0))
+        if (!grid_apply(a, gb, a.db, a.merge2 != 0))
             return false;
     }
     for (int64_t t = t0; t < a.n; t += ts)
-    {
-        const int *u = a.uloc + 5 * t;
-        jedge_one(a.bvs[u[0]], u[1], u[2], u[3], u[4], F_dBxi, F_dJxi, 1.0);
-        y[t] = a.pool[a.e[t]] - a.eta[t] * a.pool[a.dj[t]];
-    }
+        y[t] = unknown_value(a, t == t0 ? pre.u : load_unknown(a, hb, t));
     return true;
 }
 
+// What bounds the solve: the round trips of its phases (a barrier, then the
+// dependent loads of the phase's work), with the system resident in L2 and one
+// item per thread.  On 6 x 80 x 40 x 40 cells (8440 unknowns, 4 iterations, 21
+// barriers) 158 us per solve with a reset barrier, lists read in every phase and
+// every point written by every product; 120 with a counting barrier, the lists'
+// entries, scales and blocks loaded once into registers and shared memory; 96.6
+// with the points that never change written by the first product alone, a CTA
+// for every 256 items and release / acquire in place of two fences.
 __global__ void __launch_bounds__(256) k_gmres_resist(ResistSolve a)
 {
     __shared__ GmresScalars S;
     __shared__ double dv[32];
+    __shared__ HotBlock sblk[kResistBlocks];
+    __shared__ int gone;
+    GridBar gb = grid_bar(a.bar, a.err, a.h_err);
     const int tid = threadIdx.x;
+    if (tid == 0) // a solve of an earlier step gave up: the barrier's words are stale until the host clears them
+        gone = *(volatile int *)a.err == MHD_EKRYLOV;
+    for (int q = tid; q < min(a.nblocks, kResistBlocks) * int(sizeof(HotBlock) / 4); q += blockDim.x)
+        reinterpret_cast<uint32_t *>(sblk)[q] = reinterpret_cast<const uint32_t *>(a.hb)[q];
+    __syncthreads();
+    if (gone)
+        return;
+    const HotBlock *hb = a.nblocks <= kResistBlocks ? sblk : a.hb;
     const int64_t t0 = int64_t(blockIdx.x) * blockDim.x + tid, ts = int64_t(gridDim.x) * blockDim.x;
     const int64_t n = a.n;
     int pbuf = 0;
+    PreItems pre{};
+    if (t0 < n)
+        pre.u = load_unknown(a, hb, t0);
+    if (t0 < a.fa.n)
+        pre.fa = load_fused(a.fa, hb, t0);
+    if (t0 < a.fb.n)
+        pre.fb = load_fused(a.fb, hb, t0);
+    if (t0 < (a.reg.n >= 0 ? a.reg.n : int64_t(a.nblocks) * a.nreg))
+        pre.r = load_region(a, hb, t0);
     // right-hand side b = eta J at the unknowns (PackImplicitJedgeToVec_), x = 0
     for (int64_t t = t0; t < n; t += ts)
     {
         a.b[t] = 0.0 + a.eta[t] * a.pool[a.j[t]];
         a.x[t] = 0.0;
     }
-    if (!grid_dots(a, nullptr, 1, a.b, dv, pbuf))
+    if (!grid_dots(a, gb, nullptr, 1, a.b, dv, pbuf))
         return;
     if (tid == 0)
     {
@@ -700,11 +842,11 @@ __global__ void __launch_bounds__(256) k_gmres_resist(ResistSolve a)
     for (;;)
     {
         // cycle start: r = b - A x, beta = ||r||
-        if (!grid_matvec(a, a.x, 1.0, true, a.w))
+        if (!grid_matvec(a, gb, hb, pre, a.x, 1.0, true, S.cycles == 0, a.w))
             return;
         for (int64_t t = t0; t < n; t += ts)
             a.r[t] = a.b[t] - a.w[t];
-        if (!grid_dots(a, nullptr, 1, a.r, dv, pbuf))
+        if (!grid_dots(a, gb, nullptr, 1, a.r, dv, pbuf))
             return;
         if (tid == 0)
         {
@@ -736,10 +878,10 @@ __global__ void __launch_bounds__(256) k_gmres_resist(ResistSolve a)
             const int j = S.j;
             // V_j = r / beta (j = 0) or the previous step's w / ||w||, both
             // complete at the last reduction's barrier
-            if (!grid_matvec(a, j == 0 ? a.r : a.w, j == 0 ? S.beta : S.hcol[j], false, a.w))
+            if (!grid_matvec(a, gb, hb, pre, j == 0 ? a.r : a.w, j == 0 ? S.beta : S.hcol[j], false, false, a.w))
                 return;
             // classical Gram-Schmidt, twice
-            if (!grid_dots(a, a.V, j + 1, a.w, S.hcol, pbuf))
+            if (!grid_dots(a, gb, a.V, j + 1, a.w, S.hcol, pbuf))
                 return;
             for (int64_t t = t0; t < n; t += ts)
             {
@@ -750,7 +892,7 @@ __global__ void __launch_bounds__(256) k_gmres_resist(ResistSolve a)
             }
             // second pass, its dots and ||w'||^2 in one reduction: with V
             // orthonormal, ||w' - V d||^2 = ||w'||^2 - ||d||^2
-            if (!grid_dots(a, a.V, j + 1, a.w, S.d, pbuf, true))
+            if (!grid_dots(a, gb, a.V, j + 1, a.w, S.d, pbuf, true))
                 return;
             for (int64_t t = t0; t < n; t += ts)
             {
@@ -850,6 +992,7 @@ __global__ void __launch_bounds__(256) k_gmres_resist(ResistSolve a)
         st->j = S.j;
         st->total_its += S.its;
         st->total_cycles += S.cycles;
+        *(volatile unsigned *)(a.bar + 1) = gb.target; // (the count at the next launch's start)
     }
 }
 

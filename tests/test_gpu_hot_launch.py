@@ -6,9 +6,9 @@ arithmetic per point, so the fields agree bit for bit."""
 import numpy as np
 import pytest
 
-from conftest import load_golden, periodic_setup
+from conftest import load_golden, periodic_setup, slab_setup
 
-from beta1_b200 import case, solver
+from beta1_b200 import case, mhd, solver
 
 pytestmark = pytest.mark.gpu
 
@@ -70,3 +70,42 @@ def test_uploaded_eface():
             assert np.array_equal(s.field(f)[inner], g["s1/" + f][inner]), f
     finally:
         s.ctx.close()
+
+
+@pytest.mark.parametrize("group", ["dB", "Eres1form"])
+def test_resistive_operator_forms(group, monkeypatch):
+    """one more copy, without effect on the compared fields, takes the implicit
+    solve off its short lists: into divB (a field outside the group's own, so
+    every product writes every point), or of a point onto itself (a chain, so
+    the copies run as lists of their own).  It is given after the solve is set
+    up, which rebuilds the operator.  Same operations per point: the same bits."""
+    g = load_golden("slab_6x5x6_t2x2_r11_steps.npz")
+    spec, st = slab_setup(g)
+    maps, out = {}, []
+    keep = mhd.Context.set_sync_map
+
+    def record(ctx, name, dst, src):
+        maps[name] = (np.asarray(dst), np.asarray(src))
+        return keep(ctx, name, dst, src)
+
+    monkeypatch.setattr(mhd.Context, "set_sync_map", record)
+    for extra in (False, True):
+        s = solver.Solver(spec, topology="tiled")
+        try:
+            if extra:
+                dst, src = maps[group]
+                i, j = np.setdiff1d(src, dst)[:1], np.setdiff1d(src, dst)[:1]
+                if group == "dB":
+                    i = np.array([s.ctx.lib.mhd_point_id(s.ctx.h, b"divB", int(src[0]) >> 40 & 0xFFFF, 0, 1, 1, 0)])
+                    j = src[:1]
+                keep(s.ctx, group, np.concatenate([dst, i]).astype(dst.dtype),
+                     np.concatenate([src, j]).astype(src.dtype))
+            s.load_state(st)
+            s.step(3)
+            out.append({(f, b): s.field(f, b) for f in FIELDS + tuple(
+                q + x for q in ("Eres_", "dB_", "dJ_") for x in ("xi", "eta", "zeta"))
+                        for b in range(len(spec.blocks))})
+        finally:
+            s.ctx.close()
+    for k, a in out[0].items():
+        assert np.array_equal(a, out[1][k]), k
