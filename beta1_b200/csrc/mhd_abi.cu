@@ -1991,6 +1991,7 @@ int create_ctx(const mhd_block_desc *blocks, int32_t nblocks, const int32_t *run
         v.nj = blocks[b].nj;
         v.nk = blocks[b].nk;
         v.G = ctx->G;
+        v.wtiles = 1;
         const int NI = v.ni + 1 + 2 * v.G;
         v.NJ = v.nj + 1 + 2 * v.G;
         v.NK = v.nk + 1 + 2 * v.G;
@@ -2361,7 +2362,7 @@ static int64_t pool_offset(const mhd_ctx *ctx, int64_t id)
     const int j = lo[1] + int(aos % n1);
     const int i = lo[0] + int(aos / n1);
     const BlockView &v = ctx->hbv[size_t(b)];
-    return int64_t(ctx->base[size_t(f)][size_t(b)]) + int64_t(m) * v.vol + pidx(v, i, j, k);
+    return int64_t(ctx->base[size_t(f)][size_t(b)]) + field_index(v, f, nc, m, i, j, k);
 }
 
 } // extern "C"
@@ -2432,8 +2433,14 @@ struct PoolDecoder
         b = int(std::upper_bound(start.begin(), start.end() - 1, off) - start.begin()) - 1;
         const BlockView &v = ctx->hbv[size_t(b)];
         const uint64_t rel = off - start[size_t(b)];
-        const uint32_t q = uint32_t(rel / uint64_t(v.vol)), p = uint32_t(rel - q * uint64_t(v.vol));
+        const uint32_t q = uint32_t(rel / uint64_t(v.vol));
+        uint32_t p = uint32_t(rel - q * uint64_t(v.vol));
         f = field_of[q];
+        if (weight_field(f))
+        {
+            const uint64_t r = rel - uint64_t(plane_of(f)) * uint64_t(v.vol);
+            p = weight_point(v, int64_t(r / uint64_t(kWTile * kFields[f].ncomp)) * kWTile + int64_t(r % kWTile));
+        }
         const uint32_t ij = p / uint32_t(v.NK);
         k = int(p - ij * uint32_t(v.NK)) - v.G;
         const uint32_t ii = ij / uint32_t(v.NJ);

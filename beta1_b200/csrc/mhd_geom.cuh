@@ -310,7 +310,8 @@ __host__ __device__ inline void geom_point(const NodeMesh &m, const BlockView &b
     case GEOM_WB:
         if (geom_in(b, LOC_CELL, G - 1, i, j, k))
         {
-            double *W = b.f[F_WB] + p;
+            double *W = b.f[F_WB] + field_index(b, F_WB, 18, 0, i, j, k);
+            const int64_t v = b.wtiles ? kWTile : b.vol;
             if (i < 0 || j < 0 || k < 0 || i >= b.ni || j >= b.nj || k >= b.nk)
             {
                 for (int q = 0; q < 18; ++q)
@@ -349,7 +350,8 @@ __host__ __device__ inline void geom_point(const NodeMesh &m, const BlockView &b
     case GEOM_WJ:
         if (geom_in(b, LOC_CELL, G - 1, i, j, k))
         {
-            double *W = b.f[F_WJ] + p;
+            double *W = b.f[F_WJ] + field_index(b, F_WJ, 36, 0, i, j, k);
+            const int64_t v = b.wtiles ? kWTile : b.vol;
             if (i < 0 || j < 0 || k < 0 || i >= b.ni || j >= b.nj || k >= b.nk)
             {
                 for (int q = 0; q < 36; ++q)

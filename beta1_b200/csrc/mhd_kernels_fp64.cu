@@ -360,7 +360,7 @@ __global__ void k_aos_to_soa(const BlockView *__restrict__ bvs, int blk, int fid
     r /= n2;
     const int j = lo1 + int(r % n1);
     const int i = lo0 + int(r / n1);
-    b.f[fid][m * b.vol + pidx(b, i, j, k)] = aos[t];
+    b.f[fid][field_index(b, fid, ncomp, m, i, j, k)] = aos[t];
 }
 
 __global__ void k_soa_to_aos(const BlockView *__restrict__ bvs, int blk, int fid, int ncomp, int lo0, int lo1,
@@ -378,7 +378,7 @@ __global__ void k_soa_to_aos(const BlockView *__restrict__ bvs, int blk, int fid
     r /= n2;
     const int j = lo1 + int(r % n1);
     const int i = lo0 + int(r / n1);
-    aos[t] = b.f[fid][m * b.vol + pidx(b, i, j, k)];
+    aos[t] = b.f[fid][field_index(b, fid, ncomp, m, i, j, k)];
 }
 
 // ---------------------------------------------------------------------------
@@ -1390,12 +1390,13 @@ __device__ void jcell_plain(const BlockView &b, int i, int j, int k)
                           Je[pidx(b, i, j, k + 1)],     Je[pidx(b, i + 1, j, k + 1)], Jz[pidx(b, i, j, k)],
                           Jz[pidx(b, i + 1, j, k)],     Jz[pidx(b, i, j + 1, k)],     Jz[pidx(b, i + 1, j + 1, k)]};
     const int64_t p = pidx(b, i, j, k), v = b.vol;
+    const int64_t w0 = weight_tile(weight_cell(b, i, j, k), 36);
     for (int c = 0; c < 3; ++c)
     {
         double J = 0.0;
         for (int q = 0; q < 12; ++q)
         {
-            const int64_t w = (12 * c + q) * v + p;
+            const int64_t w = w0 + (12 * c + q) * kWTile;
             J += (b.w32 ? double(b.w32[W32_J * v + w]) : b.f[F_WJ][w]) * s[q];
         }
         b.f[F_Jcell][c * v + p] = J;

@@ -39,6 +39,7 @@ __global__ void k_geom32(const BlockView *__restrict__ bvs)
         for (int c = 0; c < 3; ++c)
             b.g32[(G32_NRM + 3 * a + c) * v + p] = float(b.f[F_NAxi + a][(1 + c) * v + p]);
     }
+    // the weights' order is the FP64 fields' own
     for (int q = 0; q < 18; ++q)
         b.w32[(W32_B + q) * v + p] = float(b.f[F_WB][q * v + p]);
     for (int q = 0; q < 36; ++q)

@@ -531,16 +531,21 @@ template <class A> __global__ void __launch_bounds__(kHotThreads) k_rk2_t(const 
 // in the reference touches neither input)
 // ---------------------------------------------------------------------------
 
-// least-squares weight planes of a block at the thread's point: the FP64
-// field, or its FP32 copy
-template <typename WT> __device__ __forceinline__ const WT *hot_weights(const HotBlock &b, uint32_t p, int f, int q32);
-template <> __device__ __forceinline__ const double *hot_weights<double>(const HotBlock &b, uint32_t p, int f, int)
+// an inner cell's place among the block's cells
+__device__ __forceinline__ uint32_t hot_cell(const HotBlock &b, int i, int j, int k)
 {
-    return hot_at(b, p, f);
+    return (uint32_t(i) * uint32_t(b.nj) + uint32_t(j)) * uint32_t(b.nk) + uint32_t(k);
 }
-template <> __device__ __forceinline__ const float *hot_weights<float>(const HotBlock &b, uint32_t p, int, int q32)
+// the least-squares weights of inner cell d, kWTile values apart: the FP64
+// field, or its FP32 copy
+template <typename WT> __device__ __forceinline__ const WT *hot_weights(const HotBlock &b, uint32_t d, int f, int q32);
+template <> __device__ __forceinline__ const double *hot_weights<double>(const HotBlock &b, uint32_t d, int f, int)
 {
-    return hot_plane32(b, p, kPlane32W + q32);
+    return hot_at(b, 0, f) + uint64_t(weight_tile(d, f == F_WB ? 18 : 36));
+}
+template <> __device__ __forceinline__ const float *hot_weights<float>(const HotBlock &b, uint32_t d, int f, int q32)
+{
+    return hot_plane32(b, 0, kPlane32W + q32) + uint64_t(weight_tile(d, f == F_WB ? 18 : 36));
 }
 
 // WT: double (the reference's weights, FP64 form) or float (their FP32
@@ -596,14 +601,14 @@ template <typename WT, bool EDGES, bool IND, class A> __device__ __forceinline__
         const double tot[6] = {-B0[0] - D0[0], B1[0] + D1[0], -B0[1] - D0[1],
                                B1[1] + D1[1],  -B0[2] - D0[2], B1[2] + D1[2]};
         const double ind[6] = {-B0[0], B1[0], -B0[1], B1[1], -B0[2], B1[2]};
-        const WT *W = hot_weights<WT>(b, p, F_WB, W32_B);
+        const WT *W = hot_weights<WT>(b, hot_cell(b, i, j, k), F_WB, W32_B);
         double bt[3] = {0.0, 0.0, 0.0}, bi[3] = {0.0, 0.0, 0.0};
 #pragma unroll
         for (int q = 0; q < 6; ++q)
 #pragma unroll
             for (int c = 0; c < 3; ++c)
             {
-                const double w = double(W[(6 * c + q) * v]);
+                const double w = double(W[(6 * c + q) * kWTile]);
                 bt[c] += w * tot[q];
                 if (IND)
                     bi[c] += w * ind[q];
@@ -667,27 +672,38 @@ __global__ void __launch_bounds__(kHotThreads) k_jedge_t(const __grid_constant__
 // ---------------------------------------------------------------------------
 // calc_Jcell (LunarSolver_Tools.cpp:837-892)
 // ---------------------------------------------------------------------------
-template <typename WT>
-__device__ __forceinline__ void jcell_sum(const HotBlock &b, uint32_t p, double &jx, double &jy, double &jz)
+// ALL: every weight is loaded before the first is used (72 registers; left to
+// the compiler, a few at a time)
+template <typename WT, bool ALL>
+__device__ __forceinline__ void jcell_sum(const HotBlock &b, uint32_t p, uint32_t d, double &jx, double &jy, double &jz)
 {
     const int si = int(b.si), sj = int(b.sj);
-    const uint64_t v = b.vol;
     const double *Jx = hot_at(b, p, F_Jxi), *Je = hot_at(b, p, F_Jeta), *Jz = hot_at(b, p, F_Jzeta);
-    const WT *W = hot_weights<WT>(b, p, F_WJ, W32_J);
+    const WT *W = hot_weights<WT>(b, d, F_WJ, W32_J);
+    WT w[36];
+#pragma unroll
+    for (int q = 0; q < 36; ++q)
+        w[q] = W[q * kWTile];
     const double s[12] = {Jx[0], Jx[sj], Jx[1], Jx[sj + 1], Je[0], Je[si],
                           Je[1], Je[si + 1], Jz[0], Jz[si], Jz[sj], Jz[si + sj]};
+    if (ALL)
+        asm volatile("" ::: "memory");
     jx = jy = jz = 0.0;
 #pragma unroll
     for (int q = 0; q < 12; ++q)
     {
-        jx += double(W[q * v]) * s[q];
-        jy += double(W[(12 + q) * v]) * s[q];
-        jz += double(W[(24 + q) * v]) * s[q];
+        jx += double(w[q]) * s[q];
+        jy += double(w[12 + q]) * s[q];
+        jz += double(w[24 + q]) * s[q];
     }
 }
 
-// J_cell in a pass of its own over the inner cells
-template <typename WT, class A> __global__ void __launch_bounds__(kHotThreads) k_jcell_t(const __grid_constant__ A a)
+// J_cell in a pass of its own over the inner cells: 51 values read and written
+// per cell, 36 of them weights.  A few cells per thread's worth of loads in
+// flight bound it: on 6 x 64 x 32 x 32 cells 36.2 us with the weights in planes,
+// 31.2 in tiles of the inner cells, 29.0 with every load issued first (3 CTAs per
+// SM; 2 and 4 the same); in FP32 weights on 2 x 37 x 21 x 25 cells 10.2 and 7.9.
+template <typename WT, class A> __global__ void __launch_bounds__(kHotThreads, 3) k_jcell_t(const __grid_constant__ A a)
 {
     uint32_t t, p;
     const HotBlock &b = hot_block<KIND_CELL0>(a, t);
@@ -697,7 +713,7 @@ template <typename WT, class A> __global__ void __launch_bounds__(kHotThreads) k
     if (!in_box)
         return;
     double jx, jy, jz;
-    jcell_sum<WT>(b, p, jx, jy, jz);
+    jcell_sum<WT, true>(b, p, hot_cell(b, i, j, k), jx, jy, jz);
     const uint64_t v = b.vol;
     double *Jc = hot_at(b, p, F_Jcell);
     Jc[0] = jx;
@@ -879,7 +895,7 @@ __device__ __forceinline__ void pv_uplus_dt_body(const A &a, const Consts &c, un
         constexpr bool kEarly = sizeof(WT) == sizeof(double);
         double jx, jy, jz;
         if (jc && !kEarly)
-            jcell_sum<WT>(b, p, jx, jy, jz);
+            jcell_sum<WT, false>(b, p, hot_cell(b, i, j, k), jx, jy, jz);
         const CellState s = cell_state(U, c);
         if (kEarly)
             store_cell_state<WT>(b, p, U[0], s);
@@ -927,7 +943,7 @@ __device__ __forceinline__ void pv_uplus_dt_body(const A &a, const Consts &c, un
             if (jc)
             {
                 if (kEarly)
-                    jcell_sum<WT>(b, p, jx, jy, jz);
+                    jcell_sum<WT, false>(b, p, hot_cell(b, i, j, k), jx, jy, jz);
                 double *Jc = hot_at(b, p, F_Jcell);
                 Jc[0] = jx;
                 Jc[v] = jy;

@@ -128,10 +128,11 @@ struct BlockView
     int G;            // padding ghost layers
     int NJ, NK;       // padded extents (j, k)
     int64_t vol;      // doubles per component plane
+    int wtiles;       // the weights in tiles (0: in planes, a view outside the pool)
     // mixed precision only (null otherwise): FP32 planes on the same padded box
     float *g32;       // face area xi, eta, zeta, then their unit normals
     float *q32;       // face-state quantities rho, u, v, w, p, rhoE, c
-    float *w32;       // least-squares weights: Bcell_from_Bface_w (18 planes), Jcell_from_Jedge_w (36)
+    float *w32;       // least-squares weights, in the order of the FP64 fields: Bcell_from_Bface_w (18), Jcell_from_Jedge_w (36)
     // SSP-RK2 only (null otherwise): the state at the step's start, U_H 5
     // planes then B_xi, B_eta, B_zeta, on the same padded box
     double *rk;
@@ -194,6 +195,71 @@ enum : int
 __host__ __device__ inline int64_t pidx(const BlockView &b, int i, int j, int k)
 {
     return (int64_t(i + b.G) * b.NJ + (j + b.G)) * b.NK + (k + b.G);
+}
+
+// The least-squares weights (and their FP32 copies) are not stored in planes.
+// Every pass over them takes the inner cells, 18 or 36 values each, and they are
+// the larger part of what it reads; in planes a warp's row of cells ends at the
+// ghost cells, whose bytes come along with the row's last lines.  So the inner
+// cells come first, one after another (weight_cell), then the other padded
+// points in their order, in tiles of kWTile cells: all weights of a tile's cells,
+// component by component, a constant distance apart.  On 6 x 80 x 40 x 40 cells
+// the B_cell pass takes 53.6 us (57.7 in planes) and the primitive pass 98.7
+// (103); on 6 x 64 x 32 x 32 cells J_cell alone 31.2 (36.2); with the FP32 copies
+// on 2.27 M cells the primitive pass 190 (202).  Tiles of padded points gain
+// nothing in FP64, and rows padded to 32, 64 or 128 bytes lose 1 to 5% of a step:
+// what counts is how far apart the cells lie.
+constexpr int kWTile = 32;
+__host__ __device__ constexpr bool weight_field(int f) { return f == F_WB || f == F_WJ; }
+// inner cells before the padded point (i, j, k) in the padded order
+__host__ __device__ inline int64_t inner_before(const BlockView &b, int i, int j, int k)
+{
+    auto upto = [](int x, int n) { return x < 0 ? 0 : x > n ? n : x; };
+    int64_t n = int64_t(upto(i, b.ni)) * b.nj * b.nk;
+    if (i >= 0 && i < b.ni)
+    {
+        n += int64_t(upto(j, b.nj)) * b.nk;
+        if (j >= 0 && j < b.nj)
+            n += upto(k, b.nk);
+    }
+    return n;
+}
+__host__ __device__ inline int64_t weight_cell(const BlockView &b, int i, int j, int k)
+{
+    if (i >= 0 && j >= 0 && k >= 0 && i < b.ni && j < b.nj && k < b.nk)
+        return (int64_t(i) * b.nj + j) * b.nk + k;
+    return int64_t(b.ni) * b.nj * b.nk + pidx(b, i, j, k) - inner_before(b, i, j, k);
+}
+// the padded point of weight cell d (weight_cell's inverse)
+inline uint32_t weight_point(const BlockView &v, int64_t d)
+{
+    const int64_t n = int64_t(v.ni) * v.nj * v.nk;
+    if (d < n)
+        return uint32_t(pidx(v, int(d / (int64_t(v.nj) * v.nk)), int(d / v.nk % v.nj), int(d % v.nk)));
+    // the first padded point with more than d - n points outside the cells up to it
+    int64_t lo = 0, hi = v.vol - 1;
+    while (lo < hi)
+    {
+        const int64_t p = (lo + hi) / 2, ij = p / v.NK;
+        const int i = int(ij / v.NJ) - v.G, j = int(ij % v.NJ) - v.G, k = int(p % v.NK) - v.G;
+        const bool cell = i >= 0 && j >= 0 && k >= 0 && i < v.ni && j < v.nj && k < v.nk;
+        if (p - inner_before(v, i, j, k) + (cell ? 0 : 1) > d - n)
+            hi = p;
+        else
+            lo = p + 1;
+    }
+    return uint32_t(lo);
+}
+// component 0 of cell d (the next components kWTile values on each)
+__host__ __device__ inline int64_t weight_tile(int64_t d, int ncomp)
+{
+    return (d & ~int64_t(kWTile - 1)) * ncomp + (d & (kWTile - 1));
+}
+// component m of field f at point (i, j, k), from the field's first value
+__host__ __device__ inline int64_t field_index(const BlockView &b, int f, int ncomp, int m, int i, int j, int k)
+{
+    return b.wtiles && weight_field(f) ? weight_tile(weight_cell(b, i, j, k), ncomp) + int64_t(m) * kWTile
+                                       : int64_t(m) * b.vol + pidx(b, i, j, k);
 }
 
 } // namespace mhd

@@ -38,3 +38,24 @@ def test_planes(lib):
     for f, (_, _, ncomp, _) in enumerate(mhd.field_table()):
         assert lib.hot_plane_of(f) == q
         q += ncomp
+
+
+@pytest.mark.parametrize("n", [(1, 1, 1), (2, 3, 5), (1, 33, 4), (8, 6, 31), (5, 1, 32)])
+@pytest.mark.parametrize("G", [4, 5])
+def test_weight_order(lib, n, G):
+    """every padded point has one place, the inner cells come first in their
+    own order, the place leads back to the point, and no two values of a
+    field share an index below the size of its planes"""
+    ext = [x + 1 + 2 * G for x in n]
+    vol = int(np.prod(ext))
+    cell, back = np.empty(vol, np.int64), np.empty(vol, np.int64)
+    lib.weight_order(*n, G, cell.ctypes.data_as(C.c_void_p), back.ctypes.data_as(C.c_void_p))
+    assert np.array_equal(np.sort(cell), np.arange(vol))
+    assert np.array_equal(back, np.arange(vol))
+    inner = cell.reshape(ext)[G:G + n[0], G:G + n[1], G:G + n[2]]
+    assert np.array_equal(inner.ravel(), np.arange(inner.size))
+    lib.weight_value.restype = C.c_int64
+    for nc in (18, 36):
+        at = {lib.weight_value(C.c_int64(int(d)), nc, m) for d in (0, 31, 32, vol - 1) for m in range(nc)}
+        assert len(at) == nc * len({0, 31, 32, vol - 1})
+        assert max(at) < nc * (-(-vol // 32) * 32)

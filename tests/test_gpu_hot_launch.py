@@ -109,3 +109,17 @@ def test_resistive_operator_forms(group, monkeypatch):
             s.ctx.close()
     for k, a in out[0].items():
         assert np.array_equal(a, out[1][k]), k
+
+
+@pytest.mark.parametrize("n", [(3, 4, 5), (2, 5, 33)])
+def test_weights_keep_their_points(n):
+    """the least-squares weights, stored in tiles of inner cells: every value
+    of an uploaded field, ghosts included, comes back from its own point"""
+    s = solver.Solver(case.periodic_box_case(n))
+    try:
+        for f in ("Bcell_from_Bface_w", "Jcell_from_Jedge_w"):
+            a = np.random.Generator(np.random.PCG64(5)).standard_normal(s.field(f).shape)
+            s.ctx.upload(f, 0, a)
+            assert np.array_equal(s.field(f), a), f
+    finally:
+        s.ctx.close()
