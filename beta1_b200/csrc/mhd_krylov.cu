@@ -399,6 +399,12 @@ __device__ void hall_newton_test(HallCtl *c, cudaGraphConditionalHandle h, int u
 // order.  Products are taken in chunks of at most kChunk per pass over the
 // vectors (registers per thread stay bounded whatever the basis size).
 constexpr int kChunk = 8;
+// Partials a lane of the last CTA loads per trip (592 CTAs: 19 partials a lane,
+// three trips in place of five): the end of a reduction is the last CTA's round
+// trips.  With one fence per CTA, a Hall step on 2 x 37 x 21 x 25 cells takes 536
+// us in place of 557 and on 6 x 64 x 32 x 32 cells 2127 in place of 2154; 20 per
+// trip cost the passes their occupancy (jv_dots 32 -> 46 us).
+constexpr int kLanePartials = 8;
 
 // the CTA's partial sums of products c0 + q (q < N, c0 + q < nd)
 template <int N>
@@ -435,19 +441,33 @@ __device__ bool grid_finish(int nd, const double *__restrict__ partial, double *
     constexpr int kWarps = kRedThreads / 32;
     __shared__ bool last;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    __threadfence();
     __syncthreads();
     if (threadIdx.x == 0)
+    {
+        // the CTA's partials are ordered before the count by the barrier above
+        // and the fence, the others' before the reads below likewise
+        __threadfence();
         last = (atomicAdd(done, 1u) == gridDim.x - 1);
+        __threadfence();
+    }
     __syncthreads();
     if (!last)
         return false;
-    __threadfence();
     for (int c = wid; c < nd; c += kWarps)
     {
+        // a lane's partials eight to a trip, added in CTA order
         double s = 0.0;
-        for (int b = lane; b < int(gridDim.x); b += 32)
-            s += __ldcg(&partial[int64_t(c) * gridDim.x + b]);
+        for (int b0 = lane; b0 < int(gridDim.x); b0 += 32 * kLanePartials)
+        {
+            double v[kLanePartials];
+#pragma unroll
+            for (int u = 0; u < kLanePartials; ++u)
+                v[u] = b0 + 32 * u < int(gridDim.x) ? __ldcg(&partial[int64_t(c) * gridDim.x + b0 + 32 * u]) : 0.0;
+#pragma unroll
+            for (int u = 0; u < kLanePartials; ++u)
+                if (b0 + 32 * u < int(gridDim.x))
+                    s += v[u];
+        }
         for (int o = 16; o > 0; o >>= 1)
             s += __shfl_down_sync(0xffffffffu, s, o);
         if (lane == 0)
