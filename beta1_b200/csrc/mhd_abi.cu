@@ -159,7 +159,7 @@ const char *const kKernelNames[] = {
     "k_bcell_jedge",  "k_fluid_ucontra", "k_wall_u_all",   "k_hall_cell",    "k_hall_edge",
     "k_pack_vec",     "k_geom32",       "k_fluid_mixed",  "k_gmres_resist", "k_pole",
     "k_geometry",     "k_diag_init",   "k_diag",        "k_rk2",          "k_hall_begin",    "k_hall_step_begin",
-    "k_hall_gmres_init", "k_hall_cycle_prep", "k_hall_ls_begin", "k_hall_ls_check", "k_hall_accept",
+    "k_hall_cycle_prep", "k_hall_ls_begin", "k_hall_ls_check", "k_hall_accept",
     "k_hall_trial",   "k_hall_jv_dots", "k_hall_proj_dots", "k_hall_next",  "k_hall_res_dots", "k_hall_restart_r",
     "k_hall_gmres_prologue", "k_norm2", "k_hall_take",    "k_copy_segments"};
 constexpr int kNumKernelNames = int(sizeof(kKernelNames) / sizeof(kKernelNames[0]));
@@ -1555,13 +1555,13 @@ int hall_cycle(mhd_ctx *ctx, cudaGraphConditionalHandle hout)
 {
     auto &H = ctx->hall;
     const int use = hall_use(ctx);
-    HALL_RED(k_norm2, H.dx, H.n, H.partial, H.dots + 40, H.done);
+    HALL_RED(k_norm2, H.dx, H.n, H.partial, H.dots + 40, H.done, &H.ctl->first, nullptr);
     cudaGraphConditionalHandle hr;
     RUN(new_handle(ctx, &hr));
     LAUNCH1(k_hall_cycle_prep, H.ctl, H.dots + 40, hr, use);
     RUN(hall_cond(ctx, cudaGraphCondTypeIf, hr, &H.ctl->restart, hall_restart_product, &H.kb[HALL_KB_RESTART],
                   &H.eager[HALL_KB_RESTART]));
-    HALL_RED(k_norm2, H.r, H.n, H.partial, H.dots + 44, H.done);
+    HALL_RED(k_norm2, H.r, H.n, H.partial, H.dots + 44, H.done, &H.ctl->r_is_b, H.dots + 56);
     cudaGraphConditionalHandle hin;
     RUN(new_handle(ctx, &hin));
     LAUNCH1(k_cycle_start, H.st, H.dots + 44, hin, use);
@@ -1590,12 +1590,10 @@ int hall_newton_step(mhd_ctx *ctx, cudaGraphConditionalHandle hn)
 {
     auto &H = ctx->hall;
     const int use = hall_use(ctx);
-    HALL_RED(k_norm2, H.X, H.n, H.partial, H.dots + 52, H.done);
-    LAUNCH1(k_hall_step_begin, H.ctl, H.dots + 52);
-    HALL_RED(k_hall_gmres_prologue, H.F, H.b, H.r, H.dx, H.n, H.partial, H.dots + 56, H.done);
+    HALL_RED(k_hall_gmres_prologue, H.F, H.b, H.r, H.dx, H.X, H.n, H.partial, H.dots + 56, H.done);
     cudaGraphConditionalHandle hout;
     RUN(new_handle(ctx, &hout));
-    LAUNCH1(k_hall_gmres_init, H.st, H.dots + 56, H.ksp_rtol, 0.0, H.ksp_maxit, H.restart, hout, use);
+    LAUNCH1(k_hall_step_begin, H.ctl, H.st, H.dots + 56, H.ksp_rtol, 0.0, H.ksp_maxit, H.restart, hout, use);
     RUN(hall_cond(ctx, cudaGraphCondTypeWhile, hout, &H.st->outer, hall_cycle, &H.kb[HALL_KB_CYCLE],
                   &H.eager[HALL_KB_CYCLE]));
     cudaGraphConditionalHandle hls;

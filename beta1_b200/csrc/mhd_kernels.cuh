@@ -264,7 +264,8 @@ struct HallCtl
     int it, maxit;    // Newton steps taken / allowed
     int cut;          // line-search halvings in this step
     int reason;       // 2 ||F|| <= atol, 3 ||F|| <= rtol ||F0||, -5 step limit
-    int first;        // the first GMRES cycle of the Newton step (r = b, no product)
+    int first;        // the first GMRES cycle of the Newton step (r = b, dx = 0, no product)
+    int r_is_b;       // ... the cycle under way
     int newton, ls, restart; // loop conditions
     long long lin0;          // cumulative GMRES iterations before this solve
     long long pass[3];       // cumulative: Newton steps, restart products, line-search trials
@@ -273,9 +274,8 @@ struct HallCtl
 constexpr int kMdMax = 32;
 __global__ void k_hall_begin(HallCtl *c, const double *f2, const GmresState *st, double rtol, double atol, int maxit,
                              cudaGraphConditionalHandle h, int use);
-__global__ void k_hall_step_begin(HallCtl *c, const double *x2);
-__global__ void k_hall_gmres_init(GmresState *st, const double *b2, double rtol, double atol, int maxit, int m,
-                                  cudaGraphConditionalHandle hout, int use);
+__global__ void k_hall_step_begin(HallCtl *c, GmresState *st, const double *bx2, double rtol, double atol, int maxit,
+                                  int m, cudaGraphConditionalHandle hout, int use);
 __global__ void k_hall_cycle_prep(HallCtl *c, const double *dx2, cudaGraphConditionalHandle h, int use);
 __global__ void k_hall_ls_begin(HallCtl *c, cudaGraphConditionalHandle h, int use);
 __global__ void k_hall_ls_check(HallCtl *c, const double *ft2, cudaGraphConditionalHandle h, int use);
@@ -315,10 +315,11 @@ __global__ void k_hall_res_dots(const double *pool, const uint64_t *e, const dou
 __global__ void k_hall_restart_r(const double *pool, const uint64_t *e, const double *Xt, const double *F,
                                  const double *h, const double *b, double *r, int64_t n);
 // b = -F, r = b, dx = 0; out[0] = b . b
-__global__ void k_hall_gmres_prologue(const double *F, double *b, double *r, double *dx, int64_t n, double *partial,
-                                      double *out, unsigned *done);
-// out[0] = x . x
-__global__ void k_norm2(const double *x, int64_t n, double *partial, double *out, unsigned *done);
+__global__ void k_hall_gmres_prologue(const double *F, double *b, double *r, double *dx, const double *X, int64_t n,
+                                      double *partial, double *out, unsigned *done);
+// out[0] = x . x; where *known is set the value is *val already (val null: nobody asks for it)
+__global__ void k_norm2(const double *x, int64_t n, double *partial, double *out, unsigned *done, const int *known,
+                        const double *val);
 // X = Xt, F = Ft
 __global__ void k_hall_take(double *X, const double *Xt, double *F, const double *Ft, int64_t n);
 // dst = src over nseg segments (seg: dst offset, src offset, length)

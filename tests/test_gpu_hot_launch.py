@@ -1,12 +1,14 @@
 """The hot kernels' launch forms: batches past the blocks of one launch (65
 runs and more: two launches per kernel), grids past the small argument form
-(9 blocks and more), a batch of several runs against each run alone, and the
-components of Eface the face kernel leaves alone.  Every form runs the same
-arithmetic per point, so the fields agree bit for bit."""
+(9 blocks and more), a batch of several runs against each run alone, the
+components of Eface the face kernel leaves alone, the resistive operator's
+lists, the weights' order in memory and restarts of the Hall solve.  Every form
+but the last runs the same arithmetic per point, so the fields agree bit for
+bit."""
 import numpy as np
 import pytest
 
-from conftest import load_golden, periodic_setup, slab_setup
+from conftest import load_golden, periodic_setup, rel_l2, slab_setup
 
 from beta1_b200 import case, mhd, solver
 
@@ -123,3 +125,28 @@ def test_weights_keep_their_points(n):
             assert np.array_equal(s.field(f), a), f
     finally:
         s.ctx.close()
+
+
+def test_hall_restart_cycles():
+    """linear solves held past a restart (30 basis vectors) by an unreachable
+    tolerance take the norms of dx and r that a first cycle leaves out: the
+    Newton steps reach the root that unrestarted solves reach.  Both stop at
+    1e-12 of the first residual, as the comparison with the reference's solve,
+    whose bound is 1e-10 relative L2."""
+    spec = case.slab_case(24, (5, 6), (2, 2))
+    st = case.inflow_state(spec, seed=20261205)
+    out, stats = [], []
+    for ksp in (dict(ksp_rtol=1e-10, ksp_maxit=2000), dict(ksp_rtol=1e-300, ksp_maxit=65)):
+        s = solver.Solver(spec, topology="tiled")
+        try:
+            s.load_state(st)
+            s.install_hall_implicit("tiled", rtol=1e-12, atol=1e-30, maxit=200, **ksp)
+            s.step(1)
+            stats.append(s.ctx.hall_stats())
+            out.append({(f, b): s.field(f, b) for f in ("Ehall_xi", "Ehall_eta", "B_xi", "B_zeta", "U_H")
+                        for b in range(len(spec.blocks))})
+        finally:
+            s.ctx.close()
+    assert stats[1]["reason"] in (2, 3) and stats[1]["linear_its"] > 30 * stats[1]["its"], stats
+    for k, a in out[0].items():
+        assert rel_l2(out[1][k], a) <= 1e-10, (k, stats)
