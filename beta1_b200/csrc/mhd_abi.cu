@@ -3876,7 +3876,9 @@ int mhd_set_resistive(mhd_ctx *ctx, int64_t n, const int64_t *unknowns, const do
     R.halias_of = fidx;
     R.hsign = fs;
     RUN(build_operator(ctx));
-    // every point of the solve's fields starts at zero
+    // every point of the solve's fields starts at zero (an upload of one of them
+    // may still be under way on the context's stream)
+    CK(ctx, cudaStreamSynchronize(ctx->stream));
     for (int f0 : {int(F_Eresxi), int(F_dBxi), int(F_dJxi), int(F_RBresxi)})
         for (int f = f0; f < f0 + 3; ++f)
             for (int b = 0; b < ctx->nblocks; ++b)
