@@ -69,19 +69,19 @@ ALGO_BYTES_PER_CELL = {
     "k_fluid_rhs": 31 * 8,
     # JD 9, Jac 1, U_plus 3 read; U_contra 3 written
     "k_ucontra": 16 * 8,
-    # B 3, Badd 3, U_contra 3 read; Eface 9 written
-    "k_eface": 18 * 8,
+    # B 3, Badd 3, U_contra 3 read; the 6 components of Eface that are not zero written
+    "k_eface": 15 * 8,
     # Eface 6, B 3, U_contra 3 read; E 3 written
     "k_eedge": 15 * 8,
     # E 3 read, RHS_B 3 written, B 3 read + written
     "k_curl_e2f": 12 * 8,
-    # U 5 read + written, RHS_H 5 read
-    "k_update_u": 15 * 8,
+    # the Euler update of cells and faces: U 5 read + written, RHS_H 5 read; E 3 read, RHS_B 3 written, B 3 read + written
+    "k_update_u": 27 * 8,
     # B_cell + J edges: B 3, Badd 3, W_B 18, beta 3, alpha 3 read; B_cell 3, Bind_cell 3, J 3 written
     "k_bcell_jedge": 39 * 8,
     # PV / U_plus / CFL with J_cell: U 5, Jac 1, B_cell 3, face area + normal 12, J 3, W_J 36 read;
-    # PV 5, U_plus 3, Csound 1, RhoE 1, J_cell 3 written
-    "k_pv_uplus_dt": 73 * 8,
+    # PV 4 (T is left to read-out), U_plus 3, Csound 1, RhoE 1, J_cell 3 written
+    "k_pv_uplus_dt": 72 * 8,
     # Hall EMF: B_cell 3, J_cell 3, rho 1 read; E_hall_cell 3, beta 1 written (per cell) / E_hall_cell 3,
     # beta 1, B 3, face area 3, dl 3, dr 9 read; E_hall 3 written (per edge triple)
     "k_hall_cell": 11 * 8,
@@ -119,16 +119,15 @@ ALGO_BYTES_MIXED = {"k_pv_uplus_dt": 12 * 8 + 48 * 4 + 6 * 8 + 7 * 4,
 # the dominant kernel, from one ncu capture of a smaller case of the same
 # workload, scaled by the cell count to a full launch (the kernels' traffic
 # grows with the cells they cover):
-# * C2 at half the cells per direction (165,888 cells: 114.26 MB read +
-#   10.32 MB written) to the full C2 slab (1,327,104 cells);
-# * the shell sweep's first 6 runs (2,269,318 cells; k_fluid_mixed at 3 CTAs
-#   per SM 602.60 MB read + 145.68 MB written, k_pv_uplus_dt 763.50 + 185.09
-#   MB) to all 48 runs (14,879,028 cells)
+# * C2 at half the cells per direction (165,888 cells: 95.83 MB read +
+#   10.54 MB written) to the full C2 slab (1,327,104 cells);
+# * the shell sweep's first 6 runs (2,269,318 cells; k_fluid_mixed
+#   667.88 MB read + 158.57 MB written, k_pv_uplus_dt 711.88 + 170.01 MB) to all 48 runs (14,879,028 cells)
 _SWEEP_SCALE = 14879028.0 / 2269318.0
 NCU_TRAFFIC_BYTES = {
-    ("k_pv_uplus_dt", "c2_slab6x96x48x48_implicit_resistive_fp64"): (114.25536e6 + 10.321408e6) * 8.0,
-    ("k_fluid_mixed", "c5s_sweep48_shell_runs_mixed"): (602.596096e6 + 145.683968e6) * _SWEEP_SCALE,
-    ("k_pv_uplus_dt", "c5s_sweep48_shell_runs_mixed"): (763.501568e6 + 185.093888e6) * _SWEEP_SCALE,
+    ("k_pv_uplus_dt", "c2_slab6x96x48x48_implicit_resistive_fp64"): (95.830272e6 + 10.536192e6) * 8.0,
+    ("k_fluid_mixed", "c5s_sweep48_shell_runs_mixed"): (667.88224e6 + 158.565376e6) * _SWEEP_SCALE,
+    ("k_pv_uplus_dt", "c5s_sweep48_shell_runs_mixed"): (711.876352e6 + 170.00576e6) * _SWEEP_SCALE,
 }
 
 
