@@ -8,6 +8,7 @@
 // reference bit for bit.
 #include "mhd_kernels.cuh"
 #include "mhd_hot_launch.cuh"
+#include "mhd_basis.cuh"
 
 #include <cfloat>
 #include <algorithm>
@@ -693,16 +694,17 @@ struct PreItems
     PreRegion r;
 };
 
-// y = A (src / div) (MatMultImplicitResistive_): Eres at the unknowns and
-// their aliases, Sync("Eres1form"), dB = -dt curl Eres on the region,
-// Sync("dB"), then per unknown dJ = alpha curlAdj(beta dB) at its edge and
-// y = Eres - eta dJ.  src must be complete at entry unless first_barrier:
-// the aliases read other threads' elements.  src / div is the stored basis
-// vector bit for bit (the same division), so the basis vector itself need
-// not be complete.  first: the solve's first product, which also writes the
-// points whose value no later one changes (the static tails of the lists).
+// y = A src (MatMultImplicitResistive_): Eres at the unknowns and their
+// aliases, Sync("Eres1form"), dB = -dt curl Eres on the region, Sync("dB"),
+// then per unknown dJ = alpha curlAdj(beta dB) at its edge and y = Eres - eta
+// dJ.  What src reads must be complete at entry unless first_barrier: the
+// aliases read other threads' elements.  src is the stored basis vector bit
+// for bit (the same operations), so the basis vector itself need not be
+// complete; y may be the array src reads (it is written after the last
+// barrier).  first: the solve's first product, which also writes the points
+// whose value no later one changes (the static tails of the lists).
 __device__ bool grid_matvec(const ResistSolve &a, GridBar &gb, const HotBlock *hb, const PreItems &pre,
-                            const double *src, double div, bool first_barrier, bool first, double *y)
+                            const BasisVec &src, bool first_barrier, bool first, double *y)
 {
     const int64_t t0 = int64_t(blockIdx.x) * blockDim.x + threadIdx.x, ts = int64_t(gridDim.x) * blockDim.x;
     if (first_barrier && !grid_barrier(gb))
@@ -716,9 +718,9 @@ __device__ bool grid_matvec(const ResistSolve &a, GridBar &gb, const HotBlock *h
             const PreFused x = q == t0 ? pre.fa : load_fused(a.fa, hb, q);
             double v;
             if (x.kind == FUSE_UNKNOWN)
-                v = src[x.idx] / div;
+                v = src.at(x.idx);
             else if (x.kind == FUSE_ALIAS)
-                v = x.val * (src[x.idx] / div);
+                v = x.val * src.at(x.idx);
             else if (x.kind == FUSE_CONST)
                 v = x.val;
             else
@@ -731,9 +733,9 @@ __device__ bool grid_matvec(const ResistSolve &a, GridBar &gb, const HotBlock *h
     else
     {
         for (int64_t t = t0; t < a.n; t += ts)
-            a.pool[a.e[t]] = src[t] / div;
+            a.pool[a.e[t]] = src.at(t);
         for (int64_t q = t0; q < a.nalias; q += ts)
-            a.pool[a.alias[q]] = a.sign[q] * (src[a.alias_of[q]] / div);
+            a.pool[a.alias[q]] = a.sign[q] * src.at(a.alias_of[q]);
         if (a.merge1)
             for (int64_t t = t0; t < a.eres1form.nconst; t += ts)
                 a.pool[a.eres1form.cdst[t]] = a.eres1form.cval[t];
@@ -842,7 +844,7 @@ __global__ void __launch_bounds__(256) k_gmres_resist(ResistSolve a)
     for (;;)
     {
         // cycle start: r = b - A x, beta = ||r||
-        if (!grid_matvec(a, gb, hb, pre, a.x, 1.0, true, S.cycles == 0, a.w))
+        if (!grid_matvec(a, gb, hb, pre, BasisVec{a.x, 1.0, nullptr, nullptr, 0, n}, true, S.cycles == 0, a.w))
             return;
         for (int64_t t = t0; t < n; t += ts)
             a.r[t] = a.b[t] - a.w[t];
@@ -876,9 +878,11 @@ __global__ void __launch_bounds__(256) k_gmres_resist(ResistSolve a)
         while (S.inner)
         {
             const int j = S.j;
-            // V_j = r / beta (j = 0) or the previous step's w / ||w||, both
-            // complete at the last reduction's barrier
-            if (!grid_matvec(a, gb, hb, pre, j == 0 ? a.r : a.w, j == 0 ? S.beta : S.hcol[j], false, false, a.w))
+            // V_j: r / beta (j = 0), or from the previous step's w', basis
+            // and products, complete at the last reduction's barrier
+            const BasisVec vj = j == 0 ? BasisVec{a.r, S.beta, nullptr, nullptr, 0, n}
+                                       : BasisVec{a.w, S.hcol[j], a.V, S.d, j, n};
+            if (!grid_matvec(a, gb, hb, pre, vj, false, false, a.w))
                 return;
             // classical Gram-Schmidt, twice
             if (!grid_dots(a, gb, a.V, j + 1, a.w, S.hcol, pbuf))
@@ -891,16 +895,10 @@ __global__ void __launch_bounds__(256) k_gmres_resist(ResistSolve a)
                 a.w[t] = s;
             }
             // second pass, its dots and ||w'||^2 in one reduction: with V
-            // orthonormal, ||w' - V d||^2 = ||w'||^2 - ||d||^2
+            // orthonormal, ||w' - V d||^2 = ||w'||^2 - ||d||^2; w' itself
+            // stays, for the next product's reads of other threads' elements
             if (!grid_dots(a, gb, a.V, j + 1, a.w, S.d, pbuf, true))
                 return;
-            for (int64_t t = t0; t < n; t += ts)
-            {
-                double s = a.w[t];
-                for (int c = 0; c <= j; ++c)
-                    s -= S.d[c] * a.V[int64_t(c) * n + t];
-                a.w[t] = s;
-            }
             if (tid <= j)
                 S.hcol[tid] += S.d[tid];
             __syncthreads();
@@ -933,8 +931,11 @@ __global__ void __launch_bounds__(256) k_gmres_resist(ResistSolve a)
             }
             __syncthreads();
             if (!S.breakdown)
+            {
+                const BasisVec next{a.w, S.hcol[j + 1], a.V, S.d, j + 1, n};
                 for (int64_t t = t0; t < n; t += ts)
-                    a.V[int64_t(j + 1) * n + t] = a.w[t] / S.hcol[j + 1];
+                    a.V[int64_t(j + 1) * n + t] = next.at(t);
+            }
             __syncthreads();
             if (tid == 0)
             {
