@@ -1709,32 +1709,23 @@ int launch_step(mhd_ctx *ctx)
     return launch_step_c(ctx);
 }
 
+// Error word of the steps so far, from its host copy.  After any error the
+// device words start afresh: the error word, and the barrier of the persistent
+// solve, which a solve that gave up leaves at a count no later one may build on.
 int check_err(mhd_ctx *ctx)
 {
     CK(ctx, cudaStreamSynchronize(ctx->stream));
-    if (*ctx->h_err == 0)
+    const int e = *ctx->h_err;
+    if (e == MHD_OK)
         return MHD_OK;
-    *ctx->h_err = 0;
-    int e = 0;
-    CK(ctx, cudaMemcpy(&e, ctx->err, sizeof(int), cudaMemcpyDeviceToHost));
-    if (e == MHD_EDT)
-    {
-        double d = 0.0;
-        cudaMemcpy(&d, ctx->dt, sizeof(double), cudaMemcpyDeviceToHost);
-        const int z = 0;
-        cudaMemcpy(ctx->err, &z, sizeof(int), cudaMemcpyHostToDevice);
-        return fail(ctx, MHD_EDT, "dt too small or NaN: dt=%.3e", d);
-    }
+    *ctx->h_err = MHD_OK;
+    CK(ctx, cudaMemsetAsync(ctx->err, 0, sizeof(int), ctx->stream));
+    if (ctx->res.bar)
+        CK(ctx, cudaMemsetAsync(ctx->res.bar, 0, 4 * sizeof(unsigned), ctx->stream));
+    CK(ctx, cudaStreamSynchronize(ctx->stream));
     if (e == MHD_EKRYLOV)
-    {
-        const int z = 0;
-        cudaMemcpy(ctx->err, &z, sizeof(int), cudaMemcpyHostToDevice);
-        if (ctx->res.bar)
-            cudaMemset(ctx->res.bar, 0, 4 * sizeof(unsigned));
-        cudaStreamSynchronize(cudaStreamLegacy); // (ctx->stream does not wait for it)
         return fail(ctx, MHD_EKRYLOV, "persistent Krylov solve: a grid barrier wait gave up");
-    }
-    return MHD_OK;
+    return fail(ctx, MHD_EDT, "dt too small or NaN: dt=%.3e", ctx->h_mirror[0]);
 }
 
 // dt and time of the first nr runs after nsteps steps and check_err(): from

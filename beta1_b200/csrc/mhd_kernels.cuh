@@ -43,11 +43,10 @@ __device__ __forceinline__ void begin_run(const RunClock &rc, int r)
     const double d = __longlong_as_double((long long)rc.dt_key[r]);
     rc.dt[r] = d;
     rc.h_dt[r] = d;
-    if (!isfinite(d) || d < rc.dt_abort)
-    {
-        rc.err[0] = MHD_EDT;
+    // the first error of a span stays: a solve that gave up in an earlier step
+    // must not lose its mark, by which later solves leave the barrier alone
+    if ((!isfinite(d) || d < rc.dt_abort) && atomicCAS(rc.err, MHD_OK, MHD_EDT) == MHD_OK)
         *rc.h_err = MHD_EDT;
-    }
 }
 __device__ __forceinline__ void end_run(const RunClock &rc, int r)
 {
