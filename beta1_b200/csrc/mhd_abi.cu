@@ -249,6 +249,7 @@ struct mhd_ctx
     int64_t tiles = 0;      // those CTAs
     std::map<std::string, SyncMap> syncs;
     std::map<std::string, StepSync> step_syncs; // by the groups' names joined with '+'
+    int ucell_alone = -1; // Sync("Ucell") may run beside the B_cell pass (side_ucell; -1: not looked at)
     // eta Poles: (block, direction) pairs; a context with Poles runs every
     // sync in the topology order of the Pole shell
     std::vector<int> poles;
@@ -398,6 +399,7 @@ static int materialise_all(mhd_ctx *ctx);
 static void mark_dirty(mhd_ctx *ctx);
 int build_sync(mhd_ctx *ctx, const std::string &group, SyncMap &m);
 static int step_sync(mhd_ctx *ctx, std::initializer_list<const char *> groups, SyncPart part, StepSync **out);
+static int sync_fields(mhd_ctx *ctx, const char *group, std::bitset<NFIELD> &fields);
 
 namespace
 {
@@ -821,18 +823,38 @@ struct SideScope
 // four small launches that the B_cell pass hides (with the Pole J_cell beside the
 // PV pass: a 96 x 64 x 64 shell 230 -> 216 us a step, six shells 877 -> 859, a
 // 4-block slab 34.7 -> 32.6); a copy list alone goes with Sync("Bface")'s in one
-// pass.
-bool side_ucell(const mhd_ctx *ctx)
+// pass.  Only where the tables say so: Ucell's touch U_H alone, and none of the
+// chain's Syncs touches U_H (else in order, as the merged pass does).
+bool has_side_ucell(const mhd_ctx *ctx)
 {
     const auto it = ctx->syncs.find("Ucell");
-    return forks(ctx) && it != ctx->syncs.end() && (!it->second.walls.empty() || !ctx->poles.empty());
+    return it != ctx->syncs.end() && (!it->second.walls.empty() || !ctx->poles.empty());
+}
+int side_ucell(mhd_ctx *ctx, bool &side)
+{
+    side = false;
+    if (!forks(ctx) || !has_side_ucell(ctx))
+        return MHD_OK;
+    if (ctx->ucell_alone < 0)
+    {
+        std::bitset<NFIELD> own, chain;
+        RUN(sync_fields(ctx, "Ucell", own));
+        for (const char *g : {"Bface", "B_cell", "Jedge"})
+            RUN(sync_fields(ctx, g, chain));
+        own.reset(F_U);
+        ctx->ucell_alone = own.none() && !chain.test(F_U) ? 1 : 0;
+    }
+    side = ctx->ucell_alone == 1;
+    return MHD_OK;
 }
 
 // Sync("Ucell"), Sync("Bface"), then UpdateDerivedFields_.  armed: the dt
 // reductions are (the step's update arms them).
 int launch_sync_derived(mhd_ctx *ctx, bool armed)
 {
-    if (!side_ucell(ctx))
+    bool side = false;
+    RUN(side_ucell(ctx, side));
+    if (!side)
     {
         RUN(run_syncs(ctx, {"Ucell", "Bface"}));
         return launch_update_derived(ctx, armed, false);
@@ -2517,6 +2539,7 @@ static void free_step_syncs(mhd_ctx *ctx)
                             (void *)p->cdst32, (void *)p->cval})
                 cudaFree(q);
     ctx->step_syncs.clear();
+    ctx->ucell_alone = -1;
 }
 
 static int upload_pass(mhd_ctx *ctx, const Resolved::Part &r, SyncPass &p)
@@ -3058,6 +3081,35 @@ static int build_hall_list(mhd_ctx *ctx)
     return MHD_OK;
 }
 
+// the fields a group's Sync touches in a step, added to `fields`
+static int sync_fields(mhd_ctx *ctx, const char *group, std::bitset<NFIELD> &fields)
+{
+    const auto it = ctx->syncs.find(group);
+    if (it == ctx->syncs.end())
+        return MHD_OK;
+    SyncMap &m = it->second;
+    if (!m.built)
+    {
+        if (ctx->capturing)
+            return fail(ctx, MHD_ESTATE, "sync group %s changed during capture", group);
+        RUN(build_sync(ctx, it->first, m));
+    }
+    if (!m.walls.empty())
+        fields.set(F_U);
+    if (m.res.usable)
+    {
+        fields |= m.res.fields;
+        return MHD_OK;
+    }
+    const PoolDecoder dec(ctx);
+    int f, b, i, j, k;
+    for (const auto *tab : {&m.hd, &m.hs, &m.hcd, &m.hd2, &m.hs2})
+        for (uint64_t off : *tab)
+            if (dec.decode(off, f, b, i, j, k))
+                fields.set(size_t(f));
+    return MHD_OK;
+}
+
 // every group's lists and the passes of the step (before a capture)
 static int build_all_syncs(mhd_ctx *ctx)
 {
@@ -3067,7 +3119,7 @@ static int build_all_syncs(mhd_ctx *ctx)
     StepSync *s = nullptr;
     RUN(step_sync(ctx, {"Eface"}, SYNC_HOT, &s));
     RUN(step_sync(ctx, {"Eedge"}, SYNC_HOT, &s));
-    if (ctx->syncs.count("Ucell") && (!ctx->syncs["Ucell"].walls.empty() || !ctx->poles.empty()))
+    if (has_side_ucell(ctx))
     {
         RUN(step_sync(ctx, {"Ucell"}, SYNC_HOT, &s));
         RUN(step_sync(ctx, {"Bface"}, SYNC_HOT, &s));
