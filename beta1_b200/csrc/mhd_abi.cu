@@ -139,6 +139,7 @@ struct SyncMap
     bool built = false; // device lists match the host tables
     CopyList full, hot, post;
     Resolved res; // of the hot lists
+    bool into_eface = false; // gives a zero component of Eface another value (eface_zeroed)
     // Pole contexts: the copies and fixed values a step leaves for read-out
     // (cold), written then without the rings, walls and post-wall copies
     CopyList cold;
@@ -261,7 +262,7 @@ struct mhd_ctx
     // and PV / U_plus computed on the first ghost layer only
     std::map<std::string, bool> dirty;
     bool pv_dirty = false;
-    bool eface_zero = true; // the zero components of Eface hold zero on the inner faces
+    bool eface_zero = true; // the zero components of Eface hold zero, but for what into_eface groups write
     bool geom_dirty = true; // face areas / normals to recompute from JD
     std::vector<std::string> field_group = std::vector<std::string>(NFIELD); // group that syncs a field
     double *staging = nullptr;
@@ -956,13 +957,23 @@ int launch_fluid_ucontra(mhd_ctx *ctx, const RunClock &rc = RunClock{})
     return launched(ctx, launch_k_fluid_ucontra(ctx->tune[TUNE_k_fluid_ucontra], ctx->hot, ctx->stream, ctx->c, rc));
 }
 
+int launch_eface_zero(mhd_ctx *ctx)
+{
+    prof_begin(ctx, "k_eface");
+    return launched(ctx, launch_k_eface_zero(ctx->hot, ctx->stream));
+}
 int ensure_eface_zero(mhd_ctx *ctx)
 {
     if (ctx->eface_zero)
         return MHD_OK;
     ctx->eface_zero = true;
-    prof_begin(ctx, "k_eface");
-    return launched(ctx, launch_k_eface_zero(ctx->hot, ctx->stream));
+    return launch_eface_zero(ctx);
+}
+// a table that writes one of the zero components (none of the grid families'
+// does): every step zeroes them before its Syncs run
+bool into_eface(const mhd_ctx *ctx)
+{
+    return std::any_of(ctx->syncs.begin(), ctx->syncs.end(), [](const auto &kv) { return kv.second.into_eface; });
 }
 
 // AssembleRHS_Induction_CT_ up to the edge EMF; with_ucontra unless the fluid pass computed them
@@ -976,6 +987,8 @@ int launch_edge_emf(mhd_ctx *ctx, bool with_ucontra)
         k_ucontra<<<dim3(grid_for(max_box(ctx, LOC_CELL, 1)), nb), kThreads, 0, s>>>(ctx->dbv);
         RUN(launched(ctx));
     }
+    if (into_eface(ctx))
+        RUN(launch_eface_zero(ctx));
     prof_begin(ctx, "k_eface");
     RUN(launched(ctx, launch_k_eface(ctx->tune[TUNE_k_eface], ctx->hot, s)));
     RUN(run_syncs(ctx, {"Eface"}));
@@ -2459,6 +2472,17 @@ struct PoolDecoder
         i = int(ii) - v.G;
         return true;
     }
+    // a component of Eface that the step holds at zero: component a of an inner face of axis a
+    bool eface_zero(uint64_t off) const
+    {
+        int f, b, i, j, k;
+        if (!decode(off, f, b, i, j, k) || f < F_Efxi || f > F_Efzeta)
+            return false;
+        const BlockView &v = ctx->hbv[size_t(b)];
+        const int a = f - F_Efxi;
+        return int((off - start[size_t(b)]) / uint64_t(v.vol)) == plane_of(f) + a && i >= 0 && j >= 0 && k >= 0 &&
+               i < v.ni + (a == 0) && j < v.nj + (a == 1) && k < v.nk + (a == 2);
+    }
 };
 
 // a set of offsets as a sorted list, with a mark per entry
@@ -2731,6 +2755,16 @@ static void resolve_lists(const mhd_ctx *ctx, const SyncMap &m, const PoolDecode
     r.usable = true;
 }
 
+// does a copy, or a fixed value, give a zero component of Eface another value?  (f: the destination's field)
+static bool eface_copy(const PoolDecoder &dec, int f, uint64_t dst, uint64_t src)
+{
+    return f >= F_Efxi && f <= F_Efzeta && dec.eface_zero(dst) && !dec.eface_zero(src);
+}
+static bool eface_const(const PoolDecoder &dec, int f, uint64_t dst, double val)
+{
+    return f >= F_Efxi && f <= F_Efzeta && (val != 0.0 || std::signbit(val)) && dec.eface_zero(dst);
+}
+
 // Hot and cold lists of a Pole context's group.  Its Sync runs the rings,
 // the copies, the wall handlers, the post-wall copies, then the fixed values;
 // a step runs the hot part and read-out the cold part (copies, then fixed
@@ -2758,6 +2792,7 @@ static int build_sync_pole(mhd_ctx *ctx, const std::string &group, SyncMap &m, c
         const bool at = hot_at_point(m.hd[t], f);
         if (f >= 0 && ctx->field_group[size_t(f)] != group)
             ctx->field_group[size_t(f)] = group;
+        m.into_eface |= eface_copy(dec, f, m.hd[t], m.hs[t]);
         const bool hot = all_hot || at || consts.has(m.hs[t]) || post.has(m.hs[t]) ||
                          wall_point(ctx, m, dec, m.hs[t], 0) || wall_point(ctx, m, dec, m.hd[t], 0) ||
                          post.has(m.hd[t]);
@@ -2772,11 +2807,14 @@ static int build_sync_pole(mhd_ctx *ctx, const std::string &group, SyncMap &m, c
         const bool at = hot_at_point(m.hcd[t], f);
         if (f >= 0 && ctx->field_group[size_t(f)] != group)
             ctx->field_group[size_t(f)] = group;
+        m.into_eface |= eface_const(dec, f, m.hcd[t], m.hcv[t]);
         const int64_t c = consts.find(m.hcd[t]);
         const bool hot = all_hot || at || consts.mark[size_t(c)];
         (hot ? cd : cdc).push_back(m.hcd[t]);
         (hot ? cv : cvc).push_back(m.hcv[t]);
     }
+    for (size_t t = 0; t < m.hd2.size(); ++t)
+        m.into_eface |= eface_copy(dec, F_Efxi, m.hd2[t], m.hs2[t]);
     RUN(upload_list(ctx, m.hot, cd, cv, d, s2, m.staged));
     RUN(upload_list(ctx, m.cold, cdc, cvc, dc, sc, m.staged));
     resolve_lists(ctx, m, dec, d, s2, cd, cv, m.res);
@@ -2811,6 +2849,9 @@ int build_sync(mhd_ctx *ctx, const std::string &group, SyncMap &m)
     free_step_syncs(ctx);
     if (group == "Ehall")
         ctx->hall.list_built = false;
+    if (m.into_eface) // (what the table before this one wrote)
+        ctx->eface_zero = false;
+    m.into_eface = false;
     if (!ctx->poles.empty())
         return build_sync_pole(ctx, group, m, dec);
     const HotPoints hot_at_point(ctx, dec);
@@ -2821,6 +2862,7 @@ int build_sync(mhd_ctx *ctx, const std::string &group, SyncMap &m)
         const bool at = hot_at_point(m.hd[t], f);
         if (f >= 0 && ctx->field_group[size_t(f)] != group)
             ctx->field_group[size_t(f)] = group;
+        m.into_eface |= eface_copy(dec, f, m.hd[t], m.hs[t]);
         if (!at)
             continue;
         d.push_back(m.hd[t]);
@@ -2834,6 +2876,7 @@ int build_sync(mhd_ctx *ctx, const std::string &group, SyncMap &m)
         const bool at = hot_at_point(m.hcd[t], f);
         if (f >= 0 && ctx->field_group[size_t(f)] != group)
             ctx->field_group[size_t(f)] = group;
+        m.into_eface |= eface_const(dec, f, m.hcd[t], m.hcv[t]);
         if (at || consts.mark[size_t(consts.find(m.hcd[t]))])
         {
             cd.push_back(m.hcd[t]);
