@@ -753,7 +753,8 @@ __device__ bool grid_matvec(const ResistSolve &a, GridBar &gb, const HotBlock *h
             if (r.faces & (1 << fa))
                 *hot_at(*r.b, r.p, F_dBxi + fa) = mdt * hot_curl(*r.b, r.p, plane_of(F_Eresxi), fa);
     }
-    if (a.merge2 && (first || a.fb.n < 0))
+    // (once per solve where no product writes the points otherwise, as the static tails: the region list is there)
+    if (a.merge2 && (first || a.reg.n < 0))
         for (int64_t t = t0; t < a.db.nconst; t += ts)
             a.pool[a.db.cdst[t]] = a.db.cval[t];
     if (a.fb.n >= 0)
