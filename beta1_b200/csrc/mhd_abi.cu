@@ -250,6 +250,7 @@ struct mhd_ctx
     int64_t tiles = 0;      // those CTAs
     std::map<std::string, SyncMap> syncs;
     std::map<std::string, StepSync> step_syncs; // by the groups' names joined with '+'
+    bool unsettled = false; // copies on the legacy stream may be under way (settle)
     int ucell_alone = -1; // Sync("Ucell") may run beside the B_cell pass (side_ucell; -1: not looked at)
     // eta Poles: (block, direction) pairs; a context with Poles runs every
     // sync in the topology order of the Pole shell
@@ -511,8 +512,28 @@ int ensure_staging(mhd_ctx *ctx, size_t n)
 // ---- launch helpers (all on ctx->stream) ----
 // Eager profiling: prof_begin() records an event before a launch, launched()
 // one after it, so each kernel's duration is measured on the launching stream.
+// Set-up data goes up on the legacy stream, for which the context's streams do
+// not wait, and a copy from pageable memory may return while its last part is
+// still on its way: settle() ends what is under way before the next launch.
+int h2d(mhd_ctx *ctx, void *dst, const void *src, size_t bytes)
+{
+    ctx->unsettled = true;
+    CK(ctx, cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice));
+    return MHD_OK;
+}
+int settle(mhd_ctx *ctx)
+{
+    if (!ctx->unsettled || ctx->capturing)
+        return MHD_OK;
+    CK(ctx, cudaStreamSynchronize(cudaStreamLegacy));
+    ctx->unsettled = false;
+    return MHD_OK;
+}
+
+// before every launch (an error of settle() is the device's own and stays)
 void prof_begin(mhd_ctx *ctx, const char *name)
 {
+    settle(ctx);
     if (!ctx->profiling)
         return;
     cudaEvent_t e;
@@ -1803,6 +1824,7 @@ void drop_graph(mhd_ctx *ctx)
 int capture(mhd_ctx *ctx, int (*body)(mhd_ctx *), cudaGraph_t *graph, cudaGraphExec_t *exec, int64_t *nodes)
 {
     const int64_t before = ctx->launches;
+    RUN(settle(ctx));
     CK(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
     ctx->capturing = true;
     const int rc = body(ctx);
@@ -1870,6 +1892,7 @@ int build_graph(mhd_ctx *ctx)
 int run_steps(mhd_ctx *ctx, int nsteps)
 {
     RUN(build_graph(ctx));
+    RUN(settle(ctx));
     if (nsteps > 0)
         RUN(ensure_eface_zero(ctx));
     for (int s = 0; s < nsteps; ++s)
@@ -1953,9 +1976,7 @@ int build_hot(mhd_ctx *ctx)
     std::vector<HotBlock> all;
     for (const HotChunk &c : ctx->hot.chunks)
         all.insert(all.end(), c.args.v, c.args.v + c.args.n);
-    return cudaMemcpy(ctx->dhot, all.data(), sizeof(HotBlock) * all.size(), cudaMemcpyHostToDevice) == cudaSuccess
-               ? MHD_OK
-               : MHD_ECUDA;
+    return h2d(ctx, ctx->dhot, all.data(), sizeof(HotBlock) * all.size());
 }
 
 int create_ctx(const mhd_block_desc *blocks, int32_t nblocks, const int32_t *run_of_block, int32_t nruns,
@@ -2142,8 +2163,9 @@ int create_ctx(const mhd_block_desc *blocks, int32_t nblocks, const int32_t *run
     if (cudaMemcpy(ctx->dbv, ctx->hbv.data(), sizeof(BlockView) * size_t(nblocks), cudaMemcpyHostToDevice) !=
         cudaSuccess)
         return bail(MHD_ECUDA);
-    if (cudaStreamSynchronize(ctx->stream) != cudaSuccess)
+    if (cudaStreamSynchronize(ctx->stream) != cudaSuccess || cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess)
         return bail(MHD_ECUDA);
+    ctx->unsettled = false;
     *out = ctx;
     return MHD_OK;
 }
@@ -2397,8 +2419,7 @@ template <typename T> static int upload_vec(mhd_ctx *ctx, const std::vector<T> &
     if (v.empty())
         return MHD_OK;
     CK(ctx, cudaMalloc(d, v.size() * sizeof(T)));
-    CK(ctx, cudaMemcpy(*d, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
-    return MHD_OK;
+    return h2d(ctx, *d, v.data(), v.size() * sizeof(T));
 }
 
 static void free_list(CopyList &m)
@@ -3968,14 +3989,13 @@ int mhd_set_resistive(mhd_ctx *ctx, int64_t n, const int64_t *unknowns, const do
     R.halias_of = fidx;
     R.hsign = fs;
     RUN(build_operator(ctx));
-    // every point of the solve's fields starts at zero (an upload of one of them
-    // may still be under way on the context's stream)
-    CK(ctx, cudaStreamSynchronize(ctx->stream));
+    // every point of the solve's fields starts at zero (in the stream's order:
+    // after an upload of one of them, before the next)
     for (int f0 : {int(F_Eresxi), int(F_dBxi), int(F_dJxi), int(F_RBresxi)})
         for (int f = f0; f < f0 + 3; ++f)
             for (int b = 0; b < ctx->nblocks; ++b)
-                CK(ctx, cudaMemset(ctx->pool + ctx->base[size_t(f)][size_t(b)], 0,
-                                   size_t(ctx->hbv[size_t(b)].vol) * 8 * size_t(kFields[f].ncomp)));
+                CK(ctx, cudaMemsetAsync(ctx->pool + ctx->base[size_t(f)][size_t(b)], 0,
+                                        size_t(ctx->hbv[size_t(b)].vol) * 8 * size_t(kFields[f].ncomp), ctx->stream));
     R.restart = restart;
     R.rtol = rtol;
     R.atol = atol;
@@ -3990,8 +4010,8 @@ int mhd_set_resistive(mhd_ctx *ctx, int64_t n, const int64_t *unknowns, const do
     CK(ctx, cudaMalloc(&R.partial, size_t(R.ngroups) * size_t(restart + 2) * 8));
     CK(ctx, cudaMalloc(&R.dots, 64 * 8));
     CK(ctx, cudaMalloc(&R.st, sizeof(GmresState)));
-    CK(ctx, cudaMemset(R.x, 0, nn * 8));
-    CK(ctx, cudaMemset(R.st, 0, sizeof(GmresState)));
+    CK(ctx, cudaMemsetAsync(R.x, 0, nn * 8, ctx->stream));
+    CK(ctx, cudaMemsetAsync(R.st, 0, sizeof(GmresState), ctx->stream));
     // the persistent solve: as many CTAs as the longest phase needs at an item
     // per thread (6 x 80 x 40 x 40 cells: 217 CTAs, 96.6 us per solve; 148 CTAs,
     // a second trip of each phase, 101.7), at most two per SM and no more than
@@ -4011,7 +4031,7 @@ int mhd_set_resistive(mhd_ctx *ctx, int64_t n, const int64_t *unknowns, const do
         {
             CK(ctx, cudaMalloc(&R.ppartial, size_t(2 * 32) * size_t(R.pgrid) * 8));
             CK(ctx, cudaMalloc(&R.bar, 4 * sizeof(unsigned)));
-            CK(ctx, cudaMemset(R.bar, 0, 4 * sizeof(unsigned)));
+            CK(ctx, cudaMemsetAsync(R.bar, 0, 4 * sizeof(unsigned), ctx->stream));
         }
     }
     R.its_eager = R.cycles_eager = 0;
@@ -4040,7 +4060,7 @@ int mhd_set_hall(mhd_ctx *ctx, double hall_coef, const int32_t *zero_boxes, int3
     if (nbox > 0)
     {
         CK(ctx, cudaMalloc(&ctx->hall_zb, size_t(nbox) * 8 * sizeof(int)));
-        CK(ctx, cudaMemcpy(ctx->hall_zb, zero_boxes, size_t(nbox) * 8 * sizeof(int), cudaMemcpyHostToDevice));
+        RUN(h2d(ctx, ctx->hall_zb, zero_boxes, size_t(nbox) * 8 * sizeof(int)));
     }
     ctx->hall_nzb = nbox;
     ctx->hall_coef = hall_coef;
@@ -4129,7 +4149,7 @@ int mhd_set_hall_implicit(mhd_ctx *ctx, int64_t n, const int64_t *unknowns, int6
                 bsp.push_back(H.bstar + snap[size_t(3 * b)] +
                               (int64_t(ctx->base[size_t(f)][size_t(b)]) - int64_t(ctx->base[F_Bxi][size_t(b)])));
         CK(ctx, cudaMalloc(&H.bs, bsp.size() * sizeof(double *)));
-        CK(ctx, cudaMemcpy(H.bs, bsp.data(), bsp.size() * sizeof(double *), cudaMemcpyHostToDevice));
+        RUN(h2d(ctx, H.bs, bsp.data(), bsp.size() * sizeof(double *)));
     }
     const size_t nn = size_t(H.n);
     for (double **p : {&H.X, &H.F, &H.Xt, &H.Ft, &H.dx, &H.b, &H.r, &H.w})
@@ -4138,11 +4158,11 @@ int mhd_set_hall_implicit(mhd_ctx *ctx, int64_t n, const int64_t *unknowns, int6
     CK(ctx, cudaMalloc(&H.partial, size_t(H.ngroups) * size_t(kMdMax) * 8));
     CK(ctx, cudaMalloc(&H.dots, 64 * 8));
     CK(ctx, cudaMalloc(&H.st, sizeof(GmresState)));
-    CK(ctx, cudaMemset(H.st, 0, sizeof(GmresState)));
+    CK(ctx, cudaMemsetAsync(H.st, 0, sizeof(GmresState), ctx->stream));
     CK(ctx, cudaMalloc(&H.ctl, sizeof(HallCtl)));
-    CK(ctx, cudaMemset(H.ctl, 0, sizeof(HallCtl)));
+    CK(ctx, cudaMemsetAsync(H.ctl, 0, sizeof(HallCtl), ctx->stream));
     CK(ctx, cudaMalloc(&H.done, sizeof(unsigned)));
-    CK(ctx, cudaMemset(H.done, 0, sizeof(unsigned)));
+    CK(ctx, cudaMemsetAsync(H.done, 0, sizeof(unsigned), ctx->stream));
     for (auto &sp : ctx->spare)
         if (!sp)
             CK(ctx, cudaStreamCreateWithFlags(&sp, cudaStreamNonBlocking));
@@ -4212,7 +4232,7 @@ int mhd_set_flux_reference_run(mhd_ctx *ctx, int32_t run, const double prim[5])
     const double q[6] = {rho, u, v, w, p, p / (ctx->c.gamma - 1.0) + 0.5 * rho * (u * u + v * v + w * w)};
     CK(ctx, cudaStreamSynchronize(ctx->stream));
     for (int r = (run < 0 ? 0 : run); r < (run < 0 ? ctx->nruns : run + 1); ++r)
-        CK(ctx, cudaMemcpy(ctx->qref + 6 * size_t(r), q, sizeof(q), cudaMemcpyHostToDevice));
+        RUN(h2d(ctx, ctx->qref + 6 * size_t(r), q, sizeof(q)));
     return MHD_OK;
 }
 
@@ -4229,6 +4249,7 @@ int mhd_autotune(mhd_ctx *ctx, int32_t reps, int32_t *min_ctas, int32_t n)
     if (ctx->capturing)
         return fail(ctx, MHD_ESTATE, "autotune during capture");
     RUN(ensure_geom(ctx));
+    RUN(settle(ctx));
     cudaStream_t s = ctx->stream;
     // snapshot of the state (U_H and the face B of every block; with the
     // implicit Hall solve also its edge EMF, which starts the next Newton
@@ -4442,8 +4463,7 @@ int mhd_test_stall_barrier(mhd_ctx *ctx, uint32_t spin_limit)
     // the first barrier), and a short polling limit for every wait
     const unsigned w[4] = {0xFFFFFFFFu, 0u, spin_limit, 0u};
     CK(ctx, cudaStreamSynchronize(ctx->stream));
-    CK(ctx, cudaMemcpy(R.bar, w, sizeof(w), cudaMemcpyHostToDevice));
-    return MHD_OK;
+    return h2d(ctx, R.bar, w, sizeof(w));
 }
 
 int mhd_sync(mhd_ctx *ctx, const char *group)
@@ -4700,10 +4720,9 @@ int mhd_set_time(mhd_ctx *ctx, double dt, double time, int64_t step)
     const std::vector<double> d(nr, dt), t(nr, time);
     const std::vector<long long> s(nr, step);
     CK(ctx, cudaStreamSynchronize(ctx->stream));
-    CK(ctx, cudaMemcpy(ctx->dt, d.data(), 8 * nr, cudaMemcpyHostToDevice));
-    CK(ctx, cudaMemcpy(ctx->time, t.data(), 8 * nr, cudaMemcpyHostToDevice));
-    CK(ctx, cudaMemcpy(ctx->step, s.data(), 8 * nr, cudaMemcpyHostToDevice));
-    return MHD_OK;
+    RUN(h2d(ctx, ctx->dt, d.data(), 8 * nr));
+    RUN(h2d(ctx, ctx->time, t.data(), 8 * nr));
+    return h2d(ctx, ctx->step, s.data(), 8 * nr);
 }
 
 int64_t mhd_kernel_launches(const mhd_ctx *ctx)
