@@ -2,6 +2,7 @@
 // field pool management, host<->device transfers, compiled boundary syncs,
 // and the per-step launch sequence replayed as a CUDA graph.
 #include "mhd_device_scope.h"
+#include "mhd_upload.h"
 #include "mhd_kernels.cuh"
 #include "mhd_hot_launch.cuh"
 
@@ -250,6 +251,7 @@ struct mhd_ctx
     int64_t tiles = 0;      // those CTAs
     std::map<std::string, SyncMap> syncs;
     std::map<std::string, StepSync> step_syncs; // by the groups' names joined with '+'
+    int reads_pageable = 1; // the device reads pageable host memory itself (upload_source_is_read)
     bool unsettled = false; // copies on the legacy stream may be under way (settle)
     int ucell_alone = -1; // Sync("Ucell") may run beside the B_cell pass (side_ucell; -1: not looked at)
     // eta Poles: (block, direction) pairs; a context with Poles runs every
@@ -2064,6 +2066,8 @@ int create_ctx(const mhd_block_desc *blocks, int32_t nblocks, const int32_t *run
     for (auto &e : ctx->fork_ev)
         if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess)
             return bail(MHD_ECUDA);
+    if (cudaDeviceGetAttribute(&ctx->reads_pageable, cudaDevAttrPageableMemoryAccess, ctx->device) != cudaSuccess)
+        return bail(MHD_ECUDA);
     {
         void *p = nullptr;
         if (cudaGetSymbolAddress(&p, g_noalloc_staging) != cudaSuccess)
@@ -2262,6 +2266,18 @@ int mhd_field_info(const mhd_ctx *ctx, const char *name, int32_t block, int32_t 
     return MHD_OK;
 }
 
+struct CudaPointers
+{
+    static bool unregistered(const void *p)
+    {
+        cudaPointerAttributes at{};
+        const bool ok = cudaPointerGetAttributes(&at, p) == cudaSuccess;
+        if (!ok)
+            cudaGetLastError();
+        return ok && at.type == cudaMemoryTypeUnregistered;
+    }
+};
+
 static int transfer(mhd_ctx *ctx, const char *name, int32_t block, const double *hin, double *hout, int64_t count)
 {
     const int f = field_by_name(name);
@@ -2290,11 +2306,8 @@ static int transfer(mhd_ctx *ctx, const char *name, int32_t block, const double 
                                                                 hi[0] - lo[0], hi[1] - lo[1], hi[2] - lo[2],
                                                                 ctx->staging);
         RUN(launched(ctx));
-        // a copy from pageable memory has read its source when it returns
-        cudaPointerAttributes at{};
-        if (cudaPointerGetAttributes(&at, hin) == cudaSuccess && at.type == cudaMemoryTypeUnregistered)
+        if (upload_source_is_read<CudaPointers>(hin, ctx->reads_pageable))
             return MHD_OK;
-        cudaGetLastError();
     }
     else
     {

@@ -120,7 +120,10 @@ int mhd_field_info(const mhd_ctx *ctx, const char *name, int32_t block, int32_t 
 
 /* FieldBlock host storage <-> device (the reference reads/writes FieldBlock
    storage directly, src/3_field/1_Field_Block.cpp:3-25).  `data` holds the
-   field's full logical box in AoS order; `count` must equal its size. */
+   field's full logical box in AoS order; `count` must equal its size.  An
+   upload returns when `data` has been read; the device may still be writing
+   the field (later calls come after it), and an error of that work is
+   reported by the next call that waits for the device. */
 int mhd_upload_field(mhd_ctx *ctx, const char *name, int32_t block, const double *data, int64_t count);
 int mhd_download_field(mhd_ctx *ctx, const char *name, int32_t block, double *data, int64_t count);
 
