@@ -4424,6 +4424,20 @@ int mhd_resistive_stats(const mhd_ctx *ctx, int32_t *its, double *rnorm, double 
     return MHD_OK;
 }
 
+int mhd_resistive_lists(const mhd_ctx *ctx, int64_t out[6])
+{
+    if (!ctx || !out)
+        return MHD_EINVAL;
+    const auto &R = ctx->res;
+    const int64_t n[3] = {R.fa.n, R.fb.n, R.nregpt}, dyn[3] = {R.fa.dyn, R.fb.dyn, R.regdyn};
+    for (int q = 0; q < 3; ++q)
+    {
+        out[2 * q] = n[q] < 0 ? -1 : n[q];
+        out[2 * q + 1] = n[q] < 0 ? -1 : dyn[q];
+    }
+    return MHD_OK;
+}
+
 int mhd_set_integrator(mhd_ctx *ctx, int32_t integrator)
 {
     BIND_DEVICE(ctx);

@@ -93,6 +93,7 @@ _SIGS = {
     "mhd_set_flux_reference": (C.c_int, [C.c_void_p, C.POINTER(C.c_double)]),
     "mhd_resistive_stats": (C.c_int, [C.c_void_p, C.POINTER(C.c_int32), C.POINTER(C.c_double),
                                       C.POINTER(C.c_double), C.POINTER(C.c_int32)]),
+    "mhd_resistive_lists": (C.c_int, [C.c_void_p, C.POINTER(C.c_int64)]),
     "mhd_update_derived": (C.c_int, [C.c_void_p]),
     "mhd_step": (C.c_int, [C.c_void_p, C.c_int32, C.POINTER(C.c_double), C.POINTER(C.c_double)]),
     "mhd_step_host": (C.c_int, [C.c_void_p, C.c_int32, C.c_void_p, C.c_void_p, C.c_int64, C.POINTER(C.c_double)]),
@@ -403,6 +404,13 @@ class Context:
         self._check(self.lib.mhd_resistive_stats(self.h, C.byref(its), C.byref(rn), C.byref(bn), C.byref(rs)),
                     "resistive_stats")
         return dict(its=its.value, rnorm=rn.value, bnorm=bn.value, reason=rs.value)
+
+    def resistive_lists(self):
+        """(entries, entries that change from product to product) of the
+        operator's lists: Eres, dB, region ((-1, -1): not used)"""
+        out = (C.c_int64 * 6)()
+        self._check(self.lib.mhd_resistive_lists(self.h, out), "resistive_lists")
+        return {"Eres": (out[0], out[1]), "dB": (out[2], out[3]), "region": (out[4], out[5])}
 
     def set_integrator(self, integrator: int):
         """INTEGRATOR_EULER (the reference's StepOnce) or INTEGRATOR_SSPRK2

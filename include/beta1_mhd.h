@@ -337,6 +337,13 @@ int mhd_set_tune(mhd_ctx *ctx, const int32_t *min_ctas, int32_t n);
    3 atol, -3 iteration limit, as KSPConvergedReason) of the last solve. */
 int mhd_resistive_stats(const mhd_ctx *ctx, int32_t *its, double *rnorm, double *bnorm, int32_t *reason);
 
+/* The form of the persistent solve's operator: entries of the Eres list, of
+   the dB list and of the region list, and of each how many change from
+   product to product (the others are written by a solve's first product
+   alone); -1, -1 for a list that is not used (the copies run as they are
+   given, the region as boxes).  Six values. */
+int mhd_resistive_lists(const mhd_ctx *ctx, int64_t out[6]);
+
 /* Time integrator of every following step.  The reference has one: a single
    forward-Euler stage per StepOnce (Z4_Lunar/src/LunarSolver_Driver.cpp:21-92,
    Z4_Lunar/src/physics/LunarSolver_Advance.cpp:61-122), MHD_INTEGRATOR_EULER,
