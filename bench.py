@@ -66,7 +66,6 @@ ALGO_BYTES_PER_CELL = {
     # fluid RHS: rho 1, PV 4, RhoE 1, Csound 1, JD 9, face area 3, Jac 1, B_cell 3, J_cell 3 read, RHS_H 5
     # written; with the contravariant velocities: U_plus 3 read, U_contra 3 written
     "k_fluid_ucontra": 37 * 8,
-    "k_fluid_rhs": 31 * 8,
     # JD 9, Jac 1, U_plus 3 read; U_contra 3 written
     "k_ucontra": 16 * 8,
     # B 3, Badd 3, U_contra 3 read; the 6 components of Eface that are not zero written

@@ -151,10 +151,10 @@ struct SyncMap
 constexpr int kThreads = 256;
 
 const char *const kKernelNames[] = {
-    "k_fluid_rhs",    "k_eface",       "k_eedge",        "k_curl_e2f",     "k_update_u",      "k_bcell",
-    "k_jedge",        "k_jcell",       "k_pv_uplus_dt",  "k_begin_step",   "k_arm_dt",        "k_end_step",
+    "k_eface",       "k_eedge",        "k_curl_e2f",     "k_update_u",      "k_bcell",
+    "k_jedge",        "k_jcell",       "k_pv_uplus_dt",  "k_begin_step",   "k_arm_dt",
     "k_gather",       "k_gather_stage", "k_scatter_stage", "k_aos_to_soa", "k_soa_to_aos",    "k_set_consts",
-    "k_wall_u",       "k_alias_copy",  "k_scatter_vec",  "k_resist_out",   "k_resist_rhs",    "k_dots",
+    "k_alias_copy",  "k_scatter_vec",  "k_resist_out",   "k_resist_rhs",    "k_dots",
     "k_sub_proj",    "k_add_small",    "k_div_guard",    "k_div_next",      "k_gmres_init",
     "k_cycle_start",  "k_gmres_column", "k_inner_check", "k_gmres_solve_y", "k_add_basis",    "k_outer_check",
     "k_zero",         "k_residual",    "k_ucontra",      "k_face_normals", "k_divb",          "k_eres_explicit",
@@ -185,13 +185,16 @@ enum TuneId
 const char *const kTuneNames[NTUNE] = {"k_pv_uplus_dt", "k_fluid_ucontra", "k_bcell_jedge",  "k_eface",
                                        "k_curl_e2f",    "k_eedge",         "k_fluid_mixed",  "k_gmres_resist",
                                        "k_hall_edge"};
-// per variant (variant 0, the default, first) the reported value: the minimum
-// CTAs per SM of its launch bounds (0: the default's own; 3 for the default
-// k_fluid_mixed, which now runs at 4); 12 for the
-// face-tiled k_fluid_mixed (2 CTAs per SM), 16 for the same with its face
-// states staged in shared memory, 14 for k_pv_uplus_dt with J_cell in a pass
-// of its own (the PV pass at 4); for the persistent k_gmres_resist the CTAs of
-// its grid (0: two per SM).  And the number of variants
+// per variant (variant 0, the default, first) the value that names it in a saved
+// choice: where the form is the per-point kernel, its minimum CTAs per SM when
+// the value was given, else a code.  The launch bounds of today's forms are at
+// the launchers (mhd_kernels.cuh): the default k_fluid_mixed, 3, has bounds of 4
+// CTAs, and its 0 and 2 of 1 and 2; 0 names the default where the default is not
+// named otherwise, and the uncapped k_pv_uplus_dt.  12: the face-tiled
+// k_fluid_mixed, 16: the same with its face states staged in shared memory, 14:
+// k_pv_uplus_dt with J_cell in a pass of its own; k_gmres_resist: the CTAs of
+// its grid (0: an item per thread of its longest phase, at most two per SM).
+// And the number of variants
 const int kTuneMinCtas[NTUNE][5] = {{4, 0, 5, 14, 0}, {0, 3, 0, 0, 0},        {0, 6, 0, 0, 0},
                                     {0, 6, 0, 0, 0},  {0, 6, 0, 0, 0},        {0, 8, 0, 0, 0},
                                     {3, 0, 2, 12, 16}, {0, 148, 64, 32, 0},   {0, 2, 0, 0, 0}};

@@ -313,7 +313,7 @@ __global__ void k_hall_res_dots(const double *pool, const uint64_t *e, const dou
 // r = b - ((Xt - pool[e]) - F) / *h
 __global__ void k_hall_restart_r(const double *pool, const uint64_t *e, const double *Xt, const double *F,
                                  const double *h, const double *b, double *r, int64_t n);
-// b = -F, r = b, dx = 0; out[0] = b . b
+// b = -F, r = b, dx = 0; out[0] = b . b, out[1] = X . X
 __global__ void k_hall_gmres_prologue(const double *F, double *b, double *r, double *dx, const double *X, int64_t n,
                                       double *partial, double *out, unsigned *done);
 // out[0] = x . x; where *known is set the value is *val already (val null: nobody asks for it)

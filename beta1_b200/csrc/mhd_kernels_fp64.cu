@@ -17,15 +17,9 @@
 namespace mhd
 {
 
-// std::max / std::min semantics (return the first argument unless the
-// second compares greater / smaller), which differ from fmax on NaN.
+// std::max semantics (returns the first argument unless the second compares
+// greater), which differs from fmax on NaN.
 __device__ __forceinline__ double smax(double a, double b) { return (a < b) ? b : a; }
-__device__ __forceinline__ double smin(double a, double b) { return (b < a) ? b : a; }
-
-__device__ __forceinline__ double at(const BlockView &b, int f, int m, int i, int j, int k)
-{
-    return b.f[f][m * b.vol + pidx(b, i, j, k)];
-}
 
 // Thread -> (block, i, j, k) over a box [lo, lo + n) with k fastest.
 __device__ __forceinline__ bool box_point(const int lo[3], const int n[3], int64_t t, int &i, int &j, int &k)

@@ -29,8 +29,8 @@ namespace mhd
 
 namespace
 {
-// std::max / std::min semantics (return the first argument unless the
-// second compares greater / smaller), which differ from fmax on NaN.
+// std::max semantics (returns the first argument unless the second compares
+// greater), which differs from fmax on NaN.
 __device__ __forceinline__ double smax(double a, double b) { return (a < b) ? b : a; }
 
 constexpr int kHotThreads = 256;

@@ -27,11 +27,11 @@ PREC_FP64 = 0
 PREC_MIXED = 1
 
 # the default variant of each tunable kernel, in the values mhd_autotune
-# reports (minimum CTAs per SM of its launch bounds, 0: the default's own,
-# 3: k_fluid_mixed's default; 12: the
-# face-tiled k_fluid_mixed, 16: the same with staged face states; 14:
-# k_pv_uplus_dt with J_cell in its own pass;
-# k_gmres_resist: the CTAs of the persistent grid, 0: two per SM)
+# reports (minimum CTAs per SM of the launch bounds for most variants; 0: the
+# default form where the default is not named here; 3: the default
+# k_fluid_mixed, 12: the face-tiled one, 16: the same with staged face states;
+# 14: k_pv_uplus_dt with J_cell in its own pass; k_gmres_resist: the CTAs of the
+# persistent grid, 0: as its longest phase needs, at most two per SM)
 DEFAULT_TUNE = {"k_pv_uplus_dt": 4, "k_fluid_ucontra": 0, "k_bcell_jedge": 0, "k_eface": 0, "k_curl_e2f": 0,
                 "k_eedge": 0, "k_fluid_mixed": 3, "k_gmres_resist": 0, "k_hall_edge": 0}
 

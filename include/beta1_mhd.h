@@ -311,14 +311,17 @@ int mhd_set_flux_reference_run(mhd_ctx *ctx, int32_t run, const double prim[5]);
    starts from a snapshot of the state taken
    at entry, and the state and run clocks are restored at the end, so the
    call does not advance the simulation.  Call it after the state is loaded.
-   min_ctas[i] (i < n, at most MHD_NTUNE) receives the chosen minimum CTAs
-   per SM of kernel mhd_tune_name(i) (0: the default form's own launch bounds;
-   3: the default k_fluid_mixed; 12: the face-tiled k_fluid_mixed, 16: the same with
-   its FP32 face states staged in shared memory; 14: k_pv_uplus_dt
-   with J_cell in a pass of its own).  For the persistent k_gmres_resist the
-   value is the CTAs of its grid (0: two per SM); its partial sums group
-   differently per grid, so its results agree to round-off, not bitwise.
-   */
+   min_ctas[i] (i < n, at most MHD_NTUNE) receives the value that names the
+   chosen variant of kernel mhd_tune_name(i): the minimum CTAs per SM of its
+   launch bounds for most of them; 0: the default form (of k_pv_uplus_dt and
+   k_fluid_mixed the compiler's own allocation, their defaults being 4 and 3;
+   3 keeps its meaning of the default k_fluid_mixed, whose bounds are 4 CTAs);
+   12: the face-tiled k_fluid_mixed, 16: the same with its FP32 face states
+   staged in shared memory; 14: k_pv_uplus_dt with J_cell in a pass of its own.
+   For the persistent k_gmres_resist the value is the CTAs of its grid (0: as
+   many as its longest phase has items for, at most two per SM); its partial
+   sums group differently per grid, so its results agree to round-off, not
+   bitwise. */
 #define MHD_NTUNE 9
 int mhd_autotune(mhd_ctx *ctx, int32_t reps, int32_t *min_ctas, int32_t n);
 const char *mhd_tune_name(int32_t i);
