@@ -44,9 +44,14 @@ __device__ __forceinline__ void begin_run(const RunClock &rc, int r)
     rc.dt[r] = d;
     rc.h_dt[r] = d;
     // the first error of a span stays: a solve that gave up in an earlier step
-    // must not lose its mark, by which later solves leave the barrier alone
-    if ((!isfinite(d) || d < rc.dt_abort) && atomicCAS(rc.err, MHD_OK, MHD_EDT) == MHD_OK)
+    // must not lose its mark, by which later solves leave the barrier alone (no
+    // other CTA or kernel touches the word meanwhile, the runs of a batch write
+    // one value; an atomic here costs the mixed flux pass 200 bytes of spills)
+    if ((!isfinite(d) || d < rc.dt_abort) && rc.err[0] == MHD_OK)
+    {
+        rc.err[0] = MHD_EDT;
         *rc.h_err = MHD_EDT;
+    }
 }
 __device__ __forceinline__ void end_run(const RunClock &rc, int r)
 {
