@@ -118,15 +118,17 @@ ALGO_BYTES_MIXED = {"k_pv_uplus_dt": 12 * 8 + 48 * 4 + 6 * 8 + 7 * 4,
 # the dominant kernel, from one ncu capture of a smaller case of the same
 # workload, scaled by the cell count to a full launch (the kernels' traffic
 # grows with the cells they cover):
-# * C2 at half the cells per direction (165,888 cells: 95.83 MB read +
-#   10.54 MB written) to the full C2 slab (1,327,104 cells);
-# * the shell sweep's first 6 runs (2,269,318 cells; k_fluid_mixed
-#   667.88 MB read + 158.57 MB written, k_pv_uplus_dt 711.88 + 170.01 MB) to all 48 runs (14,879,028 cells)
+# * C2 at half the cells per direction (165,888 cells: 96.15 MB read +
+#   12.19 MB written, profiles/hot_kernels_c2small_fp64.md) to the full C2
+#   slab (1,327,104 cells);
+# * the shell sweep's first 6 runs (2,269,318 cells; k_fluid_mixed 668.00 MB
+#   read + 162.08 MB written, k_pv_uplus_dt 711.87 + 170.04 MB,
+#   profiles/hot_kernels_c5s6_mixed.md) to all 48 runs (14,879,028 cells)
 _SWEEP_SCALE = 14879028.0 / 2269318.0
 NCU_TRAFFIC_BYTES = {
-    ("k_pv_uplus_dt", "c2_slab6x96x48x48_implicit_resistive_fp64"): (95.830272e6 + 10.536192e6) * 8.0,
-    ("k_fluid_mixed", "c5s_sweep48_shell_runs_mixed"): (667.88224e6 + 158.565376e6) * _SWEEP_SCALE,
-    ("k_pv_uplus_dt", "c5s_sweep48_shell_runs_mixed"): (711.876352e6 + 170.00576e6) * _SWEEP_SCALE,
+    ("k_pv_uplus_dt", "c2_slab6x96x48x48_implicit_resistive_fp64"): (96.1536e6 + 12.194048e6) * 8.0,
+    ("k_fluid_mixed", "c5s_sweep48_shell_runs_mixed"): (667.995648e6 + 162.084864e6) * _SWEEP_SCALE,
+    ("k_pv_uplus_dt", "c5s_sweep48_shell_runs_mixed"): (711.872256e6 + 170.043904e6) * _SWEEP_SCALE,
 }
 
 
