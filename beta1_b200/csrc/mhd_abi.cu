@@ -140,6 +140,7 @@ struct SyncMap
     bool built = false; // device lists match the host tables
     CopyList full, hot, post;
     Resolved res; // of the hot lists
+    int reads_t = -1; // some copy of the tables reads PV_H's temperature (-1: not looked at)
     bool into_eface = false; // gives a zero component of Eface another value (eface_zeroed)
     // Pole contexts: the copies and fixed values a step leaves for read-out
     // (cold), written then without the rings, walls and post-wall copies
@@ -407,6 +408,7 @@ static void mark_dirty(mhd_ctx *ctx);
 int build_sync(mhd_ctx *ctx, const std::string &group, SyncMap &m);
 static int step_sync(mhd_ctx *ctx, std::initializer_list<const char *> groups, SyncPart part, StepSync **out);
 static int sync_fields(mhd_ctx *ctx, const char *group, std::bitset<NFIELD> &fields);
+static bool reads_temperature(const mhd_ctx *ctx, SyncMap &m);
 
 namespace
 {
@@ -797,6 +799,7 @@ int ensure_geom(mhd_ctx *ctx)
 // stream beside PV's FP64 work).  Each sync runs after the pass that writes
 // its fields and before any pass that reads them; the reference's order
 // among these independent fields does not change any value.
+int launch_temperature(mhd_ctx *ctx);
 int launch_update_derived(mhd_ctx *ctx, bool armed, bool joined);
 int launch_update_derived_pole(mhd_ctx *ctx, bool joined);
 
@@ -917,7 +920,23 @@ int launch_update_derived(mhd_ctx *ctx, bool armed, bool joined)
     ctx->pv_dirty = true;
     RUN(launched(ctx, launch_k_pv_uplus_dt(ctx->tune[TUNE_k_pv_uplus_dt], ctx->pool32 != nullptr, ctx->hot, s, ctx->c,
                                            ctx->dt_key)));
+    RUN(launch_temperature(ctx));
     return run_syncs(ctx, {"J_cell", "Uplus"});
+}
+
+// A table of the step that reads the temperature of PV_H (none of the grid
+// families' does): the read-out pass, which forms it, right behind the primitive
+// pass that leaves it out
+int launch_temperature(mhd_ctx *ctx)
+{
+    bool read = false;
+    for (auto &kv : ctx->syncs)
+        read = read || (kv.second.built && !(kv.second.res.usable && !kv.second.res.fields.test(F_PV)) &&
+                        reads_temperature(ctx, kv.second));
+    if (!read)
+        return MHD_OK;
+    prof_begin(ctx, "k_pv_uplus_dt");
+    return launched(ctx, launch_k_pv_all(ctx->hot, ctx->stream, ctx->c));
 }
 
 // UpdateDerivedFields_ with Poles, in the reference's order: calc_Bcell and
@@ -959,6 +978,7 @@ int launch_update_derived_pole(mhd_ctx *ctx, bool joined)
         RUN(join_side(ctx, 2));
     else
         RUN(launch_pole(ctx, split ? int(POLE_JCELL) : POLE_JCELL_FIRST));
+    RUN(launch_temperature(ctx));
     return run_syncs(ctx, {"J_cell", "Uplus"});
 }
 
@@ -3196,6 +3216,26 @@ static int sync_fields(mhd_ctx *ctx, const char *group, std::bitset<NFIELD> &fie
     return MHD_OK;
 }
 
+// Does a copy of the group's tables read the temperature of PV_H (its plane 4)?
+// The step leaves that plane to read-out.
+static bool reads_temperature(const mhd_ctx *ctx, SyncMap &m)
+{
+    if (m.reads_t < 0)
+    {
+        const PoolDecoder dec(ctx);
+        auto temperature = [&](uint64_t off) {
+            const size_t b = size_t(std::upper_bound(dec.start.begin(), dec.start.end() - 1, off) - dec.start.begin()) - 1;
+            const uint64_t vol = uint64_t(ctx->hbv[b].vol), lo = dec.start[b] + uint64_t(plane_of(F_PV) + 4) * vol;
+            return off >= lo && off - lo < vol;
+        };
+        m.reads_t = std::any_of(m.hs.begin(), m.hs.end(), temperature) ||
+                            std::any_of(m.hs2.begin(), m.hs2.end(), temperature)
+                        ? 1
+                        : 0;
+    }
+    return m.reads_t == 1;
+}
+
 // every group's lists and the passes of the step (before a capture)
 static int build_all_syncs(mhd_ctx *ctx)
 {
@@ -3754,6 +3794,7 @@ int mhd_set_sync_map(mhd_ctx *ctx, const char *group, const int64_t *dst, const 
     SyncMap &m = ctx->syncs[group];
     m.hd.swap(d);
     m.hs.swap(s);
+    m.reads_t = -1;
     m.staged = staged;
     m.built = false;
     drop_graph(ctx);
@@ -3814,6 +3855,7 @@ int mhd_set_sync_map_post(mhd_ctx *ctx, const char *group, const int64_t *dst, c
     SyncMap &m = ctx->syncs[group];
     m.hd2.swap(d);
     m.hs2.swap(s);
+    m.reads_t = -1;
     m.built = false;
     drop_graph(ctx);
     return MHD_OK;
@@ -4502,6 +4544,8 @@ int mhd_sync(mhd_ctx *ctx, const char *group)
     if (!ctx || !group)
         return MHD_EINVAL;
     RUN(ensure_geom(ctx));
+    if (const auto it = ctx->syncs.find(group); ctx->pv_dirty && it != ctx->syncs.end() && reads_temperature(ctx, it->second))
+        RUN(materialise_pv(ctx));
     RUN(run_sync(ctx, group, true));
     CK(ctx, cudaStreamSynchronize(ctx->stream));
     return MHD_OK;
