@@ -789,7 +789,9 @@ __device__ bool grid_matvec(const ResistSolve &a, GridBar &gb, const HotBlock *h
 // every point written by every product; 120 with a counting barrier, the lists'
 // entries, scales and blocks loaded once into registers and shared memory; 96.6
 // with the points that never change written by the first product alone, a CTA
-// for every 256 items and release / acquire in place of two fences.
+// for every 256 items and release / acquire in place of two fences; 98.6 with the
+// elements of other CTAs formed where they are read (BasisVec: before, the
+// second pass's result was read without a barrier behind its store).
 __global__ void __launch_bounds__(256) k_gmres_resist(ResistSolve a)
 {
     __shared__ GmresScalars S;

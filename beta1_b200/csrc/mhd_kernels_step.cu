@@ -15,9 +15,9 @@
 // whole steps on a 64^3 box, the 6 x 80 x 40 x 40 slab and shell and slab
 // sweeps: more registers keep more loads in flight, fewer hide more latency.
 // Measured on six shells (2.27 M cells, mixed form), against the kernels that
-// loaded views and pointers and stored between loads: PV / CFL 267 -> 199 us,
-// mixed flux 241 -> 207, face EMF 104 -> 91, edge EMF 95 -> 72, curl 74 -> 45,
-// cell update 63 -> 54, B_cell and J edges 127 -> 121 us.
+// loaded views and pointers and stored between loads: PV / CFL 267 -> 191 us,
+// mixed flux 241 -> 189, face EMF 104 -> 87, edge EMF 95 -> 73, curl and cell
+// update (one pass, before: two) 137 -> 89, B_cell and J edges 127 -> 120 us.
 #include "mhd_kernels.cuh"
 #include "mhd_hot_launch.cuh"
 
@@ -288,7 +288,7 @@ template <class A> __device__ __forceinline__ void eface_body(const A &a)
 }
 
 // the zero components of Eface: zero in a new pool; written again after an
-// Eface field was uploaded
+// upload of Eface or a table that wrote them, in every step while one does
 template <class A> __global__ void __launch_bounds__(kHotThreads) k_eface_zero_t(const __grid_constant__ A a)
 {
     uint32_t t, p;
@@ -803,8 +803,10 @@ __device__ __forceinline__ CellState cell_state(const double U[5], const Consts 
 // WT double: PV_H without its temperature, U_plus and the FP64 face states;
 // float (mixed form): U_plus.  No kernel of a step reads the temperature, and
 // none of the mixed form PV_H (its flux reads the FP32 face states, its J x B
-// source the velocities from U); the read-out pass forms PV_H anew (k_pv_all).  In a mixed context also the FP32 face
-// states, deviations from the reference state (formed in FP64), sound speed.
+// source the velocities from U); the read-out pass forms PV_H anew (k_pv_all),
+// and runs inside a step where a Sync table copies the temperature.  In a mixed
+// context also the FP32 face states, deviations from the reference state
+// (formed in FP64), sound speed.
 template <typename WT>
 __device__ __forceinline__ void store_cell_state(const HotBlock &b, uint32_t p, double U0, const CellState &s)
 {
