@@ -140,8 +140,8 @@ struct SyncMap
     bool built = false; // device lists match the host tables
     CopyList full, hot, post;
     Resolved res; // of the hot lists
-    int reads_t = -1; // some copy of the tables reads PV_H's temperature (-1: not looked at)
-    bool into_eface = false; // gives a zero component of Eface another value (eface_zeroed)
+    bool t_map = false, t_post = false; // a copy of hs / hs2 reads PV_H's temperature (launch_temperature)
+    bool into_eface = false; // gives a zero component of Eface another value (launch_eface_zero)
     // Pole contexts: the copies and fixed values a step leaves for read-out
     // (cold), written then without the rings, walls and post-wall copies
     CopyList cold;
@@ -408,7 +408,6 @@ static void mark_dirty(mhd_ctx *ctx);
 int build_sync(mhd_ctx *ctx, const std::string &group, SyncMap &m);
 static int step_sync(mhd_ctx *ctx, std::initializer_list<const char *> groups, SyncPart part, StepSync **out);
 static int sync_fields(mhd_ctx *ctx, const char *group, std::bitset<NFIELD> &fields);
-static bool reads_temperature(const mhd_ctx *ctx, SyncMap &m);
 
 namespace
 {
@@ -929,11 +928,8 @@ int launch_update_derived(mhd_ctx *ctx, bool armed, bool joined)
 // pass that leaves it out
 int launch_temperature(mhd_ctx *ctx)
 {
-    bool read = false;
-    for (auto &kv : ctx->syncs)
-        read = read || (kv.second.built && !(kv.second.res.usable && !kv.second.res.fields.test(F_PV)) &&
-                        reads_temperature(ctx, kv.second));
-    if (!read)
+    if (std::none_of(ctx->syncs.begin(), ctx->syncs.end(),
+                     [](const auto &kv) { return kv.second.t_map || kv.second.t_post; }))
         return MHD_OK;
     prof_begin(ctx, "k_pv_uplus_dt");
     return launched(ctx, launch_k_pv_all(ctx->hot, ctx->stream, ctx->c));
@@ -2421,6 +2417,12 @@ int64_t mhd_point_id(const mhd_ctx *ctx, const char *name, int32_t block, int32_
     return (int64_t(f) << 56) | (int64_t(block) << 40) | aos;
 }
 
+// is the point id one of PV_H's temperature
+static bool is_temperature(int64_t id)
+{
+    return int(id >> 56) == F_PV && (id & ((int64_t(1) << 40) - 1)) % kFields[F_PV].ncomp == 4;
+}
+
 // point id -> pool offset (-1 if invalid)
 static int64_t pool_offset(const mhd_ctx *ctx, int64_t id)
 {
@@ -3216,26 +3218,6 @@ static int sync_fields(mhd_ctx *ctx, const char *group, std::bitset<NFIELD> &fie
     return MHD_OK;
 }
 
-// Does a copy of the group's tables read the temperature of PV_H (its plane 4)?
-// The step leaves that plane to read-out.
-static bool reads_temperature(const mhd_ctx *ctx, SyncMap &m)
-{
-    if (m.reads_t < 0)
-    {
-        const PoolDecoder dec(ctx);
-        auto temperature = [&](uint64_t off) {
-            const size_t b = size_t(std::upper_bound(dec.start.begin(), dec.start.end() - 1, off) - dec.start.begin()) - 1;
-            const uint64_t vol = uint64_t(ctx->hbv[b].vol), lo = dec.start[b] + uint64_t(plane_of(F_PV) + 4) * vol;
-            return off >= lo && off - lo < vol;
-        };
-        m.reads_t = std::any_of(m.hs.begin(), m.hs.end(), temperature) ||
-                            std::any_of(m.hs2.begin(), m.hs2.end(), temperature)
-                        ? 1
-                        : 0;
-    }
-    return m.reads_t == 1;
-}
-
 // every group's lists and the passes of the step (before a capture)
 static int build_all_syncs(mhd_ctx *ctx)
 {
@@ -3776,6 +3758,7 @@ int mhd_set_sync_map(mhd_ctx *ctx, const char *group, const int64_t *dst, const 
     if (!ctx || !group || n < 0 || (n > 0 && (!dst || !src)))
         return fail(ctx, MHD_EINVAL, "bad sync map arguments");
     std::vector<uint64_t> d(static_cast<size_t>(n)), s(static_cast<size_t>(n));
+    bool temperature = false;
     for (int64_t t = 0; t < n; ++t)
     {
         const int64_t od = pool_offset(ctx, dst[t]);
@@ -3784,6 +3767,7 @@ int mhd_set_sync_map(mhd_ctx *ctx, const char *group, const int64_t *dst, const 
             return fail(ctx, MHD_EINVAL, "sync map entry %lld has an invalid point id", (long long)t);
         d[size_t(t)] = uint64_t(od);
         s[size_t(t)] = uint64_t(os);
+        temperature = temperature || is_temperature(src[t]);
     }
     // staged (gather, then scatter) when a source is also a destination
     std::vector<uint64_t> sorted_d(d);
@@ -3794,7 +3778,7 @@ int mhd_set_sync_map(mhd_ctx *ctx, const char *group, const int64_t *dst, const 
     SyncMap &m = ctx->syncs[group];
     m.hd.swap(d);
     m.hs.swap(s);
-    m.reads_t = -1;
+    m.t_map = temperature;
     m.staged = staged;
     m.built = false;
     drop_graph(ctx);
@@ -3837,6 +3821,7 @@ int mhd_set_sync_map_post(mhd_ctx *ctx, const char *group, const int64_t *dst, c
     if (!ctx || !group || n < 0 || (n > 0 && (!dst || !src)))
         return fail(ctx, MHD_EINVAL, "bad sync map arguments");
     std::vector<uint64_t> d(static_cast<size_t>(n)), s(static_cast<size_t>(n));
+    bool temperature = false;
     for (int64_t t = 0; t < n; ++t)
     {
         const int64_t od = pool_offset(ctx, dst[t]);
@@ -3845,6 +3830,7 @@ int mhd_set_sync_map_post(mhd_ctx *ctx, const char *group, const int64_t *dst, c
             return fail(ctx, MHD_EINVAL, "sync map entry %lld has an invalid point id", (long long)t);
         d[size_t(t)] = uint64_t(od);
         s[size_t(t)] = uint64_t(os);
+        temperature = temperature || is_temperature(src[t]);
     }
     // one gather: no source may be a destination
     std::vector<uint64_t> sorted_d(d);
@@ -3855,7 +3841,7 @@ int mhd_set_sync_map_post(mhd_ctx *ctx, const char *group, const int64_t *dst, c
     SyncMap &m = ctx->syncs[group];
     m.hd2.swap(d);
     m.hs2.swap(s);
-    m.reads_t = -1;
+    m.t_post = temperature;
     m.built = false;
     drop_graph(ctx);
     return MHD_OK;
@@ -4544,7 +4530,7 @@ int mhd_sync(mhd_ctx *ctx, const char *group)
     if (!ctx || !group)
         return MHD_EINVAL;
     RUN(ensure_geom(ctx));
-    if (const auto it = ctx->syncs.find(group); ctx->pv_dirty && it != ctx->syncs.end() && reads_temperature(ctx, it->second))
+    if (const auto it = ctx->syncs.find(group); it != ctx->syncs.end() && (it->second.t_map || it->second.t_post))
         RUN(materialise_pv(ctx));
     RUN(run_sync(ctx, group, true));
     CK(ctx, cudaStreamSynchronize(ctx->stream));
